@@ -303,6 +303,45 @@ def test_long_portions_run_as_segments_side_by_side(dtype, H, P, N, G):
             at[s] += n
 
 
+@pytest.mark.parametrize("H,P,N,G", [(4, 64, 128, 2), (2, 128, 64, 1), (3, 64, 64, 3), (2, 128, 128, 1)])
+def test_segments_in_matrix_form(H, P, N, G):
+    """bfloat16 inputs at the sizes that the segments' matrix form takes: outputs and states to the bound of the float32
+    recurrence above, since only the inputs are 16-bit. Last segments of 1, 16 and 37 tokens; a head that forgets almost
+    nothing, one that forgets everything within a token, one whose step sizes are large."""
+    from types import SimpleNamespace
+    from dynalm_b200.kernels import ops
+    rng = np.random.RandomState(7 * H + P + N)
+    seg, inner, dt_col = ops.SSM_SEGMENT, H * P, 8
+    a_log, dt_bias, d_skip = rng.randn(H) * 0.3, rng.randn(H) * 0.3, 1 + 0.2 * rng.randn(H)
+    a_log[0], a_log[-1], dt_bias[1] = -7.0, 6.0, 3.0
+    steps = [{0: 2 * seg + 37, 1: seg + 1, 2: 5}, {0: seg + 16, 2: 3 * seg, 1: 1}]
+    states = {s: None for s in range(3)}
+    state = torch.zeros(3, inner * N + 8, device=DEV)
+    plan, most = ops.SSM_SEGMENTS, ops.SSM_SEGMENTS.most_segments(640)
+    for st in steps:
+        rows = sum(st.values())
+        u = _t(rng.randn(rows, inner + 2 * G * N) * 0.7, torch.bfloat16)
+        proj = _t(rng.randn(rows, dt_col + H), torch.bfloat16)
+        _, _, _, q_start, _, slots = _step_arrays([(0, n) for n in st.values()], list(st))
+        host = np.zeros(plan.ints(640, 3), dtype=np.int32)
+        meta = plan.fill(host, SimpleNamespace(q_len=list(st.values()), q_start=[int(v) for v in q_start.cpu()[:-1]], slots=list(st)))
+        scratch = torch.full((most * inner * N,), float("nan"), device=DEV)
+        decay = torch.full((most * H,), float("nan"), device=DEV)
+        y = torch.full((rows, inner), float("nan"), device=DEV)
+        ops.ssm_scan(u, proj, dt_col, _t(dt_bias), _t(a_log), _t(d_skip), state, q_start, slots, y, len(st), H, P, N, G,
+                     (torch.from_numpy(host).to(DEV), meta), scratch, decay)
+        r0 = 0
+        for s, n in st.items():
+            u_t, dt_t = _np(u[r0:r0 + n]), _np(proj[r0:r0 + n, dt_col:])
+            B, C = (np.repeat(v.reshape(n, G, N), H // G, axis=1) for v in (u_t[:, inner:inner + G * N], u_t[:, inner + G * N:]))
+            want, states[s] = plain.ssm_scan(u_t[:, :inner].reshape(n, H, P), plain.softplus(dt_t + dt_bias), B, C, a_log, d_skip,
+                                             states[s])
+            assert np.abs(_np(y[r0:r0 + n]) - want.reshape(n, inner)).max() <= 2e-5 * max(1.0, np.abs(want).max())
+            got = _np(state[s, :inner * N]).reshape(H, N, P)
+            assert np.abs(got - states[s]).max() <= 2e-5 * max(1.0, np.abs(states[s]).max())
+            r0 += n
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gate_comes_before_the_norm_of_every_part(dtype):
     from dynalm_b200.kernels import ops
