@@ -1,11 +1,10 @@
 // y = x W^T on the 5th-generation tensor cores: tcgen05.mma with the accumulator in tensor memory,
 // operands brought to shared memory by TMA. bf16 operands, fp32 accumulation.
 //
-// The kernel and its launcher are in gemm_tcgen05_impl.cuh; this file instantiates them with every block loading
-// its own operands (gemm_tcgen05_cluster.cu: with pairs of blocks sharing W tiles).
+// The kernel and its launcher are in gemm_tcgen05_impl.cuh.
 //
-// A thread block computes 128 x BN tiles of y (BN = 256, 192 or 128; for SwiGLU two halves of gate and up
-// columns), one after another. Roles (warps 0 and 1 run their loops as whole warps; one elected lane issues):
+// A thread block computes 128 x bn tiles of y, or a pair of blocks 256 x bn tiles (bn up to 256; for SwiGLU two halves of
+// gate and up columns), one after another. Roles (warps 0 and 1 run their loops as whole warps; one elected lane issues):
 //   warp 0             TMA producer: for each 64-wide slice of K, waits for a free stage, arms the stage's
 //                      mbarrier with the byte count and issues the tile loads (x: 128 rows, W: BN rows), both
 //                      K-major with the 128-byte swizzle that the tensor core reads directly
@@ -27,17 +26,6 @@
 // (matmul_gated, dynacore/include/dynacore/device/device.h:188-199).
 #include "gemm_tcgen05_impl.cuh"
 
-namespace dl {
-
-// Every block loads its own operands; a stage is free when this block's MMAs have read it.
-struct T5Alone {
-  static constexpr int CLUSTER = 1;
-  static __device__ __forceinline__ void load_shared_half(void*, const CUtensorMap*, int, int, uint64_t*) {}
-  static __device__ __forceinline__ void commit_stage_free(uint64_t* bar) { umma_commit(bar); }
-};
-
-}  // namespace dl
-
 // The output tile (row block, column block) that tile number `tile` stands for when num_tiles tiles in tiles_n
 // columns are numbered in groups of group_m row blocks: the kernel's own numbering, for tests on the host.
 DL_EXPORT int dl_gemm_tcgen05_tile_coords(int tile, int tiles_n, int num_tiles, int group_m, int* m_tile, int* n_tile) {
@@ -46,11 +34,22 @@ DL_EXPORT int dl_gemm_tcgen05_tile_coords(int tile, int tiles_n, int num_tiles, 
   return 0;
 }
 
+// The tile a product of M rows and `feats` output features (mode as below) would run with: its columns, and whether a pair of
+// blocks computes it. For tests.
+DL_EXPORT int dl_gemm_tcgen05_choice(int M, int feats, int mode, int head_dim, int sms, int pairs, int* bn, int* pair) {
+  if (M <= 0 || feats <= 0 || sms <= 1 || head_dim <= 0) return DL_ERR_UNSUPPORTED;
+  const T5Choice c = t5_choose((M + dl::T5_BM - 1) / dl::T5_BM, feats, mode, head_dim, sms, pairs);
+  *bn = c.bn;
+  *pair = c.pair;
+  return 0;
+}
+
+// pairs: two blocks to a tile (cta_group::2) never (0), always (1) or where that costs less (-1).
 DL_EXPORT int dl_gemm_tcgen05(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, int mode,
-                              float out_scale, const float* coeffs, int* status, cudaStream_t stream) {
+                              float out_scale, const float* coeffs, int* status, int pairs, cudaStream_t stream) {
   if (mode < 0 || (mode > 2 && mode != dl::T5_OUT_RELU2 && mode != dl::T5_OUT_GELU && mode != dl::T5_OUT_XIELU)) return DL_ERR_UNSUPPORTED;
   const dl::QkvRope none = {};
-  return t5_launch<dl::T5Alone>(x, ldx, w, y, ldy, M, N, K, mode, out_scale, status, none, stream, coeffs);
+  return t5_launch(x, ldx, w, y, ldy, M, N, K, mode, out_scale, status, none, pairs, stream, coeffs);
 }
 
 // A grouped product on the same kernel: runs of a's rows, listed on the device as row tiles (matrix, first row, rows <=
@@ -60,7 +59,7 @@ DL_EXPORT int dl_gemm_tcgen05(const void* x, int ldx, const void* w, void* y, in
 DL_EXPORT int dl_gemm_tcgen05_grouped(const void* a, int lda, int rows, const void* w, int matrices, int N, int K, void* y,
                                       int ldy, int mode, const int* tiles, const int* n_tiles, int max_row_tiles, int* status,
                                       cudaStream_t stream) {
-  return t5_launch_grouped<dl::T5Alone>(a, lda, rows, w, matrices, N, K, y, ldy, mode, tiles, n_tiles, max_row_tiles, status,
+  return t5_launch_grouped(a, lda, rows, w, matrices, N, K, y, ldy, mode, tiles, n_tiles, max_row_tiles, status,
                                         stream);
 }
 
@@ -72,8 +71,8 @@ DL_EXPORT int dl_gemm_tcgen05_qkv_rope(const void* x, int ldx, const void* w, vo
                                        const int* positions, const int* row_request, const int* block_table, int max_blocks,
                                        void* k_cache, void* v_cache, const float* inv_freq, const void* angles,
                                        float pos_scale, int n_heads, int n_kv_heads, int head_dim, int page_size,
-                                       int* status, cudaStream_t stream) {
-  return t5_launch_qkv_rope<dl::T5Alone>(x, ldx, w, q_out, ldq, M, K, positions, row_request, block_table, max_blocks, k_cache,
+                                       int* status, int pairs, cudaStream_t stream) {
+  return t5_launch_qkv_rope(x, ldx, w, q_out, ldq, M, K, positions, row_request, block_table, max_blocks, k_cache,
                                          v_cache, inv_freq, angles, pos_scale, n_heads, n_kv_heads, head_dim, page_size, status,
-                                         stream);
+                            pairs, stream);
 }

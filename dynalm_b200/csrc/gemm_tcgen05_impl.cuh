@@ -1,5 +1,5 @@
-// The tcgen05 matrix product, shared by gemm_tcgen05.cu (every block for itself) and the cluster variant (two blocks
-// share each W tile): the kernel, templated on how a block gets its operands, and its host-side launcher.
+// The tcgen05 matrix product of gemm_tcgen05.cu: the kernel, templated on whether a block works alone or two blocks of a
+// cluster work on one tile (cta_group::2), and its host-side launchers.
 #pragma once
 
 #include "qkv_rope.cuh"
@@ -13,15 +13,17 @@ constexpr int T5_THREADS = 192;           // 6 warps
 constexpr uint32_t T5_A_BYTES = T5_BM * T5_BK * 2;    // 16 KiB
 constexpr uint32_t T5_STORE_BYTES = 4 * 32 * 128;     // per epilogue warp: 32 rows x 128 bytes of output, staged for coalesced stores
 
-// Tile width BN is 256 (4 stages of 48 KiB), 192 (5 stages of 40 KiB) or 128 (6 stages of 32 KiB); the narrower
-// ones are for shapes whose tile count fits the SMs badly at 256. SwiGLU takes 256 or 128 only.
-template <int BN> struct T5 {
-  static constexpr int STAGES = BN == 256 ? 4 : (BN == 192 ? 5 : 6);
-  static constexpr uint32_t B_BYTES = BN * T5_BK * 2;
-  static constexpr uint32_t STAGE_BYTES = T5_A_BYTES + B_BYTES;
-  static constexpr uint32_t TMEM_COLS = BN == 128 ? 256 : 512;      // two accumulators (a power of two)
-  static constexpr size_t SMEM = static_cast<size_t>(STAGES) * STAGE_BYTES + T5_STORE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
-};
+// A tile is 128 rows (256 for a pair of blocks, 128 each) by `bn` columns, a multiple of 32 up to 256, chosen per product
+// (t5_launch). As many stages as fit: a stage is 128 rows of x and bn rows of W (bn / 2 for each block of a pair).
+constexpr int T5_MAX_STAGES = 8;
+constexpr uint32_t T5_TMEM_COLS = 512;                // two accumulators of up to 256 columns
+constexpr uint32_t T5_BAR_BYTES = 256;
+constexpr uint32_t T5_SMEM = 232448;                  // the 227 KiB a block may have
+constexpr uint32_t T5_STAGE_ROOM = T5_SMEM - T5_STORE_BYTES - 1024 /* alignment */ - T5_BAR_BYTES;
+__host__ __device__ constexpr uint32_t t5_stage_bytes(int bn, int cluster) { return T5_A_BYTES + bn / cluster * T5_BK * 2; }
+__host__ __device__ constexpr int t5_stages(int bn, int cluster) {
+  return T5_STAGE_ROOM / t5_stage_bytes(bn, cluster) < T5_MAX_STAGES ? T5_STAGE_ROOM / t5_stage_bytes(bn, cluster) : T5_MAX_STAGES;
+}
 
 enum { T5_OUT_BF16 = 0, T5_OUT_F32 = 1, T5_OUT_SWIGLU = 2, T5_OUT_QKV_ROPE = 3, T5_OUT_RELU2 = 4, T5_OUT_GELU = 5, T5_OUT_PAIRS = 6, T5_OUT_XIELU = 7 };
 enum { T5_ERR_PRODUCER = 1, T5_ERR_MMA = 2, T5_ERR_EPILOGUE = 3 };
@@ -52,12 +54,12 @@ __host__ __device__ __forceinline__ void t5_tile_coords(int tile, int tiles_n, i
 // The accumulator is double-buffered in tensor memory (2 x 256 columns): the epilogue warps drain
 // one tile while the MMA warp fills the next.
 //
-// `P` says how a block gets its operands. P::CLUSTER == 1: every block loads both halves of its W tile itself.
-// P::CLUSTER == 2: the two blocks of a thread-block cluster take row blocks 2i and 2i + 1 of the same column
-// block; each loads one half of the shared W tile and its copy lands in both blocks' shared memory, so W crosses
-// from L2 once per pair (measured: the kernel is bound by operand traffic from L2; loading a third less made it
-// a fifth faster). A stage is then free only when both blocks' MMAs have read it: each block's commit arrives on
-// the stage's barrier in both blocks, and the barrier counts two arrivals.
+// PAIR: the two blocks of a thread-block cluster compute one tile of 256 rows: each loads its own 128 rows of x and one half
+// of the tile's W (for SwiGLU one the gate rows, the other the up rows), and the first block's tensor core instructions
+// (cta_group::2) read both blocks' shared memory and write both blocks' tensor memory, 128 rows each. An SM so takes in
+// 128 + bn / 2 rows a slice where a block alone takes in 128 + bn: the product is bound by that traffic from L2. The copies
+// of both blocks count on the first block's "full" barrier (it expects the bytes of both); its commits arrive on the
+// "empty" and "accumulator full" barriers of both; both blocks' epilogues arrive on its "accumulator empty" barrier.
 // A grouped product: the rows of x come in runs, each run multiplied by a matrix of its own (the experts of a mixture),
 // and which rows form a run is known on the device only. `tiles` lists row tiles as (matrix, first row, rows <= 128),
 // `n_tiles[0]` says how many; matrix g lies w_rows rows below the first in the tensor map of W. A row tile may start at
@@ -69,32 +71,31 @@ struct T5Groups {
   int w_rows;
 };
 
-template <int T5_BN, class P>
+template <bool PAIR>
 __global__ void __launch_bounds__(T5_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     void* __restrict__ y, int ldy, int M, int N, int K, int mode, float out_scale, int gate_rows,
                     int tiles_n, int num_tiles_plain, int group_m, int* __restrict__ status, const QkvRope rope,
-                    const T5Groups groups, const float* __restrict__ coeffs) {
-  constexpr int T5_STAGES = T5<T5_BN>::STAGES;
-  constexpr uint32_t T5_B_BYTES = T5<T5_BN>::B_BYTES, T5_STAGE_BYTES = T5<T5_BN>::STAGE_BYTES, T5_TMEM_COLS = T5<T5_BN>::TMEM_COLS;
+                    const T5Groups groups, const float* __restrict__ coeffs, const int bn) {
+  constexpr int CLUSTER = PAIR ? 2 : 1;
+  const int stages = t5_stages(bn, CLUSTER);
+  const uint32_t stage_bytes = t5_stage_bytes(bn, CLUSTER);
   extern __shared__ unsigned char t5_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(t5_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* store_stage = tiles + static_cast<size_t>(T5_STAGES) * T5_STAGE_BYTES;
+  unsigned char* store_stage = tiles + static_cast<size_t>(stages) * stage_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(store_stage + T5_STORE_BYTES);
-  uint64_t* full_bar = bars;                        // [T5_STAGES] stage loaded
-  uint64_t* empty_bar = bars + T5_STAGES;           // [T5_STAGES] stage consumed
-  uint64_t* acc_full = bars + 2 * T5_STAGES;        // [2] accumulator complete
-  uint64_t* acc_empty = bars + 2 * T5_STAGES + 2;   // [2] accumulator drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T5_STAGES + 4);
+  uint64_t* full_bar = bars;                        // [stages] stage loaded (a pair: the first block's)
+  uint64_t* empty_bar = bars + T5_MAX_STAGES;       // [stages] stage consumed
+  uint64_t* acc_full = bars + 2 * T5_MAX_STAGES;        // [2] accumulator complete
+  uint64_t* acc_empty = bars + 2 * T5_MAX_STAGES + 2;   // [2] accumulator drained (a pair: the first block's)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T5_MAX_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // in a cluster: this block's rank, and the walk over pairs of row blocks instead of single tiles
-  const int rank = P::CLUSTER == 2 ? static_cast<int>(cluster_rank()) : 0;
-  const int first_tile = P::CLUSTER == 2 ? static_cast<int>(blockIdx.x) / 2 : static_cast<int>(blockIdx.x);
-  const int tile_step = P::CLUSTER == 2 ? static_cast<int>(gridDim.x) / 2 : static_cast<int>(gridDim.x);
+  const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
+  const int first_tile = static_cast<int>(blockIdx.x) / CLUSTER, tile_step = static_cast<int>(gridDim.x) / CLUSTER;
   const bool swiglu = mode == T5_OUT_SWIGLU;
-  const int n_per_tile = swiglu ? T5_BN / 2 : T5_BN;      // output features per tile
+  const int n_per_tile = swiglu ? bn / 2 : bn;            // output features per tile
   const int k_tiles = (K + T5_BK - 1) / T5_BK;
   const bool grouped = groups.tiles != nullptr;
   // (first row, first feature, first row of W's matrix, one past the last row to store) of a tile
@@ -108,7 +109,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else {
       int m_tile, n_tile;
       t5_tile_coords(tile, tiles_n, num_tiles, group_m, &m_tile, &n_tile);
-      *m0 = (m_tile * P::CLUSTER + rank) * T5_BM;
+      *m0 = (m_tile * CLUSTER + rank) * T5_BM;
       *n0 = n_tile * n_per_tile;
       *w0 = 0;
       *m_end = M;
@@ -116,52 +117,63 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   };
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < T5_STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], P::CLUSTER);
+      mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 4);                  // one arrival per epilogue warp
+      mbar_init(&acc_empty[b], 4 * CLUSTER);        // one arrival per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T5_TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T5_TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(T5_TMEM_COLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (P::CLUSTER == 2) cluster_sync_all();      // the partner's barriers exist before anything is sent to them
+  if constexpr (PAIR) cluster_sync_all();              // both blocks' barriers exist before anything is sent to them
 
   if (warp == 0) {
     // TMA producer: the whole warp runs the loop (every lane polls the barrier), one elected lane issues the copies
     // The first stages' slices of W are requested before the wait on the kernel in front (programmatic dependent
     // launch): W does not depend on it. x, which does, follows after the wait.
+    const uint32_t full0 = PAIR ? in_first_block(smem_u32(full_bar)) : smem_u32(full_bar);
     auto load_w = [&](int s, int kt, int n0) {
-      unsigned char* b_dst = tiles + static_cast<size_t>(s) * T5_STAGE_BYTES + T5_A_BYTES;
-      const int second_half = swiglu ? gate_rows + n0 : n0 + T5_BN / 2;      // W row of the tile's second half
-      if constexpr (P::CLUSTER == 2) {
-        // this block's half of the W tile, into both blocks (the partner sends the other half)
-        P::load_shared_half(b_dst + rank * (T5_B_BYTES / 2), &map_w, kt * T5_BK, rank == 0 ? n0 : second_half, &full_bar[s]);
+      unsigned char* b_dst = tiles + static_cast<size_t>(s) * stage_bytes + T5_A_BYTES;
+      const int second_half = swiglu ? gate_rows + n0 : n0 + bn / 2;      // W row of the tile's second half
+      if constexpr (PAIR) {
+        tma_load_2d_pair(b_dst, &map_w, kt * T5_BK, rank == 0 ? n0 : second_half, full0 + s * 8);
       } else {
         tma_load_2d(b_dst, &map_w, kt * T5_BK, n0, &full_bar[s]);
-        tma_load_2d(b_dst + T5_B_BYTES / 2, &map_w, kt * T5_BK, second_half, &full_bar[s]);
+        tma_load_2d(b_dst + bn / 2 * (T5_BK * 2), &map_w, kt * T5_BK, second_half, &full_bar[s]);
       }
     };
     auto load_x = [&](int s, int kt, int m0) {
-      tma_load_2d(tiles + static_cast<size_t>(s) * T5_STAGE_BYTES, &map_x, kt * T5_BK, m0, &full_bar[s]);
+      unsigned char* a_dst = tiles + static_cast<size_t>(s) * stage_bytes;
+      if constexpr (PAIR) tma_load_2d_pair(a_dst, &map_x, kt * T5_BK, m0, full0 + s * 8);
+      else tma_load_2d(a_dst, &map_x, kt * T5_BK, m0, &full_bar[s]);
     };
-    const int ahead = (!grouped && first_tile < num_tiles_plain) ? min(k_tiles, T5_STAGES) : 0;
+    // the first block of a pair expects the bytes of both
+    auto expect = [&](int s) {
+      if (rank == 0) mbar_expect_tx(&full_bar[s], CLUSTER * stage_bytes);
+    };
+    const int ahead = (!grouped && first_tile < num_tiles_plain) ? min(k_tiles, stages) : 0;
     if (ahead > 0) {
       int m0, n0, w0, m_end;
       coords(first_tile, num_tiles_plain, &m0, &n0, &w0, &m_end);
       if (elect_one()) {
         for (int kt = 0; kt < ahead; ++kt) {
-          mbar_expect_tx(&full_bar[kt], T5_STAGE_BYTES);
+          expect(kt);
           load_w(kt, kt, n0);
         }
       }
@@ -177,61 +189,67 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       pdl_trigger();
     }
     const int num_tiles = grouped ? groups.n_tiles[0] * tiles_n : num_tiles_plain;      // (after the wait)
-    uint32_t it = ahead;                           // k-slices issued so far, over all tiles
+    int s = ahead % stages, round = ahead / stages;      // the next slice's stage, and how often the stages have gone round
     bool ok = true;
     for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step) {
       int m0, n0, w0, m_end;
       coords(tile, num_tiles, &m0, &n0, &w0, &m_end);
       n0 += w0;                                    // the row of W's tensor map
-      for (int kt = tile == first_tile ? ahead : 0; kt < k_tiles; ++kt, ++it) {
-        const int s = it % T5_STAGES;
-        if (it >= T5_STAGES && !warp_wait(&empty_bar[s], ((it / T5_STAGES) & 1) ^ 1, status, T5_ERR_PRODUCER, abort_flag)) {
+      for (int kt = tile == first_tile ? ahead : 0; kt < k_tiles; ++kt) {
+        if (round > 0 && !warp_wait(&empty_bar[s], (round & 1) ^ 1, status, T5_ERR_PRODUCER, abort_flag)) {
           ok = false;
           break;
         }
         if (elect_one()) {
-          mbar_expect_tx(&full_bar[s], T5_STAGE_BYTES);
+          expect(s);
           load_x(s, kt, m0);
           load_w(s, kt, n0);
         }
         __syncwarp();
+        if (++s == stages) s = 0, ++round;
       }
     }
   } else if (warp == 1) {
     pdl_wait();
     pdl_trigger();
     // MMA issue: the whole warp runs the loop, one elected lane issues the instructions
-    constexpr uint32_t idesc = umma_idesc(T5_BM, T5_BN);
+    const uint32_t idesc = umma_idesc(T5_BM * CLUSTER, bn);
     const uint64_t desc0 = umma_desc_sw128(smem_u32(tiles));      // a step along the tiles adds (bytes >> 4)
     const int num_tiles = grouped ? groups.n_tiles[0] * tiles_n : num_tiles_plain;
-    uint32_t it = 0, local = 0;                    // k-slices consumed; tiles done by this block
-    bool ok = true;
+    uint32_t local = 0;                            // tiles done by this block
+    int s = 0, round = 0;
+    bool ok = rank == 0;                           // (the second block of a pair issues nothing)
     for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++local) {
       const uint32_t buf = local & 1;
       // the epilogue must have drained this buffer (its previous use was tile local - 2)
       if (local >= 2 && !warp_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, status, T5_ERR_MMA, abort_flag)) break;
       tcgen05_after_sync();
-      const uint32_t acc = tmem_base + buf * T5_BN;
-      for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-        const int s = it % T5_STAGES;
-        if (!warp_wait(&full_bar[s], (it / T5_STAGES) & 1, status, T5_ERR_MMA, abort_flag)) {
+      const uint32_t acc = tmem_base + buf * 256;
+      for (int kt = 0; kt < k_tiles; ++kt) {
+        if (!warp_wait(&full_bar[s], round & 1, status, T5_ERR_MMA, abort_flag)) {
           ok = false;
           break;
         }
         tcgen05_after_sync();
         if (elect_one()) {
-          const uint64_t a_desc = desc0 + ((static_cast<uint32_t>(s) * T5_STAGE_BYTES) >> 4);
+          const uint64_t a_desc = desc0 + ((static_cast<uint32_t>(s) * stage_bytes) >> 4);
           const uint64_t b_desc = a_desc + (T5_A_BYTES >> 4);
 #pragma unroll
           for (int k = 0; k < T5_BK / 16; ++k) {
             // 16 elements of K = 32 bytes further along the swizzled row
-            umma_bf16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            if constexpr (PAIR) umma_bf16_pair(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
+            else umma_bf16(acc, a_desc + 2 * k, b_desc + 2 * k, idesc, (kt > 0 || k > 0) ? 1u : 0u);
           }
-          P::commit_stage_free(&empty_bar[s]);       // arrives (in both blocks of a pair) when these MMAs have read the stage
+          if constexpr (PAIR) umma_commit_pair(&empty_bar[s]);      // arrives when these MMAs have read the stage
+          else umma_commit(&empty_bar[s]);
         }
         __syncwarp();
+        if (++s == stages) s = 0, ++round;
       }
-      if (ok && elect_one()) umma_commit(&acc_full[buf]);    // arrives when every MMA issued so far has completed
+      if (ok && elect_one()) {                     // arrives when every MMA issued so far has completed
+        if constexpr (PAIR) umma_commit_pair(&acc_full[buf]);
+        else umma_commit(&acc_full[buf]);
+      }
       __syncwarp();
     }
   } else {
@@ -250,21 +268,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const int row = m0 + quarter * 32 + lane;
       if (!warp_wait(&acc_full[buf], (local >> 1) & 1, status, T5_ERR_EPILOGUE, abort_flag)) break;
       tcgen05_after_sync();
-      const uint32_t lane_addr = tmem_base + buf * T5_BN + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t lane_addr = tmem_base + buf * 256 + (static_cast<uint32_t>(quarter * 32) << 16);
       unsigned char* my_stage = store_stage + (warp - 2) * (T5_STORE_BYTES / 4);
       const int row0 = m0 + quarter * 32;
+      const int n_end = min(swiglu ? gate_rows : N, n0 + n_per_tile);      // one past the last feature this tile may store
       if (swiglu && coeffs != nullptr) {
         // clamped halves with biases: a branch of its own, so that the plain epilogue stays as small as it was
         const float limit = coeffs[0], gate_scale = coeffs[1];
         const float* bias_g = coeffs + CLAMPED_HEADER;
         const float* bias_u = bias_g + gate_rows;            // (gate_rows is a multiple of 8)
-        for (int c0 = 0; c0 < T5_BN / 2; c0 += 64) {
+        for (int c0 = 0; c0 < bn / 2; c0 += 64) {
           uint4 w[8];
 #pragma unroll 1
           for (int hh = 0; hh < 2; ++hh) {
             uint32_t g[32], u[32];
             tmem_ld32(lane_addr + c0 + hh * 32, g);
-            tmem_ld32(lane_addr + T5_BN / 2 + c0 + hh * 32, u);
+            tmem_ld32(lane_addr + bn / 2 + c0 + hh * 32, u);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -283,17 +302,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
               else w[4 + j / 8] = q;
             }
           }
-          store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, gate_rows);
+          store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, n_end);
         }
       } else if (swiglu) {
         bf16* out = static_cast<bf16*>(y);
-        for (int c0 = 0; c0 < T5_BN / 2; c0 += 64) {
+        for (int c0 = 0; c0 < bn / 2; c0 += 64) {
           uint4 w[8];
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             uint32_t g[32], u[32];
             tmem_ld32(lane_addr + c0 + hh * 32, g);
-            tmem_ld32(lane_addr + T5_BN / 2 + c0 + hh * 32, u);
+            tmem_ld32(lane_addr + bn / 2 + c0 + hh * 32, u);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -307,7 +326,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
               w[hh * 4 + j / 8] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
           }
-          store_rows_bf16(w, my_stage, lane, out, ldy, row0, M, n0 + c0, gate_rows);   // gate_rows is a multiple of 8
+          store_rows_bf16(w, my_stage, lane, out, ldy, row0, M, n0 + c0, n_end);   // a multiple of 8
         }
       } else if (mode == T5_OUT_QKV_ROPE) {
         // W = [Wq; Wk; Wv]: a tile holds whole heads (head_dim 64 or 128 divides the tile width). Thread = row:
@@ -323,7 +342,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         // A warp past the last row has nothing to read or write; a row past it inside a live warp is carried along
         // unrotated (its sines and cosines are not looked up or worked out).
         const bool warp_live = row - lane < M;
-        for (int h0 = 0; warp_live && h0 < T5_BN && n0 + h0 < N; h0 += hd) {
+        for (int h0 = 0; warp_live && h0 < bn && n0 + h0 < N; h0 += hd) {
           const int head = (n0 + h0) / hd;                // q heads, then k heads, then v heads
           const bool rotated = head < rope.n_heads + rope.n_kv_heads;
           bf16* dst = nullptr;
@@ -381,7 +400,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       } else if (mode == T5_OUT_XIELU) {
         // xIELU with the two coefficients in memory; a branch of its own, so that the plain epilogue stays as small as it was
         const float c0_x = coeffs[0], c1_x = coeffs[1];
-        for (int c0 = 0; c0 < T5_BN; c0 += 64) {
+        for (int c0 = 0; c0 < bn; c0 += 64) {
           uint4 w[8];
 #pragma unroll 1
           for (int hh = 0; hh < 2; ++hh) {
@@ -397,11 +416,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
               else w[4 + j / 8] = q;
             }
           }
-          store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, N);   // N is a multiple of 8
+          store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, n_end);   // a multiple of 8
         }
       } else if (mode == T5_OUT_PAIRS) {
         // rows 2j and 2j + 1 of W are the gate and up rows of feature j: 128 columns of the tile give 64 of the output
-        for (int c0 = 0; c0 < T5_BN; c0 += 128) {
+        for (int c0 = 0; c0 < bn; c0 += 128) {
           uint4 w[8];
 #pragma unroll
           for (int hh = 0; hh < 4; ++hh) {
@@ -420,7 +439,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
           store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, (n0 + c0) / 2, N / 2);   // N / 2 is a multiple of 8
         }
       } else {
-        for (int c0 = 0; c0 < T5_BN; c0 += 64) {
+        for (int c0 = 0; c0 < bn; c0 += 64) {
           uint32_t va[32], vb[32];
           tmem_ld32(lane_addr + c0, va);
           tmem_ld32(lane_addr + c0 + 32, vb);
@@ -434,7 +453,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
                   const int col = n0 + c0 + hh * 32 + j;
-                  if (col < N)                    // N is a multiple of 4 in this mode
+                  if (col < n_end)                // a multiple of 4 in this mode
                     *reinterpret_cast<float4*>(out + col) =
                         make_float4(__uint_as_float(v[j]) * out_scale, __uint_as_float(v[j + 1]) * out_scale,
                                     __uint_as_float(v[j + 2]) * out_scale, __uint_as_float(v[j + 3]) * out_scale);
@@ -464,23 +483,27 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 w[hh * 4 + j / 8] = make_uint4(pack2_bf16(fin(v[j]), fin(v[j + 1])), pack2_bf16(fin(v[j + 2]), fin(v[j + 3])),
                                                pack2_bf16(fin(v[j + 4]), fin(v[j + 5])), pack2_bf16(fin(v[j + 6]), fin(v[j + 7])));
             }
-            store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, N);   // N is a multiple of 8
+            store_rows_bf16(w, my_stage, lane, static_cast<bf16*>(y), ldy, row0, M, n0 + c0, n_end);   // a multiple of 8
           }
         }
       }
       // this warp has read its part of the buffer: let the MMA warp reuse it
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_first_block(&acc_empty[buf]);
+        else mbar_arrive(&acc_empty[buf]);
+      }
     }
   }
   // common exit: every role arrives here, with or without a timeout
   drain_after_abort(abort_flag);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if constexpr (P::CLUSTER == 2) cluster_sync_all();      // nobody leaves while its partner may still send to it
+  if constexpr (PAIR) cluster_sync_all();              // nobody leaves while its partner may still send to it or read from it
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T5_TMEM_COLS) : "memory");
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T5_TMEM_COLS) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T5_TMEM_COLS) : "memory");
   }
 }
 
@@ -508,9 +531,82 @@ static inline int make_map(CUtensorMap* map, const void* base, int rows, int col
 // CLAMPED_HEADER) the gated activation with clamped halves and biases; mode 4: y bf16 [M, N] = max(x W^T, 0)^2; mode 5: = gelu_tanh(x W^T);
 // mode 7: = xIELU(x W^T) with coeffs = two float32 on the device. status: one device int, set to a nonzero code if a wait
 // inside the kernel timed out (left untouched otherwise).
-template <class P>
+static int t5_sm_count() {
+  static int sm_count = 0;
+  if (sm_count == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
+  }
+  return sm_count;
+}
+
+// What a round of tiles of bn columns takes, of blocks alone or of pairs, in rounds of 256-wide tiles of pairs (24.1 us at K
+// 4096). Measured on B200 over all widths at 2499 x 28672 (SwiGLU) x 4096; at 23 products from 64 to 2,499 rows the width and
+// kind with the least rounds x cost is the fastest measured or within 5 % of it. Below 128 columns a round no longer gets
+// shorter: the 128 rows of x of every block are what it brings in. Against blocks alone at 256, 192 or 128 columns, with pairs
+// that only shared W's loads for the largest products (us, cold caches, same order of sums): 2048 x 16384 (SwiGLU) x 2048 98
+// -> 86; 2048 x 2048 x 8192 70 -> 57; 2499 x 28672 (SwiGLU) x 4096 395 -> 382; 2499 x 4096 x 14336 230 -> 202; 543 x 16384
+// (SwiGLU) x 3072 72 -> 57; 543 x 3072 x 8192 53 -> 43.
+static double t5_tile_cost(int bn, bool pair) {
+  static const double alone[] = {0.65, 0.63, 0.672, 0.755, 0.813, 0.963, 1.025};       // 64, 96, .. 256
+  static const double paired[] = {0.62, 0.637, 0.643, 0.68, 0.755, 0.88, 1.0};
+  return (pair ? paired : alone)[(bn - 64) / 32];
+}
+
+struct T5Choice {
+  int bn;
+  bool pair;
+};
+
+// The width and kind of tile whose rounds over the SMs cost least. SwiGLU pairs gate and up columns, so a tile holds bn / 2
+// features; the q | k | v epilogue needs whole heads (or, at head size 128, whole tiles of heads) in a tile.
+// pairs: 0 never, 1 always, -1 by cost.
+static T5Choice t5_choose(long long m_blocks, int feats, int mode, int head_dim, int sms, int pairs) {
+  // DYNALM_GEMM_TILE=<multiple of 32, 64 to 256> overrides the width where it is allowed
+  static int forced = -1;
+  if (forced < 0) {
+    const char* e = getenv("DYNALM_GEMM_TILE");
+    forced = e ? atoi(e) : 0;
+  }
+  T5Choice best = {256, false};
+  double least = 1e300;
+  for (int pair = 0; pair < 2; ++pair) {
+    if (pairs >= 0 && pairs != pair) continue;
+    for (int bn = 256; bn >= 64; bn -= 32) {
+      if (mode == dl::T5_OUT_QKV_ROPE && bn % head_dim != 0) continue;
+      if (forced >= 64 && forced <= 256 && forced % 32 == 0 && forced != bn && (mode != dl::T5_OUT_QKV_ROPE || forced % head_dim == 0)) continue;
+      const int per = mode == dl::T5_OUT_SWIGLU ? bn / 2 : bn;
+      const long long t = (m_blocks + pair) / (1 + pair) * ((feats + per - 1) / per);
+      const int units = sms / (1 + pair);
+      const double c = static_cast<double>((t + units - 1) / units) * t5_tile_cost(bn, pair != 0);
+      if (c < least) {
+        least = c;
+        best = {bn, pair != 0};
+      }
+    }
+  }
+  return best;
+}
+
+template <bool PAIR>
+static int t5_run(cudaLaunchConfig_t cfg, const CUtensorMap& map_x, const CUtensorMap& map_w, void* y, int ldy, int M, int N,
+                  int K, int mode, float out_scale, int gate_rows, int tiles_n, int tiles, int group_m, int* status,
+                  const dl::QkvRope& rope, const dl::T5Groups& groups, const float* coeffs, int bn) {
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(dl::T5_SMEM));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  cfg.dynamicSmemBytes = dl::T5_SMEM;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<PAIR>, map_x, map_w, y, ldy, M, N, K, mode, out_scale,
+                                             gate_rows, tiles_n, tiles, group_m, status, rope, groups, coeffs, bn));
+}
+
 static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, int mode, float out_scale,
-                     int* status, const dl::QkvRope& rope, cudaStream_t stream, const float* coeffs = nullptr) {
+                     int* status, const dl::QkvRope& rope, int pairs, cudaStream_t stream, const float* coeffs = nullptr) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || (K & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) ||
       status == nullptr || mode < 0 || (mode > 5 && mode != dl::T5_OUT_XIELU) || (mode == dl::T5_OUT_XIELU && coeffs == nullptr))
@@ -520,34 +616,12 @@ static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, in
   if ((mode == dl::T5_OUT_SWIGLU && (N & 1)) || (mode == dl::T5_OUT_F32 ? (feats & 3) || (ldy & 3) : (feats & 7) || (ldy & 7)) ||
       (reinterpret_cast<uintptr_t>(y) & 15))
     return DL_ERR_UNSUPPORTED;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
-  }
+  const int sms = t5_sm_count();
   const long long m_blocks = (M + dl::T5_BM - 1) / dl::T5_BM;
-  const long long m_tiles = (m_blocks + P::CLUSTER - 1) / P::CLUSTER;      // pairs of row blocks in a cluster
-  // Tile width: the one whose rounds over the SMs cost least, a round of 192- or 128-wide tiles taking about 0.78
-  // or 0.7 of a round of 256-wide ones (measured). SwiGLU pairs gate and up columns in halves of 64: 256 or 128. The
-  // q | k | v epilogue needs whole heads in a tile.
-  const int units = sm_count / P::CLUSTER;                                  // blocks, or clusters of two
-  auto cost = [&](int bn, double per_round) {
-    const int per = mode == dl::T5_OUT_SWIGLU ? bn / 2 : bn;
-    const long long t = m_tiles * ((feats + per - 1) / per);
-    return static_cast<double>((t + units - 1) / units) * per_round;
-  };
-  static int forced = -1;      // DYNALM_GEMM_TILE=128|192|256 overrides the choice where the width is allowed (for measurements)
-  if (forced < 0) { const char* e = getenv("DYNALM_GEMM_TILE"); forced = e ? atoi(e) : 0; }
-  int bn = 256;
-  double best = cost(256, 1.0);
-  const bool can192 = mode != dl::T5_OUT_SWIGLU && (mode != dl::T5_OUT_QKV_ROPE || 192 % rope.head_dim == 0);
-  if (can192 && cost(192, 0.78) < best) {
-    bn = 192;
-    best = cost(192, 0.78);
-  }
-  if (cost(128, 0.7) < best) bn = 128;
-  if (forced == 128 || forced == 256 || (forced == 192 && can192)) bn = forced;
+  const T5Choice choice = t5_choose(m_blocks, feats, mode, rope.head_dim, sms, pairs);
+  const int cluster = choice.pair ? 2 : 1, bn = choice.bn;
+  const long long m_tiles = (m_blocks + cluster - 1) / cluster;
+  const int units = sms / cluster;                                          // blocks, or pairs of them
   const int per_tile = mode == dl::T5_OUT_SWIGLU ? bn / 2 : bn;
   const int tiles_n = (feats + per_tile - 1) / per_tile;
   const long long tiles = m_tiles * tiles_n;
@@ -561,20 +635,20 @@ static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, in
   // 4 to 16. DYNALM_GEMM_GROUP_M overrides it (1: along the columns first).
   static int forced_group = -1;
   if (forced_group < 0) { const char* e = getenv("DYNALM_GEMM_GROUP_M"); forced_group = e ? atoi(e) : 0; }
-  long long group = (32ll << 20) / (2ll * dl::T5_BM * P::CLUSTER * K);
+  long long group = (32ll << 20) / (2ll * dl::T5_BM * cluster * K);
   group = group < 4 ? 4 : (group > 16 ? 16 : group);
   if (forced_group > 0) group = forced_group;
   const int group_m = static_cast<int>(group < m_tiles ? group : m_tiles);
-  const int blocks = static_cast<int>(tiles < units ? tiles : units) * P::CLUSTER;
+  const int blocks = static_cast<int>(tiles < units ? tiles : units) * cluster;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(dl::T5_THREADS);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   int n_attr = 0;
-  if (P::CLUSTER > 1) {
+  if (choice.pair) {
     attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-    attr[n_attr].val.clusterDim.x = P::CLUSTER;
+    attr[n_attr].val.clusterDim.x = 2;
     attr[n_attr].val.clusterDim.y = 1;
     attr[n_attr].val.clusterDim.z = 1;
     ++n_attr;
@@ -587,51 +661,20 @@ static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, in
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
   const int gate_rows = mode == dl::T5_OUT_SWIGLU ? N / 2 : 0;
-  if (bn == 256) {
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<256, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(dl::T5<256>::SMEM));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured = true;
-    }
-    cfg.dynamicSmemBytes = dl::T5<256>::SMEM;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<256, P>, map_x, map_w, y, ldy, M, N, K, mode,
-                                               out_scale, gate_rows, tiles_n, static_cast<int>(tiles), group_m, status, rope, dl::T5Groups{nullptr, nullptr, 0}, coeffs));
-  } else if (bn == 192) {
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<192, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(dl::T5<192>::SMEM));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured = true;
-    }
-    cfg.dynamicSmemBytes = dl::T5<192>::SMEM;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<192, P>, map_x, map_w, y, ldy, M, N, K, mode,
-                                               out_scale, gate_rows, tiles_n, static_cast<int>(tiles), group_m, status, rope, dl::T5Groups{nullptr, nullptr, 0}, coeffs));
-  } else {
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<128, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(dl::T5<128>::SMEM));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured = true;
-    }
-    cfg.dynamicSmemBytes = dl::T5<128>::SMEM;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<128, P>, map_x, map_w, y, ldy, M, N, K, mode,
-                                               out_scale, gate_rows, tiles_n, static_cast<int>(tiles), group_m, status, rope, dl::T5Groups{nullptr, nullptr, 0}, coeffs));
-  }
+  const dl::T5Groups plain = {nullptr, nullptr, 0};
+  return choice.pair ? t5_run<true>(cfg, map_x, map_w, y, ldy, M, N, K, mode, out_scale, gate_rows, tiles_n, static_cast<int>(tiles),
+                                    group_m, status, rope, plain, coeffs, bn)
+                     : t5_run<false>(cfg, map_x, map_w, y, ldy, M, N, K, mode, out_scale, gate_rows, tiles_n, static_cast<int>(tiles),
+                                     group_m, status, rope, plain, coeffs, bn);
 }
 
 // A grouped product (see T5Groups): a bf16 [rows, K] whose runs of rows are listed in `tiles`, w bf16 [matrices, N, K]
 // contiguous, y [rows, N] bf16 (mode 0, or 4 with the squared ReLU) or fp32 (mode 1), or with mode 6 (gate and up rows of w
 // in turn, N a multiple of 16) y [rows, N / 2] bf16. max_row_tiles: the most row tiles
 // the list can hold; the grid is sized for it and blocks past the list's end do nothing.
-template <class P>
 static int t5_launch_grouped(const void* a, int lda, int rows, const void* w, int matrices, int N, int K, void* y, int ldy,
                              int mode, const int* tiles, const int* n_tiles, int max_row_tiles, int* status,
                              cudaStream_t stream) {
-  static_assert(P::CLUSTER == 1, "a grouped product runs every block for itself");
   if (rows <= 0 || N <= 0 || max_row_tiles <= 0) return 0;
   if (K <= 0 || (K & 7) || (lda & 7) || (reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) ||
       (reinterpret_cast<uintptr_t>(y) & 15) || status == nullptr || tiles == nullptr || n_tiles == nullptr || matrices <= 0 ||
@@ -640,12 +683,6 @@ static int t5_launch_grouped(const void* a, int lda, int rows, const void* w, in
       (mode == dl::T5_OUT_F32 ? (N & 3) || (ldy & 3) : (N & 7) || (ldy & 7)) ||
       static_cast<long long>(matrices) * N > (1ll << 30))
     return DL_ERR_UNSUPPORTED;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
-  }
   const int bn = N >= 256 ? 256 : 128;
   const int tiles_n = (N + bn - 1) / bn;
   const long long most = static_cast<long long>(max_row_tiles) * tiles_n;
@@ -656,41 +693,19 @@ static int t5_launch_grouped(const void* a, int lda, int rows, const void* w, in
   rc = dl::make_map(&map_w, w, matrices * N, K, K, bn / 2);
   if (rc != 0) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(most < sm_count ? most : sm_count));
+  cfg.gridDim = dim3(static_cast<unsigned>(most < t5_sm_count() ? most : t5_sm_count()));
   cfg.blockDim = dim3(dl::T5_THREADS);
   cfg.stream = stream;
   const dl::QkvRope none = {};
   const dl::T5Groups groups = {tiles, n_tiles, N};
-  if (bn == 256) {
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<256, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(dl::T5<256>::SMEM));
-      if (e != cudaSuccess) return static_cast<int>(e);
-      configured = true;
-    }
-    cfg.dynamicSmemBytes = dl::T5<256>::SMEM;
-    return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<256, P>, map_x, map_w, y, ldy, rows, N, K, mode,
-                                               1.0f, 0, tiles_n, 0, 1, status, none, groups, nullptr));
-  }
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(dl::gemm_tcgen05_kernel<128, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(dl::T5<128>::SMEM));
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
-  cfg.dynamicSmemBytes = dl::T5<128>::SMEM;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, dl::gemm_tcgen05_kernel<128, P>, map_x, map_w, y, ldy, rows, N, K, mode,
-                                             1.0f, 0, tiles_n, 0, 1, status, none, groups, nullptr));
+  return t5_run<false>(cfg, map_x, map_w, y, ldy, rows, N, K, mode, 1.0f, 0, tiles_n, 0, 1, status, none, groups, nullptr, bn);
 }
 
 // Fills the epilogue's parameters for the q | k | v product and launches it (see dl_gemm_tcgen05_qkv_rope).
-template <class P>
 static int t5_launch_qkv_rope(const void* x, int ldx, const void* w, void* q_out, int ldq, int M, int K, const int* positions,
                               const int* row_request, const int* block_table, int max_blocks, void* k_cache, void* v_cache,
                               const float* inv_freq, const void* angles, float pos_scale, int n_heads, int n_kv_heads,
-                              int head_dim, int page_size, int* status, cudaStream_t stream) {
+                              int head_dim, int page_size, int* status, int pairs, cudaStream_t stream) {
   if ((head_dim != 64 && head_dim != 128) || n_heads <= 0 || n_kv_heads <= 0 || page_size <= 0 || inv_freq == nullptr ||
       (reinterpret_cast<uintptr_t>(k_cache) & 15) || (reinterpret_cast<uintptr_t>(v_cache) & 15) ||
       (reinterpret_cast<uintptr_t>(angles) & 15))
@@ -709,6 +724,6 @@ static int t5_launch_qkv_rope(const void* x, int ldx, const void* w, void* q_out
   p.n_kv_heads = n_kv_heads;
   p.head_dim = head_dim;
   p.page_size = page_size;
-  return t5_launch<P>(x, ldx, w, q_out, ldq, M, (n_heads + 2 * n_kv_heads) * head_dim, K, dl::T5_OUT_QKV_ROPE, 1.0f, status, p,
-                      stream);
+  return t5_launch(x, ldx, w, q_out, ldq, M, (n_heads + 2 * n_kv_heads) * head_dim, K, dl::T5_OUT_QKV_ROPE, 1.0f, status, p,
+                   pairs, stream);
 }

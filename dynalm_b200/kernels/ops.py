@@ -133,13 +133,11 @@ _SIGNATURES = {
         "dl_gemm_skinny": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _L, _P, _P],
         "dl_gemm_skinny_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _F, _I, _I, _I, _I, _P]},
     "gemm_tcgen05": {
-        "dl_gemm_tcgen05": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _P],
+        "dl_gemm_tcgen05": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _I, _P],
         "dl_gemm_tcgen05_tile_coords": [_I, _I, _I, _I, _P, _P],
+        "dl_gemm_tcgen05_choice": [_I, _I, _I, _I, _I, _I, _P, _P],
         "dl_gemm_tcgen05_grouped": [_P, _I, _I, _P, _I, _I, _I, _P, _I, _I, _P, _P, _I, _P, _P],
-        "dl_gemm_tcgen05_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _F, _I, _I, _I, _I, _P, _P]},
-    "gemm_tcgen05_cluster": {
-        "dl_gemm_tcgen05_cluster": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _P],
-        "dl_gemm_tcgen05_cluster_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _F, _I, _I, _I, _I, _P, _P]},
+        "dl_gemm_tcgen05_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _F, _I, _I, _I, _I, _P, _I, _P]},
     "gemm_stream_tcgen05": {
         "dl_gemm_stream": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _P, _P]},
     "gemm_simt": {"dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P]},
@@ -1220,13 +1218,12 @@ def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, pos
             or row_request.dtype != torch.int32:
         raise InvalidArgument("gemm_qkv_rope: positions, row_request and block_table must be int32")
     if not few:
-        library, name = (("gemm_tcgen05_cluster", "dl_gemm_tcgen05_cluster_qkv_rope") if tcgen05_pairs(M, w_qkv.shape[0])
-                         else ("gemm_tcgen05", "dl_gemm_tcgen05_qkv_rope"))
-        check_limits(library, pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
-        _check(_fn(library, name)(
+        check_limits("gemm_tcgen05", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
+        _check(_fn("gemm_tcgen05", "dl_gemm_tcgen05_qkv_rope")(
             _p(x), x.stride(0), _p(w_qkv), _p(q_out), q_out.stride(0), M, K, _p(positions), _p(row_request),
             _p(block_table), block_table.stride(0), _p(k_cache), _p(v_cache), _p(inv_freq), _p(angles), pos_scale, n_heads,
-            n_kv_heads, head_dim, page_size, _p(_status_word(x.device)), _stream()), "gemm_tcgen05_qkv_rope")
+            n_kv_heads, head_dim, page_size, _p(_status_word(x.device)), tcgen05_pairs(M, w_qkv.shape[0]), _stream()),
+               "gemm_tcgen05_qkv_rope")
         return
     check_limits("gemm_skinny", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
     _check(_fn("gemm_skinny", "dl_gemm_skinny_qkv_rope")(
@@ -1236,24 +1233,20 @@ def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, pos
 
 
 _tcgen05_status = {}
-_pairs: Optional[bool] = None      # whether the variant with pairs of blocks sharing W tiles can be used
 
 
-# rounds of 128 x 256 tiles over the SMs from which sharing W tiles between two blocks pays (measured on B200)
-PAIRS_MIN_WAVES = float(os.environ.get("DYNALM_GEMM_PAIRS_MIN_WAVES", "4"))
+# None: the tcgen05 product has two blocks work on a tile where that costs least (csrc/gemm_tcgen05_impl.cuh); a number: exactly
+# from that many rounds of 128 x 256 tiles over the SMs on.
+_waves = os.environ.get("DYNALM_GEMM_PAIRS_MIN_WAVES")
+PAIRS_MIN_WAVES: Optional[float] = float(_waves) if _waves else {"0": float(1 << 30), "1": 0.0}.get(os.environ.get("DYNALM_GEMM_PAIRS", ""))
 
 
-def tcgen05_pairs(rows: int, features: int) -> bool:
-    """Large products run the tcgen05 kernel in which two thread blocks share each tile of W
-    (csrc/gemm_tcgen05_cluster.cu: 108 us against 119 us for 2048 x 16384 x 2048, 423 against 454 for 8192 rows),
-    unless DYNALM_GEMM_PAIRS=0 or that source file is not there; smaller ones, where the pairing only couples the
-    blocks' pipelines (54 us against 52 us for 2048 x 2048 x 8192), run csrc/gemm_tcgen05.cu."""
-    global _pairs
-    if _pairs is None:
-        _pairs = os.environ.get("DYNALM_GEMM_PAIRS", "1") != "0" and \
-            os.path.isfile(os.path.join(_lib.CSRC, "gemm_tcgen05_cluster.cu"))
+def tcgen05_pairs(rows: int, features: int) -> int:
+    """-1: by cost, 0 or 1: blocks alone or in pairs (see PAIRS_MIN_WAVES)."""
+    if PAIRS_MIN_WAVES is None:
+        return -1
     from .device import sm_count
-    return _pairs and -(-rows // 128) * -(-features // 256) >= PAIRS_MIN_WAVES * sm_count()
+    return int(-(-rows // 128) * -(-features // 256) >= PAIRS_MIN_WAVES * sm_count())
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -1459,10 +1452,8 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str 
         else:
             raise InvalidArgument("gemm_tcgen05: out bfloat16 or float32")
     status = _status_word(x.device)
-    library, name = (("gemm_tcgen05_cluster", "dl_gemm_tcgen05_cluster") if tcgen05_pairs(M, N)
-                     else ("gemm_tcgen05", "dl_gemm_tcgen05"))
-    _check(_fn(library, name)(_p(x), x.stride(0), _p(w), _p(out), out.stride(0), M, N, K, code, out_scale, _p(coeffs), _p(status),
-                              _stream()), "gemm_tcgen05")
+    _check(_fn("gemm_tcgen05", "dl_gemm_tcgen05")(_p(x), x.stride(0), _p(w), _p(out), out.stride(0), M, N, K, code, out_scale, _p(coeffs), _p(status),
+                                                   tcgen05_pairs(M, N), _stream()), "gemm_tcgen05")
 
 
 def gemm_tcgen05_tile_coords(tile: int, tiles_n: int, num_tiles: int, group_m: int):
@@ -1474,6 +1465,17 @@ def gemm_tcgen05_tile_coords(tile: int, tiles_n: int, num_tiles: int, group_m: i
     _check(_fn("gemm_tcgen05", "dl_gemm_tcgen05_tile_coords")(tile, tiles_n, num_tiles, group_m, byref(m), byref(n)),
            "gemm_tcgen05_tile_coords")
     return m.value, n.value
+
+
+def gemm_tcgen05_choice(rows: int, features: int, mode: str = "store", head_dim: int = 64, sms: int = 148, pairs: int = -1):
+    """(columns of a tile, whether a pair of blocks computes it) of the tcgen05 product at these sizes; `features` counts outputs
+    (for "swiglu" half of W's rows). Runs on the host."""
+    from ctypes import byref, c_int
+    bn, pair = c_int(-1), c_int(-1)
+    code = {"store": 0, "f32": 1, "swiglu": 2, "qkv_rope": 3}[mode]
+    _check(_fn("gemm_tcgen05", "dl_gemm_tcgen05_choice")(rows, features, code, head_dim, sms, pairs, byref(bn), byref(pair)),
+           "gemm_tcgen05_choice")
+    return bn.value, bool(pair.value)
 
 
 STREAM_MAX_ROWS = 64       # what the tcgen05 weight-streaming product takes

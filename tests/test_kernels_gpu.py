@@ -839,6 +839,33 @@ def tile_sharing(request, ops, monkeypatch):
     return request.param
 
 
+@pytest.mark.parametrize("mode", ["store", "f32", "swiglu"])
+def test_gemm_tcgen05_every_tile(ops, mode, monkeypatch):
+    """Every width of tile that the cost rule takes at some size, of blocks alone and of pairs, with rows and columns that end
+    inside a tile: bf16 operands, sums in float32 (K 200: a bound of 2^-24 K on them), the result rounded to bf16."""
+    g = torch.Generator(device="cpu").manual_seed(77)
+    found = {}
+    for pairs in (0, 1):
+        for rows in (130, 200, 383, 641, 1100):
+            for feats in range(136, 5000, 264):
+                found.setdefault(ops.gemm_tcgen05_choice(rows, feats, mode, pairs=pairs), (rows, feats))
+    assert len(found) >= 12, found
+    K = 200
+    for (bn, pair), (rows, feats) in found.items():
+        monkeypatch.setattr(ops, "PAIRS_MIN_WAVES", 0 if pair else 1 << 30)
+        n = 2 * feats if mode == "swiglu" else feats
+        x = torch.randn(rows, K, generator=g).to(DEV, torch.bfloat16)
+        w = (torch.randn(n, K, generator=g) * 0.2).to(DEV, torch.bfloat16)
+        out = torch.full((rows, feats), 9.0, dtype=torch.float32 if mode == "f32" else torch.bfloat16, device=DEV)
+        ops.gemm_tcgen05(x, w, out, "swiglu" if mode == "swiglu" else "store")
+        z = x.double() @ w.double().T
+        ref = torch.nn.functional.silu(z[:, :feats]) * z[:, feats:] if mode == "swiglu" else z
+        tol_ = 2.0 ** -24 * K * (x.double().abs() @ w.double().abs().T).max().item() if mode == "f32" else None
+        err = (out.double() - ref).abs()
+        assert (err <= (tol_ if tol_ is not None else 2.0 ** -7 * ref.abs() + 2e-3)).all(), (bn, pair, rows, feats, err.max())
+    assert ops.gemm_tcgen05_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (128, 256, 256), (100, 264, 200), (300, 1000, 136), (17, 48, 8),
                                    (2048, 3072, 2048), (513, 4096, 1024)])
 def test_gemm_tcgen05(ops, tile_sharing, M, N, K):
