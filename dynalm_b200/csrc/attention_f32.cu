@@ -1,0 +1,517 @@
+// Paged causal attention of the 32-bit path over a step's query tiles and its single-token rows.
+//
+// The masks, the sink and the distance bias are those of attention_generic.cu, which stays for sizes that these kernels do
+// not take (heads above 128 numbers, sizes or addresses off the 16-byte grid) and for steps without query tiles. All
+// arithmetic is float32 on the multiply-add lanes, expf and no faster exponential.
+//
+// What a row computes depends on its own query, position and keys alone, in the same order in both kernels: keys in tiles of
+// 64 at absolute multiples of 64; a score is a running fma over the head; of a tile m_t = the largest score, p = exp(s - m_t),
+// l_t = the p's of keys j, j + 16, j + 32, j + 48 in their order and those 16 sums as a tree, a_t = a running fma over the
+// keys; tiles are merged in their order by the (max, sum, weighted sum) rule (dynacore/cpu/cpu_device.cpp:1782-1845). So it
+// makes no difference how a prompt was cut nor which kernel took a row. A key that a row does not see is not multiplied in,
+// so that no infinity reaches a row that does not see it.
+//
+// * f32_tiles_kernel: 64 query rows of one request and one head a block, 256 threads, 4 x 4 scores and 4 rows x D / 16
+//   values a thread; keys and values by cp.async, the next tile's keys on their way while the values are multiplied.
+// * f32_rows_kernel: a row's keys over the warps of up to eight blocks (a cluster along the keys), a tile of 64 a warp, for
+//   up to four query heads of one KV head at once, so that a key is read once for them. A warp asks for its whole tile of
+//   keys and values at once (cp.async), and for the next tile's as soon as a buffer has been read: with a few rows it is the
+//   trips to memory that the time goes into. The warps' (m, l, a) meet in shared memory, over the cluster where it has
+//   several blocks, and are merged in the order of the keys.
+//
+// Bound by the multiply-add lanes (tiles) and by trips to memory (rows). Measured on B200, a layer of 32:8 heads of 64, against
+// attention_generic.cu: a prompt of 700 tokens 1,410 -> 146 us; four single tokens of 500 keys 94 -> 15 us.
+#include "common.cuh"
+
+#include <cooperative_groups.h>
+
+namespace dl {
+
+namespace cg = cooperative_groups;
+
+constexpr int FT = 64;                 // keys of a tile, query rows of a block
+
+struct F32Attention {
+  const float *q, *k_cache, *v_cache;
+  float* out;
+  const int* table;
+  const float *rate, *dstep;
+  long long k_row, v_row;
+  int q_stride, out_stride, max_blocks, n_heads, n_kv_heads, head_dim, vdim, page_size, window, keep_first, sink, chunk;
+  float scale;
+};
+
+// the first key a position sees (beside the kept ones in front of it)
+__device__ __forceinline__ int first_key(const F32Attention& a, int pos) {
+  return a.chunk > 0 ? pos / a.chunk * a.chunk : (a.window > 0 ? max(0, pos - a.window + 1) : 0);
+}
+
+__device__ __forceinline__ float biased(const F32Attention& a, float s, int head, int gap) {
+  return a.rate == nullptr ? s : __fsub_rn(s, __fmul_rn(a.rate[head], logf(__fadd_rn(1.0f, __fmul_rn(a.dstep[head], static_cast<float>(gap))))));
+}
+
+// x c + y d with both products rounded: the two kernels' sums agree however the compiler would contract them
+__device__ __forceinline__ float two_products(float x, float c, float y, float d) {
+  return __fadd_rn(__fmul_rn(x, c), __fmul_rn(y, d));
+}
+
+// (M, L, A) <- the tile (m, l, a) behind it; scale factors of the two sides. A side without a key leaves the other as it is.
+__device__ __forceinline__ void merge_factors(float& m_run, float m, float& c_run, float& c) {
+  const float top = fmaxf(m_run, m);
+  c_run = m_run == -INFINITY ? 0.0f : expf(m_run - top);
+  c = m == -INFINITY ? 0.0f : expf(m - top);
+  m_run = top;
+}
+
+__device__ __forceinline__ void cp_async16_f32(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(bytes)
+               : "memory");
+}
+
+template <int D>
+__global__ void __launch_bounds__(256)
+f32_tiles_kernel(F32Attention at, const int4* __restrict__ tiles) {
+  constexpr int KS = D + 4, PS = FT + 4, DV = D / 16;        // DV values of a row a thread: tx * 4 + 64 j, or tx * DV below 64
+  constexpr int RUN = DV < 4 ? DV : 4;
+  extern __shared__ __align__(16) float f32_smem[];
+  float* sq = f32_smem;                  // [FT][KS]
+  float* sk = sq + FT * KS;              // [FT][KS]
+  float* sv = sk + FT * KS;              // [FT][D]
+  float* sp = sv + FT * D;               // [FT][PS]
+  const int4 tile = ck_tile(tiles[blockIdx.x >> 1]);
+  const int half = blockIdx.x & 1, rows = min(FT, tile.z - half * FT);
+  if (rows <= 0) return;
+  const int row0 = tile.y + half * FT, pos0 = tile.w + half * FT, head = blockIdx.y;
+  const int kvh = head / (at.n_heads / at.n_kv_heads);
+  const int* table = at.table + static_cast<size_t>(ck_request(tile.x)) * at.max_blocks;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int d4 = at.head_dim >> 2, e4 = at.vdim >> 2;
+
+  const int last = pos0 + rows - 1, lo = first_key(at, pos0);
+  const int kept = lo > 0 ? min(at.keep_first, lo) : 0;      // (keys that a later row's window has passed are kept ones too)
+  const int kept_last = first_key(at, last) > 0 ? min(at.keep_first, first_key(at, last)) : 0;
+  const int kept_most = max(kept, kept_last);
+  // one run of 16 bytes of key or value t; zeros for a key that no row of the block sees
+  auto fetch = [&](float* dst, int stride, const float* cache, long long row, int size, int per, int t0) {
+    for (int e = tid; e < FT * per; e += 256) {
+      const int r = e / per, c = (e - r * per) * 4, t = t0 + r;
+      const bool there = t <= last && (t >= lo || t < kept_most);
+      const float* src = cache;
+      if (there) {
+        const size_t slot = static_cast<size_t>(ck_page(table, t / at.page_size, at.max_blocks)) * at.page_size + t % at.page_size;
+        src = cache + slot * row + static_cast<size_t>(kvh) * size + c;
+      }
+      cp_async16_f32(dst + r * stride + c, src, there ? 16 : 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto seen_tile = [&](int t0) { return t0 + FT > lo || t0 < kept_most; };
+
+  for (int e = tid; e < FT * d4; e += 256) {
+    const int r = e / d4, c = (e - r * d4) * 4;
+    cp_async16_f32(sq + r * KS + c, at.q + static_cast<size_t>(row0 + min(r, rows - 1)) * at.q_stride + static_cast<size_t>(head) * at.head_dim + c, 16);
+  }
+  int t0 = kept_most > 0 ? 0 : lo / FT * FT;
+  fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, t0);
+
+  float o[4][DV], m_run[4], l_run[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_run[i] = -INFINITY, l_run[i] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < DV; ++j) o[i][j] = 0.0f;
+  }
+  while (t0 <= last) {
+    int next = t0 + FT;
+    while (next <= last && !seen_tile(next)) next += FT;
+    fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, t0);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    // scores of rows ty * 4 .. + 3 and keys tx + 16 j
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 4
+    for (int c = 0; c < d4; ++c) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sq + (ty * 4 + i) * KS + c * 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * KS + c * 4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+          s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+          s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+          s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+        }
+    }
+    float c_run[4], c_tile[4], l_tile[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int pos = pos0 + ty * 4 + i, from = first_key(at, pos), keep = from > 0 ? min(at.keep_first, from) : 0;
+      float m = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = t0 + tx + 16 * j;
+        const bool seen = t <= pos && (t >= from || t < keep);
+        s[i][j] = seen ? biased(at, __fmul_rn(s[i][j], at.scale), head, pos - t) : -INFINITY;
+        m = fmaxf(m, s[i][j]);
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, w));
+      float l = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = s[i][j] == -INFINITY ? 0.0f : expf(s[i][j] - m);
+        sp[(ty * 4 + i) * PS + tx + 16 * j] = p;
+        l = j == 0 ? p : l + p;
+      }
+#pragma unroll
+      for (int w = 8; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+      l_tile[i] = l;
+      merge_factors(m_run[i], m, c_run[i], c_tile[i]);
+    }
+    __syncthreads();                       // the keys have been read, the p's are there
+    if (next <= last) fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, next);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    float acc[4][DV];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < DV; ++j) acc[i][j] = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < FT; k += 4) {
+      float4 p[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(sp + (ty * 4 + i) * PS + k);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float v[DV];
+#pragma unroll
+        for (int j = 0; j < DV / RUN; ++j)
+#pragma unroll
+          for (int h = 0; h < RUN; ++h) v[j * RUN + h] = sv[(k + kk) * D + tx * RUN + 64 * j + h];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+#pragma unroll
+          for (int j = 0; j < DV; ++j) acc[i][j] = w != 0.0f ? fmaf(w, v[j], acc[i][j]) : acc[i][j];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      l_run[i] = two_products(l_run[i], c_run[i], l_tile[i], c_tile[i]);
+#pragma unroll
+      for (int j = 0; j < DV; ++j) o[i][j] = two_products(o[i][j], c_run[i], acc[i][j], c_tile[i]);
+    }
+    t0 = next;
+    __syncthreads();                       // the values and the p's have been read
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = ty * 4 + i;
+    if (at.sink) {                         // one more score of 0 in the denominator; it carries no value
+      float c_run, c_tile;
+      merge_factors(m_run[i], 0.0f, c_run, c_tile);
+      l_run[i] = two_products(l_run[i], c_run, 1.0f, c_tile);
+#pragma unroll
+      for (int j = 0; j < DV; ++j) o[i][j] *= c_run;
+    }
+    if (r >= rows) continue;
+    float* orow = at.out + static_cast<size_t>(row0 + r) * at.out_stride + static_cast<size_t>(head) * at.vdim;
+#pragma unroll
+    for (int j = 0; j < DV / RUN; ++j)
+#pragma unroll
+      for (int h = 0; h < RUN; ++h) {
+        const int d = tx * RUN + 64 * j + h;
+        if (d < at.vdim) orow[d] = o[i][j * RUN + h] / l_run[i];
+      }
+  }
+}
+
+constexpr int FG = 4;                  // query heads of a block
+
+template <int D> struct FRows {
+  static constexpr int WARPS = D <= 64 ? 4 : 2;
+  static constexpr int K_FLOATS = FT * (D + 4), V_FLOATS = FT * D;          // a warp's tile of keys, of values
+  static constexpr int SMEM = (FG * D + WARPS * (K_FLOATS + V_FLOATS + FG * FT + FG * (D + 2))) * 4;
+};
+
+// grid (parts, KV heads x runs of FG query heads, rows); a cluster is the parts of a row. A round takes parts x WARPS tiles in
+// a row, tile j to warp j / parts of part j % parts, so that few tiles spread over the SMs.
+template <int D>
+__global__ void __launch_bounds__(FRows<D>::WARPS * 32)
+f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* __restrict__ row_request) {
+  constexpr int DL = D / 32;             // values a lane
+  constexpr int FW = FRows<D>::WARPS, KS = D + 4, REC = D + 2;
+  extern __shared__ __align__(16) float f32_smem[];
+  float* sq = f32_smem;                                  // [FG][D]
+  float* sk_all = sq + FG * D;                           // [FW][FT][KS]
+  float* sv_all = sk_all + FW * FRows<D>::K_FLOATS;      // [FW][FT][D]
+  float* sp_all = sv_all + FW * FRows<D>::V_FLOATS;      // [FW][FG][FT]
+  float* records = sp_all + FW * FG * FT;                // [FW][FG][REC]: a tile's weighted sum, largest score, sum
+  cg::cluster_group cluster = cg::this_cluster();
+  const int part = blockIdx.x, n_parts = gridDim.x, row = blockIdx.z;
+  const int group = at.n_heads / at.n_kv_heads, runs = (group + FG - 1) / FG;
+  const int kvh = blockIdx.y / runs, g0 = (blockIdx.y % runs) * FG, heads = min(FG, group - g0), head0 = kvh * group + g0;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pos = positions[row], lo = first_key(at, pos), kept = lo > 0 ? min(at.keep_first, lo) : 0;
+  const int* table = at.table + static_cast<size_t>(ck_request(row_request[row])) * at.max_blocks;
+  const int d4 = at.head_dim >> 2, e4 = at.vdim >> 2;
+  float* sk = sk_all + warp * FRows<D>::K_FLOATS;
+  float* sv = sv_all + warp * FRows<D>::V_FLOATS;
+  float* sp = sp_all + warp * FG * FT;
+
+  const int step = n_parts * FW * FT;
+  auto tile_of = [&](int base) { return base + (warp * n_parts + part) * FT; };
+  auto in_tile = [&](int t0) { return t0 <= pos && (t0 + FT > lo || t0 < kept); };
+  auto seen = [&](int t) { return t <= pos && (t >= lo || t < kept); };
+  auto next_base = [&](int base) {                       // (the same for every block of the cluster)
+    for (base += step; base <= pos && base + step <= lo && base >= kept; base += step) {}
+    return base;
+  };
+  // the warp's tile of keys or values, 16 bytes a lane and trip; zeros for a key that the row does not see
+  auto fetch = [&](float* dst, int stride, const float* cache, long long cache_row, int size, int per, int t0) {
+    if (in_tile(t0)) {
+      int slot[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t0 + lane + 32 * h;
+        slot[h] = seen(t) ? ck_page(table, t / at.page_size, at.max_blocks) * at.page_size + t % at.page_size : -1;
+      }
+      for (int e0 = 0; e0 < FT * per; e0 += 32) {        // (FT * per is a multiple of 32)
+        const int e = e0 + lane, r = e / per, c = (e - r * per) * 4;
+        const int a = __shfl_sync(0xffffffffu, slot[0], r & 31), b = __shfl_sync(0xffffffffu, slot[1], r & 31);
+        const int place = r < 32 ? a : b;
+        cp_async16_f32(dst + r * stride + c, cache + (place < 0 ? 0 : place * cache_row + static_cast<size_t>(kvh) * size + c), place < 0 ? 0 : 16);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  int base = kept > 0 ? 0 : lo / FT * FT;
+  fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, tile_of(base));
+  fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, tile_of(base));
+  for (int e = tid; e < FG * D; e += FW * 32) {
+    const int g = e / D, d = e % D;
+    sq[e] = g < heads && d < at.head_dim ? at.q[static_cast<size_t>(row) * at.q_stride + static_cast<size_t>(head0 + g) * at.head_dim + d] : 0.0f;
+  }
+  __syncthreads();
+  // the thread's outputs in the merge: numbers e of [heads][vdim], dealt over the cluster's threads
+  constexpr int MOST = FG * D / (FW * 32);
+  float m_run[MOST], l_run[MOST], o[MOST];
+#pragma unroll
+  for (int i = 0; i < MOST; ++i) m_run[i] = -INFINITY, l_run[i] = 0.0f, o[i] = 0.0f;
+
+  while (base <= pos) {
+    const int t0 = tile_of(base), next = next_base(base);
+    float m_t[FG], l_t[FG], acc[FG][DL];
+#pragma unroll
+    for (int g = 0; g < FG; ++g) {
+      m_t[g] = -INFINITY, l_t[g] = 0.0f;
+#pragma unroll
+      for (int j = 0; j < DL; ++j) acc[g][j] = 0.0f;
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    if (in_tile(t0)) {
+      float s[2][FG];
+#pragma unroll
+      for (int g = 0; g < FG; ++g) s[0][g] = s[1][g] = 0.0f;
+#pragma unroll 4
+      for (int c = 0; c < d4; ++c) {
+        const float4 k0 = *reinterpret_cast<const float4*>(sk + lane * KS + c * 4);
+        const float4 k1 = *reinterpret_cast<const float4*>(sk + (lane + 32) * KS + c * 4);
+#pragma unroll
+        for (int g = 0; g < FG; ++g) {
+          const float4 a = *reinterpret_cast<const float4*>(sq + g * D + c * 4);
+          s[0][g] = fmaf(a.x, k0.x, s[0][g]);
+          s[0][g] = fmaf(a.y, k0.y, s[0][g]);
+          s[0][g] = fmaf(a.z, k0.z, s[0][g]);
+          s[0][g] = fmaf(a.w, k0.w, s[0][g]);
+          s[1][g] = fmaf(a.x, k1.x, s[1][g]);
+          s[1][g] = fmaf(a.y, k1.y, s[1][g]);
+          s[1][g] = fmaf(a.z, k1.z, s[1][g]);
+          s[1][g] = fmaf(a.w, k1.w, s[1][g]);
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < FG; ++g) {
+        if (g >= heads) break;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int t = t0 + lane + 32 * h;
+          s[h][g] = seen(t) ? biased(at, __fmul_rn(s[h][g], at.scale), head0 + g, pos - t) : -INFINITY;
+        }
+        m_t[g] = warp_max(fmaxf(s[0][g], s[1][g]));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) sp[g * FT + lane + 32 * h] = s[h][g] == -INFINITY ? 0.0f : expf(s[h][g] - m_t[g]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int g = 0; g < FG; ++g) {
+        if (g >= heads) break;
+        const int x = lane & 15;
+        float l = sp[g * FT + x];
+#pragma unroll
+        for (int j = 1; j < 4; ++j) l += sp[g * FT + x + 16 * j];
+#pragma unroll
+        for (int w = 8; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
+        l_t[g] = l;
+      }
+    }
+    __syncwarp();                                          // the keys have been read
+    fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, next <= pos ? tile_of(next) : pos + 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    if (in_tile(t0)) {
+#pragma unroll 8
+      for (int k = 0; k < FT; ++k) {
+        float v[DL];
+#pragma unroll
+        for (int j = 0; j < DL; ++j) v[j] = sv[k * D + lane * DL + j];
+#pragma unroll
+        for (int g = 0; g < FG; ++g) {
+          const float p = g < heads ? sp[g * FT + k] : 0.0f;
+#pragma unroll
+          for (int j = 0; j < DL; ++j) acc[g][j] = p != 0.0f ? fmaf(p, v[j], acc[g][j]) : acc[g][j];
+        }
+      }
+    }
+    __syncwarp();                                          // the values have been read
+    fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, next <= pos ? tile_of(next) : pos + 1);
+    float* mine = records + warp * FG * REC;
+#pragma unroll
+    for (int g = 0; g < FG; ++g) {
+#pragma unroll
+      for (int j = 0; j < DL; ++j) mine[g * REC + lane * DL + j] = acc[g][j];
+      if (lane == 0) mine[g * REC + D] = m_t[g], mine[g * REC + D + 1] = l_t[g];
+    }
+    if (n_parts > 1) cluster.sync();
+    else __syncthreads();
+    const int tiles = min(n_parts * FW, (pos - base) / FT + 1);
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) {
+      const int e = (i * n_parts + part) * FW * 32 + tid, g = e / at.vdim, d = e - g * at.vdim;
+      if (g >= heads) break;
+      for (int j0 = 0; j0 < tiles; j0 += 4) {              // four tiles' numbers at a time: none waits for another
+        float m[4], l[4], a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int j = min(j0 + k, tiles - 1), b = j % n_parts;
+          const float* pt = (n_parts > 1 ? cluster.map_shared_rank(records, b) : records) + (j / n_parts * FG + g) * REC;
+          m[k] = j0 + k < tiles ? pt[D] : -INFINITY, l[k] = pt[D + 1], a[k] = pt[d];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (m[k] == -INFINITY) continue;
+          float c_run, c_tile;
+          merge_factors(m_run[i], m[k], c_run, c_tile);
+          l_run[i] = two_products(l_run[i], c_run, l[k], c_tile);
+          o[i] = two_products(o[i], c_run, a[k], c_tile);
+        }
+      }
+    }
+    if (n_parts > 1) cluster.sync();
+    else __syncthreads();
+    base = next;
+  }
+#pragma unroll
+  for (int i = 0; i < MOST; ++i) {
+    const int e = (i * n_parts + part) * FW * 32 + tid, g = e / at.vdim, d = e - g * at.vdim;
+    if (g >= heads) break;
+    if (at.sink) {
+      float c_run, c_tile;
+      merge_factors(m_run[i], 0.0f, c_run, c_tile);
+      l_run[i] = two_products(l_run[i], c_run, 1.0f, c_tile);
+      o[i] *= c_run;
+    }
+    at.out[static_cast<size_t>(row) * at.out_stride + static_cast<size_t>(head0 + g) * at.vdim + d] = o[i] / l_run[i];
+  }
+}
+
+template <int D>
+int launch_f32_tiles(const F32Attention& at, const int4* tiles, int n_tiles, cudaStream_t stream) {
+  constexpr int SMEM = (2 * FT * (D + 4) + FT * D + FT * (FT + 4)) * 4;
+  const cudaError_t e = cudaFuncSetAttribute(f32_tiles_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  f32_tiles_kernel<D><<<dim3(2 * n_tiles, at.n_heads), 256, SMEM, stream>>>(at, tiles);
+  return launch_status();
+}
+
+template <int D>
+int launch_f32_rows(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts,
+                    cudaStream_t stream) {
+  const int group = at.n_heads / at.n_kv_heads;
+  const cudaError_t e = cudaFuncSetAttribute(f32_rows_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRows<D>::SMEM);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(parts, at.n_kv_heads * ((group + FG - 1) / FG), rows);
+  cfg.blockDim = FRows<D>::WARPS * 32;
+  cfg.dynamicSmemBytes = FRows<D>::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, f32_rows_kernel<D>, at, positions, row_request));
+}
+
+inline bool f32_sizes(const F32Attention& a) {
+  return a.head_dim > 0 && a.vdim > 0 && a.head_dim <= 128 && a.vdim <= 128 && a.head_dim % 4 == 0 && a.vdim % 4 == 0 &&
+         a.k_row % 4 == 0 && a.v_row % 4 == 0 && a.q_stride % 4 == 0 && a.n_kv_heads > 0 && a.n_heads % a.n_kv_heads == 0 &&
+         a.page_size > 0 && a.n_heads <= 65535 && a.keep_first >= 0 && (a.rate != nullptr) == (a.dstep != nullptr) && a.chunk >= 0 &&
+         !(a.chunk > 0 && (a.window > 0 || a.keep_first > 0)) &&
+         ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & 15) == 0;
+}
+
+}  // namespace dl
+
+// Arguments as dl_paged_attention_generic_masked's, all float32. tiles: int4 [n_tiles] of (request slot, first row, rows up
+// to 128, first position).
+DL_EXPORT int dl_attention_f32_tiles(const void* q, int q_stride, const void* k_cache, long long k_row, const void* v_cache,
+                                     long long v_row, const int* block_table, int max_blocks, const int* tiles, int n_tiles,
+                                     void* out, int out_stride, int n_heads, int n_kv_heads, int head_dim, int vdim,
+                                     int page_size, float scale, int window, int keep_first, int sink, const float* rate,
+                                     const float* dstep, int chunk, cudaStream_t stream) {
+  if (n_tiles <= 0) return 0;
+  const dl::F32Attention at = {static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
+                               static_cast<float*>(out), block_table, rate, dstep, k_row, v_row, q_stride, out_stride, max_blocks,
+                               n_heads, n_kv_heads, head_dim, vdim, page_size, window, keep_first, sink, chunk, scale};
+  if (!dl::f32_sizes(at) || (reinterpret_cast<uintptr_t>(tiles) & 15) != 0) return DL_ERR_UNSUPPORTED;
+  const int4* list = reinterpret_cast<const int4*>(tiles);
+  const int most = head_dim > vdim ? head_dim : vdim;
+  if (most <= 32) return dl::launch_f32_tiles<32>(at, list, n_tiles, stream);
+  if (most <= 64) return dl::launch_f32_tiles<64>(at, list, n_tiles, stream);
+  return dl::launch_f32_tiles<128>(at, list, n_tiles, stream);
+}
+
+// Rows 0 .. rows - 1, each the newest token of its request; `parts` (1, 2, 4 or 8): blocks over a row's keys.
+DL_EXPORT int dl_attention_f32_rows(const void* q, int q_stride, const void* k_cache, long long k_row, const void* v_cache,
+                                    long long v_row, const int* block_table, int max_blocks, const int* positions,
+                                    const int* row_request, int rows, int parts, void* out, int out_stride, int n_heads,
+                                    int n_kv_heads, int head_dim, int vdim, int page_size, float scale, int window,
+                                    int keep_first, int sink, const float* rate, const float* dstep, int chunk,
+                                    cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  const dl::F32Attention at = {static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
+                               static_cast<float*>(out), block_table, rate, dstep, k_row, v_row, q_stride, out_stride, max_blocks,
+                               n_heads, n_kv_heads, head_dim, vdim, page_size, window, keep_first, sink, chunk, scale};
+  if (!dl::f32_sizes(at) || rows > 65535 || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return DL_ERR_UNSUPPORTED;
+  const int most = head_dim > vdim ? head_dim : vdim;
+  if (most <= 32) return dl::launch_f32_rows<32>(at, positions, row_request, rows, parts, stream);
+  if (most <= 64) return dl::launch_f32_rows<64>(at, positions, row_request, rows, parts, stream);
+  return dl::launch_f32_rows<128>(at, positions, row_request, rows, parts, stream);
+}

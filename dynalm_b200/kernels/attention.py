@@ -1,7 +1,7 @@
 """Chooses the attention kernel for a step.
 
-float32 always runs the plain kernel (csrc/attention_generic.cu), whose arithmetic for a row is
-fixed by the row alone. bfloat16 steps in which every request brings one token run the split-KV
+float32 runs the 32-bit kernels (csrc/attention_f32.cu; the plain kernel, csrc/attention_generic.cu, for sizes they do not
+take), whose arithmetic for a row is fixed by the row alone. bfloat16 steps in which every request brings one token run the split-KV
 kernel (csrc/attention_decode.cu); other bfloat16 steps (prompt portions, alone or beside decode
 rows) run a flash kernel: the tcgen05 one (csrc/attention_prefill_tcgen05.cu) for head sizes 64 and
 128 with pages of at least 16 keys, else the mma.sync one (csrc/attention_prefill.cu). Every shape
@@ -338,9 +338,50 @@ def _decode_rows(qkv: torch.Tensor, cache, ctx, out: torch.Tensor, spec, runtime
                                tensor_cores=decode_uses_tensor_cores(spec) and qkv.stride(0) % 8 == 0)
 
 
+# Steps of up to this many rows run row by row: a query tile of the other kernel then has mostly empty rows. A layer of 32:8
+# heads of 64 on B200, the plain kernel / these: a prompt of 700 tokens in tiles 1,410 / 146 us; four single tokens of 500
+# keys 94 / 15 us.
+F32_ROWS = 64
+
+
+def f32_parts(rows: int, n_heads: int, n_kv_heads: int, sms: int = 0) -> int:
+    """Blocks over a row's keys: as many (a power of two up to a cluster's 8) as keep the grid within a block an SM (one fits)."""
+    blocks = max(1, rows) * n_kv_heads * -(-(n_heads // n_kv_heads) // 4)
+    parts = 8
+    while parts > 1 and blocks * parts > (sms or sm_count()):
+        parts //= 2
+    return parts
+
+
+def attention_f32(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: torch.Tensor, v_row: int, cache, ctx,
+                  out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, vdim: int, scale: float, window: int = 0,
+                  keep_first: int = 0, sink: bool = False, rate=None, step=None, chunk: int = 0) -> bool:
+    """The 32-bit kernels on a step, False where they do not take it: single tokens (and any step of few rows) row by row,
+    prompt portions in query tiles."""
+    rows = q.shape[0]
+    if not ops.attention_f32_takes(q, k_cache, k_row, v_cache, v_row, head_dim, vdim):
+        return False
+    single, n_tiles, tiles = rows, 0, None
+    if rows > F32_ROWS and not ctx.decode_only:
+        if query_tiles(ctx) is None:
+            return False
+        tiles, _, n_tiles, single = query_tiles(ctx)
+    args = (n_heads, n_kv_heads, head_dim, vdim, cache.page_size, scale, window, keep_first, sink, rate, step, chunk)
+    if single > 0:
+        ops.attention_f32_rows(q, k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions, ctx.row_slot, single,
+                               f32_parts(single, n_heads, n_kv_heads), out, *args)
+    if n_tiles > 0:
+        ops.attention_f32_tiles(q, k_cache, k_row, v_cache, v_row, cache.block_table, tiles, n_tiles, out, *args)
+    return True
+
+
 def paged_attention(qkv: torch.Tensor, cache, ctx, out: torch.Tensor, spec, runtime) -> bool:
     """Run the fast kernel(s) for this step if they apply; False means the caller runs the plain one."""
     k_cache, v_cache = cache.arrays
+    if qkv.dtype == torch.float32:
+        kv_row = spec.num_kv_heads * spec.head_dim
+        return attention_f32(qkv, k_cache, kv_row, v_cache, kv_row, cache, ctx, out, spec.num_heads, spec.num_kv_heads,
+                             spec.head_dim, spec.head_dim, float(spec.scale), spec.get("window", 0))
     if use_decode_kernel(ctx, spec, qkv.dtype, cache.page_size):
         _decode_rows(qkv, cache, ctx, out, spec, runtime, qkv.shape[0])
         return True

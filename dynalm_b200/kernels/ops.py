@@ -140,6 +140,10 @@ _SIGNATURES = {
         "dl_gemm_tcgen05_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _P, _F, _I, _I, _I, _I, _P, _I, _P]},
     "gemm_stream_tcgen05": {
         "dl_gemm_stream": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _P, _P]},
+    "attention_f32": {
+        "dl_attention_f32_tiles": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _P],
+        "dl_attention_f32_rows": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
+                                  _I, _P]},
     "gemm_simt": {"dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P]},
     "sampling": {
         "dl_argmax": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
@@ -1877,6 +1881,57 @@ def paged_attention_generic_kv(q: torch.Tensor, k_cache: torch.Tensor, k_row: in
         block_table.stride(0), _p(positions), _p(row_request), _p(out), out.stride(0), q.shape[0], n_heads, n_kv_heads,
         head_dim, vdim, page_size, scale, window, int(keep_first), 1 if sink else 0, _p(rate), _p(step), int(chunk), _stream()),
            "paged_attention_generic_kv")
+
+
+ATTENTION_F32_MAX = 128      # most numbers of a key or value
+
+
+def attention_f32_takes(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: torch.Tensor, v_row: int, head_dim: int,
+                        vdim: int) -> bool:
+    """Whether the 32-bit attention kernels of csrc/attention_f32.cu take these sizes: whole runs of 16 bytes everywhere."""
+    return (q.dtype == torch.float32 and 0 < head_dim <= ATTENTION_F32_MAX and 0 < vdim <= ATTENTION_F32_MAX
+            and head_dim % 4 == 0 and vdim % 4 == 0 and k_row % 4 == 0 and v_row % 4 == 0 and q.stride(0) % 4 == 0
+            and q.data_ptr() % 16 == 0 and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0)
+
+
+def _attention_f32_args(q, k_cache, v_cache, block_table, out, n_heads, n_kv_heads, rate, step):
+    _cuda(q, k_cache, v_cache, block_table, out, rate, step)
+    _distance_bias(rate, step, n_heads)
+    _rows_contiguous(q, "q")
+    _rows_contiguous(out, "out")
+    if n_heads % n_kv_heads:
+        raise Unsupported(f"attention: {n_heads} heads do not divide into {n_kv_heads} KV heads")
+    if not q.dtype == out.dtype == k_cache.dtype == v_cache.dtype == torch.float32:
+        raise InvalidArgument("attention_f32: q, out and the cache are float32")
+    check_limits("attention_f32", pages=k_cache.shape[0], requests=block_table.shape[0], rows=q.shape[0])
+
+
+def attention_f32_tiles(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: torch.Tensor, v_row: int,
+                        block_table: torch.Tensor, q_tiles: torch.Tensor, n_tiles: int, out: torch.Tensor, n_heads: int,
+                        n_kv_heads: int, head_dim: int, vdim: int, page_size: int, scale: float, window: int = 0,
+                        keep_first: int = 0, sink: bool = False, rate: Optional[torch.Tensor] = None,
+                        step: Optional[torch.Tensor] = None, chunk: int = 0) -> None:
+    """paged_attention_generic_kv for the rows of the first n_tiles of the step's query tiles (float32)."""
+    _attention_f32_args(q, k_cache, v_cache, block_table, out, n_heads, n_kv_heads, rate, step)
+    _check(_fn("attention_f32", "dl_attention_f32_tiles")(
+        _p(q), q.stride(0), _p(k_cache), k_row, _p(v_cache), v_row, _p(block_table), block_table.stride(0), _p(q_tiles), n_tiles,
+        _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, vdim, page_size, scale, window, int(keep_first), 1 if sink else 0,
+        _p(rate), _p(step), int(chunk), _stream()), "attention_f32_tiles")
+
+
+def attention_f32_rows(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: torch.Tensor, v_row: int,
+                       block_table: torch.Tensor, positions: torch.Tensor, row_request: torch.Tensor, rows: int, parts: int,
+                       out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, vdim: int, page_size: int, scale: float,
+                       window: int = 0, keep_first: int = 0, sink: bool = False, rate: Optional[torch.Tensor] = None,
+                       step: Optional[torch.Tensor] = None, chunk: int = 0) -> None:
+    """The same for the first `rows` rows of the step one by one, each row's keys over `parts` (1, 2, 4 or 8) blocks; the
+    result's bits do not depend on `parts`."""
+    _attention_f32_args(q, k_cache, v_cache, block_table, out, n_heads, n_kv_heads, rate, step)
+    _cuda(positions, row_request)
+    _check(_fn("attention_f32", "dl_attention_f32_rows")(
+        _p(q), q.stride(0), _p(k_cache), k_row, _p(v_cache), v_row, _p(block_table), block_table.stride(0), _p(positions),
+        _p(row_request), rows, parts, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, vdim, page_size, scale, window,
+        int(keep_first), 1 if sink else 0, _p(rate), _p(step), int(chunk), _stream()), "attention_f32_rows")
 
 
 def gelu_mul(gate_up: torch.Tensor, out: torch.Tensor) -> None:

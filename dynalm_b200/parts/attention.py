@@ -461,6 +461,12 @@ class GatedNormedAttention(PagedAttention):
             if fast.paged_attention(qkv, cache, ctx, out, s, self.rt):
                 return False
         k_cache, k_row, v_cache, v_row = self._kv(cache)
+        if not (self.same and self.plain_mask) and qkv.dtype == torch.float32:
+            from ..kernels import attention as fast
+            if fast.attention_f32(qkv, k_cache, k_row, v_cache, v_row, cache, ctx, out, s.num_heads, s.num_kv_heads, s.head_dim,
+                                  s.value_dim, float(s.scale), self.window, self.keep_first, self.sink, self.rate, self.dstep,
+                                  self.chunk):
+                return False
         ops.paged_attention_generic_kv(qkv, k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions, ctx.row_slot,
                                        out, s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, cache.page_size,
                                        float(s.scale), self.window, self.keep_first, self.sink, rate=self.rate, step=self.dstep,

@@ -223,6 +223,55 @@ def test_paged_attention_generic(ops, dtype, heads, kvh, hd, page, window):
         assert err <= tol(dtype, 2), f"row {i} (request {r}, position {p}): {err}"
 
 
+@pytest.mark.parametrize("heads,kvh,d,e,window,keep,sink,bias,chunk", [
+    (4, 2, 16, 16, 0, 0, False, False, 0), (6, 1, 48, 20, 0, 0, True, False, 0), (8, 2, 64, 64, 100, 0, False, True, 0),
+    (5, 5, 128, 128, 64, 70, True, False, 0), (8, 1, 64, 128, 33, 3, False, False, 0), (4, 4, 36, 100, 0, 0, True, True, 96)])
+def test_attention_f32(ops, heads, kvh, d, e, window, keep, sink, bias, chunk):
+    """The 32-bit kernels against the plain one under every mask: three requests in scattered pages of 16 (slots nobody wrote
+    hold infinities), tiles that start and end anywhere; a row's bits are the same from tiles, alone, and with its keys over
+    1, 2, 4 or 8 blocks. Bound: two sums of the same terms in other orders, weights that add up to one."""
+    g = torch.Generator(device="cpu").manual_seed(61)
+    lens, page = [60, 1300, 131], 16
+    blocks = [-(-n // page) for n in lens]
+    perm = torch.randperm(sum(blocks), generator=g)
+    table = torch.zeros(3, max(blocks), dtype=torch.int32)
+    kc = torch.full((sum(blocks), page, kvh * (d + e)), float("inf"))
+    at = 0
+    for r, n in enumerate(lens):
+        kv = torch.randn(n, kvh * (d + e), generator=g)
+        kv[3, :kvh * d] *= 4.0
+        for b in range(blocks[r]):
+            table[r, b] = perm[at]
+            m = min(page, n - b * page)
+            kc[perm[at], :m] = kv[b * page:b * page + m]
+            at += 1
+    tiles = [(1, 5, 128, 1300 - 205), (1, 133, 77, 1300 - 77), (2, 210, 31, 100), (0, 241, 1, 0), (1, 242, 70, 0)]
+    rows = [(0, 59), (1, 700), (2, 0), (2, 130), (1, 63)] + [(slot, p0 + i) for slot, _, n, p0 in tiles for i in range(n)]
+    req = torch.tensor([r for r, _ in rows], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p for _, p in rows], dtype=torch.int32, device=DEV)
+    n = len(rows)
+    q = torch.randn(n, heads * d, generator=g).to(DEV)
+    kc, table = kc.to(DEV), table.to(DEV)
+    vc = kc.view(-1)[kvh * d:]
+    rate, step = ((torch.rand(heads, generator=g) + 0.5).to(DEV), (torch.rand(heads, generator=g) * 0.2).to(DEV)) if bias else (None, None)
+    row = kvh * (d + e)
+    args = (heads, kvh, d, e, page, d ** -0.5, window, keep, sink, rate, step, chunk)
+    ref = torch.empty(n, heads * e, device=DEV)
+    ops.paged_attention_generic_kv(q, kc, row, vc, row, table, pos, req, ref, *args)
+    assert torch.isfinite(ref).all()
+    alone = []
+    for parts in (1, 2, 4, 8):
+        out = torch.full((n, heads * e), 7.0, device=DEV)
+        ops.attention_f32_rows(q, kc, row, vc, row, table, pos, req, n, parts, out, *args)
+        alone.append(out)
+    assert (alone[0] - ref).abs().max() <= 4e-5
+    for out in alone[1:]:
+        assert torch.equal(out, alone[0])
+    out = torch.full((n, heads * e), 7.0, device=DEV)
+    ops.attention_f32_tiles(q, kc, row, vc, row, table, torch.tensor(tiles, dtype=torch.int32, device=DEV).view(-1), len(tiles), out, *args)
+    assert torch.equal(out[5:], alone[0][5:]) and (out[:5] == 7.0).all()
+
+
 def test_argmax_ties_and_sizes(ops):
     g = torch.Generator(device="cpu").manual_seed(7)
     # 50,001: rows that do not start on 16 bytes and a last slice that is no multiple of 4 (the scan's scalar ends)
