@@ -4,7 +4,7 @@ float32 always runs the plain kernel (csrc/attention_diff.cu), whose arithmetic 
 bfloat16 with map and value sizes that are multiples of 16 up to 128 runs the tensor-core kernels
 (csrc/attention_diff_flash.cu): the rows at the head of a step that bring a single token each go through the
 split-KV kernel, prompt portions through the flash kernel, cut into the step's query tiles
-(kernels/attention.QueryTilePlan). Every other shape runs the plain kernel.
+(kernels/attention.QueryTilePlan); at the sizes of ops.DIFF_TCGEN05_SIZES through the tcgen05 flash kernel. Every other shape runs the plain kernel.
 """
 
 from __future__ import annotations
@@ -83,7 +83,15 @@ def attend(q: torch.Tensor, cache, ctx, out: torch.Tensor, spec, lam: torch.Tens
     if leading > 0:
         _single(q, records, k_off, cache, ctx, out, spec, lam, out_scale, eps, runtime, leading)
         n_tiles = n_prompt_tiles
-    if n_tiles > 0:
+    if n_tiles > 0 and (spec.head_dim, spec.value_dim) in ops.DIFF_TCGEN05_SIZES and cache.page_size >= 16 and \
+            q.data_ptr() % 16 == 0 and float(spec.scale) > 0:
+        # a layer of 2,048 rows, 16:4 heads of 2 x 64 with values of 128: 88 us, both maps of a head in one block of the
+        # mma.sync kernel 137
+        maps = runtime.buffer("diff_maps", (q.shape[0], spec.num_heads * 2 * spec.value_dim), torch.float32)
+        ops.diff_attention_tcgen05(q, records, 0, k_off, cache.block_table, q_tiles, n_tiles, out, spec.num_heads,
+                                   spec.num_kv_heads, spec.head_dim, spec.value_dim, cache.page_size, float(spec.scale),
+                                   float(spec.get("softcap", 0.0)), lam, out_scale, eps, maps)
+    elif n_tiles > 0:
         ops.diff_attention_prefill(q, records, 0, k_off, cache.block_table, q_tiles, n_tiles, out, spec.num_heads,
                                    spec.num_kv_heads, spec.head_dim, spec.value_dim, cache.page_size, float(spec.scale),
                                    float(spec.get("softcap", 0.0)), lam, out_scale, eps)

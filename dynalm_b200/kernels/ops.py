@@ -127,8 +127,12 @@ _SIGNATURES = {
     "attention_prefill": {
         "dl_paged_attention_prefill": [_P, _I, _P, _P, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _P]},
     "attention_prefill_tcgen05": {
-        "dl_paged_attention_prefill_tcgen05": [_P, _I, _I, _P, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P,
-                                               _P, _P, _I, _P]},
+        "dl_paged_attention_prefill_tcgen05": [_P, _I, _I, _P, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
+                                               _P, _P, _I, _P],
+        "dl_latent_gather": [_P, _I, _P, _I, _I, _P, _I, _P, _P],
+        "dl_latent_attention_tcgen05": [_P, _I, _P, _I, _P, _I, _I, _P, _I, _P, _P, _I, _P, _I, _I, _F, _I, _P, _P, _P],
+        "dl_diff_attention_tcgen05": [_P, _I, _I, _P, _L, _I, _I, _I, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _F, _F,
+                                      _P, _P, _P]},
     "gemm_skinny": {
         "dl_gemm_skinny": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _L, _P, _P],
         "dl_gemm_skinny_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _F, _I, _I, _I, _I, _P]},
@@ -898,6 +902,47 @@ def latent_attention_flash(qw: torch.Tensor, cache: torch.Tensor, block_table: t
         LAUNCHES += 1
 
 
+def latent_gather(records: torch.Tensor, block_table: torch.Tensor, page_size: int, pieces: torch.Tensor, n_pieces: int,
+                  out: torch.Tensor) -> None:
+    """The records of pieces of up to 16 keys, int32 [n_pieces, 4] = (request slot, first key, keys, -), to rows 16 i .. of `out`
+    (zeros past a piece's keys); bfloat16."""
+    _cuda(records, block_table, pieces, out)
+    record = records.shape[-1]
+    if records.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or not records.is_contiguous() or not out.is_contiguous() \
+            or out.shape[-1] != record or out.shape[0] < 16 * n_pieces or pieces.dtype != torch.int32 or pieces.numel() < 4 * n_pieces:
+        raise InvalidArgument("latent_gather: bfloat16 records [pages, page_size, record], out [16 * pieces, record], pieces int32")
+    check_limits("attention_prefill_tcgen05", pages=records.shape[0], requests=block_table.shape[0], rows=0)
+    _check(_fn("attention_prefill_tcgen05", "dl_latent_gather")(
+        _p(records), record, _p(block_table), block_table.stride(0), page_size, _p(pieces), n_pieces, _p(out), _stream()),
+        "latent_gather")
+
+
+def latent_attention_tcgen05(q: torch.Tensor, q_rot: torch.Tensor, latents: torch.Tensor, k2_off: int, kv: torch.Tensor,
+                             bases: torch.Tensor, tiles: torch.Tensor, n_tiles: int, out: torch.Tensor, heads: int, scale: float,
+                             window: int, sink: Optional[torch.Tensor]) -> None:
+    """Latent attention of query tiles over expanded keys and values on tcgen05, heads of 128 + 64 and values of 128 numbers; see
+    csrc/attention_prefill_tcgen05.cu. q [rows, >= heads * 192] (own numbers of head h at h * 192), q_rot [rows, heads * 64],
+    latents [keys, row] (the shared turned piece at k2_off), kv [keys, heads * 256], bases int32 per request slot."""
+    _cuda(q, q_rot, latents, kv, bases, tiles, out, sink)
+    _rows_contiguous(q, "q")
+    _rows_contiguous(out, "out")
+    if any(t.dtype != torch.bfloat16 for t in (q, q_rot, latents, kv, out)):
+        raise Unsupported("latent_attention_tcgen05: bfloat16 only")
+    if q.shape[1] < heads * 192 or tuple(q_rot.shape) != (q.shape[0], heads * 64) or not q_rot.is_contiguous() or not kv.is_contiguous() \
+            or kv.shape[1] != heads * 256 or latents.shape[0] < kv.shape[0] or not latents.is_contiguous() \
+            or latents.shape[1] < k2_off + 64 or out.shape[1] < heads * 128 or out.shape[0] < q.shape[0]:
+        raise InvalidArgument("latent_attention_tcgen05: q [rows, heads * 192], q_rot [rows, heads * 64], kv [keys, heads * 256]")
+    if tiles.dtype != torch.int32 or tiles.numel() < 4 * n_tiles or bases.dtype != torch.int32:
+        raise InvalidArgument("latent_attention_tcgen05: tiles int32 [n_tiles, 4], bases int32")
+    if sink is not None and (sink.dtype != torch.float32 or sink.numel() != heads):
+        raise InvalidArgument("latent_attention_tcgen05: sinks float32 [heads]")
+    check_limits("attention_prefill_tcgen05", pages=0, requests=bases.numel(), rows=q.shape[0])
+    _check(_fn("attention_prefill_tcgen05", "dl_latent_attention_tcgen05")(
+        _p(q), q.stride(0), _p(q_rot), q.shape[0], _p(latents), latents.shape[1], k2_off, _p(kv), kv.shape[0], _p(bases), _p(tiles),
+        n_tiles, _p(out), out.stride(0), heads, scale, window, _p(sink), _p(_status_word(q.device)), _stream()),
+        "latent_attention_tcgen05")
+
+
 def qk_norm_cache_write(qkv: torch.Tensor, positions: torch.Tensor, row_slot: torch.Tensor,
                         block_table: Optional[torch.Tensor], cache: Optional[torch.Tensor], k_off: int, v_off: int,
                         q_weight: torch.Tensor, k_weight: Optional[torch.Tensor], eps: float, temp_coef: float,
@@ -993,6 +1038,32 @@ def diff_attention_prefill(q: torch.Tensor, cache: torch.Tensor, k_off: int, v_o
         _p(q), q.stride(0), _p(cache), cache.shape[2], k_off, v_off, _p(block_table), block_table.stride(0), _p(q_tiles),
         n_tiles, _p(out), out.stride(0), n_heads, n_kv_heads, dim, vdim, page_size, scale, softcap, _p(lam), out_scale, eps,
         _stream()), "diff_attention_prefill")
+
+
+DIFF_TCGEN05_SIZES = ((64, 64), (64, 128), (128, 128))     # (map, value) sizes of the tcgen05 kernel
+
+
+def diff_attention_tcgen05(q: torch.Tensor, cache: torch.Tensor, k_off: int, v_off: int, block_table: torch.Tensor,
+                           q_tiles: torch.Tensor, n_tiles: int, out: torch.Tensor, n_heads: int, n_kv_heads: int, dim: int,
+                           vdim: int, page_size: int, scale: float, softcap: float, lam: torch.Tensor, out_scale: float,
+                           eps: float, maps: torch.Tensor) -> None:
+    """diff_attention_prefill on tcgen05 tensor cores, the two maps of a head as heads of their own whose rows go to `maps`
+    (float32 [rows, heads, 2, vdim]) and are combined from there; see csrc/attention_prefill_tcgen05.cu. Sizes
+    DIFF_TCGEN05_SIZES, pages of at least 16 keys."""
+    _cuda(q, cache, block_table, q_tiles, out, lam, maps)
+    _diff_fast_checks(q, cache, out, block_table, lam, k_off, v_off, n_heads, n_kv_heads, dim, vdim, page_size,
+                      "diff attention (tcgen05)")
+    if (dim, vdim) not in DIFF_TCGEN05_SIZES or page_size < 16:
+        raise Unsupported(f"diff attention (tcgen05): maps of {dim}, values of {vdim}, pages of {page_size}")
+    if q_tiles.dtype != torch.int32 or q_tiles.numel() < 4 * n_tiles or q_tiles.data_ptr() % 16:
+        raise InvalidArgument("diff attention (tcgen05): q_tiles must be int32 [n_tiles, 4], 16-byte aligned")
+    if maps.dtype != torch.float32 or not maps.is_contiguous() or maps.numel() < q.shape[0] * n_heads * 2 * vdim:
+        raise InvalidArgument("diff attention (tcgen05): maps float32 [rows, heads, 2, vdim]")
+    check_limits("attention_prefill_tcgen05", pages=cache.shape[0], requests=block_table.shape[0], rows=q.shape[0])
+    _check(_fn("attention_prefill_tcgen05", "dl_diff_attention_tcgen05")(
+        _p(q), q.stride(0), q.shape[0], _p(cache), cache.shape[0] * page_size, cache.shape[2], k_off, v_off, _p(block_table),
+        block_table.stride(0), _p(q_tiles), n_tiles, _p(out), out.stride(0), n_heads, n_kv_heads, dim, vdim, page_size, scale,
+        softcap, _p(lam), out_scale, eps, _p(maps), _p(_status_word(q.device)), _stream()), "diff_attention_tcgen05")
 
 
 def diff_decode_scratch_floats(rows: int, n_heads: int, vdim: int, n_split: int) -> int:
@@ -1278,12 +1349,13 @@ def paged_attention_prefill_tcgen05(q: torch.Tensor, k_cache: torch.Tensor, v_ca
                                     q_tiles: torch.Tensor, n_tiles: int, out: torch.Tensor, n_heads: int, n_kv_heads: int,
                                     head_dim: int, page_size: int, scale: float, window: int = 0,
                                     unit_parts: Optional[torch.Tensor] = None, partial: Optional[torch.Tensor] = None,
-                                    counters: Optional[torch.Tensor] = None) -> None:
+                                    counters: Optional[torch.Tensor] = None, chunk: int = 0, sink: bool = False) -> None:
     """Flash attention of query tiles over the paged cache on tcgen05 tensor cores, bfloat16, head_dim 64 or
     128, pages of at least 16 keys; see csrc/attention_prefill_tcgen05.cu. Arguments as paged_attention_prefill.
 
     unit_parts: int32 [n_tiles], when the keys of some tiles are dealt over several entries of q_tiles (see
-    kernels/attention.QueryTileParts): part | parts << 8 | scratch slot << 16 per entry, 0 = whole. Then partial:
+    kernels/attention.QueryTileParts): part | parts << 8 | scratch slot << 16 per entry, 0 = whole. chunk, sink: as
+    masked_flash_attention's. Then partial:
     float32, (slots in use) * n_heads * (head_dim + 2) * 128 elements; counters: int32, (slots in use) * n_heads, zero."""
     _cuda(q, k_cache, v_cache, block_table, q_tiles, out, unit_parts, partial, counters)
     _rows_contiguous(q, "q")
@@ -1311,8 +1383,8 @@ def paged_attention_prefill_tcgen05(q: torch.Tensor, k_cache: torch.Tensor, v_ca
     check_limits("attention_prefill_tcgen05", pages=k_cache.shape[0], requests=block_table.shape[0], rows=q.shape[0])
     _check(_fn("attention_prefill_tcgen05", "dl_paged_attention_prefill_tcgen05")(
         _p(q), q.stride(0), q.shape[0], _p(k_cache), _p(v_cache), k_cache.shape[0], _p(block_table), block_table.stride(0),
-        _p(q_tiles), n_tiles, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, page_size, scale, window,
-        _p(_status_word(q.device)), _p(unit_parts), _p(partial), _p(counters), records, _stream()),
+        _p(q_tiles), n_tiles, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, page_size, scale, window, int(chunk),
+        1 if sink else 0, _p(_status_word(q.device)), _p(unit_parts), _p(partial), _p(counters), records, _stream()),
         "paged_attention_prefill_tcgen05")
 
 

@@ -319,12 +319,10 @@ class GatedNormedAttention(PagedAttention):
     def graph_key(self, ctx) -> tuple:
         if self.same and self.plain_mask:
             return super().graph_key(ctx) if self.rt.dtype == torch.bfloat16 else ()
-        return (("masked_flash_parts", self._decode_parts(ctx)),) if self.rt.dtype == torch.bfloat16 else ()
+        return (("masked_flash_parts", self._decode_parts(ctx, ctx.num_tokens)),) if self.rt.dtype == torch.bfloat16 else ()
 
-    def _decode_parts(self, ctx) -> int:
-        """Into how many parts a step of single tokens deals a row's keys (part of the launch shape, so of the graph key)."""
-        if not ctx.decode_only:
-            return 1
+    def _decode_parts(self, ctx, rows: int) -> int:
+        """Into how many parts the keys of `rows` single tokens are dealt (part of the launch shape, so of the graph key)."""
         s = self.spec
         span = ctx.max_kv_len
         if self.window > 0 or self.chunk > 0:
@@ -333,7 +331,7 @@ class GatedNormedAttention(PagedAttention):
         while bucket < span:
             bucket *= 2
         group = s.num_heads // s.num_kv_heads
-        return ops.masked_flash_parts(ctx.num_tokens, s.num_kv_heads if 1 < group <= 64 else s.num_heads, bucket)
+        return ops.masked_flash_parts(rows, s.num_kv_heads if 1 < group <= 64 else s.num_heads, bucket)
 
     def cache_spec(self) -> Optional[CacheSpec]:
         s = self.spec
@@ -437,24 +435,54 @@ class GatedNormedAttention(PagedAttention):
                 and fast.query_tiles(ctx) is not None and cache.page_size & (cache.page_size - 1) == 0
                 and qkv.stride(0) % 8 == 0 and self.kv_width % 8 == 0 and self.v_width % 8 == 0)
 
+    def _tcgen05_applies(self, qkv: torch.Tensor, cache, out: torch.Tensor, gate) -> bool:
+        """The tcgen05 prompt kernel knows a window, chunks and a sink, over keys and values of one size in two arrays. Measured
+        on B200, 700 rows of a prompt beside 8 single tokens, 16:4 heads of 128: all rows on the mma.sync kernel 72 us a layer;
+        the prompt here 21 us, beside it the single tokens there, their keys in parts, 20 us."""
+        from ..kernels import attention as fast
+        return (self.same and self.keep_first == 0 and self.rate is None and gate is None and float(self.spec.scale) > 0
+                and fast.use_prefill_tcgen05(self.spec, qkv, out, cache.page_size))
+
+    def _masked_flash(self, qkv: torch.Tensor, cache, ctx, out: torch.Tensor, tiles: torch.Tensor, n_tiles: int, single: bool,
+                      rows: int, gate: Optional[torch.Tensor]) -> None:
+        """The masked flash kernel on `tiles`; `single`: they are the single tokens of rows 0 .. rows - 1."""
+        s = self.spec
+        k_cache, k_row, v_cache, v_row = self._kv(cache)
+        parts = self._decode_parts(ctx, rows) if single else 1
+        partial = None
+        if parts > 1:
+            most = max(self.rt.max_requests, rows)
+            partial = self.rt.flat(f"masked_flash_parts_{s.num_heads}x{s.value_dim}",
+                                   ops.masked_flash_partial_floats(most, s.num_heads, s.value_dim, ops.MASKED_FLASH_MAX_PARTS))
+        ops.masked_flash_attention(qkv, k_cache, k_row, v_cache, v_row, cache.block_table, tiles, n_tiles, out,
+                                   s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, cache.page_size,
+                                   float(s.scale), self.window, self.keep_first, self.sink,
+                                   one_token_tiles=single, parts=parts, partial=partial, rate=self.rate, step=self.dstep,
+                                   gate=gate, chunk=self.chunk)
+
     def attend(self, qkv: torch.Tensor, cache, ctx, out: torch.Tensor, gate: Optional[torch.Tensor] = None) -> bool:
         """True when the output gate has been applied on the way out."""
         s = self.spec
         if not (self.same and self.plain_mask) and self._flash_applies(qkv, cache, ctx):
             from ..kernels import attention as fast
-            q_tiles, n_tiles, _, _ = fast.query_tiles(ctx)
-            k_cache, k_row, v_cache, v_row = self._kv(cache)
-            parts = self._decode_parts(ctx)
-            partial = None
-            if parts > 1:
-                most = max(self.rt.max_requests, qkv.shape[0])
-                partial = self.rt.flat(f"masked_flash_parts_{s.num_heads}x{s.value_dim}",
-                                       ops.masked_flash_partial_floats(most, s.num_heads, s.value_dim, ops.MASKED_FLASH_MAX_PARTS))
-            ops.masked_flash_attention(qkv, k_cache, k_row, v_cache, v_row, cache.block_table, q_tiles, n_tiles, out,
-                                       s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim, cache.page_size,
-                                       float(s.scale), self.window, self.keep_first, self.sink,
-                                       one_token_tiles=ctx.decode_only, parts=parts, partial=partial, rate=self.rate, step=self.dstep,
-                                       gate=gate, chunk=self.chunk)
+            q_tiles, n_tiles, n_prompt, lead = fast.query_tiles(ctx)
+            if self._tcgen05_applies(qkv, cache, out, gate) and n_prompt > 0:
+                # prompt portions on the tcgen05 kernel; beside it, on a second stream, the single tokens at the step's head
+                side = self.rt.side_stream if lead > 0 and fast.SIDE_BY_SIDE else None
+                if side is not None:
+                    ops.stream_fork(side)
+                    with ops.on_stream(side):
+                        self._masked_flash(qkv, cache, ctx, out, q_tiles[4 * n_prompt:], lead, True, lead, None)
+                elif lead > 0:
+                    self._masked_flash(qkv, cache, ctx, out, q_tiles[4 * n_prompt:], lead, True, lead, None)
+                k_cache, v_cache = cache.arrays
+                ops.paged_attention_prefill_tcgen05(qkv, k_cache, v_cache, cache.block_table, q_tiles, n_prompt, out, s.num_heads,
+                                                    s.num_kv_heads, s.head_dim, cache.page_size, float(s.scale), self.window,
+                                                    chunk=self.chunk, sink=self.sink)
+                if side is not None:
+                    ops.stream_join(side)
+                return False
+            self._masked_flash(qkv, cache, ctx, out, q_tiles, n_tiles, ctx.decode_only, ctx.num_tokens if ctx.decode_only else 0, gate)
             return gate is not None
         if self.same and self.plain_mask:
             from ..kernels import attention as fast

@@ -759,6 +759,82 @@ def test_paged_attention_prefill_tcgen05_keys_dealt_over_blocks(ops, heads, kvh,
         assert torch.equal(out[128 + 70:], ref_out[128 + 70:])                   # the whole tile among them: the same bits
 
 
+def _portions(g, width, page, lens, dtype):
+    """Requests' records on shuffled pages and query tiles over them: portions from the
+    middle of a page and of a key tile, of one row, of a whole tile."""
+    blocks = [-(-n // page) for n in lens]
+    perm = torch.randperm(sum(blocks), generator=g)
+    table = torch.zeros(len(lens), max(blocks), dtype=torch.int32)
+    cache = torch.zeros(sum(blocks), page, width, dtype=dtype)
+    at = 0
+    for r, n in enumerate(lens):
+        rec = torch.randn(n, width, generator=g).to(dtype)
+        for b in range(blocks[r]):
+            table[r, b] = perm[at]
+            m = min(page, n - b * page)
+            cache[perm[at], :m] = rec[b * page:b * page + m]
+            at += 1
+    tiles, row = [], 0
+    for slot, pos, n in [(1, lens[1] - 205, 128), (1, lens[1] - 77, 77), (2, 100, 31), (0, 0, 1), (1, 0, 128), (1, 128, 70), (2, 63, 2)]:
+        tiles.append((slot, row, n, pos))
+        row += n
+    req = torch.tensor([t[0] for t in tiles for _ in range(t[2])], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([t[3] + i for t in tiles for i in range(t[2])], dtype=torch.int32, device=DEV)
+    return cache.to(DEV), table.to(DEV), torch.tensor(tiles, dtype=torch.int32, device=DEV).view(-1), len(tiles), req, pos
+
+
+@pytest.mark.parametrize("heads,kvh,hd,page,window,chunk,sink", [(4, 2, 64, 16, 0, 0, True), (4, 1, 64, 32, 0, 100, True),
+                                                                 (2, 2, 128, 16, 0, 64, False), (4, 2, 128, 64, 77, 0, True),
+                                                                 (4, 4, 64, 16, 0, 1, True), (2, 1, 64, 16, 0, 333, False)])
+def test_paged_attention_prefill_tcgen05_chunks_and_sink(ops, heads, kvh, hd, page, window, chunk, sink):
+    """Against the plain 32-bit kernel on the same numbers. Weights and results are rounded to 8 bits of mantissa, 2^-9 of a
+    weighted mean of values each."""
+    g = torch.Generator(device="cpu").manual_seed(19)
+    cache, table, tiles, n_tiles, req, pos = _portions(g, kvh * hd, page, [60, 900, 131], torch.bfloat16)
+    kc = cache.view(-1, page, kvh, hd)
+    vc = torch.randn(kc.shape, generator=g).to(torch.bfloat16).to(DEV)
+    n = pos.numel()
+    q = torch.randn(n, heads * hd, generator=g).to(torch.bfloat16).to(DEV)
+    out = torch.empty(n, heads * hd, dtype=torch.bfloat16, device=DEV)
+    ops.paged_attention_prefill_tcgen05(q, kc, vc, table, tiles, n_tiles, out, heads, kvh, hd, page, hd ** -0.5, window,
+                                        chunk=chunk, sink=sink)
+    assert ops.gemm_tcgen05_status() == 0
+    ref = torch.empty(n, heads * hd, device=DEV)
+    ops.paged_attention_generic_kv(q.float(), kc.float(), kvh * hd, vc.float(), kvh * hd, table, pos, req, ref, heads, kvh, hd, hd,
+                                   page, hd ** -0.5, window, 0, sink, chunk=chunk)
+    largest = vc.abs().max().item()
+    assert (out.float() - ref).abs().max().item() <= 1.1 * 2 * 2 ** -9 * largest
+
+
+@pytest.mark.parametrize("heads,groups,dim,vdim,page,cap", [(4, 2, 64, 64, 16, 0.0), (6, 2, 64, 128, 32, 3.0), (2, 2, 128, 128, 16, 30.0),
+                                                            (3, 1, 64, 128, 16, 0.0)])
+def test_diff_attention_tcgen05(ops, heads, groups, dim, vdim, page, cap):
+    """Against the plain kernel in 32 bits on the same numbers. Each map is off by the rounding of its weights, 2^-9 of the
+    largest value; the norm behind their difference o turns an error e into at most (1 + |y|) e / rms(o)."""
+    g = torch.Generator(device="cpu").manual_seed(23)
+    kw, vw, lam, out_scale = groups * 2 * dim, groups * vdim, 0.37, 0.6
+    cache, table, tiles, n_tiles, req, pos = _portions(g, kw + vw, page, [60, 900, 131], torch.bfloat16)
+    n = pos.numel()
+    q = torch.randn(n, heads * 2 * dim, generator=g).to(torch.bfloat16).to(DEV)
+    out = torch.empty(n, heads * vdim, dtype=torch.bfloat16, device=DEV)
+    lam_t = torch.tensor([lam], device=DEV)
+    maps = torch.empty(n, heads * 2 * vdim, device=DEV)
+    ops.diff_attention_tcgen05(q, cache, 0, kw, table, tiles, n_tiles, out, heads, groups, dim, vdim, page, dim ** -0.5, cap, lam_t,
+                               out_scale, 1e-5, maps)
+    assert ops.gemm_tcgen05_status() == 0
+    ref, o = torch.empty(n, heads * vdim, device=DEV), torch.empty(n, heads * vdim, device=DEV)
+    args = (table, pos, req)
+    sizes = (heads, groups, dim, vdim, page, dim ** -0.5, cap, lam_t)
+    ops.diff_attention(q.float(), cache.float(), 0, kw, *args, ref, *sizes, out_scale, 1e-5)
+    ops.diff_attention(q.float(), cache.float(), 0, kw, *args, o, *sizes, 1e4, 1e8)         # an eps this large leaves o as it is
+    rms = o.view(n, heads, vdim).pow(2).mean(-1, keepdim=True).add(1e-5).sqrt()
+    values = cache[..., kw:]
+    e = 1.1 * (1 + lam) * 2 ** -9 * values.abs().max().item()
+    y = (ref / out_scale).view(n, heads, vdim)
+    bound = out_scale * ((1 + y.abs()) * e / rms + 2 ** -8 * y.abs())
+    assert ((out.float() - ref).view(n, heads, vdim).abs() <= bound).all()
+
+
 def test_paged_attention_prefill_tcgen05_refuses_other_shapes(ops):
     q = torch.zeros(4, 2 * 48, dtype=torch.bfloat16, device=DEV)
     kc = torch.zeros(3, 16, 1, 48, dtype=torch.bfloat16, device=DEV)
