@@ -106,6 +106,35 @@ def test_gemm_simt(ops, dtype, M, N, K):
         assert torch.equal(one[0], full[M - 1])
 
 
+@pytest.mark.parametrize("N,K", [(40, 96), (16, 4), (130, 516), (65, 2052), (2048, 1000), (70, 77), (3, 8192)])
+def test_gemm_simt_rows_and_tiles_agree(ops, N, K):
+    """float32: the few-row kernel (aligned rows, alone or in groups of 16) and the tiles of 64 and of 128 rows give a row
+    the same bits. Error: spans of at most K / 16 + 32 numbers, then 16 sums."""
+    g = torch.Generator(device="cpu").manual_seed(41)
+    x = torch.randn(2000, K, generator=g).to(DEV)
+    w = torch.randn(N, K, generator=g).to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    ref = (x.double() @ w.double().T + bias.double()) * 0.5
+    bound = 2.0 ** -24 * (K / 16 + 50) * (x.double().abs() @ w.double().abs().T + bias.double().abs())
+    first = None
+    for M in (1, 2, 3, 7, 16, 17, 64, 65, 129, 2000):
+        out = torch.empty(M, N, device=DEV)
+        ops.gemm_simt(x[:M], w, out, bias, 0.5)
+        assert ((out.double() - ref[:M]).abs() <= bound[:M]).all()
+        first = out[0].clone() if first is None else first
+        assert torch.equal(out[0], first)
+        if M > 3:
+            two = torch.empty(2, N, device=DEV)
+            ops.gemm_simt(x[M - 2:M], w, two, bias, 0.5)
+            assert torch.equal(two, out[M - 2:])
+    # rows that lie apart by more than a row, at an address that is no multiple of 16 bytes
+    wide = torch.zeros(20, K + 9, device=DEV)
+    wide[:, 1:K + 1] = x[:20]
+    out = torch.empty(20, N, device=DEV)
+    ops.gemm_simt(wide[:, 1:K + 1], w, out, bias, 0.5)
+    assert torch.equal(out[0], first)
+
+
 def _rope_ref(x, pos, inv_freq, rot, pos_scale):
     """x [n, heads, hd] fp64; half-split rotation of the first `rot` dims."""
     half = rot // 2
