@@ -4,11 +4,14 @@ float32 always runs the plain kernel (csrc/latent_attention.cu), whose arithmeti
 alone. bfloat16 runs the tensor-core kernel (csrc/latent_attention_flash.cu) when the record's two pieces are
 multiples of 8 numbers and the latent has at most 512: its blocks take 32 query units, a unit being (row, head), so
 the host cuts every request of the step into tiles of 32 / heads-to-a-block consecutive rows (a step plan, sent with
-the step's integers). Prompt portions and single decoded tokens go through the same launch.
+the step's integers). Prompt portions and single decoded tokens go through the same launch, unless the heads have the sizes
+EXPAND_SIZES: then a portion's keys and values are worked out for every head (one product over the records its rows see) and
+attended by the tcgen05 flash kernel (csrc/attention_prefill_tcgen05.cu), a fifth of the operations a row and key.
 """
 
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from . import ops
@@ -46,6 +49,75 @@ class LatentTilePlan:
         return len(tiles)
 
 
+class LatentExpandPlan:
+    """Prompt portions whose keys and values are worked out for the heads before the attention: for every request behind the
+    single tokens at the head of the step, the keys its rows may see, from a multiple of 16 on, as pieces of 16. On the
+    device: per request slot what a key's position is added to for its row among the expanded ones, then int32 [pieces, 4] =
+    (request slot, first key, keys, 0). `fill` returns the pieces, 0 when the step is to go the other way: no portions, one
+    of fewer than EXPAND_MIN_ROWS rows, or more keys than there is room for."""
+
+    def __init__(self, window: int):
+        self.window = int(window)
+        self.name = f"latent_expand:{self.window}"
+
+    @staticmethod
+    def most_pieces(max_tokens: int) -> int:
+        return (2 * max_tokens + 2048) // 16
+
+    def ints(self, max_tokens: int, max_requests: int) -> int:
+        return (max_requests + 3) // 4 * 4 + 4 * self.most_pieces(max_tokens)
+
+    def fill(self, host, shape) -> tuple:
+        requests = (self.max_requests + 3) // 4 * 4
+        room = (len(host) - requests) // 4
+        lead = 0
+        while lead < len(shape.q_len) and shape.q_len[lead] == 1:
+            lead += 1
+        portions = list(zip(shape.q_len, shape.pos_start, shape.slots))[lead:]
+        if not portions or min(n for n, _, _ in portions) < EXPAND_MIN_ROWS:
+            return 0, requests
+        spans, total = [], 0
+        for n, start, slot in portions:
+            lo = max(0, start - self.window + 1) // 16 * 16 if self.window > 0 else 0
+            count = -(-(start + n - lo) // 16)
+            spans.append((slot, lo, start + n, count))
+            total += count
+        if total > room:
+            return 0, requests
+        at = 0
+        pieces = host[requests:requests + 4 * total].reshape(total, 4)
+        for slot, lo, hi, count in spans:
+            keys = np.arange(lo, lo + 16 * count, 16, dtype=np.int32)
+            host[slot] = 16 * at - lo
+            part = pieces[at:at + count]
+            part[:, 0], part[:, 1], part[:, 2], part[:, 3] = slot, keys, np.minimum(16, hi - keys), 0
+            at += count
+        return total, requests
+
+
+# Rows of a portion from which its keys and values are expanded: expanding costs a key 2 R heads (d + e) operations once, and
+# saves a row 2 heads (2 R - d - e) for every key it sees, on a kernel four times as fast: even at some 45 rows when all keys
+# are new to the step. Measured on B200, three steps of a Rematar model (width 2,048) that bring a prompt in portions beside
+# four single tokens, expanded / absorbed: portions of 64 1,685 / 1,843 us, of 256 2,019 / 2,170; two prompts of 394 and 1,383
+# tokens, the attention of a layer 38 + 4 us and the product / 299 us.
+EXPAND_MIN_ROWS = 64
+EXPAND_SIZES = (128, 64, 128)      # (own numbers of a key, turned piece, values) of the tcgen05 kernel
+
+_expand_plans = {}
+
+
+def expand_plan(spec, max_requests: int):
+    """The plan for a layer of these sizes, or None where the tcgen05 kernel has no such sizes."""
+    if (spec.head_dim, spec.rot_dim, spec.value_dim) != EXPAND_SIZES or spec.kv_rank % 8:
+        return None
+    key = (int(spec.get("window", 0)), int(max_requests))
+    plan = _expand_plans.get(key)
+    if plan is None:
+        plan = _expand_plans[key] = LatentExpandPlan(key[0])
+        plan.max_requests = key[1]
+    return plan
+
+
 _plans = {}
 
 
@@ -67,12 +139,13 @@ PART_ROWS = 64          # steps of single tokens up to this many rows may deal t
 MAX_PARTS = 16
 
 
-def key_parts(ctx, spec, sms: int = 0) -> int:
-    """Into how many parts the keys of every query tile are dealt. Only steps in which every request brings one token,
-    and few of them: such a step has one block per request and group of heads, each walking all of its keys alone. The
+def key_parts(ctx, spec, sms: int = 0, single_rows: int = 0) -> int:
+    """Into how many parts the keys of every query tile are dealt. Only steps in which every request brings one token (or the
+    single_rows single tokens of a step by themselves), and few of them: such a step has one block per request and group of heads, each walking all of its keys alone. The
     count follows the step's longest span of keys in powers of two (cut off at the window), so that a growing context
     keeps its launch shape, gives every part at least two key tiles, and aims at two blocks per SM."""
-    if not ctx.decode_only or ctx.num_tokens > PART_ROWS:
+    rows = single_rows or (ctx.num_tokens if ctx.decode_only else PART_ROWS + 1)
+    if rows > PART_ROWS:
         return 1
     window = int(spec.get("window", 0))
     span = 256
@@ -81,21 +154,22 @@ def key_parts(ctx, spec, sms: int = 0) -> int:
     if window > 0:
         span = min(span, window)
     tiles = span // KEY_TILE + 1
-    blocks = ctx.num_tokens * -(-spec.num_heads // heads_per_block(spec.num_heads))
+    blocks = rows * -(-spec.num_heads // heads_per_block(spec.num_heads))
     want = -(-2 * (sms or sm_count()) // blocks)
     return max(1, min(want, tiles // 2, MAX_PARTS))
 
 
-def attend(wide: torch.Tensor, cache, ctx, out: torch.Tensor, spec, sink, runtime=None) -> bool:
-    """The tensor-core kernel over the step's tiles; False (nothing done) when it does not take this model or step."""
+def attend(wide: torch.Tensor, cache, ctx, out: torch.Tensor, spec, sink, runtime=None, single=None) -> bool:
+    """The tensor-core kernel over the step's tiles, or over `single` = (tiles, number) of one row each, the first rows of the
+    step; False (nothing done) when it does not take this model or step."""
     if not flash_applies(spec, wide.dtype):
         return False
-    planned = ctx.extras.get(tile_plan(spec).name)
+    planned = single or ctx.extras.get(tile_plan(spec).name)
     if planned is None:
         return False
     tiles, n_tiles = planned
     (records,) = cache.arrays
-    parts = key_parts(ctx, spec) if runtime is not None else 1
+    parts = key_parts(ctx, spec, single_rows=n_tiles if single else 0) if runtime is not None else 1
     scratch = None
     if parts > 1:
         scratch = runtime.flat(f"latent_parts_{spec.num_heads}_{spec.kv_rank}",

@@ -32,7 +32,8 @@ import torch
 
 from ..errors import Unsupported
 from ..kernels import linear, ops
-from ..kernels.gemm import linear_partial
+from ..kernels.attention import QUERY_TILES
+from ..kernels.gemm import linear_partial, linear_short
 from .base import POSITIONS, CacheSpec, TensorDecl, register_mixer
 
 
@@ -86,6 +87,12 @@ class LatentAttention:
         self.joined_col = self.w_down.shape[0]
         self.w_uk = tensors["uk"].reshape(H, d, R).contiguous()                          # [H, in = d, out = R] as stored
         self.w_uv = tensors["uv"].reshape(H, e, R).transpose(1, 2).contiguous()          # [H, in = R, out = e]
+        # for prompt portions at the sizes of the tcgen05 kernel: one product gives every head's keys and values of a record
+        from ..kernels import latent_attention as fast
+        self.expand = None
+        if self.rt.dtype == torch.bfloat16 and fast.flash_applies(spec, self.rt.dtype):
+            self.expand = fast.expand_plan(spec, runtime.max_requests)
+        self.w_kv = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self.expand is not None else None
         self.sink = tensors.get("sink")
         self.w_o = tensors["o"]
         self.eps = float(spec.eps)
@@ -107,7 +114,8 @@ class LatentAttention:
     def step_plans(self) -> list:
         """The query tiles of the step, for the tensor-core kernel (kernels/latent_attention.py)."""
         from ..kernels import latent_attention as fast
-        return [fast.tile_plan(self.spec)] if fast.flash_applies(self.spec, self.rt.dtype) else []
+        plans = [fast.tile_plan(self.spec)] if fast.flash_applies(self.spec, self.rt.dtype) else []
+        return plans + ([QUERY_TILES, self.expand] if self.expand is not None else [])
 
     def graph_key(self, ctx) -> tuple:
         from ..kernels import latent_attention as fast
@@ -137,22 +145,68 @@ class LatentAttention:
             q = down[:, :self.q_cols]
             ops.latent_prep(down[:, self.q_cols:], 0, R, r, self.rot, None, self.dkv_norm, self.eps, self.freq, ctx.positions,
                             ctx.row_slot, cache.block_table, records, cache.page_size, None, self.mag)
+        heads = rt.buffer("latent_heads", (rows, H * e))
+        gate = down[:, self.q_cols + R + r:] if self.has_gate else None
+        if not self._expanded(q, gate, cache, ctx, heads):
+            self._absorbed(q, gate, cache, ctx, heads, rows, None)
+        return linear_partial(heads, self.w_o, rt, "mixer_out")
+
+    def _absorbed(self, q: torch.Tensor, gate: Optional[torch.Tensor], cache, ctx, heads: torch.Tensor, rows: int, single) -> None:
+        """The first `rows` rows with the up-projections on the queries' and the results' side, over the records as they are."""
+        s, rt = self.spec, self.rt
+        H, d, r, e, R = s.num_heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank
+        q, heads = q[:rows], heads[:rows]
         wide = rt.buffer("latent_wide_q", (rows, H * (R + r)))
         ops.head_linear(q, d + r, d, self.w_uk, wide, R + r)
         if r:
             ops.rotate_pairs(q, d + r, d, wide, R + r, R, r, self.rot, self.freq, ctx.positions, H, self.mag)
         mixed = rt.buffer("latent_mixed", (rows, H * R))
-        self.attend(wide, cache, ctx, mixed)
-        heads = rt.buffer("latent_heads", (rows, H * e))
-        gate = down[:, self.q_cols + R + r:] if self.has_gate else None
+        self.attend(wide, cache, ctx, mixed, single)
         ops.head_linear(mixed, R, R, self.w_uv, heads, e, gate, e)
-        return linear_partial(heads, self.w_o, rt, "mixer_out")
 
-    def attend(self, wide: torch.Tensor, cache, ctx, out: torch.Tensor) -> None:
+    def _expanded(self, q: torch.Tensor, gate: Optional[torch.Tensor], cache, ctx, heads: torch.Tensor) -> bool:
+        """A step whose portions' keys and values are worked out first (kernels/latent_attention.LatentExpandPlan): the portions
+        through the tcgen05 kernel, the single tokens at the step's head beside them the other way. False: nothing done."""
+        planned = ctx.extras.get(self.expand.name) if self.expand is not None else None
+        tiles = ctx.extras.get(QUERY_TILES.name)
+        if planned is None or tiles is None or planned[1][0] == 0 or cache.page_size < 16 or cache.page_size & (cache.page_size - 1) \
+                or q.stride(0) % 8 or q.data_ptr() % 16:
+            return False
+        s, rt = self.spec, self.rt
+        H, d, r, e, R = s.num_heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank
+        (records,) = cache.arrays
+        ints, (pieces, first_piece) = planned
+        q_tiles, (_, n_tiles, lead) = tiles
+        from ..kernels import attention
+        side = rt.side_stream if lead > 0 and attention.SIDE_BY_SIDE else None
+        if side is not None:
+            ops.stream_fork(side)
+            with ops.on_stream(side):
+                self._absorbed(q, gate, cache, ctx, heads, lead, (q_tiles[4 * n_tiles:], lead))
+        elif lead > 0:
+            self._absorbed(q, gate, cache, ctx, heads, lead, (q_tiles[4 * n_tiles:], lead))
+        most = 16 * self.expand.most_pieces(rt.max_tokens)
+        keys = 16 * pieces
+        latents = rt.flat(f"latent_rows_{R + r}", most * (R + r), torch.bfloat16)[:keys * (R + r)].view(keys, R + r)
+        kv = rt.flat(f"latent_kv_{H * (d + e)}", most * H * (d + e), torch.bfloat16)[:keys * H * (d + e)].view(keys, H * (d + e))
+        ops.latent_gather(records, cache.block_table, cache.page_size, ints[first_piece:], pieces, latents)
+        linear_short(latents[:, :R], self.w_kv, kv)
+        rows = q.shape[0]
+        q_rot = rt.buffer("latent_q_rot", (rows, H * r))
+        ops.rotate_pairs(q, d + r, d, q_rot, r, 0, r, self.rot, self.freq, ctx.positions, H, self.mag)
+        ops.latent_attention_tcgen05(q, q_rot, latents, R, kv, ints, q_tiles, n_tiles, heads, H, float(s.scale),
+                                     int(s.get("window", 0)), self.sink)
+        if gate is not None:
+            ops.sigmoid_gate(heads[lead:], gate[lead:])
+        if side is not None:
+            ops.stream_join(side)
+        return True
+
+    def attend(self, wide: torch.Tensor, cache, ctx, out: torch.Tensor, single=None) -> None:
         s = self.spec
         (records,) = cache.arrays
         from ..kernels import latent_attention as fast
-        if fast.attend(wide, cache, ctx, out, s, self.sink, self.rt):
+        if fast.attend(wide, cache, ctx, out, s, self.sink, self.rt, single):
             return
         ops.latent_attention(wide, records, cache.block_table, ctx.positions, ctx.row_slot, self.sink, out, s.num_heads,
                              s.kv_rank, s.rot_dim, cache.page_size, float(s.scale), int(s.get("window", 0)))

@@ -699,3 +699,90 @@ def test_command_line_generates(folders):
     assert len(ids) == 8 and all(0 <= t < REMATAR["ra"][0]["vocab"] for t in ids)
     from dynalm_b200 import Engine
     assert Engine(folders["bfloat16"]["ra"], ctx=256, batch=64).generate([5, 9, 200, 31], max_tokens=8).tokens == ids
+
+
+@pytest.mark.parametrize("window,with_sink", [(0, False), (100, True), (64, False), (333, True)])
+def test_expanded_latent_attention(window, with_sink):
+    """Portions over expanded keys and values (tcgen05) against float64: gathered records, bases per slot, keys that start in
+    the middle of a request, a tile of one row, a window that begins inside a piece. bf16 operands as given, probabilities
+    rounded to bf16 (2^-9 of weights that add up to one), the result to bf16."""
+    from types import SimpleNamespace
+    from dynalm_b200.kernels import latent_attention as fast
+    from dynalm_b200.kernels import ops
+    g = torch.Generator().manual_seed(window + 5)
+    H, R, page, slots = 3, 40, 16, 4
+    plan = fast.LatentExpandPlan(window)
+    plan.max_requests = slots
+    requests = {2: (0, 129), 0: (210, 64), 3: (55, 200)}                    # slot -> (first position, rows)
+    blocks = {s: -(-(p + n) // page) for s, (p, n) in requests.items()}
+    perm = torch.randperm(sum(blocks.values()) + 3, generator=g)
+    table = torch.full((slots, max(blocks.values())), -1, dtype=torch.int32)
+    records = torch.randn(len(perm), page, R + 64, generator=g).to(torch.bfloat16)
+    at = 0
+    for s, n in blocks.items():
+        table[s, :n] = perm[at:at + n].to(torch.int32)
+        at += n
+    shape = SimpleNamespace(q_len=[1] + [n for _, n in requests.values()], pos_start=[9] + [p for p, _ in requests.values()],
+                            slots=[1] + list(requests), q_start=[0, 1, 130, 194])
+    host = np.zeros(plan.ints(512, slots), dtype=np.int32)
+    pieces, first = plan.fill(host, shape)
+    tiles = [t for s, r0 in zip(requests, (1, 130, 194)) for t in
+             [(s, r0 + i, min(128, requests[s][1] - i), requests[s][0] + i) for i in range(0, requests[s][1], 128)]]
+    ints = torch.from_numpy(host).to(DEV)
+    latents = torch.full((16 * pieces, R + 64), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.latent_gather(records.to(DEV), table.to(DEV), page, ints[first:], pieces, latents)
+    assert torch.isfinite(latents).all()
+    w = (torch.randn(H * 256, R, generator=g) * 0.3).to(DEV, torch.bfloat16)
+    kv = (latents[:, :R].float() @ w.float().T).to(torch.bfloat16).contiguous()
+    q = torch.randn(394, H * 192, generator=g).to(DEV, torch.bfloat16)
+    q_rot = torch.randn(394, H * 64, generator=g).to(DEV, torch.bfloat16)
+    sink = torch.randn(H, generator=g).to(DEV) if with_sink else None
+    out = torch.full((394, H * 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    scale = 0.09
+    ops.latent_attention_tcgen05(q, q_rot, latents, R, kv, ints, torch.tensor(tiles, dtype=torch.int32, device=DEV).view(-1), len(tiles),
+                                 out, H, scale, window, sink)
+    assert (out[0] == 7.0).all()
+    for s, r0 in zip(requests, (1, 130, 194)):
+        p0, n = requests[s]
+        rec = torch.stack([records[table[s, t // page], t % page] for t in range(p0 + n)]).to(DEV)
+        both = (rec[:, :R].float() @ w.float().T).to(torch.bfloat16).double()
+        k, v = both[:, :H * 128].view(-1, H, 128), both[:, H * 128:].view(-1, H, 128)
+        qq = q[r0:r0 + n].double().view(n, H, 192)[:, :, :128]
+        sc = torch.einsum("qhd,khd->hqk", qq, k) + torch.einsum("qhr,kr->hqk", q_rot[r0:r0 + n].double().view(n, H, 64), rec[:, R:].double())
+        gap = (p0 + torch.arange(n, device=DEV))[:, None] - torch.arange(p0 + n, device=DEV)[None, :]
+        seen = (gap >= 0) & ((gap < window) if window else True)
+        sc = (sc * scale).masked_fill(~seen, -torch.inf)
+        if with_sink:
+            sc = torch.cat([sc, sink.double()[:, None, None].expand(H, n, 1)], -1)
+        pr = torch.softmax(sc, -1)[..., :p0 + n]
+        want = torch.einsum("hqk,khe->qhe", pr, v).reshape(n, -1)
+        bound = 2.0 ** -7 * torch.einsum("hqk,khe->qhe", pr, v.abs()).reshape(n, -1) + 1e-3
+        assert ((out[r0:r0 + n].double() - want).abs() <= bound).all()
+
+
+def test_portions_go_through_expanded_latents_and_back(monkeypatch):
+    """The same steps with portions long enough to be expanded and with the other way: single tokens beside portions, a gate, a
+    sink, a window, a portion too short for it; logits agree to the rounding of 16-bit activations."""
+    from dynalm_b200 import Engine, StepEntry
+    from dynalm_b200.kernels import latent_attention as fast
+    lat = {"heads": 2, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 64, "kv_rank": 48, "scale": 0.07,
+           "rot": {"base": 10000.0, "dims": 64}, "mask": {"size": 150}}
+    cfg = {"architecture": "Rematar", "vocab": 300, "width": 128, "norm": {"eps": 1e-5}, "postln_alpha": 2.0, "embedding": {"scale": 8.0},
+           "layers": [{"type": "latent_attention", "mixer": dict(lat), "mlp": {"kind": "dense", "ff": 128}} for _ in range(2)]}
+    ids = torch.randint(0, 300, (900,), generator=torch.Generator().manual_seed(2)).tolist()
+    got = {}
+    for rows in (64, 1 << 30):
+        monkeypatch.setattr(fast, "EXPAND_MIN_ROWS", rows)
+        calls = []
+        from dynalm_b200.kernels import ops
+        real = ops.latent_attention_tcgen05
+        monkeypatch.setattr(ops, "latent_attention_tcgen05", lambda *a, **k: (calls.append(1), real(*a, **k))[1])
+        eng = Engine(config=cfg, random_seed=3, dtype="bfloat16", ctx=2048, batch=420, max_running=4)
+        out = got[rows] = []
+        out.append(eng.step([StepEntry("a", ids[:200], [199]), StepEntry("b", ids[200:290], [0, 89])]).clone())
+        out.append(eng.step([StepEntry("b", ids[290:291], [0]), StepEntry("a", ids[300:400], [50, 99]), StepEntry("c", ids[400:665], [264])]).clone())
+        out.append(eng.step([StepEntry("a", ids[700:701], [0]), StepEntry("c", ids[710:725], [14])]).clone())
+        monkeypatch.setattr(ops, "latent_attention_tcgen05", real)
+        assert len(calls) == (4 if rows == 64 else 0)
+    for a, b in zip(got[64], got[1 << 30]):
+        assert (a - b).abs().max() <= 2e-2 * b.abs().max()
