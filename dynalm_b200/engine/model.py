@@ -51,6 +51,13 @@ class Decoder:
         `graph_key` covers, so that a decode step can be captured once and replayed."""
         return all(getattr(b, "graph_safe", False) for b in self.blocks)
 
+    @property
+    def portions_graph_safe(self) -> bool:
+        """True when every part says that the launches of ANY step depend only on the numbers of rows of its requests, on
+        the numbers of wanted rows, on what the step plans answered and on the longest context in powers of two from 256:
+        steps with prompt portions can then be captured and replayed as well."""
+        return self.graph_safe and all(getattr(b, "portions_graph_safe", False) for b in self.blocks)
+
     def graph_key(self, ctx) -> tuple:
         """What, beyond the numbers of rows, the parts' launch shapes depend on for this step."""
         key = ()

@@ -340,17 +340,20 @@ class StepFunction:
         self._caches = None
         # Decode-only steps (one token per request) are captured once per (requests, wanted rows,
         # span bucket) as a CUDA graph and replayed: the kernels read the step's integers from the
-        # packed device buffer, whose addresses never change. The reference's GPU path keeps one
+        # packed device buffer, whose addresses never change. So are steps with prompt portions whose
+        # requests bring the same numbers of rows again (a server's portions of one size beside the same
+        # number of decoding requests): their key holds all that the launches can depend on. The reference's GPU path keeps one
         # prepared graph per step structure in the same way, at most 64 of them
         # (dynacore/include/dynacore/gpu/ggml_device.h:8-13,39-48).
         from ..kernels import ops as _ops
         self.use_graphs = bool(use_graphs) and model.graph_safe and not _ops.CHECKED     # a checked build reads a record after every launch
+        self.portion_graphs = self.use_graphs and model.portions_graph_safe
         self._graphs: Dict[tuple, torch.cuda.CUDAGraph] = {}
         self._decode_logits: Optional[torch.Tensor] = None
         self.graph_kernel_launches = 0     # kernels replayed through graphs so far
         self._graph_nodes: Dict[tuple, int] = {}
         self._captured_logits: Dict[tuple, bool] = {}     # whether a captured step leaves logits (or only chosen ids)
-        self._shape_seen: Dict[tuple, int] = {}     # decode-only launch shape -> how often it has come
+        self._shape_seen: Dict[tuple, int] = {}     # launch shape -> how often it has come (the SHAPES_KEPT last new ones)
         self._capture_stream: Optional[torch.cuda.Stream] = None
         self.graph_captures = 0            # graphs captured so far, and the host time that took
         self.graph_capture_ms = 0.0
@@ -405,7 +408,7 @@ class StepFunction:
             chosen, src = token_feedback
             ctx = self.batcher.build(entries, reserve, feedback_src=src)
             ops.feedback_tokens(ctx.token_ids, chosen, ctx.extras["step:feedback_src"], len(entries))
-        if self.use_graphs and ctx.decode_only:
+        if self.use_graphs and (ctx.decode_only or (self.portion_graphs and ctx.num_logit_rows <= self.max_requests)):
             logits = self._replay(ctx, choose)
         else:
             out = self._logits_buffer(ctx.num_logit_rows) if ctx.num_logit_rows else None
@@ -442,12 +445,22 @@ class StepFunction:
         self.graph_capture_ms += (time.perf_counter() - started) * 1e3
         return graph
 
+    def _plan_answers(self, ctx: StepContext) -> tuple:
+        """What the step plans answered, as far as launches depend on it (a plan's `launch_key`; by default all of it)."""
+        out = []
+        for plan in self.batcher.buffers.plans:
+            got = ctx.extras[plan.name][1]
+            key = getattr(plan, "launch_key", None)
+            out.append(got if key is None else key(got))
+        return tuple(out)
+
     def _forward(self, ctx: StepContext, out: Optional[torch.Tensor], choose=None) -> Optional[torch.Tensor]:
         from ..kernels import ops
         with ops.pinned_stream():
             return self.model.forward(ctx, self.caches(), out, choose)
 
     MAX_GRAPHS = 64
+    SHAPES_KEPT = 4096
     # A launch shape is captured when it comes for the eighth time. A capture costs 5 to 15 ms on the host; shapes
     # that pass by (the last requests of a batch ending one after the other: 64, 63, 62, ... rows for two steps
     # each) are cheaper run as they are, and the plain runs before a capture have allocated every workspace and
@@ -461,12 +474,20 @@ class StepFunction:
                                               device=self.rt.device)
         # a graph holds the addresses it was captured with: the tensors of `choose` are part of its key
         chosen = None if choose is None else tuple(None if t is None else t.data_ptr() for t in choose)
-        key = (ctx.num_requests, ctx.num_logit_rows, chosen) + self.model.graph_key(ctx)
+        if ctx.decode_only:
+            key = (ctx.num_requests, ctx.num_logit_rows, chosen) + self.model.graph_key(ctx)
+        else:
+            key = ("portions", tuple(ctx.h_q_len), ctx.num_logit_rows, chosen, self._plan_answers(ctx),
+                   max(256, 1 << (ctx.max_kv_len - 1).bit_length()))
         out = self._decode_logits if ctx.num_logit_rows else None
-        graph = self._graphs.get(key)
-        if graph is None:
-            seen = self._shape_seen.get(key, 0) + 1
+        graph = self._graphs.pop(key, None)
+        if graph is not None:
+            self._graphs[key] = graph          # the one used last goes last (`_capture` drops the first)
+        else:
+            seen = self._shape_seen.pop(key, 0) + 1
             self._shape_seen[key] = seen
+            if len(self._shape_seen) > self.SHAPES_KEPT:
+                del self._shape_seen[next(iter(self._shape_seen))]
             if seen < self.GRAPH_AFTER:
                 got = self._forward(ctx, out, choose)
                 return got[:ctx.num_logit_rows] if got is not None else None

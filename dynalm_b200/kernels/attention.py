@@ -86,6 +86,11 @@ class QueryTileParts:
     def ints(self, max_tokens: int, max_requests: int) -> int:
         return 4 + 5 * (max_tokens // Q_TILE + max_requests + PART_SLOTS)
 
+    @staticmethod
+    def launch_key(answer) -> tuple:
+        """Without a split tile the attention walks QueryTilePlan's tiles."""
+        return (answer[0], answer[1] > 0) if answer[1] else (0, False)
+
     def key_tiles(self, pos0: int, rows: int) -> int:
         lo = max(0, pos0 - self.window + 1) if self.window > 0 else 0
         return (pos0 + rows - 1) // KEY_TILE - lo // KEY_TILE + 1
@@ -169,6 +174,11 @@ class DecodeUnits:
     def __init__(self, chunks: int, tile_keys: int, window: int):
         self.chunks, self.tile, self.window = int(chunks), int(tile_keys), int(window)
         self.name = f"attention_decode_units:{chunks}:{tile_keys}:{window}"
+
+    @staticmethod
+    def launch_key(answer) -> tuple:
+        """The grid follows the rows; the number of units is read on the device."""
+        return (answer[0] > 0, answer[1])
 
     def slots(self) -> int:
         return sm_count() * DECODE_BLOCKS_PER_SM

@@ -100,6 +100,7 @@ class Block:
         inner = [getattr(p, "position", None) for p in parts]
         self.replay_safe = all(getattr(p, "replay_safe", False) for p in parts + [p for p in inner if p is not None])
         self.graph_safe = all(getattr(p, "graph_safe", False) for p in parts)
+        self.portions_graph_safe = self.replay_safe and all(getattr(p, "portions_graph_safe", False) for p in parts)
 
     def parts(self):
         return [getattr(self, n) for n in self.part_names]
@@ -261,6 +262,7 @@ class SigmoidGate:
 
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
     post_weight, post_eps = None, 0.0
 
     @staticmethod
@@ -347,6 +349,7 @@ class HyperConnection:
 
     replay_safe = True     # it launches nothing itself
     graph_safe = True
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
 
     @staticmethod
     def declare(spec):

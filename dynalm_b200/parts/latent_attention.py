@@ -41,6 +41,7 @@ from .base import POSITIONS, CacheSpec, TensorDecl, register_mixer
 class LatentAttention:
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True      # launches depend on row counts only
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
 
     @staticmethod
     def declare(spec) -> Dict[str, TensorDecl]:

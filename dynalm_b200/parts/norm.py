@@ -16,6 +16,7 @@ from .base import TensorDecl, register_norm
 class RMSNorm:
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True      # launches depend on row counts only
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
 
     @staticmethod
     def declare(spec) -> Dict[str, TensorDecl]:
@@ -57,6 +58,7 @@ class RMSNormAfterSum:
 
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True      # launches depend on row counts only
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
 
     @staticmethod
     def declare(spec) -> Dict[str, TensorDecl]:
@@ -85,6 +87,7 @@ class LayerNorm:
 
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True      # launches depend on row counts only
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
 
     @staticmethod
     def declare(spec) -> Dict[str, TensorDecl]:

@@ -31,6 +31,7 @@ from .base import CacheSpec, TensorDecl, register_mixer
 class GatedLinearRecurrence:
     replay_safe = True     # all device work goes through the recorded launches of kernels/ops.py (engine/launch_memo.py)
     graph_safe = True      # launches depend on row and request counts only
+    portions_graph_safe = True      # the same of steps with prompt portions, given the plans' answers and the span (engine/step.py)
     out_name = "mixer_out"     # the workspace buffer of the result; a mixer that holds this one may name another
 
     @staticmethod

@@ -53,6 +53,7 @@ class SideBySideMixer:
         self.eps = float(spec.get("eps", 1e-6))
         self.replay_safe = all(getattr(getattr(self, s), "replay_safe", False) for s in SIDES)
         self.graph_safe = all(getattr(getattr(self, s), "graph_safe", False) for s in SIDES)
+        self.portions_graph_safe = all(getattr(getattr(self, s), "portions_graph_safe", False) for s in SIDES)
         specs = [getattr(self, s).cache_spec() for s in SIDES]
         kinds = [c.kind for c in specs if c is not None]
         if len(kinds) != len(set(kinds)):
