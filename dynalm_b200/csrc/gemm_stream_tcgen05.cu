@@ -182,33 +182,31 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc[c0 + j] = __uint_as_float(v[j]);
       }
-      if (mode == GS_OUT_BF16 || mode == GS_OUT_F32 || mode == GS_OUT_RELU2 || mode == GS_OUT_GELU || mode == GS_OUT_XIELU) {
+      if (mode != GS_OUT_SWIGLU) {
+        // every kind a loop of its own: the activations' code between the plain store's instructions costs their fetching
         const int f = f0 + fl;
-        if (f < N) {
-          if (mode == GS_OUT_F32) {
-            float* out = static_cast<float*>(y) + static_cast<size_t>(split) * split_stride + f;
+        auto write = [&](auto fin) {
+          bf16* out = static_cast<bf16*>(y) + f;
 #pragma unroll
-            for (int b = 0; b < NB; ++b)
-              if (b < M) out[static_cast<size_t>(b) * ldy] = acc[b] * out_scale;
-          } else {
-            bf16* out = static_cast<bf16*>(y) + f;
+          for (int b = 0; b < NB; ++b)
+            if (b < M && f < N) out[static_cast<size_t>(b) * ldy] = __float2bfloat16_rn(fin(acc[b]));
+        };
+        if (mode == GS_OUT_F32) {
+          float* out = static_cast<float*>(y) + static_cast<size_t>(split) * split_stride + f;
 #pragma unroll
-            for (int b = 0; b < NB; ++b)
-              if (b < M) {
-                float v = acc[b] * out_scale;
-                if (mode == GS_OUT_RELU2) {      // the squared ReLU of an ungated feed-forward
-                  v = fmaxf(v, 0.0f);
-                  v *= v;
-                } else if (mode == GS_OUT_GELU) {  // or its GELU in the tanh form
-                  v = gelu_tanh_bf16(v);
-                } else if (mode == GS_OUT_XIELU) {
-                  v = xielu_bf16(v, coeffs[0], coeffs[1]);
-                }
-                out[static_cast<size_t>(b) * ldy] = __float2bfloat16_rn(v);
-              }
-          }
+          for (int b = 0; b < NB; ++b)
+            if (b < M && f < N) out[static_cast<size_t>(b) * ldy] = acc[b] * out_scale;
+        } else if (mode == GS_OUT_RELU2) {      // the squared ReLU of an ungated feed-forward
+          write([&](float v) { v = fmaxf(v * out_scale, 0.0f); return v * v; });
+        } else if (mode == GS_OUT_GELU) {       // or its GELU in the tanh form
+          write([&](float v) { return gelu_tanh_bf16(v * out_scale); });
+        } else if (mode == GS_OUT_XIELU) {
+          const float c0 = coeffs[0], c1 = coeffs[1];
+          write([&](float v) { return xielu_bf16(v * out_scale, c0, c1); });
+        } else {
+          write([&](float v) { return v * out_scale; });
         }
-      } else if (mode == GS_OUT_SWIGLU) {
+      } else {
         // lanes 0..63 hold gate features f0 + fl, lanes 64..127 the matching up features. The two halves swap half of
         // their batch columns through shared memory (every MMA has completed, so the stages are free): a gate thread
         // finishes columns [0, NB / 2) of its feature, the up thread of the same feature columns [NB / 2, NB).
@@ -230,17 +228,19 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             bias_g = coeffs[CLAMPED_HEADER + f0 + feat];
             bias_u = coeffs[CLAMPED_HEADER + gate_rows + f0 + feat];
           }
+          auto write = [&](auto fin) {
 #pragma unroll
-          for (int b = 0; b < HALF; ++b) {
-            const int col = is_gate ? b : HALF + b;
-            if (col < M) {
-              const float other = exchange[col * 64 + feat];
-              const float g = is_gate ? acc[b] : other, u = is_gate ? other : acc[HALF + b];
-              const float v = coeffs != nullptr ? clamped_swiglu_bf16(g + bias_g, u + bias_u, limit, gate_scale)
-                                                : __fdividef(g, 1.0f + __expf(-g)) * u;
-              out[static_cast<size_t>(col) * ldy] = __float2bfloat16_rn(v);
+            for (int b = 0; b < HALF; ++b) {
+              const int col = is_gate ? b : HALF + b;
+              if (col < M) {
+                const float other = exchange[col * 64 + feat];
+                const float g = is_gate ? acc[b] : other, u = is_gate ? other : acc[HALF + b];
+                out[static_cast<size_t>(col) * ldy] = __float2bfloat16_rn(fin(g, u));
+              }
             }
-          }
+          };
+          if (coeffs != nullptr) write([&](float g, float u) { return clamped_swiglu_bf16(g + bias_g, u + bias_u, limit, gate_scale); });
+          else write([](float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; });
         }
       }
     }

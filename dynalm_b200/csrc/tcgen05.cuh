@@ -61,6 +61,10 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int* s
   return __all_sync(0xffffffffu, ok);
 }
 
+__device__ __forceinline__ void prefetch_tensor_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -182,26 +186,37 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void tcgen05_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Writes this warp's 32 rows x 64 bf16 columns (one row per lane, `w` = the lane's 8 x 16 bytes) through a
-// swizzled shared staging area, so that each store instruction covers four whole 128-byte row pieces.
+// Writes this warp's 32 rows x 64 bf16 columns, one row per lane, through a swizzled shared staging area, so that each store
+// instruction covers four whole 128-byte row pieces. In two steps, for code that works out 32 columns at a time: a lane's 4 x
+// 16 bytes of columns 32 `half` .. go to the staging area; then both halves are stored.
 // `col0` is the first of the 64 columns, `n_valid` the number of valid output columns overall.
-__device__ __forceinline__ void store_rows_bf16(const uint4 (&w)[8], unsigned char* stage, int lane, bf16* out, int ldy,
-                                                int row0, int M, int col0, int n_valid) {
+__device__ __forceinline__ void stage_half_row(const uint4 (&w)[4], unsigned char* stage, int lane, int half) {
   uint4* st = reinterpret_cast<uint4*>(stage);
 #pragma unroll
-  for (int ch = 0; ch < 8; ++ch) st[lane * 8 + (ch ^ (lane & 7))] = w[ch];
+  for (int ch = 0; ch < 4; ++ch) st[lane * 8 + ((half * 4 + ch) ^ (lane & 7))] = w[ch];
+}
+__device__ __forceinline__ void store_staged_rows(const unsigned char* stage, int lane, bf16* out, int ldy, int row0, int M, int col0,
+                                                  int n_valid) {
+  const uint4* st = reinterpret_cast<const uint4*>(stage);
   __syncwarp();
+  const int ch = lane & 7, col = col0 + ch * 8;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int r = i * 4 + (lane >> 3), ch = lane & 7;
+    const int r = i * 4 + (lane >> 3);
     const uint4 v = st[r * 8 + (ch ^ (r & 7))];
-    const int col = col0 + ch * 8;
     if (row0 + r < M && col < n_valid) *reinterpret_cast<uint4*>(out + static_cast<size_t>(row0 + r) * ldy + col) = v;
   }
   __syncwarp();
 }
 
-// As store_rows_bf16 for rows that lie anywhere: lane r holds two pieces of 32 bf16 (`lo`, `hi`: 4 x 16 bytes each)
+__device__ __forceinline__ void store_rows_bf16(const uint4 (&w)[8], unsigned char* stage, int lane, bf16* out, int ldy,
+                                                int row0, int M, int col0, int n_valid) {
+  stage_half_row({w[0], w[1], w[2], w[3]}, stage, lane, 0);
+  stage_half_row({w[4], w[5], w[6], w[7]}, stage, lane, 1);
+  store_staged_rows(stage, lane, out, ldy, row0, M, col0, n_valid);
+}
+
+// As store_staged_rows for rows that lie anywhere: lane r holds two pieces of 32 bf16 (`lo`, `hi`: 4 x 16 bytes each)
 // of its row and the row's base pointer `dst` (null: nothing is written); the pieces go to dst + off_lo and
 // dst + off_hi (elements, multiples of 8). Each store instruction covers four rows' pieces of 64 bytes.
 __device__ __forceinline__ void store_rows_pieces(const uint4 (&lo)[4], const uint4 (&hi)[4], unsigned char* stage, int lane,
