@@ -523,16 +523,16 @@ static int t5_sm_count() {
   return sm_count;
 }
 
-// What a round of tiles of bn columns takes, of blocks alone or of pairs, in rounds of 256-wide tiles of pairs (24.1 us at K
-// 4096). Measured on B200 over all widths at 2499 x 28672 (SwiGLU) x 4096; at 23 products from 64 to 2,499 rows the width and
-// kind with the least rounds x cost is the fastest measured or within 5 % of it. Below 128 columns a round no longer gets
-// shorter: the 128 rows of x of every block are what it brings in. Against blocks alone at 256, 192 or 128 columns, with pairs
-// that only shared W's loads for the largest products (us, cold caches, same order of sums): 2048 x 16384 (SwiGLU) x 2048 98
-// -> 86; 2048 x 2048 x 8192 70 -> 57; 2499 x 28672 (SwiGLU) x 4096 395 -> 382; 2499 x 4096 x 14336 230 -> 202; 543 x 16384
-// (SwiGLU) x 3072 72 -> 57; 543 x 3072 x 8192 53 -> 43.
-static double t5_tile_cost(int bn, bool pair) {
-  static const double alone[] = {0.65, 0.63, 0.672, 0.755, 0.813, 0.963, 1.025};       // 64, 96, .. 256
-  static const double paired[] = {0.62, 0.637, 0.643, 0.68, 0.755, 0.88, 1.0};
+// What a slice of 64 k takes a round of tiles of bn columns, of blocks alone or of pairs, in us: from products of 543 to 2,048
+// rows by 2,048 or 3,072 features, between K 2048 and K 8192, on B200. At 35 products from 64 to 2,048 rows the width and kind
+// with the least rounds x cost is the fastest measured or within 5 % of it. Against blocks alone at 256, 192 or 128 columns,
+// with pairs that only shared W's loads for the largest products (us, cold caches, same order of sums): 2048 x 16384 (SwiGLU) x
+// 2048 98 -> 86; 2048 x 2048 x 8192 70 -> 57; 2499 x 28672 (SwiGLU) x 4096 395 -> 382; 2499 x 4096 x 14336 230 -> 202. (K in 2
+// to 8 pieces over a cluster, the sums added through distributed shared memory, takes 25.5 us for 700 x 2048 x 8192 against
+// 29.8 here, but no whole step gained from it by more than its runs differ.)
+static double t5_slice_us(int bn, bool pair) {
+  static const double alone[] = {0.215, 0.222, 0.244, 0.293, 0.321, 0.361, 0.402};       // 64, 96, .. 256
+  static const double paired[] = {0.183, 0.190, 0.209, 0.240, 0.268, 0.295, 0.325};
   return (pair ? paired : alone)[(bn - 64) / 32];
 }
 
@@ -561,7 +561,7 @@ static T5Choice t5_choose(long long m_blocks, int feats, int mode, int head_dim,
       const int per = mode == dl::T5_OUT_SWIGLU ? bn / 2 : bn;
       const long long t = (m_blocks + pair) / (1 + pair) * ((feats + per - 1) / per);
       const int units = sms / (1 + pair);
-      const double c = static_cast<double>((t + units - 1) / units) * t5_tile_cost(bn, pair != 0);
+      const double c = static_cast<double>((t + units - 1) / units) * t5_slice_us(bn, pair != 0);
       if (c < least) {
         least = c;
         best = {bn, pair != 0};
