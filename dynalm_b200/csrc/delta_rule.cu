@@ -246,7 +246,7 @@ delta_rule_kernel(const T* __restrict__ u, int u_stride, int q_col, int k_col, i
                   const int* __restrict__ state_slots, float* __restrict__ out, int H, int G, int d, int e) {
   using L = DrTile<R, P>;
   extern __shared__ __align__(16) float sm[];   // two tiles
-  const int h = blockIdx.y, r = blockIdx.z;
+  const int h = blockIdx.y, r = static_cast<int>(gridDim.z) - 1 - static_cast<int>(blockIdx.z);      // (see the launch)
   const int j = h / (H / G);
   const int tid = threadIdx.x;
   const int col0 = blockIdx.x * L::COLS;
@@ -570,6 +570,9 @@ int delta_rule_launch(const void* u, int u_stride, int q_col, int k_col, int v_c
     const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return static_cast<int>(err);
   }
+  // The requests from the last to the first: a step's single tokens stand at its head, and the blocks of a portion, which take
+  // as long as it is, start first, one to an SM (700 tokens beside eight single ones, 16 heads of 128 with 128 columns, a decay per channel: 135 us
+  // a layer from the first to the last, 122 from the last).
   dim3 grid((e + L::COLS - 1) / L::COLS, H, requests);
   kernel<<<grid, DR_THREADS, smem, stream>>>(static_cast<const T*>(u), u_stride, q_col, k_col, v_col,
                                              static_cast<const T*>(proj), proj_stride, b_col, a_col, a_log, dt_bias, decays,
