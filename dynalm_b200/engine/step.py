@@ -408,7 +408,10 @@ class StepFunction:
             chosen, src = token_feedback
             ctx = self.batcher.build(entries, reserve, feedback_src=src)
             ops.feedback_tokens(ctx.token_ids, chosen, ctx.extras["step:feedback_src"], len(entries))
-        if self.use_graphs and (ctx.decode_only or (self.portion_graphs and ctx.num_logit_rows <= self.max_requests)):
+        # (A step that leaves nothing, a portion from the middle of a prompt with no decoding request beside it, is not captured:
+        # nobody waits for it, so its launches are issued while the step in front runs. Bringing in eight prompts of 1,500
+        # tokens for a Nisotar model took 24.5 ms without a capture among them and 29.4 with one.)
+        if self.use_graphs and (ctx.decode_only or (self.portion_graphs and 0 < ctx.num_logit_rows <= self.max_requests)):
             logits = self._replay(ctx, choose)
         else:
             out = self._logits_buffer(ctx.num_logit_rows) if ctx.num_logit_rows else None

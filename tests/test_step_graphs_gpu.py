@@ -50,6 +50,22 @@ def test_portions_replayed_give_the_same_bits(name, dtype, monkeypatch):
         assert torch.equal(a, b), f"step {step}"
 
 
+def test_portions_that_leave_nothing_are_not_captured(monkeypatch):
+    from dynalm_b200 import Engine, StepEntry
+    from dynalm_b200.engine.step import StepFunction
+    monkeypatch.setattr(StepFunction, "GRAPH_AFTER", 2)
+    cfg, seed = TINY["a"]
+    eng = Engine(config=cfg, random_seed=seed, dtype="bfloat16", ctx=512, batch=64, max_running=2)
+    for _ in range(4):
+        eng.step([StepEntry("r", list(range(20)))])
+        eng.end("r")
+    assert eng.step_fn.graph_captures == 0
+    for _ in range(4):
+        eng.step([StepEntry("r", list(range(20)), [19])])
+        eng.end("r")
+    assert eng.step_fn.graph_captures == 1
+
+
 def test_shapes_that_pass_by_are_forgotten(monkeypatch):
     from dynalm_b200 import Engine, StepEntry
     from dynalm_b200.engine.step import StepFunction
