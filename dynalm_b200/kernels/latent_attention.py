@@ -141,8 +141,8 @@ MAX_PARTS = 16
 
 def key_parts(ctx, spec, sms: int = 0, single_rows: int = 0) -> int:
     """Into how many parts the keys of every query tile are dealt. Only steps in which every request brings one token (or the
-    single_rows single tokens of a step by themselves), and few of them: such a step has one block per request and group of heads, each walking all of its keys alone. The
-    count follows the step's longest span of keys in powers of two (cut off at the window), so that a growing context
+    single_rows single tokens of a step by themselves), and few of them: such a step has one block per request and group of
+    heads, each walking all of its keys alone. The count follows the step's longest span of keys in powers of two (cut off at the window), so that a growing context
     keeps its launch shape, gives every part at least two key tiles, and aims at two blocks per SM."""
     rows = single_rows or (ctx.num_tokens if ctx.decode_only else PART_ROWS + 1)
     if rows > PART_ROWS:
