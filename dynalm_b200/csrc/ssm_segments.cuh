@@ -50,6 +50,13 @@ __device__ __forceinline__ void seg_split(float a, float b, uint32_t (&out)[3]) 
   }
 }
 
+// Whether one of eight bfloat16 numbers is an infinity or no number.
+__device__ __forceinline__ bool seg_not_finite(const uint4& v) {
+  constexpr unsigned EXPONENTS = 0x7f807f80u;
+  return (__vcmpeq2(v.x & EXPONENTS, EXPONENTS) | __vcmpeq2(v.y & EXPONENTS, EXPONENTS) | __vcmpeq2(v.z & EXPONENTS, EXPONENTS) |
+          __vcmpeq2(v.w & EXPONENTS, EXPONENTS)) != 0u;
+}
+
 // The segment's step sizes and running exponents: at[t] = (exponent, what it misses, step size, 0); zeros past the end.
 // Called by the whole block (at least SEG_T threads); ends with a barrier.
 __device__ __forceinline__ void seg_exponents(float4* at, double* warp_sums, const bf16* proj, int proj_stride, int col, int r0,
@@ -158,6 +165,7 @@ ssm_outputs_kernel(const bf16* __restrict__ u, int u_stride, const bf16* __restr
   bf16* ss = sx + SEG_T * XS;                         // C [SEG_T][BS] first, then the start state's terms [3][N][XS]
   __shared__ float4 at[SEG_T];
   __shared__ double warp_sums[SEG_T / 32];
+  __shared__ unsigned not_finite;                     // bit i: of the tokens 16 i .. 16 i + 15 one has an x that is not finite
   static_assert(START > 0, "");
   const int4 seg = reinterpret_cast<const int4*>(segments)[blockIdx.x];
   const int h = blockIdx.y, g = h / (H / G), r0 = seg.y, n = seg.z, inner = H * P, tid = threadIdx.x;
@@ -173,14 +181,18 @@ ssm_outputs_kernel(const bf16* __restrict__ u, int u_stride, const bf16* __restr
     *reinterpret_cast<Vec16*>(sb + t * BS + c) = b;
     *reinterpret_cast<Vec16*>(ss + t * BS + c) = cc;
   }
+  if (tid == 0) not_finite = 0u;
+  unsigned mine = 0u;
   for (int e = tid; e < SEG_T * (P / 8); e += 256) {
     const int t = e / (P / 8), c = e % (P / 8) * 8;
     Vec16 v;
     v.raw = make_uint4(0, 0, 0, 0);
     if (t < n) v = *reinterpret_cast<const Vec16*>(u + static_cast<size_t>(r0 + t) * u_stride + h * P + c);
     *reinterpret_cast<Vec16*>(sx + t * XS + c) = v;
+    if (seg_not_finite(v.raw)) mine |= 1u << (t >> 4);
   }
   seg_exponents(at, warp_sums, proj, proj_stride, dt_col + h, r0, n, dt_bias[h], expf(a_log[h]));
+  if (mine != 0u) atomicOr(&not_finite, mine);        // (set to zero in front of the barriers of seg_exponents, read behind the next two)
   const int warp = tid >> 5, lane = tid & 31, j = lane >> 3, l8 = lane & 7;
   const int tile = warp < 4 ? warp : 11 - warp;        // 16 tokens; a scheduler's two warps have nine steps together
   const int t0 = tile * 16, ta = t0 + (lane >> 2), tb = ta + 8;
@@ -239,20 +251,41 @@ ssm_outputs_kernel(const bf16* __restrict__ u, int u_stride, const bf16* __restr
       seg_mma(gc[0], c_frag[k], b[0], b[1]);
       seg_mma(gc[1], c_frag[k], b[2], b[3]);
     }
-    uint32_t a[3][4];
+    float v[2][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float v[4];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const int s = s0 + i * 8 + (lane & 3) * 2 + k;
         const float4 es = at[s];
-        v[k] = s <= ta ? gc[i][k] * (expf(-((ea.x - es.x) + (ea.y - es.y))) * es.z) : 0.0f;
-        v[2 + k] = s <= tb ? gc[i][2 + k] * (expf(-((eb.x - es.x) + (eb.y - es.y))) * es.z) : 0.0f;
+        v[i][k] = s <= ta ? gc[i][k] * (expf(-((ea.x - es.x) + (ea.y - es.y))) * es.z) : 0.0f;
+        v[i][2 + k] = s <= tb ? gc[i][2 + k] * (expf(-((eb.x - es.x) + (eb.y - es.y))) * es.z) : 0.0f;
       }
+    if (not_finite >> (s0 >> 4) & 1u) {
+      // In the product the weight 0 of a token that a row does not see, or of a term of a weight that needs no third one, would
+      // meet the infinity: these sixteen tokens are added one by one, each to the rows that see it.
+#pragma unroll 1
+      for (int k = 0; k < 16; ++k) {
+        const int from = (lane & ~3) | (k >> 1 & 3);
+        const float wa = __shfl_sync(0xffffffffu, k & 8 ? (k & 1 ? v[1][1] : v[1][0]) : (k & 1 ? v[0][1] : v[0][0]), from);
+        const float wb = __shfl_sync(0xffffffffu, k & 8 ? (k & 1 ? v[1][3] : v[1][2]) : (k & 1 ? v[0][3] : v[0][2]), from);
+        const bool seen_a = s0 + k <= ta, seen_b = s0 + k <= tb;
+        const bf16* xr = sx + (s0 + k) * XS + (lane & 3) * 2;
+#pragma unroll
+        for (int i = 0; i < P / 8; ++i) {
+          const __nv_bfloat162 xv = *reinterpret_cast<const __nv_bfloat162*>(xr + i * 8);
+          if (seen_a) acc[i][0] = fmaf(wa, __low2float(xv), acc[i][0]), acc[i][1] = fmaf(wa, __high2float(xv), acc[i][1]);
+          if (seen_b) acc[i][2] = fmaf(wb, __low2float(xv), acc[i][2]), acc[i][3] = fmaf(wb, __high2float(xv), acc[i][3]);
+        }
+      }
+      continue;
+    }
+    uint32_t a[3][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
       uint32_t p0[3], p1[3];
-      seg_split(v[0], v[1], p0);
-      seg_split(v[2], v[3], p1);
+      seg_split(v[i][0], v[i][1], p0);
+      seg_split(v[i][2], v[i][3], p1);
 #pragma unroll
       for (int m = 0; m < 3; ++m) a[m][2 * i] = p0[m], a[m][2 * i + 1] = p1[m];
     }

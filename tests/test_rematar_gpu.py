@@ -342,6 +342,37 @@ def test_segments_in_matrix_form(H, P, N, G):
             r0 += n
 
 
+@pytest.mark.parametrize("P,N", [(64, 128), (128, 64)])
+def test_segments_in_matrix_form_keep_what_is_not_finite_behind_its_token(P, N):
+    """Infinities and a NaN in x: the numbers of the tokens in front of them, of the other channels and of the other head are
+    those of the recurrence, what the recurrence leaves without a number is not finite here either. Bound as above."""
+    from types import SimpleNamespace
+    from dynalm_b200.kernels import ops
+    H, G, seg, dt_col = 2, 1, ops.SSM_SEGMENT, 8
+    rng = np.random.RandomState(P + 3)
+    inner, n = H * P, 2 * seg + 37
+    a_log, dt_bias, d_skip = rng.randn(H) * 0.3, rng.randn(H) * 0.3, 1 + 0.2 * rng.randn(H)
+    x = rng.randn(n, inner + 2 * N) * 0.7
+    x[40, 3], x[seg + 30, 9], x[2 * seg + 36, P - 1], x[47, 20] = np.inf, np.nan, -np.inf, -np.inf
+    u, proj = _t(x, torch.bfloat16), _t(rng.randn(n, dt_col + H), torch.bfloat16)
+    _, _, _, q_start, _, slots = _step_arrays([(0, n)], [0])
+    plan, most = ops.SSM_SEGMENTS, ops.SSM_SEGMENTS.most_segments(640)
+    host = np.zeros(plan.ints(640, 1), dtype=np.int32)
+    meta = plan.fill(host, SimpleNamespace(q_len=[n], q_start=[0], slots=[0]))
+    state = torch.zeros(1, inner * N, device=DEV)
+    y = torch.full((n, inner), 7.0, device=DEV)
+    ops.ssm_scan(u, proj, dt_col, _t(dt_bias), _t(a_log), _t(d_skip), state, q_start, slots, y, 1, H, P, N, G,
+                 (torch.from_numpy(host).to(DEV), meta), torch.zeros(most * inner * N, device=DEV), torch.zeros(most * H, device=DEV))
+    ut = _np(u)
+    B, C = (np.repeat(v.reshape(n, G, N), H // G, axis=1) for v in (ut[:, inner:inner + N], ut[:, inner + N:]))
+    with np.errstate(invalid="ignore"):
+        want, kept = plain.ssm_scan(ut[:, :inner].reshape(n, H, P), plain.softplus(_np(proj[:, dt_col:]) + dt_bias), B, C, a_log, d_skip, None)
+    for got, ref in ((_np(y), want.reshape(n, inner)), (_np(state[0]).reshape(H, N, P), kept)):
+        fine = np.isfinite(ref)
+        assert (np.isfinite(got) == fine).all() and (~fine).any()
+        assert np.abs(got[fine] - ref[fine]).max() <= 2e-5 * max(1.0, np.abs(ref[fine]).max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gate_comes_before_the_norm_of_every_part(dtype):
     from dynalm_b200.kernels import ops
