@@ -409,11 +409,13 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
         for (int k = 0; k < 4; ++k) {
           const int j = min(j0 + k, tiles - 1), b = j % n_parts;
           const float* pt = (n_parts > 1 ? cluster.map_shared_rank(records, b) : records) + (j / n_parts * FG + g) * REC;
-          m[k] = j0 + k < tiles ? pt[D] : -INFINITY, l[k] = pt[D + 1], a[k] = pt[d];
+          m[k] = pt[D], l[k] = pt[D + 1], a[k] = pt[d];
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          if (m[k] == -INFINITY) continue;
+          // (a tile whose seen scores are no numbers has no largest one either: it counts, and only one without a key
+          // changes nothing)
+          if (j0 + k >= tiles) break;
           float c_run, c_tile;
           merge_factors(m_run[i], m[k], c_run, c_tile);
           l_run[i] = two_products(l_run[i], c_run, l[k], c_tile);

@@ -301,6 +301,41 @@ def test_attention_f32(ops, heads, kvh, d, e, window, keep, sink, bias, chunk):
     assert torch.equal(out[5:], alone[0][5:]) and (out[:5] == 7.0).all()
 
 
+@pytest.mark.parametrize("window", [0, 5])
+def test_attention_f32_lets_no_key_without_a_number_pass(ops, window):
+    """Keys that are no numbers, all that a row sees of a tile of 64: rows that see one give no numbers in every kernel and
+    with any number of blocks over the keys, the others the same numbers as ever."""
+    g = torch.Generator(device="cpu").manual_seed(67)
+    heads, kvh, d, page, length = 4, 2, 32, 16, 400
+    kc = torch.randn(length // page, page, kvh * 2 * d, generator=g)
+    flat = kc.view(length, 2 * kvh * d)
+    bad = [64, 65, 66, 128, 320, 321]
+    flat[bad, :d] = float("nan")                   # the first KV head's keys
+    table = torch.arange(length // page, dtype=torch.int32).view(1, -1).to(DEV)
+    kc = kc.to(DEV)
+    row, vc = 2 * kvh * d, kc.view(-1)[kvh * d:]
+    q = torch.randn(length, heads * d, generator=g).to(DEV)
+    pos = torch.arange(length, dtype=torch.int32, device=DEV)
+    req = torch.zeros(length, dtype=torch.int32, device=DEV)
+    args = (heads, kvh, d, d, page, d ** -0.5, window)
+    sees = torch.tensor([any(max(0, p - window + 1 if window else 0) <= b <= p for b in bad) for p in range(length)], device=DEV)
+    outs = []
+    for parts in (1, 2, 4, 8):
+        outs.append(torch.empty(length, heads * d, device=DEV))
+        ops.attention_f32_rows(q, kc, row, vc, row, table, pos, req, length, parts, outs[-1], *args)
+    outs.append(torch.empty(length, heads * d, device=DEV))
+    tiles = torch.tensor([(0, t0, min(128, length - t0), t0) for t0 in range(0, length, 128)], dtype=torch.int32, device=DEV)
+    ops.attention_f32_tiles(q, kc, row, vc, row, table, tiles.view(-1), tiles.shape[0], outs[-1], *args)
+    outs.append(torch.empty(length, heads * d, device=DEV))
+    ops.paged_attention_generic_kv(q, kc, row, vc, row, table, pos, req, outs[-1], *args)
+    half = heads // 2 * d
+    for out in outs:
+        assert torch.equal(torch.isnan(out[:, :half]).all(dim=1), sees) and not torch.isnan(out[~sees]).any()
+        assert not torch.isnan(out[:, half:]).any()
+    for out in outs[1:5]:
+        assert torch.equal(torch.nan_to_num(out), torch.nan_to_num(outs[0]))
+
+
 def test_argmax_ties_and_sizes(ops):
     g = torch.Generator(device="cpu").manual_seed(7)
     # 50,001: rows that do not start on 16 bytes and a last slice that is no multiple of 4 (the scan's scalar ends)
