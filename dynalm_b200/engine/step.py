@@ -21,6 +21,7 @@ import torch
 from ..cache import CacheManager
 from ..errors import InvalidArgument
 from .context import StepContext
+from .kept_graphs import KeptGraphs
 from .model import Decoder
 from .runtime import Runtime
 
@@ -342,18 +343,16 @@ class StepFunction:
         # span bucket) as a CUDA graph and replayed: the kernels read the step's integers from the
         # packed device buffer, whose addresses never change. So are steps with prompt portions whose
         # requests bring the same numbers of rows again (a server's portions of one size beside the same
-        # number of decoding requests): their key holds all that the launches can depend on. The reference's GPU path keeps one
-        # prepared graph per step structure in the same way, at most 64 of them
+        # number of decoding requests): their key holds all that the launches can depend on. Which are kept: kept_graphs.py.
+        # The reference's GPU path keeps one prepared graph per step structure in the same way, at most 64 of them
         # (dynacore/include/dynacore/gpu/ggml_device.h:8-13,39-48).
         from ..kernels import ops as _ops
         self.use_graphs = bool(use_graphs) and model.graph_safe and not _ops.CHECKED     # a checked build reads a record after every launch
         self.portion_graphs = self.use_graphs and model.portions_graph_safe
-        self._graphs: Dict[tuple, torch.cuda.CUDAGraph] = {}
+        self._graphs = KeptGraphs({"decode": self.MAX_GRAPHS, "portions": self.MAX_PORTION_GRAPHS}, self.GRAPH_AFTER, self.SHAPES_KEPT)
         self._decode_logits: Optional[torch.Tensor] = None
         self.graph_kernel_launches = 0     # kernels replayed through graphs so far
-        self._graph_nodes: Dict[tuple, int] = {}
-        self._captured_logits: Dict[tuple, bool] = {}     # whether a captured step leaves logits (or only chosen ids)
-        self._shape_seen: Dict[tuple, int] = {}     # launch shape -> how often it has come (the SHAPES_KEPT last new ones)
+        self._shape_seen = self._graphs.seen
         self._capture_stream: Optional[torch.cuda.Stream] = None
         self.graph_captures = 0            # graphs captured so far, and the host time that took
         self.graph_capture_ms = 0.0
@@ -419,16 +418,13 @@ class StepFunction:
         self.batcher.finish(entries)
         return logits
 
-    def _capture(self, key: tuple, ctx: StepContext, out: Optional[torch.Tensor], choose=None) -> torch.cuda.CUDAGraph:
-        """The step's launches as a CUDA graph (nothing runs yet). Captured on a stream of its own between
+    def _capture(self, ctx: StepContext, out: Optional[torch.Tensor], choose=None) -> tuple:
+        """The step's launches as a CUDA graph (nothing runs yet), how many kernels it holds, and whether it leaves logits (or
+        only chosen ids). Captured on a stream of its own between
         capture_begin and capture_end, without the collection of garbage and the emptying of the allocator's
         cache that torch's context manager does first: nothing is allocated in here."""
         from ..kernels import ops
         started = time.perf_counter()
-        if len(self._graphs) >= self.MAX_GRAPHS:
-            old = next(iter(self._graphs))
-            del self._graphs[old]
-            self._graph_nodes.pop(old, None)
         if self._capture_stream is None:
             self._capture_stream = torch.cuda.Stream(device=self.rt.device)
         graph = torch.cuda.CUDAGraph()
@@ -438,15 +434,13 @@ class StepFunction:
         with torch.cuda.stream(self._capture_stream):
             graph.capture_begin()
             try:
-                self._captured_logits[key] = self._forward(ctx, out, choose) is not None
+                leaves_logits = self._forward(ctx, out, choose) is not None
             finally:
                 graph.capture_end()
         current.wait_stream(self._capture_stream)
-        self._graph_nodes[key] = ops.LAUNCHES - before
-        self._graphs[key] = graph
         self.graph_captures += 1
         self.graph_capture_ms += (time.perf_counter() - started) * 1e3
-        return graph
+        return graph, ops.LAUNCHES - before, leaves_logits
 
     def _plan_answers(self, ctx: StepContext) -> tuple:
         """What the step plans answered, as far as launches depend on it (a plan's `launch_key`; by default all of it)."""
@@ -462,7 +456,8 @@ class StepFunction:
         with ops.pinned_stream():
             return self.model.forward(ctx, self.caches(), out, choose)
 
-    MAX_GRAPHS = 64
+    MAX_GRAPHS = 64             # of steps of single tokens
+    MAX_PORTION_GRAPHS = 32     # of steps with prompt portions
     SHAPES_KEPT = 4096
     # A launch shape is captured when it comes for the eighth time. A capture costs 5 to 15 ms on the host; shapes
     # that pass by (the last requests of a batch ending one after the other: 64, 63, 62, ... rows for two steps
@@ -478,23 +473,19 @@ class StepFunction:
         # a graph holds the addresses it was captured with: the tensors of `choose` are part of its key
         chosen = None if choose is None else tuple(None if t is None else t.data_ptr() for t in choose)
         if ctx.decode_only:
-            key = (ctx.num_requests, ctx.num_logit_rows, chosen) + self.model.graph_key(ctx)
+            kind, key = "decode", (ctx.num_requests, ctx.num_logit_rows, chosen) + self.model.graph_key(ctx)
         else:
-            key = ("portions", tuple(ctx.h_q_len), ctx.num_logit_rows, chosen, self._plan_answers(ctx),
-                   max(256, 1 << (ctx.max_kv_len - 1).bit_length()))
+            kind, key = "portions", (tuple(ctx.h_q_len), ctx.num_logit_rows, chosen, self._plan_answers(ctx),
+                                     max(256, 1 << (ctx.max_kv_len - 1).bit_length()))
         out = self._decode_logits if ctx.num_logit_rows else None
-        graph = self._graphs.pop(key, None)
-        if graph is not None:
-            self._graphs[key] = graph          # the one used last goes last (`_capture` drops the first)
-        else:
-            seen = self._shape_seen.pop(key, 0) + 1
-            self._shape_seen[key] = seen
-            if len(self._shape_seen) > self.SHAPES_KEPT:
-                del self._shape_seen[next(iter(self._shape_seen))]
-            if seen < self.GRAPH_AFTER:
+        kept = self._graphs.use(kind, key)
+        if kept is None:
+            if not self._graphs.wants(kind, key):
                 got = self._forward(ctx, out, choose)
                 return got[:ctx.num_logit_rows] if got is not None else None
-            graph = self._capture(key, ctx, out, choose)
+            kept = self._capture(ctx, out, choose)
+            self._graphs.keep(kind, key, kept)
+        graph, kernels, leaves_logits = kept
         graph.replay()
-        self.graph_kernel_launches += self._graph_nodes[key]
-        return out[:ctx.num_logit_rows] if (out is not None and self._captured_logits[key]) else None
+        self.graph_kernel_launches += kernels
+        return out[:ctx.num_logit_rows] if (out is not None and leaves_logits) else None
