@@ -529,10 +529,10 @@ DL_EXPORT int dl_ssm_scan(int dtype, const void* u, int u_stride, const void* pr
   if (dtype != 0 && dtype != 1) return DL_ERR_UNSUPPORTED;
   DL_MODE(dl::SCAN_WHOLE, requests);
   // The matrix form takes bfloat16 inputs with 64 or 128 rows of state and channels a head, in whole runs of 16 bytes; other
-  // sizes and float32 inputs (whose terms would not be exact) are walked. Measured on B200 (64 heads of 64, 128 rows, 8 groups;
+  // sizes, float32 inputs (whose terms would not be exact) and segments that may be longer than its fixed arrays are walked. Measured on B200 (64 heads of 64, 128 rows, 8 groups;
   // prompts of 394 and 1,383 tokens; us a layer): first pass 41 against 167 walked, outputs 70 against 219; the carry between
   // them, with the segments' numbers asked for eight at a time, 21 against 39.
-  const bool matrices = dtype == 1 && (N == 64 || N == 128) && (P == 64 || P == 128) && u_stride % 8 == 0 &&
+  const bool matrices = dtype == 1 && (N == 64 || N == 128) && (P == 64 || P == 128) && whole_up_to <= dl::SEG_T && u_stride % 8 == 0 &&
                         (reinterpret_cast<uintptr_t>(u) & 15) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 &&
                         (reinterpret_cast<uintptr_t>(y) & 7) == 0;
 #define DL_SIZES(CALL)                                         \

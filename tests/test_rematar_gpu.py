@@ -373,6 +373,13 @@ def test_segments_in_matrix_form_keep_what_is_not_finite_behind_its_token(P, N):
         assert np.abs(got[fine] - ref[fine]).max() <= 2e-5 * max(1.0, np.abs(ref[fine]).max())
 
 
+def test_segments_longer_than_the_matrix_form_holds_are_walked(monkeypatch):
+    """The length of a segment is the step plan's; the matrix form's arrays end at 128 tokens."""
+    from dynalm_b200.kernels import ops
+    monkeypatch.setattr(ops, "SSM_SEGMENT", 160)
+    test_segments_in_matrix_form(2, 64, 64, 1)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gate_comes_before_the_norm_of_every_part(dtype):
     from dynalm_b200.kernels import ops
