@@ -54,10 +54,13 @@ class LatentExpandPlan:
     single tokens at the head of the step, the keys its rows may see, from a multiple of 16 on, as pieces of 16. On the
     device: per request slot what a key's position is added to for its row among the expanded ones, then int32 [pieces, 4] =
     (request slot, first key, keys, 0). `fill` returns the pieces, 0 when the step is to go the other way: no portions, one
-    of fewer than EXPAND_MIN_ROWS rows, or more keys than there is room for."""
+    of fewer than EXPAND_MIN_ROWS rows, or more keys than there is room for: 2 x the most tokens of a step + 2,048, as many as
+    the expanded keys and values have scratch for (6,144 keys take 50 MB with 16 heads where a step brings up to 2,048 tokens).
+    A layer without a window so goes back to the records once a prompt is longer than that."""
 
-    def __init__(self, window: int):
+    def __init__(self, window: int, max_requests: int = 0, max_tokens: int = 0):
         self.window = int(window)
+        self.max_requests, self.max_tokens = int(max_requests), int(max_tokens)
         self.name = f"latent_expand:{self.window}"
 
     @staticmethod
@@ -65,7 +68,8 @@ class LatentExpandPlan:
         return (2 * max_tokens + 2048) // 16
 
     def ints(self, max_tokens: int, max_requests: int) -> int:
-        return (max_requests + 3) // 4 * 4 + 4 * self.most_pieces(max_tokens)
+        # (the same in the buffers of small steps: which way a prompt goes must not change with the size of its portions)
+        return (max_requests + 3) // 4 * 4 + 4 * self.most_pieces(max(max_tokens, self.max_tokens))
 
     def fill(self, host, shape) -> tuple:
         requests = (self.max_requests + 3) // 4 * 4
@@ -106,15 +110,14 @@ EXPAND_SIZES = (128, 64, 128)      # (own numbers of a key, turned piece, values
 _expand_plans = {}
 
 
-def expand_plan(spec, max_requests: int):
+def expand_plan(spec, max_requests: int, max_tokens: int):
     """The plan for a layer of these sizes, or None where the tcgen05 kernel has no such sizes."""
     if (spec.head_dim, spec.rot_dim, spec.value_dim) != EXPAND_SIZES or spec.kv_rank % 8:
         return None
-    key = (int(spec.get("window", 0)), int(max_requests))
+    key = (int(spec.get("window", 0)), int(max_requests), int(max_tokens))
     plan = _expand_plans.get(key)
     if plan is None:
-        plan = _expand_plans[key] = LatentExpandPlan(key[0])
-        plan.max_requests = key[1]
+        plan = _expand_plans[key] = LatentExpandPlan(*key)
     return plan
 
 

@@ -92,7 +92,7 @@ class LatentAttention:
         from ..kernels import latent_attention as fast
         self.expand = None
         if self.rt.dtype == torch.bfloat16 and fast.flash_applies(spec, self.rt.dtype):
-            self.expand = fast.expand_plan(spec, runtime.max_requests)
+            self.expand = fast.expand_plan(spec, runtime.max_requests, runtime.max_tokens)
         self.w_kv = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self.expand is not None else None
         self.sink = tensors.get("sink")
         self.w_o = tensors["o"]

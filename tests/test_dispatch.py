@@ -3,6 +3,7 @@ kernels/attention.py on tensors that are never touched (no GPU needed)."""
 
 import os
 
+import numpy as np
 import torch
 
 from dynalm_b200.kernels import attention, gemm
@@ -195,3 +196,25 @@ def test_query_tile_parts_deal_long_tiles(monkeypatch):
                                                        len({(n, r) for _, n, r in got}) == 1)
     firsts = sorted(got[0][2] for got in seen.values() if got[0][1] > 1)
     assert firsts == list(range(0, records, 4))                                # records of the split tiles do not overlap
+
+
+def test_expanding_latents_depends_on_the_request_not_on_the_step_buffers():
+    """A portion's keys are worked out for the heads up to 2 x the most tokens of a step + 2,048 keys, in a step of few rows as in
+    a large one; beyond, and for portions of fewer rows than pay, the layer goes over the records."""
+    from dynalm_b200.engine.step import SMALL_STEP_ROWS, StepShape
+    from dynalm_b200.kernels import latent_attention as latent
+    from types import SimpleNamespace
+    spec = SimpleNamespace(head_dim=128, rot_dim=64, value_dim=128, kv_rank=512, get=lambda name, default=0: 0)
+    plan = latent.expand_plan(spec, 6, 2048)
+    small, large = (np.zeros(plan.ints(n, 6), dtype=np.int32) for n in (SMALL_STEP_ROWS, 2048))
+    room = 2 * 2048 + 2048
+    for rows in (latent.EXPAND_MIN_ROWS, 200):
+        for host in (small, large):
+            # two single tokens, then a portion that ends at the last key there is room for, or one behind it
+            within = StepShape([1, 1, rows], [0, 1, 2], [9, 9999, room - rows], [0, 1, 4], rows + 2)
+            beyond = StepShape([1, 1, rows], [0, 1, 2], [9, 9999, room - rows + 1], [0, 1, 4], rows + 2)
+            assert plan.fill(host, within) == (room // 16, 8) and plan.fill(host, beyond) == (0, 8)
+            assert host[4] == 0 and host[8:8 + 4].tolist() == [4, 0, 16, 0]
+            assert host[8 + 4 * (room // 16 - 1):8 + 4 * (room // 16)].tolist() == [4, room - 16, 16, 0]
+    short = StepShape([1, latent.EXPAND_MIN_ROWS - 1], [0, 1], [3, 100], [0, 1], latent.EXPAND_MIN_ROWS)
+    assert plan.fill(small, short)[0] == 0
