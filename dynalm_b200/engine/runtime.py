@@ -2,7 +2,7 @@
 
 from __future__ import annotations
 
-from typing import Dict, Tuple
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -44,6 +44,7 @@ class Runtime:
         self._buffers: Dict[Tuple, torch.Tensor] = {}
         self._views: Dict[Tuple, torch.Tensor] = {}      # (name, shape, dtype) -> the first rows of a buffer
         self._side_stream = None
+        self._refused = set()                            # what `spare` had no memory for
 
     @property
     def side_stream(self) -> int:
@@ -82,6 +83,17 @@ class Runtime:
         if buf.numel() < numel:
             raise InvalidArgument(f"scratch '{name}' was made for {buf.numel()} elements, {numel} are asked for")
         return buf
+
+    def spare(self, name: str, numel: int, dtype: torch.dtype = torch.float32) -> Optional[torch.Tensor]:
+        """`flat` for scratch that a step can do without: None where the device has no memory left for it (now and at every later
+        call, so that a model keeps to one way). The cache pool may take all but 5 % of the memory."""
+        if (name, dtype) in self._refused:
+            return None
+        try:
+            return self.flat(name, numel, dtype)
+        except torch.OutOfMemoryError:
+            self._refused.add((name, dtype))
+            return None
 
     def workspace_bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._buffers.values())

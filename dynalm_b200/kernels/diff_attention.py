@@ -83,11 +83,14 @@ def attend(q: torch.Tensor, cache, ctx, out: torch.Tensor, spec, lam: torch.Tens
     if leading > 0:
         _single(q, records, k_off, cache, ctx, out, spec, lam, out_scale, eps, runtime, leading)
         n_tiles = n_prompt_tiles
+    maps = None
     if n_tiles > 0 and (spec.head_dim, spec.value_dim) in ops.DIFF_TCGEN05_SIZES and cache.page_size >= 16 and \
             q.data_ptr() % 16 == 0 and float(spec.scale) > 0:
+        width = spec.num_heads * 2 * spec.value_dim
+        maps = runtime.spare(f"diff_maps_{width}", runtime.max_tokens * width)
+    if maps is not None:
         # a layer of 2,048 rows, 16:4 heads of 2 x 64 with values of 128: 88 us, both maps of a head in one block of the
         # mma.sync kernel 137
-        maps = runtime.buffer("diff_maps", (q.shape[0], spec.num_heads * 2 * spec.value_dim), torch.float32)
         ops.diff_attention_tcgen05(q, records, 0, k_off, cache.block_table, q_tiles, n_tiles, out, spec.num_heads,
                                    spec.num_kv_heads, spec.head_dim, spec.value_dim, cache.page_size, float(spec.scale),
                                    float(spec.get("softcap", 0.0)), lam, out_scale, eps, maps)

@@ -177,6 +177,11 @@ class LatentAttention:
         H, d, r, e, R = s.num_heads, s.head_dim, s.rot_dim, s.value_dim, s.kv_rank
         (records,) = cache.arrays
         ints, (pieces, first_piece) = planned
+        most = 16 * self.expand.most_pieces(rt.max_tokens)
+        latents = rt.spare(f"latent_rows_{R + r}", most * (R + r), torch.bfloat16)
+        kv = rt.spare(f"latent_kv_{H * (d + e)}", most * H * (d + e), torch.bfloat16) if latents is not None else None
+        if kv is None:
+            return False
         q_tiles, (_, n_tiles, lead) = tiles
         from ..kernels import attention
         side = rt.side_stream if lead > 0 and attention.SIDE_BY_SIDE else None
@@ -186,10 +191,9 @@ class LatentAttention:
                 self._absorbed(q, gate, cache, ctx, heads, lead, (q_tiles[4 * n_tiles:], lead))
         elif lead > 0:
             self._absorbed(q, gate, cache, ctx, heads, lead, (q_tiles[4 * n_tiles:], lead))
-        most = 16 * self.expand.most_pieces(rt.max_tokens)
         keys = 16 * pieces
-        latents = rt.flat(f"latent_rows_{R + r}", most * (R + r), torch.bfloat16)[:keys * (R + r)].view(keys, R + r)
-        kv = rt.flat(f"latent_kv_{H * (d + e)}", most * H * (d + e), torch.bfloat16)[:keys * H * (d + e)].view(keys, H * (d + e))
+        latents = latents[:keys * (R + r)].view(keys, R + r)
+        kv = kv[:keys * H * (d + e)].view(keys, H * (d + e))
         ops.latent_gather(records, cache.block_table, cache.page_size, ints[first_piece:], pieces, latents)
         linear_short(latents[:, :R], self.w_kv, kv)
         rows = q.shape[0]

@@ -218,3 +218,39 @@ def test_expanding_latents_depends_on_the_request_not_on_the_step_buffers():
             assert host[8 + 4 * (room // 16 - 1):8 + 4 * (room // 16)].tolist() == [4, room - 16, 16, 0]
     short = StepShape([1, latent.EXPAND_MIN_ROWS - 1], [0, 1], [3, 100], [0, 1], latent.EXPAND_MIN_ROWS)
     assert plan.fill(small, short)[0] == 0
+
+
+def test_scratch_that_a_step_can_do_without(monkeypatch):
+    """No memory for it: None, then and later, and nothing else of the runtime changes; else as `flat`."""
+    from dynalm_b200.engine.runtime import Runtime
+    rt = object.__new__(Runtime)
+    rt.device, rt._buffers, rt._refused = torch.device("cpu"), {}, set()
+    a = rt.spare("a", 100)
+    assert a.numel() == 100 and a.dtype == torch.float32 and rt.spare("a", 50) is a
+
+    def full(*args, **kwargs):
+        raise torch.OutOfMemoryError("full")
+    with monkeypatch.context() as m:
+        m.setattr(torch, "zeros", full)
+        assert rt.spare("b", 100, torch.bfloat16) is None and rt.spare("a", 100) is a
+    assert rt.spare("b", 100, torch.bfloat16) is None          # (memory is back, but the model has taken the other way)
+    assert rt.spare("b", 100) is not None and rt.workspace_bytes() == 800
+
+
+def test_prompts_without_scratch_for_the_faster_kernels_take_the_others(monkeypatch):
+    """Differential attention with no memory for its maps goes to the kernel that needs none."""
+    from types import SimpleNamespace
+    from dynalm_b200.kernels import diff_attention, ops
+    spec = SimpleNamespace(head_dim=64, value_dim=128, num_heads=4, num_kv_heads=2, scale=0.1, get=lambda name, default=0: default)
+    taken = []
+    monkeypatch.setattr(ops, "diff_attention_tcgen05", lambda *a: taken.append("tcgen05"))
+    monkeypatch.setattr(ops, "diff_attention_prefill", lambda *a: taken.append("mma.sync"))
+    q = torch.zeros(130, 4 * 2 * 64, dtype=torch.bfloat16)
+    out = torch.zeros(130, 4 * 128, dtype=torch.bfloat16)
+    cache = SimpleNamespace(arrays=(torch.zeros(9, 16, 512, dtype=torch.bfloat16),), page_size=16, block_table=None)
+    ctx = SimpleNamespace(decode_only=False, extras={"query_tiles": (torch.zeros(64, dtype=torch.int32), (2, 2, 0))})
+    monkeypatch.setattr(diff_attention, "query_tiles", lambda c: (torch.zeros(64, dtype=torch.int32), 2, 2, 0))
+    for room in (True, False):
+        rt = SimpleNamespace(max_tokens=256, spare=lambda name, n, dtype=None: torch.zeros(n) if room else None)
+        assert diff_attention.attend(q, cache, ctx, out, spec, None, 1.0, 1e-5, rt)
+    assert taken == ["tcgen05", "mma.sync"]

@@ -824,3 +824,25 @@ def test_portions_go_through_expanded_latents_and_back(monkeypatch):
         assert len(calls) == (4 if rows == 64 else 0)
     for a, b in zip(got[64], got[1 << 30]):
         assert (a - b).abs().max() <= 2e-2 * b.abs().max()
+
+
+def test_portions_whose_expanded_keys_have_no_memory_go_over_the_records(monkeypatch):
+    """The bits of a model that expands nothing."""
+    from dynalm_b200 import Engine, StepEntry
+    from dynalm_b200.engine.runtime import Runtime
+    from dynalm_b200.kernels import latent_attention as fast
+    lat = {"heads": 2, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 64, "kv_rank": 48, "scale": 0.07,
+           "rot": {"base": 10000.0, "dims": 64}, "mask": {"size": 150}}
+    cfg = {"architecture": "Rematar", "vocab": 300, "width": 128, "norm": {"eps": 1e-5}, "postln_alpha": 2.0, "embedding": {"scale": 8.0},
+           "layers": [{"type": "latent_attention", "mixer": dict(lat), "mlp": {"kind": "dense", "ff": 128}} for _ in range(2)]}
+    ids = torch.randint(0, 300, (400,), generator=torch.Generator().manual_seed(2)).tolist()
+    spare, got = Runtime.spare, []
+    for refused, rows in ((("latent_rows_112", "latent_kv_512"), 64), (("latent_kv_512",), 64), ((), 1 << 30)):
+        monkeypatch.setattr(Runtime, "spare", lambda rt, name, *a: None if name in refused else spare(rt, name, *a))
+        monkeypatch.setattr(fast, "EXPAND_MIN_ROWS", rows)
+        eng = Engine(config=cfg, random_seed=3, dtype="bfloat16", ctx=1024, batch=300, max_running=3)
+        out = [eng.step([StepEntry("a", ids[:200], [199]), StepEntry("b", ids[200:290], [0, 89])]).clone()]
+        out.append(eng.step([StepEntry("b", ids[290:291], [0]), StepEntry("a", ids[300:400], [50, 99])]).clone())
+        got.append(out)
+    for other in got[:2]:
+        assert all(torch.equal(a, b) for a, b in zip(other, got[2]))
