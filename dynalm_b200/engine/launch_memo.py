@@ -74,13 +74,15 @@ class _Layout:
 
 
 class _Record:
-    __slots__ = ("calls", "own", "library", "pending", "pending_scale", "pending2", "as_input", "streams", "parts", "gate", "via")
+    __slots__ = ("calls", "layout", "own", "library", "pending", "pending_scale", "pending2", "as_input", "streams", "parts", "gate", "via")
 
-    def __init__(self, calls, pending, pending_scale, pending2=None, as_input=None, streams=None, parts=1, gate=None, via=False):
-        # [(function, arguments, ((argument index, tensor index, offset or None for the tensor itself), ...))]
+    def __init__(self, calls, layout, pending, pending_scale, pending2=None, as_input=None, streams=None, parts=1, gate=None, via=False):
+        # [(function, arguments)], and with the layer that comes again (most kinds of a mixed model do not within a step) what
+        # `_patches` adds: ((argument index, tensor index, offset or None for the tensor itself), ...)
         self.calls = calls
-        self.library = sum(1 for f, _, _ in calls if f is ops.library_mm_again)
-        self.own = sum(1 for f, _, _ in calls if ops.counts_as_kernel(f))
+        self.layout = layout        # the recorded layer's; None: the patches are there
+        self.library = sum(1 for f, _ in calls if f is ops.library_mm_again)
+        self.own = sum(1 for f, _ in calls if ops.counts_as_kernel(f))
         self.pending = pending
         self.pending_scale = pending_scale
         self.pending2 = pending2
@@ -157,6 +159,8 @@ class LayerLaunchMemo:
             record = self.records[key]
             if record is None:
                 return block.forward(stream, ctx, cache, owns_cache)
+            if record.layout is not None:
+                record.calls, record.layout = _patches(record.calls, record.layout), None
             pointers, tensors = layout.pointers, layout.tensors
             for f, args, patch in record.calls:
                 if patch:
@@ -183,7 +187,7 @@ class LayerLaunchMemo:
         if any(f is None for f, _ in recording.calls):
             self.records[key] = None             # some work was not written down: this kind runs through its parts
         else:
-            self.records[key] = _Record(_patches(recording.calls, layout), stream.pending, stream.pending_scale,
+            self.records[key] = _Record(recording.calls, layout, stream.pending, stream.pending_scale,
                                         stream.pending2, stream.as_input, stream.streams, stream.parts, stream.gate,
                                         stream.via is not None)
         return stream

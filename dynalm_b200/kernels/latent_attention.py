@@ -20,6 +20,9 @@ from .device import sm_count
 UNITS = 32          # query units (row, head) to a block of the tensor-core kernel
 
 
+NUMPY_TILES = 64    # more tiles than this are worked out in numpy (two rows a tile: 258 rows 27 us against 54, 708 rows 33 against 142)
+
+
 def heads_per_block(heads: int) -> int:
     """Heads to a block: all of them up to 32, else the heads dealt evenly over the fewest blocks."""
     groups = -(-heads // UNITS)
@@ -39,6 +42,15 @@ class LatentTilePlan:
         return 4 * (max_tokens // self.rows + max_requests)
 
     def fill(self, host, shape) -> int:
+        if sum(shape.q_len) > NUMPY_TILES * self.rows:
+            n, r0, start, slot = (np.asarray(v, dtype=np.int32) for v in (shape.q_len, shape.q_start, shape.pos_start, shape.slots))
+            count = -(-n // self.rows)
+            of = np.repeat(np.arange(len(n)), count)
+            t0 = (np.arange(len(of), dtype=np.int32) - np.repeat(np.cumsum(count) - count, count)) * self.rows
+            rows, pos = np.minimum(self.rows, n[of] - t0), start[of] + t0
+            order = np.argsort(-(pos + rows), kind="stable")
+            host[:4 * len(of)].reshape(-1, 4)[:] = np.stack([slot[of], r0[of] + t0, rows, pos], axis=1)[order]
+            return len(of)
         tiles = []
         for n, r0, start, slot in zip(shape.q_len, shape.q_start, shape.pos_start, shape.slots):
             for t0 in range(0, n, self.rows):

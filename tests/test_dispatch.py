@@ -254,3 +254,21 @@ def test_prompts_without_scratch_for_the_faster_kernels_take_the_others(monkeypa
         rt = SimpleNamespace(max_tokens=256, spare=lambda name, n, dtype=None: torch.zeros(n) if room else None)
         assert diff_attention.attend(q, cache, ctx, out, spec, None, 1.0, 1e-5, rt)
     assert taken == ["tcgen05", "mma.sync"]
+
+
+def test_latent_tiles_are_the_same_from_numpy_and_from_a_loop(monkeypatch):
+    from dynalm_b200.engine.step import StepShape
+    from dynalm_b200.kernels import latent_attention as latent
+    rng = np.random.RandomState(4)
+    for rows in (1, 2, 3, 32):
+        plan = latent.LatentTilePlan(rows)
+        for lens in ([1] * 9, [1, 1, 300], [2, 1, 130, 1, 64], [2048], [5], [33, 32, 31, 1]):
+            first = np.cumsum([0] + lens)
+            shape = StepShape(lens, first[:-1].tolist(), rng.randint(0, 5000, len(lens)).tolist(), rng.permutation(90)[:len(lens)].tolist(),
+                              int(first[-1]))
+            hosts = []
+            for most in (0, 1 << 30):
+                monkeypatch.setattr(latent, "NUMPY_TILES", most)
+                hosts.append(np.full(plan.ints(shape.num_tokens, 9), -7, dtype=np.int32))
+                assert plan.fill(hosts[-1], shape) == sum(-(-n // rows) for n in lens)
+            assert (hosts[0] == hosts[1]).all()
