@@ -1354,9 +1354,9 @@ def paged_attention_prefill_tcgen05(q: torch.Tensor, k_cache: torch.Tensor, v_ca
     128, pages of at least 16 keys; see csrc/attention_prefill_tcgen05.cu. Arguments as paged_attention_prefill.
 
     unit_parts: int32 [n_tiles], when the keys of some tiles are dealt over several entries of q_tiles (see
-    kernels/attention.QueryTileParts): part | parts << 8 | scratch slot << 16 per entry, 0 = whole. chunk, sink: as
-    masked_flash_attention's. Then partial:
-    float32, (slots in use) * n_heads * (head_dim + 2) * 128 elements; counters: int32, (slots in use) * n_heads, zero."""
+    kernels/attention.QueryTileParts): part | parts << 8 | scratch slot << 16 per entry, 0 = whole. Then partial:
+    float32, (slots in use) * n_heads * (head_dim + 2) * 128 elements; counters: int32, (slots in use) * n_heads, zero.
+    chunk, sink: as masked_flash_attention's."""
     _cuda(q, k_cache, v_cache, block_table, q_tiles, out, unit_parts, partial, counters)
     _rows_contiguous(q, "q")
     _rows_contiguous(out, "out")

@@ -870,6 +870,35 @@ def test_paged_attention_prefill_tcgen05_chunks_and_sink(ops, heads, kvh, hd, pa
     assert (out.float() - ref).abs().max().item() <= 1.1 * 2 * 2 ** -9 * largest
 
 
+@pytest.mark.parametrize("heads,kvh,hd,page,window,chunk", [(4, 2, 64, 16, 0, 0), (2, 1, 128, 32, 0, 300), (4, 4, 64, 16, 500, 0)])
+def test_paged_attention_prefill_tcgen05_sink_with_dealt_keys(ops, heads, kvh, hd, page, window, chunk):
+    """The sink joins where the parts of a tile's keys are added up, once. Bound as above."""
+    g = torch.Generator(device="cpu").manual_seed(29)
+    cache, table, tiles, n_tiles, req, pos = _portions(g, kvh * hd, page, [60, 900, 131], torch.bfloat16)
+    kc = cache.view(-1, page, kvh, hd)
+    vc = torch.randn(kc.shape, generator=g).to(torch.bfloat16).to(DEV)
+    n = pos.numel()
+    q = torch.randn(n, heads * hd, generator=g).to(torch.bfloat16).to(DEV)
+    entries, words, record = [], [], 0
+    for i, t in enumerate(tiles.view(-1, 4).tolist()):
+        parts = (3, 2, 1, 1, 2, 1, 2)[i]
+        for p in range(parts):
+            entries.append(t)
+            words.append(0 if parts == 1 else (p | parts << 8 | record << 16))
+        record += parts if parts > 1 else 0
+    partial = torch.full((record * heads * (hd + 2) * 128,), float("nan"), device=DEV)
+    counters = torch.zeros(record * heads, dtype=torch.int32, device=DEV)
+    out = torch.empty(n, heads * hd, dtype=torch.bfloat16, device=DEV)
+    ops.paged_attention_prefill_tcgen05(q, kc, vc, table, torch.tensor(entries, dtype=torch.int32, device=DEV).view(-1), len(entries), out,
+                                        heads, kvh, hd, page, hd ** -0.5, window, unit_parts=torch.tensor(words, dtype=torch.int32, device=DEV),
+                                        partial=partial, counters=counters, chunk=chunk, sink=True)
+    assert ops.gemm_tcgen05_status() == 0
+    ref = torch.empty(n, heads * hd, device=DEV)
+    ops.paged_attention_generic_kv(q.float(), kc.float(), kvh * hd, vc.float(), kvh * hd, table, pos, req, ref, heads, kvh, hd, hd,
+                                   page, hd ** -0.5, window, 0, True, chunk=chunk)
+    assert (out.float() - ref).abs().max().item() <= 1.1 * 2 * 2 ** -9 * vc.abs().max().item()
+
+
 @pytest.mark.parametrize("heads,groups,dim,vdim,page,cap", [(4, 2, 64, 64, 16, 0.0), (6, 2, 64, 128, 32, 3.0), (2, 2, 128, 128, 16, 30.0),
                                                             (3, 1, 64, 128, 16, 0.0)])
 def test_diff_attention_tcgen05(ops, heads, groups, dim, vdim, page, cap):
