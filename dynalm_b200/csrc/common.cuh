@@ -10,6 +10,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #define DL_EXPORT extern "C" __attribute__((visibility("default")))
 
 // Return code for "this size is not supported by the kernel" (never a wrong result).
@@ -160,6 +162,19 @@ __device__ __forceinline__ float clamped_swiglu_bf16(float g, float u, float lim
 constexpr int CLAMPED_HEADER = 4;
 
 inline int launch_status() { return static_cast<int>(cudaGetLastError()); }
+
+// SMs of the current device, and of B200 where that cannot be read.
+inline int sm_count() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0)
+      n = 148;
+    known.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 
 // Programmatic dependent launch. A kernel launched with the attribute may begin while the kernel before it on
 // the stream is still running; it must call pdl_wait() before it reads anything an earlier kernel wrote and

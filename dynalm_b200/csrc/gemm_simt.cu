@@ -355,7 +355,7 @@ DL_EXPORT int dl_gemm_simt(int in_dtype, int out_dtype, const void* x, int ldx, 
   // four blocks an SM. Measured, groups / tiles, us: 64 x 2048 x 2048 41 / 45, 48 x 3072 x 2048 41 / 46, 64 x 3072 x 2048 57 /
   // 45, 32 x 2048 x 8192 66 / 143, 32 x 16384 x 2048 125 / 119; 16 x 128256 x 2048 461 / 735.
   const long long row_blocks = static_cast<long long>((N + dl::RF - 1) / dl::RF) * ((M + 15) / 16);
-  if (aligned && out_dtype == 0 && (M <= 16 || (M <= 64 && row_blocks <= 4 * 148))) {
+  if (aligned && out_dtype == 0 && (M <= 16 || (M <= 64 && row_blocks <= 4 * dl::sm_count()))) {
     const float* xf = static_cast<const float*>(x);
     const float* wf = static_cast<const float*>(w);
     float* yf = static_cast<float*>(y);
@@ -367,11 +367,12 @@ DL_EXPORT int dl_gemm_simt(int in_dtype, int out_dtype, const void* x, int ldx, 
     DL_ROWS(16);
 #undef DL_ROWS
   }
-  // Tiles of 128 rows or of 64, by the rounds of blocks over the SMs (148, of which clusters of four leave a few idle): an SM
+  // Tiles of 128 rows or of 64, by the rounds of blocks over the SMs (of 148, clusters of four fill 140): an SM
   // takes about 33 us for every block of 64 rows and 50 for one of 128 that it gets, at k 2048. Measured, 64 / 128, us: 128 x
   // 2048 x 2048 46 / 69, 128 x 16384 x 2048 237 / 218, 300 x 3072 x 2048 131 / 159, 700 x 2048 x 2048 181 / 162, 1000 x 16384
   // x 2048 1,656 / 1,382.
-  auto rounds = [&](int rows) { return (4ll * ((N + dl::BN - 1) / dl::BN) * ((M + rows - 1) / rows) + 139) / 140; };
+  const long long filled = (dl::sm_count() * 35ll + 36) / 37;
+  auto rounds = [&](int rows) { return (4ll * ((N + dl::BN - 1) / dl::BN) * ((M + rows - 1) / rows) + filled - 1) / filled; };
   const bool tall = 50 * rounds(128) < 33 * rounds(64);
 #define DL_LAUNCH(TI, TO)                                                                                              \
   return tall ? dl::launch_tiles<TI, TO, 128, 16>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, aligned, stream)        \

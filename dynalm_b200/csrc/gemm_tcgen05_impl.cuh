@@ -507,22 +507,6 @@ static inline int make_map(CUtensorMap* map, const void* base, int rows, int col
 
 }  // namespace dl
 
-// x: bf16 [M, K] rows of ldx elements; w: bf16 [N, K] contiguous; both 16-byte aligned with K and ldx multiples of 8.
-// mode 0: y bf16 [M, N] (N % 8 == 0); mode 1: y fp32 [M, N] (N % 4 == 0); mode 2: w = [gate; up] with N = 2F rows,
-// y bf16 [M, F] = silu(x Wg^T) * (x Wu^T) (F % 8 == 0), or with coeffs (N + 4 float32, 16-byte aligned: common.cuh,
-// CLAMPED_HEADER) the gated activation with clamped halves and biases; mode 4: y bf16 [M, N] = max(x W^T, 0)^2; mode 5: = gelu_tanh(x W^T);
-// mode 7: = xIELU(x W^T) with coeffs = two float32 on the device. status: one device int, set to a nonzero code if a wait
-// inside the kernel timed out (left untouched otherwise).
-static int t5_sm_count() {
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0) sm_count = 148;
-  }
-  return sm_count;
-}
-
 // What a slice of 64 k takes a round of tiles of bn columns, of blocks alone or of pairs, in us: from products of 543 to 2,048
 // rows by 2,048 or 3,072 features, between K 2048 and K 8192, on B200. At 35 products from 64 to 2,048 rows the width and kind
 // with the least rounds x cost is the fastest measured or within 5 % of it. Against blocks alone at 256, 192 or 128 columns,
@@ -587,6 +571,12 @@ static int t5_run(cudaLaunchConfig_t cfg, const CUtensorMap& map_x, const CUtens
                                              gate_rows, tiles_n, tiles, group_m, status, rope, groups, coeffs, bn));
 }
 
+// x: bf16 [M, K] rows of ldx elements; w: bf16 [N, K] contiguous; both 16-byte aligned with K and ldx multiples of 8.
+// mode 0: y bf16 [M, N] (N % 8 == 0); mode 1: y fp32 [M, N] (N % 4 == 0); mode 2: w = [gate; up] with N = 2F rows,
+// y bf16 [M, F] = silu(x Wg^T) * (x Wu^T) (F % 8 == 0), or with coeffs (N + 4 float32, 16-byte aligned: common.cuh,
+// CLAMPED_HEADER) the gated activation with clamped halves and biases; mode 4: y bf16 [M, N] = max(x W^T, 0)^2; mode 5: = gelu_tanh(x W^T);
+// mode 7: = xIELU(x W^T) with coeffs = two float32 on the device. status: one device int, set to a nonzero code if a wait
+// inside the kernel timed out (left untouched otherwise).
 static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, int mode, float out_scale,
                      int* status, const dl::QkvRope& rope, int pairs, cudaStream_t stream, const float* coeffs = nullptr) {
   if (M <= 0 || N <= 0) return 0;
@@ -598,7 +588,7 @@ static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, in
   if ((mode == dl::T5_OUT_SWIGLU && (N & 1)) || (mode == dl::T5_OUT_F32 ? (feats & 3) || (ldy & 3) : (feats & 7) || (ldy & 7)) ||
       (reinterpret_cast<uintptr_t>(y) & 15))
     return DL_ERR_UNSUPPORTED;
-  const int sms = t5_sm_count();
+  const int sms = dl::sm_count();
   const long long m_blocks = (M + dl::T5_BM - 1) / dl::T5_BM;
   const T5Choice choice = t5_choose(m_blocks, feats, mode, rope.head_dim, sms, pairs);
   const int cluster = choice.pair ? 2 : 1, bn = choice.bn;
@@ -675,7 +665,7 @@ static int t5_launch_grouped(const void* a, int lda, int rows, const void* w, in
   rc = dl::make_map(&map_w, w, matrices * N, K, K, bn / 2);
   if (rc != 0) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(most < t5_sm_count() ? most : t5_sm_count()));
+  cfg.gridDim = dim3(static_cast<unsigned>(most < dl::sm_count() ? most : dl::sm_count()));
   cfg.blockDim = dim3(dl::T5_THREADS);
   cfg.stream = stream;
   const dl::QkvRope none = {};
