@@ -11,8 +11,12 @@
 //
 // ssm_added_kernel: block = (segment, head), a warp 16 rows of the state. ssm_outputs_kernel: block = (segment, head), a warp
 // 16 tokens: C S_start first, then over the tokens up to its own in steps of 16 the scores C B^T (from registers to
-// registers, as in a flash attention: a score tile's accumulator is the next product's left operand). Both are bound by the
-// mma.sync pipe and the conversions, no longer by a chain over the tokens.
+// registers, as in a flash attention: a score tile's accumulator is the next product's left operand). No chain over the tokens is
+// left; a block's loads, conversions and products follow one another, and two blocks an SM hide little of that (the tensor pipe
+// is busy a quarter of the time, warps wait for memory most of it).
+//
+// A token's numbers reach itself and the tokens behind it alone, infinities and NaNs among them: runs of sixteen tokens with such
+// an x are added token by token (ssm_outputs_kernel).
 //
 // Both passes of the walk in ssm.cu issue five multiply-adds per number of the state and token; here it is about two and a half,
 // three times over, on the tensor pipe. Figures at the launch rule in ssm.cu.
@@ -158,7 +162,6 @@ ssm_outputs_kernel(const bf16* __restrict__ u, int u_stride, const bf16* __restr
                    const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                    const int* __restrict__ segments, const float* __restrict__ scratch, float* __restrict__ y, int H, int G) {
   constexpr int BS = N + 8, XS = P + 8;
-  constexpr int START = (3 * N * XS > SEG_T * BS ? 3 * N * XS : SEG_T * BS);
   extern __shared__ __align__(16) unsigned char seg_smem[];
   bf16* sb = reinterpret_cast<bf16*>(seg_smem);       // [SEG_T][BS]
   bf16* sx = sb + SEG_T * BS;                         // [SEG_T][XS]
@@ -166,7 +169,6 @@ ssm_outputs_kernel(const bf16* __restrict__ u, int u_stride, const bf16* __restr
   __shared__ float4 at[SEG_T];
   __shared__ double warp_sums[SEG_T / 32];
   __shared__ unsigned not_finite;                     // bit i: of the tokens 16 i .. 16 i + 15 one has an x that is not finite
-  static_assert(START > 0, "");
   const int4 seg = reinterpret_cast<const int4*>(segments)[blockIdx.x];
   const int h = blockIdx.y, g = h / (H / G), r0 = seg.y, n = seg.z, inner = H * P, tid = threadIdx.x;
   for (int e = tid; e < SEG_T * (N / 8); e += 256) {
@@ -332,8 +334,9 @@ template <int N, int P>
 int launch_outputs(const bf16* u, int u_stride, const bf16* proj, int proj_stride, int dt_col, const float* dt_bias,
                    const float* a_log, const float* d_skip, const int* segments, int n_segments, const float* scratch, float* y,
                    int H, int G, cudaStream_t stream) {
-  constexpr int START = (3 * N * (P + 8) > SEG_T * (N + 8) ? 3 * N * (P + 8) : SEG_T * (N + 8));
-  constexpr int SMEM = (SEG_T * (N + 8) + SEG_T * (P + 8) + START) * 2;
+  constexpr int SHARED_PLACE = 3 * N * (P + 8) > SEG_T * (N + 8) ? 3 * N * (P + 8) : SEG_T * (N + 8);      // C, then the start state
+  constexpr int SMEM = (SEG_T * (N + 8) + SEG_T * (P + 8) + SHARED_PLACE) * 2;
+  static_assert(SMEM + 4096 <= 232448, "with the static arrays within the 227 KiB of a block");
   const cudaError_t e = cudaFuncSetAttribute(ssm_outputs_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   ssm_outputs_kernel<N, P><<<dim3(n_segments, H), 256, SMEM, stream>>>(u, u_stride, proj, proj_stride, dt_col, dt_bias, a_log,
