@@ -123,8 +123,9 @@ _expand_plans = {}
 
 
 def expand_plan(spec, max_requests: int, max_tokens: int):
-    """The plan for a layer of these sizes, or None where the tcgen05 kernel has no such sizes."""
-    if (spec.head_dim, spec.rot_dim, spec.value_dim) != EXPAND_SIZES or spec.kv_rank % 8:
+    """The plan for a layer of these sizes, or None where the tcgen05 kernel has no such sizes, or not its scale: it takes a row's
+    largest score before it scales the scores, the kernel over the records after."""
+    if (spec.head_dim, spec.rot_dim, spec.value_dim) != EXPAND_SIZES or spec.kv_rank % 8 or not float(spec.scale) > 0:
         return None
     key = (int(spec.get("window", 0)), int(max_requests), int(max_tokens))
     plan = _expand_plans.get(key)

@@ -204,7 +204,7 @@ def test_expanding_latents_depends_on_the_request_not_on_the_step_buffers():
     from dynalm_b200.engine.step import SMALL_STEP_ROWS, StepShape
     from dynalm_b200.kernels import latent_attention as latent
     from types import SimpleNamespace
-    spec = SimpleNamespace(head_dim=128, rot_dim=64, value_dim=128, kv_rank=512, get=lambda name, default=0: 0)
+    spec = SimpleNamespace(head_dim=128, rot_dim=64, value_dim=128, kv_rank=512, scale=0.1, get=lambda name, default=0: 0)
     plan = latent.expand_plan(spec, 6, 2048)
     small, large = (np.zeros(plan.ints(n, 6), dtype=np.int32) for n in (SMALL_STEP_ROWS, 2048))
     room = 2 * 2048 + 2048
@@ -272,3 +272,12 @@ def test_latent_tiles_are_the_same_from_numpy_and_from_a_loop(monkeypatch):
                 hosts.append(np.full(plan.ints(shape.num_tokens, 9), -7, dtype=np.int32))
                 assert plan.fill(hosts[-1], shape) == sum(-(-n // rows) for n in lens)
             assert (hosts[0] == hosts[1]).all()
+
+
+def test_latents_with_a_scale_that_is_not_positive_go_over_the_records():
+    """Two designs read any scale; the kernel over expanded keys and values refuses one that is not positive."""
+    from types import SimpleNamespace
+    from dynalm_b200.kernels import latent_attention as latent
+    for scale, expanded in ((0.07, True), (0.0, False), (-0.07, False)):
+        spec = SimpleNamespace(head_dim=128, rot_dim=64, value_dim=128, kv_rank=48, scale=scale, get=lambda name, default=0: default)
+        assert (latent.expand_plan(spec, 4, 512) is not None) == expanded
