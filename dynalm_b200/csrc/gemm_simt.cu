@@ -33,6 +33,8 @@
 
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 namespace dl {
 
 namespace cg = cooperative_groups;
@@ -163,8 +165,9 @@ __device__ __forceinline__ unsigned long long twice(float a) {
 constexpr int BN = 128;
 
 // BM x 128 outputs, 8 x TN a thread (BM 128: TN 16; BM 64: TN 8), 128 threads; `wide`: four numbers of a row of x and of W may
-// be loaded at once. A quarter of k for each of the cluster's QUARTERS blocks.
-template <typename TX, typename TO, int BM, int TN>
+// be loaded at once. A quarter of k for each of the CL blocks of a cluster: QUARTERS, or one where k has no more than a quarter (up
+// to 128: 1,000 x 499 x 80 float32 took 20.3 us with three blocks of four that had nothing to do, 11.0 without).
+template <typename TX, typename TO, int BM, int TN, int CL>
 __global__ void __launch_bounds__(128, 2)
 gemm_tile_kernel(const TX* __restrict__ x, int ldx, const TX* __restrict__ w, const float* __restrict__ bias,
                  TO* __restrict__ y, int ldy, int M, int N, int K, float out_scale, int wide) {
@@ -176,40 +179,79 @@ gemm_tile_kernel(const TX* __restrict__ x, int ldx, const TX* __restrict__ w, co
   float* ws = xs + 2 * TK * XS;                       // [2][TK][WS]
   float* quarter = ws + 2 * TK * WS;                  // [8 TN][THREADS]: the running quarter
   const int tid = threadIdx.x;
-  const int part = blockIdx.x % QUARTERS;
-  const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / QUARTERS) * BN;
+  const int part = blockIdx.x % CL;
+  const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / CL) * BN;
   const int tm = tid / COLS * 4, tn = tid % COLS * 4;    // rows tm.. and BM/2 + tm.., columns tn + 4 COLS j ..
   const int span = span_length(K), quarter_k = span * (SPANS / QUARTERS);
   const int k_begin = part * quarter_k, k_end = min(K, k_begin + quarter_k);
 
+  // the next tile's numbers on their way: float32, or bfloat16 as they lie, which are converted only when they are kept (with the
+  // conversion beside the load every run waited for its own: 40 x 499 x 80 15.0 us, now 11.3)
   float xv[XV][4], wv[WV][4];
+  ushort4 xh[XV], wh[WV];
   auto fetch = [&](int k0) {
+    if constexpr (sizeof(TX) == 2) {
+      auto run = [&](ushort4& v, const TX* base, int ld, int row, int rows, int e, bool at_once) {
+        const int k = k0 + e % (TK / 4) * 4, there = row < rows ? K - k : 0;
+        const TX* p = base + static_cast<size_t>(row) * ld + k;
+        v = make_ushort4(0, 0, 0, 0);
+        if (at_once) {                                  // (K is a multiple of four)
+          if (there > 0) v = *reinterpret_cast<const ushort4*>(p);
+        } else {
+          const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+          if (there > 0) v.x = q[0];
+          if (there > 1) v.y = q[1];
+          if (there > 2) v.z = q[2];
+          if (there > 3) v.w = q[3];
+        }
+      };
+      auto all = [&](auto at_once) {
+        constexpr bool O = decltype(at_once)::value;
 #pragma unroll
-    for (int i = 0; i < XV; ++i) {
-      const int e = i * THREADS + tid, k = k0 + (e % (TK / 4)) * 4, m = m0 + e / (TK / 4);
-      const TX* p = x + static_cast<size_t>(m) * ldx + k;
-      if (sizeof(TX) == 4 && wide && m < M && k + 3 < K) {
-        const float4 v = *reinterpret_cast<const float4*>(p);
-        xv[i][0] = v.x, xv[i][1] = v.y, xv[i][2] = v.z, xv[i][3] = v.w;
-      } else {
+        for (int i = 0; i < XV; ++i) run(xh[i], x, ldx, m0 + (i * THREADS + tid) / (TK / 4), M, i * THREADS + tid, O);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) xv[i][j] = (m < M && k + j < K) ? to_float(p[j]) : 0.0f;
+        for (int i = 0; i < WV; ++i) run(wh[i], w, K, n0 + (i * THREADS + tid) / (TK / 4), N, i * THREADS + tid, O);
+      };
+      if (wide) all(std::true_type());
+      else all(std::false_type());
+    } else {
+#pragma unroll
+      for (int i = 0; i < XV; ++i) {
+        const int e = i * THREADS + tid, k = k0 + (e % (TK / 4)) * 4, m = m0 + e / (TK / 4);
+        const TX* p = x + static_cast<size_t>(m) * ldx + k;
+        if (wide && m < M && k + 3 < K) {
+          const float4 v = *reinterpret_cast<const float4*>(p);
+          xv[i][0] = v.x, xv[i][1] = v.y, xv[i][2] = v.z, xv[i][3] = v.w;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) xv[i][j] = (m < M && k + j < K) ? to_float(p[j]) : 0.0f;
+        }
       }
-    }
 #pragma unroll
-    for (int i = 0; i < WV; ++i) {
-      const int e = i * THREADS + tid, k = k0 + (e % (TK / 4)) * 4, n = n0 + e / (TK / 4);
-      const TX* p = w + static_cast<size_t>(n) * K + k;
-      if (sizeof(TX) == 4 && wide && n < N && k + 3 < K) {
-        const float4 v = *reinterpret_cast<const float4*>(p);
-        wv[i][0] = v.x, wv[i][1] = v.y, wv[i][2] = v.z, wv[i][3] = v.w;
-      } else {
+      for (int i = 0; i < WV; ++i) {
+        const int e = i * THREADS + tid, k = k0 + (e % (TK / 4)) * 4, n = n0 + e / (TK / 4);
+        const TX* p = w + static_cast<size_t>(n) * K + k;
+        if (wide && n < N && k + 3 < K) {
+          const float4 v = *reinterpret_cast<const float4*>(p);
+          wv[i][0] = v.x, wv[i][1] = v.y, wv[i][2] = v.z, wv[i][3] = v.w;
+        } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) wv[i][j] = (n < N && k + j < K) ? to_float(p[j]) : 0.0f;
+          for (int j = 0; j < 4; ++j) wv[i][j] = (n < N && k + j < K) ? to_float(p[j]) : 0.0f;
+        }
       }
     }
   };
   auto keep = [&](int buf) {
+    if constexpr (sizeof(TX) == 2) {
+      auto numbers = [](float (&v)[4], const ushort4& h) {
+        v[0] = __bfloat162float(__ushort_as_bfloat16(h.x)), v[1] = __bfloat162float(__ushort_as_bfloat16(h.y));
+        v[2] = __bfloat162float(__ushort_as_bfloat16(h.z)), v[3] = __bfloat162float(__ushort_as_bfloat16(h.w));
+      };
+#pragma unroll
+      for (int i = 0; i < XV; ++i) numbers(xv[i], xh[i]);
+#pragma unroll
+      for (int i = 0; i < WV; ++i) numbers(wv[i], wh[i]);
+    }
 #pragma unroll
     for (int i = 0; i < XV; ++i) {
       const int e = i * THREADS + tid, k = (e % (TK / 4)) * 4, r = e / (TK / 4);
@@ -281,20 +323,20 @@ gemm_tile_kernel(const TX* __restrict__ x, int ldx, const TX* __restrict__ w, co
 
   // every block of the cluster adds up the quarters of a share of the outputs
   cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  const int have = min(QUARTERS, (K + quarter_k - 1) / quarter_k);      // quarters that hold any k
-  const float* theirs[QUARTERS];
+  if constexpr (CL > 1) cluster.sync();
+  const int have = min(CL, (K + quarter_k - 1) / quarter_k);      // quarters that hold any k
+  const float* theirs[CL];
 #pragma unroll
-  for (int q = 0; q < QUARTERS; ++q) theirs[q] = cluster.map_shared_rank(quarter, q);
+  for (int q = 0; q < CL; ++q) theirs[q] = CL > 1 ? cluster.map_shared_rank(quarter, q) : quarter;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    if (i % QUARTERS != part) continue;
+    if (i % CL != part) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int at = (i * TN + j) * THREADS + tid;
       float v = theirs[0][at];
 #pragma unroll
-      for (int q = 1; q < QUARTERS; ++q)
+      for (int q = 1; q < CL; ++q)
         if (q < have) v += theirs[q][at];
       const int m = m0 + (i < 4 ? tm + i : BM / 2 + tm + i - 4), n = n0 + tn + j / 4 * 4 * COLS + j % 4;
       if (m < M && n < N) {
@@ -303,29 +345,29 @@ gemm_tile_kernel(const TX* __restrict__ x, int ldx, const TX* __restrict__ w, co
       }
     }
   }
-  cluster.sync();                                       // nobody leaves while its quarter is being read
+  if constexpr (CL > 1) cluster.sync();                 // nobody leaves while its quarter is being read
 }
 
-template <typename TX, typename TO, int BM, int TN>
+template <typename TX, typename TO, int BM, int TN, int CL>
 int launch_tiles(const void* x, int ldx, const void* w, const float* bias, void* y, int ldy, int M, int N, int K,
                  float out_scale, int wide, cudaStream_t stream) {
   constexpr int THREADS = 128;
   constexpr int SMEM = (2 * TK * (BM + 4 + BN + 4) + 8 * TN * THREADS) * 4;
-  auto kernel = gemm_tile_kernel<TX, TO, BM, TN>;
+  auto kernel = gemm_tile_kernel<TX, TO, BM, TN, CL>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((N + BN - 1) / BN * QUARTERS, (M + BM - 1) / BM, 1);
+  cfg.gridDim = dim3((N + BN - 1) / BN * CL, (M + BM - 1) / BM, 1);
   cfg.blockDim = THREADS;
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = QUARTERS;
+  attr[0].val.clusterDim.x = CL;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, static_cast<const TX*>(x), ldx, static_cast<const TX*>(w), bias,
                                              static_cast<TO*>(y), ldy, M, N, K, out_scale, wide));
 }
@@ -349,13 +391,14 @@ DL_EXPORT int dl_gemm_simt(int in_dtype, int out_dtype, const void* x, int ldx, 
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return DL_ERR_UNSUPPORTED;
   if ((M + 63) / 64 > 65535) return DL_ERR_UNSUPPORTED;
-  const bool aligned = in_dtype == 0 && K % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-                       (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+  // four numbers of a row at once: 16 bytes of float32, 8 of bfloat16
+  const bool aligned = K % 4 == 0 && ldx % 4 == 0 &&
+                       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & (in_dtype == 0 ? 15 : 7)) == 0;
   // The few-row kernel up to 16 rows, and for narrow products of up to 64 rows in groups of 16 that share W in L2, up to about
   // four blocks an SM. Measured, groups / tiles, us: 64 x 2048 x 2048 41 / 45, 48 x 3072 x 2048 41 / 46, 64 x 3072 x 2048 57 /
   // 45, 32 x 2048 x 8192 66 / 143, 32 x 16384 x 2048 125 / 119; 16 x 128256 x 2048 461 / 735.
   const long long row_blocks = static_cast<long long>((N + dl::RF - 1) / dl::RF) * ((M + 15) / 16);
-  if (aligned && out_dtype == 0 && (M <= 16 || (M <= 64 && row_blocks <= 4 * dl::sm_count()))) {
+  if (aligned && in_dtype == 0 && out_dtype == 0 && (M <= 16 || (M <= 64 && row_blocks <= 4 * dl::sm_count()))) {
     const float* xf = static_cast<const float*>(x);
     const float* wf = static_cast<const float*>(w);
     float* yf = static_cast<float*>(y);
@@ -371,15 +414,22 @@ DL_EXPORT int dl_gemm_simt(int in_dtype, int out_dtype, const void* x, int ldx, 
   // takes about 33 us for every block of 64 rows and 50 for one of 128 that it gets, at k 2048. Measured, 64 / 128, us: 128 x
   // 2048 x 2048 46 / 69, 128 x 16384 x 2048 237 / 218, 300 x 3072 x 2048 131 / 159, 700 x 2048 x 2048 181 / 162, 1000 x 16384
   // x 2048 1,656 / 1,382.
-  const long long filled = (dl::sm_count() * 35ll + 36) / 37;
-  auto rounds = [&](int rows) { return (4ll * ((N + dl::BN - 1) / dl::BN) * ((M + rows - 1) / rows) + filled - 1) / filled; };
+  const bool alone = K <= dl::span_length(K) * (dl::SPANS / dl::QUARTERS);
+  const long long blocks = alone ? 1 : dl::QUARTERS, filled = alone ? dl::sm_count() : (dl::sm_count() * 35ll + 36) / 37;
+  auto rounds = [&](int rows) { return (blocks * ((N + dl::BN - 1) / dl::BN) * ((M + rows - 1) / rows) + filled - 1) / filled; };
   const bool tall = 50 * rounds(128) < 33 * rounds(64);
-#define DL_LAUNCH(TI, TO)                                                                                              \
-  return tall ? dl::launch_tiles<TI, TO, 128, 16>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, aligned, stream)        \
-              : dl::launch_tiles<TI, TO, 64, 8>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, aligned, stream)
+#define DL_TILES(TI, TO, CL)                                                                                           \
+  return tall ? dl::launch_tiles<TI, TO, 128, 16, CL>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, aligned, stream)    \
+              : dl::launch_tiles<TI, TO, 64, 8, CL>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, aligned, stream)
+#define DL_LAUNCH(TI, TO)                       \
+  do {                                          \
+    if (alone) DL_TILES(TI, TO, 1);             \
+    DL_TILES(TI, TO, dl::QUARTERS);             \
+  } while (0)
   if (in_dtype == 0 && out_dtype == 0) DL_LAUNCH(float, float);
   if (in_dtype == 1 && out_dtype == 1) DL_LAUNCH(dl::bf16, dl::bf16);
   if (in_dtype == 1 && out_dtype == 0) DL_LAUNCH(dl::bf16, float);
 #undef DL_LAUNCH
+#undef DL_TILES
   return DL_ERR_UNSUPPORTED;
 }

@@ -135,6 +135,28 @@ def test_gemm_simt_rows_and_tiles_agree(ops, N, K):
     assert torch.equal(out[0], first)
 
 
+@pytest.mark.parametrize("N,K", [(64, 128), (499, 80), (33, 129), (130, 77), (8, 4), (70, 516)])
+def test_gemm_simt_bfloat16_runs_of_four_and_single_numbers(ops, N, K):
+    """bfloat16 operands, in runs of four numbers where K, the rows and the addresses allow it and one by one elsewhere, K within
+    one quarter and beyond: the bits of the float32 kernel on the same numbers."""
+    g = torch.Generator(device="cpu").manual_seed(43)
+    x = torch.randn(300, K, generator=g).to(DEV, torch.bfloat16)
+    w = torch.randn(N, K, generator=g).to(DEV, torch.bfloat16)
+    bias = torch.randn(N, generator=g).to(DEV)
+    for M in (1, 17, 64, 65, 300):
+        want, out, half = (torch.empty(M, N, dtype=d, device=DEV) for d in (torch.float32, torch.float32, torch.bfloat16))
+        ops.gemm_simt(x[:M].float(), w.float(), want, bias, 0.5)
+        ops.gemm_simt(x[:M], w, out, bias, 0.5)
+        assert torch.equal(out, want)
+        ops.gemm_simt(x[:M], w, half, bias, 0.5)
+        assert torch.equal(half, want.to(torch.bfloat16))
+        for col in (1, 2, 4):                       # rows of an odd stride, or off the 8-byte grid
+            wide = torch.full((M, K + 5 + col % 2), 3.0, dtype=torch.bfloat16, device=DEV)
+            wide[:, col:K + col] = x[:M]
+            ops.gemm_simt(wide[:, col:K + col], w, out.zero_(), bias, 0.5)
+            assert torch.equal(out, want)
+
+
 def _rope_ref(x, pos, inv_freq, rot, pos_scale):
     """x [n, heads, hd] fp64; half-split rotation of the first `rot` dims."""
     half = rot // 2
