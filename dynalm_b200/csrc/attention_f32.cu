@@ -17,13 +17,18 @@
 //   up to four query heads of one KV head at once, so that a key is read once for them. A warp asks for its whole tile of
 //   keys and values at once (cp.async), and for the next tile's as soon as a buffer has been read: with a few rows it is the
 //   trips to memory that the time goes into. The warps' (m, l, a) meet in shared memory, over the cluster where it has
-//   several blocks, and are merged in the order of the keys.
+//   several blocks, and are merged in the order of the keys. Which of its launches is taken, and where query tiles give
+//   way to rows: F32Cost in kernels/attention.py.
 //
-// Bound by the multiply-add lanes (tiles) and by trips to memory (rows). Measured on B200, a layer of 32:8 heads of 64, against
-// attention_generic.cu: a prompt of 700 tokens 1,410 -> 146 us; four single tokens of 500 keys 94 -> 15 us.
+// Bound by the multiply-add lanes (tiles) and by trips to memory (rows). Measured on B200 against attention_generic.cu, us a
+// layer: 32:8 heads of 64, a prompt of 700 tokens 1,410 -> 146, single tokens: five of 450 keys 70 -> 12, 64 of 3,000 1,573 ->
+// 389; 24:8 heads of 128, 64 of 3,000 2,157 -> 754; six heads of 96, 256 of 700 546 -> 347; 4:2 heads of 16, 100 rows behind
+// 3,000 keys 102 -> 64. Behind the plain kernel with a handful of keys alone: 256 rows of 8 keys, 24:8 heads of 128, 56 -> 86.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 namespace dl {
 
@@ -238,26 +243,29 @@ f32_tiles_kernel(F32Attention at, const int4* __restrict__ tiles) {
   }
 }
 
-constexpr int FG = 4;                  // query heads of a block
-
-template <int D> struct FRows {
-  static constexpr int WARPS = D <= 64 ? 4 : 2;
+// G query heads of one KV head a block: the group where it has one or two, else four of it (a key or value read from shared
+// memory serves G of them; with places for four heads a group of one took 839 us for 256 rows of 700 keys, 6 heads of 96,
+// and the plain kernel 547).
+template <int D, int G, int W> struct FRows {
+  static constexpr int WARPS = W;
   static constexpr int K_FLOATS = FT * (D + 4), V_FLOATS = FT * D;          // a warp's tile of keys, of values
-  static constexpr int SMEM = (FG * D + WARPS * (K_FLOATS + V_FLOATS + FG * FT + FG * (D + 2))) * 4;
+  static constexpr int SMEM = (G * D + WARPS * (K_FLOATS + V_FLOATS + G * FT + G * (D + 2))) * 4;
 };
 
-// grid (parts, KV heads x runs of FG query heads, rows); a cluster is the parts of a row. A round takes parts x WARPS tiles in
-// a row, tile j to warp j / parts of part j % parts, so that few tiles spread over the SMs.
-template <int D>
-__global__ void __launch_bounds__(FRows<D>::WARPS * 32)
+// grid (parts, KV heads x runs of G query heads, rows); a cluster is the parts of a row. A round takes parts x WARPS tiles in
+// a row, tile j to warp j / parts of part j % parts, so that few tiles spread over the SMs. Of a tile only the keys from the
+// first to the last that the row sees are fetched and walked.
+template <int D, int FG, int FW>
+__global__ void __launch_bounds__(FW * 32)
 f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* __restrict__ row_request) {
   constexpr int DL = D / 32;             // values a lane
-  constexpr int FW = FRows<D>::WARPS, KS = D + 4, REC = D + 2;
+  using F = FRows<D, FG, FW>;
+  constexpr int KS = D + 4, REC = D + 2;
   extern __shared__ __align__(16) float f32_smem[];
   float* sq = f32_smem;                                  // [FG][D]
   float* sk_all = sq + FG * D;                           // [FW][FT][KS]
-  float* sv_all = sk_all + FW * FRows<D>::K_FLOATS;      // [FW][FT][D]
-  float* sp_all = sv_all + FW * FRows<D>::V_FLOATS;      // [FW][FG][FT]
+  float* sv_all = sk_all + FW * F::K_FLOATS;      // [FW][FT][D]
+  float* sp_all = sv_all + FW * F::V_FLOATS;      // [FW][FG][FT]
   float* records = sp_all + FW * FG * FT;                // [FW][FG][REC]: a tile's weighted sum, largest score, sum
   cg::cluster_group cluster = cg::this_cluster();
   const int part = blockIdx.x, n_parts = gridDim.x, row = blockIdx.z;
@@ -267,8 +275,8 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
   const int pos = positions[row], lo = first_key(at, pos), kept = lo > 0 ? min(at.keep_first, lo) : 0;
   const int* table = at.table + static_cast<size_t>(ck_request(row_request[row])) * at.max_blocks;
   const int d4 = at.head_dim >> 2, e4 = at.vdim >> 2;
-  float* sk = sk_all + warp * FRows<D>::K_FLOATS;
-  float* sv = sv_all + warp * FRows<D>::V_FLOATS;
+  float* sk = sk_all + warp * F::K_FLOATS;
+  float* sv = sv_all + warp * F::V_FLOATS;
   float* sp = sp_all + warp * FG * FT;
 
   const int step = n_parts * FW * FT;
@@ -279,7 +287,11 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
     for (base += step; base <= pos && base + step <= lo && base >= kept; base += step) {}
     return base;
   };
-  // the warp's tile of keys or values, 16 bytes a lane and trip; zeros for a key that the row does not see
+  // the keys of a tile from the first to behind the last that the row sees
+  auto first_of = [&](int t0) { return kept > t0 ? 0 : max(0, lo - t0); };
+  auto end_of = [&](int t0) { return min(FT, pos + 1 - t0); };
+  // those keys or values of the warp's tile, 16 bytes a lane and trip (D / 4 lanes a key, whatever its size: a division for every
+  // 16 bytes took longer than the products); zeros for one among them that the row does not see
   auto fetch = [&](float* dst, int stride, const float* cache, long long cache_row, int size, int per, int t0) {
     if (in_tile(t0)) {
       int slot[2];
@@ -288,11 +300,14 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
         const int t = t0 + lane + 32 * h;
         slot[h] = seen(t) ? ck_page(table, t / at.page_size, at.max_blocks) * at.page_size + t % at.page_size : -1;
       }
-      for (int e0 = 0; e0 < FT * per; e0 += 32) {        // (FT * per is a multiple of 32)
-        const int e = e0 + lane, r = e / per, c = (e - r * per) * 4;
-        const int a = __shfl_sync(0xffffffffu, slot[0], r & 31), b = __shfl_sync(0xffffffffu, slot[1], r & 31);
-        const int place = r < 32 ? a : b;
-        cp_async16_f32(dst + r * stride + c, cache + (place < 0 ? 0 : place * cache_row + static_cast<size_t>(kvh) * size + c), place < 0 ? 0 : 16);
+      constexpr int LANES = D / 4, KEYS = 32 / LANES;
+      const int c = lane % LANES, r0 = lane / LANES, end = (end_of(t0) + KEYS - 1) / KEYS;
+      const float* from = cache + static_cast<size_t>(kvh) * size + c * 4;
+      float* to = dst + r0 * stride + c * 4;
+#pragma unroll 8
+      for (int i = first_of(t0) / KEYS; i < end; ++i) {
+        const int place = __shfl_sync(0xffffffffu, i * KEYS < 32 ? slot[0] : slot[1], (i * KEYS + r0) & 31);
+        if (c < per) cp_async16_f32(to + i * KEYS * stride, from + (place < 0 ? 0 : place * cache_row), place < 0 ? 0 : 16);
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -307,7 +322,7 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
   }
   __syncthreads();
   // the thread's outputs in the merge: numbers e of [heads][vdim], dealt over the cluster's threads
-  constexpr int MOST = FG * D / (FW * 32);
+  constexpr int MOST = (FG * D + FW * 32 - 1) / (FW * 32);
   float m_run[MOST], l_run[MOST], o[MOST];
 #pragma unroll
   for (int i = 0; i < MOST; ++i) m_run[i] = -INFINITY, l_run[i] = 0.0f, o[i] = 0.0f;
@@ -327,23 +342,28 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
       float s[2][FG];
 #pragma unroll
       for (int g = 0; g < FG; ++g) s[0][g] = s[1][g] = 0.0f;
+      auto scores = [&](auto halves) {                     // (keys behind the last are not read: what lies there is left over)
+        constexpr int H = decltype(halves)::value;
 #pragma unroll 4
-      for (int c = 0; c < d4; ++c) {
-        const float4 k0 = *reinterpret_cast<const float4*>(sk + lane * KS + c * 4);
-        const float4 k1 = *reinterpret_cast<const float4*>(sk + (lane + 32) * KS + c * 4);
+        for (int c = 0; c < d4; ++c) {
+          float4 k[H];
 #pragma unroll
-        for (int g = 0; g < FG; ++g) {
-          const float4 a = *reinterpret_cast<const float4*>(sq + g * D + c * 4);
-          s[0][g] = fmaf(a.x, k0.x, s[0][g]);
-          s[0][g] = fmaf(a.y, k0.y, s[0][g]);
-          s[0][g] = fmaf(a.z, k0.z, s[0][g]);
-          s[0][g] = fmaf(a.w, k0.w, s[0][g]);
-          s[1][g] = fmaf(a.x, k1.x, s[1][g]);
-          s[1][g] = fmaf(a.y, k1.y, s[1][g]);
-          s[1][g] = fmaf(a.z, k1.z, s[1][g]);
-          s[1][g] = fmaf(a.w, k1.w, s[1][g]);
+          for (int h = 0; h < H; ++h) k[h] = *reinterpret_cast<const float4*>(sk + (lane + 32 * h) * KS + c * 4);
+#pragma unroll
+          for (int g = 0; g < FG; ++g) {
+            const float4 a = *reinterpret_cast<const float4*>(sq + g * D + c * 4);
+#pragma unroll
+            for (int h = 0; h < H; ++h) {
+              s[h][g] = fmaf(a.x, k[h].x, s[h][g]);
+              s[h][g] = fmaf(a.y, k[h].y, s[h][g]);
+              s[h][g] = fmaf(a.z, k[h].z, s[h][g]);
+              s[h][g] = fmaf(a.w, k[h].w, s[h][g]);
+            }
+          }
         }
-      }
+      };
+      if (end_of(t0) > 32) scores(std::integral_constant<int, 2>());
+      else scores(std::integral_constant<int, 1>());
 #pragma unroll
       for (int g = 0; g < FG; ++g) {
         if (g >= heads) break;
@@ -374,18 +394,30 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
     if (in_tile(t0)) {
-#pragma unroll 8
-      for (int k = 0; k < FT; ++k) {
-        float v[DL];
+      auto weigh = [&](int first, int end) {
+#pragma unroll 4
+        for (int k = first; k < end; k += 4) {             // (the weights of keys that are not seen are there, and 0)
+          float4 p[FG];
 #pragma unroll
-        for (int j = 0; j < DL; ++j) v[j] = sv[k * D + lane * DL + j];
+          for (int g = 0; g < FG; ++g)
+            p[g] = g < heads ? *reinterpret_cast<const float4*>(sp + g * FT + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-        for (int g = 0; g < FG; ++g) {
-          const float p = g < heads ? sp[g * FT + k] : 0.0f;
+          for (int kk = 0; kk < 4; ++kk) {
+            float v[DL];
 #pragma unroll
-          for (int j = 0; j < DL; ++j) acc[g][j] = p != 0.0f ? fmaf(p, v[j], acc[g][j]) : acc[g][j];
+            for (int j = 0; j < DL; ++j) v[j] = sv[(k + kk) * D + lane * DL + j];
+#pragma unroll
+            for (int g = 0; g < FG; ++g) {
+              const float w = kk == 0 ? p[g].x : kk == 1 ? p[g].y : kk == 2 ? p[g].z : p[g].w;
+#pragma unroll
+              for (int j = 0; j < DL; ++j) acc[g][j] = w != 0.0f ? fmaf(w, v[j], acc[g][j]) : acc[g][j];
+            }
+          }
         }
-      }
+      };
+      const int first = first_of(t0) & ~3, end = end_of(t0);
+      if (first == 0 && end == FT) weigh(0, FT);
+      else weigh(first, end);
     }
     __syncwarp();                                          // the values have been read
     fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, next <= pos ? tile_of(next) : pos + 1);
@@ -450,16 +482,16 @@ int launch_f32_tiles(const F32Attention& at, const int4* tiles, int n_tiles, cud
   return launch_status();
 }
 
-template <int D>
-int launch_f32_rows(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts,
-                    cudaStream_t stream) {
+template <int D, int FG, int FW>
+int launch_f32_rows_of(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts,
+                       cudaStream_t stream) {
   const int group = at.n_heads / at.n_kv_heads;
-  const cudaError_t e = cudaFuncSetAttribute(f32_rows_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRows<D>::SMEM);
+  const cudaError_t e = cudaFuncSetAttribute(f32_rows_kernel<D, FG, FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRows<D, FG, FW>::SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(parts, at.n_kv_heads * ((group + FG - 1) / FG), rows);
-  cfg.blockDim = FRows<D>::WARPS * 32;
-  cfg.dynamicSmemBytes = FRows<D>::SMEM;
+  cfg.blockDim = FW * 32;
+  cfg.dynamicSmemBytes = FRows<D, FG, FW>::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -467,8 +499,22 @@ int launch_f32_rows(const F32Attention& at, const int* positions, const int* row
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, f32_rows_kernel<D>, at, positions, row_request));
+  cfg.numAttrs = parts > 1 ? 1 : 0;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, f32_rows_kernel<D, FG, FW>, at, positions, row_request));
+}
+
+template <int D>
+int launch_f32_rows(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts, int warps,
+                    cudaStream_t stream) {
+  constexpr int MOST_WARPS = D <= 64 ? 4 : 2;
+  const int group = at.n_heads / at.n_kv_heads;
+#define DL_ROWS(G)                                                                                          \
+  return warps == 1 ? launch_f32_rows_of<D, G, 1>(at, positions, row_request, rows, parts, stream)          \
+                    : launch_f32_rows_of<D, G, MOST_WARPS>(at, positions, row_request, rows, parts, stream)
+  if (group == 1) DL_ROWS(1);
+  if (group == 2) DL_ROWS(2);
+  DL_ROWS(4);
+#undef DL_ROWS
 }
 
 inline bool f32_sizes(const F32Attention& a) {
@@ -500,10 +546,11 @@ DL_EXPORT int dl_attention_f32_tiles(const void* q, int q_stride, const void* k_
   return dl::launch_f32_tiles<128>(at, list, n_tiles, stream);
 }
 
-// Rows 0 .. rows - 1, each the newest token of its request; `parts` (1, 2, 4 or 8): blocks over a row's keys.
+// Rows 0 .. rows - 1, each the newest token of its request; `parts` (1, 2, 4 or 8): blocks over a row's keys; warps of a block: 1,
+// or 0 for as many as have room for a tile each (4, with more than 64 numbers 2).
 DL_EXPORT int dl_attention_f32_rows(const void* q, int q_stride, const void* k_cache, long long k_row, const void* v_cache,
                                     long long v_row, const int* block_table, int max_blocks, const int* positions,
-                                    const int* row_request, int rows, int parts, void* out, int out_stride, int n_heads,
+                                    const int* row_request, int rows, int parts, int warps, void* out, int out_stride, int n_heads,
                                     int n_kv_heads, int head_dim, int vdim, int page_size, float scale, int window,
                                     int keep_first, int sink, const float* rate, const float* dstep, int chunk,
                                     cudaStream_t stream) {
@@ -511,9 +558,10 @@ DL_EXPORT int dl_attention_f32_rows(const void* q, int q_stride, const void* k_c
   const dl::F32Attention at = {static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
                                static_cast<float*>(out), block_table, rate, dstep, k_row, v_row, q_stride, out_stride, max_blocks,
                                n_heads, n_kv_heads, head_dim, vdim, page_size, window, keep_first, sink, chunk, scale};
-  if (!dl::f32_sizes(at) || rows > 65535 || (parts != 1 && parts != 2 && parts != 4 && parts != 8)) return DL_ERR_UNSUPPORTED;
+  if (!dl::f32_sizes(at) || rows > 65535 || (parts != 1 && parts != 2 && parts != 4 && parts != 8) || warps < 0 || warps > 1)
+    return DL_ERR_UNSUPPORTED;
   const int most = head_dim > vdim ? head_dim : vdim;
-  if (most <= 32) return dl::launch_f32_rows<32>(at, positions, row_request, rows, parts, stream);
-  if (most <= 64) return dl::launch_f32_rows<64>(at, positions, row_request, rows, parts, stream);
-  return dl::launch_f32_rows<128>(at, positions, row_request, rows, parts, stream);
+  if (most <= 32) return dl::launch_f32_rows<32>(at, positions, row_request, rows, parts, warps, stream);
+  if (most <= 64) return dl::launch_f32_rows<64>(at, positions, row_request, rows, parts, warps, stream);
+  return dl::launch_f32_rows<128>(at, positions, row_request, rows, parts, warps, stream);
 }

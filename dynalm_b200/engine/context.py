@@ -58,6 +58,7 @@ class StepContext:
     decode_only: bool = False        # every request brings exactly one token
     max_q_len: int = 0
     max_kv_len: int = 0
+    portions_kv_len: int = 0         # max_kv_len over the requests behind the single tokens at the head of the step
     # per-step scratch that parts share. A part's step plan (see StepShape in engine/step.py) is found under its name
     # as (the plan's integers on the device, what its `fill` returned); parts may add entries of their own.
     extras: Dict[str, object] = field(default_factory=dict)

@@ -262,6 +262,7 @@ class BatchBuilder:
         slots = h[off["state_slots"]]
         r0 = 0
         n_logit = 0
+        portions_kv_len = 0
         h_q_len, h_q_start, h_pos_start, h_slots = [], [], [], []
         for r, e in enumerate(entries):
             n = len(e.tokens)
@@ -277,6 +278,8 @@ class BatchBuilder:
             q_start[r] = r0
             pos_start[r] = start
             kv_len[r] = start + n
+            if n > 1 or portions_kv_len > 0:
+                portions_kv_len = max(portions_kv_len, start + n)
             slots[r] = slot
             h_q_len.append(n)
             h_q_start.append(r0)
@@ -313,7 +316,7 @@ class BatchBuilder:
             kv_len=d["kv_len"], state_slots=d["state_slots"], logit_rows=d["logit_rows"], num_logit_rows=n_logit,
             h_q_len=h_q_len, h_pos_start=h_pos_start, h_state_slots=h_slots, block_tables=self.tables,
             decode_only=all(n == 1 for n in h_q_len), max_q_len=max(h_q_len),
-            max_kv_len=max(s + n for s, n in zip(h_pos_start, h_q_len)), extras=extras)
+            max_kv_len=max(s + n for s, n in zip(h_pos_start, h_q_len)), portions_kv_len=portions_kv_len, extras=extras)
 
     def finish(self, entries: Sequence[StepEntry]) -> None:
         """The step has been issued: count its tokens and let windows give pages back."""
@@ -477,6 +480,8 @@ class StepFunction:
         else:
             kind, key = "portions", (tuple(ctx.h_q_len), ctx.num_logit_rows, chosen, self._plan_answers(ctx),
                                      max(256, 1 << (ctx.max_kv_len - 1).bit_length()))
+            if self.rt.dtype == torch.float32:          # (what the 32-bit attention's launches follow: kernels/attention.f32_launches)
+                key += (max(64, 1 << (ctx.max_kv_len - 1).bit_length()), max(64, 1 << (ctx.portions_kv_len - 1).bit_length()))
         out = self._decode_logits if ctx.num_logit_rows else None
         kept = self._graphs.use(kind, key)
         if kept is None:

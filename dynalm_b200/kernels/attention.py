@@ -10,6 +10,7 @@ the faster kernels refuse falls to the plain kernel.
 
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
@@ -348,40 +349,108 @@ def _decode_rows(qkv: torch.Tensor, cache, ctx, out: torch.Tensor, spec, runtime
                                tensor_cores=decode_uses_tensor_cores(spec) and qkv.stride(0) % 8 == 0)
 
 
-# Steps of up to this many rows run row by row: a query tile of the other kernel then has mostly empty rows. A layer of 32:8
-# heads of 64 on B200, the plain kernel / these: a prompt of 700 tokens in tiles 1,410 / 146 us; four single tokens of 500
-# keys 94 / 15 us.
-F32_ROWS = 64
+class F32Cost:
+    """What a 32-bit attention layer takes, for choosing between its two kernels and how the row kernel is launched
+    (csrc/attention_f32.cu; a row's bits are the same from all of them): rounds of blocks over the SMs times tiles of 64 keys
+    that a block walks one after the other times what one takes, in us. `span`: the most keys a row sees, in powers of two from
+    64, so that what follows from it changes a CUDA graph only now and then.
+
+    Measured on B200 over 1 to 256 rows of 8 to 3,000 keys, nine shapes of heads: the launch with the least cost is on average 3 %
+    behind the fastest of all. Blocks of one warp, several to an SM, are the better ones for many rows (64 rows of 3,000 keys, 24:8
+    heads of 128: 1,210 us with two warps a block, 754 in four blocks of one), blocks of several warps for few (one row of 3,000
+    keys: 79 and 43 us). Query tiles against rows, us: 70 rows behind 900 keys, 4:2 heads of 16 81 / 16, 32:8 heads of 64 132 /
+    135, 24:8 heads of 128 219 / 407; a prompt of 300 rows 28 / 17, 64 / 165, 72 / 381."""
+
+    WARPS = {32: 4, 64: 4, 128: 2}                      # of a block that is not one warp, a tile each
+    ROUND = {32: (6.5, 6.5), 64: (8.4, 11.6), 128: (12.8, 14.0)}      # a tile for each warp of the block; for its only one
+    FIT = {32: (2, 11), 64: (1, 6), 128: (1, 3)}        # blocks an SM holds, likewise
+    ONE_HEAD = 0.6                                      # of ROUND where a KV head has one query head
+    # SMs of 148 that clusters of 1, 2, 4 and 8 blocks fill round after round (with eight of 144 KB one of two stays empty)
+    FILLED = {32: ((148, 148, 140, 112), (148, 148, 140, 128)), 64: ((148, 148, 128, 64), (148, 148, 140, 128)),
+              128: ((148, 148, 128, 112), (148, 148, 140, 128))}
+    TILE, TILES_FIT = {32: 5.0, 64: 8.1, 128: 13.6}, {32: 2, 64: 2, 128: 1}      # a tile of keys of a block of 64 query rows
+    LAUNCH = 5.0
+
+    def __init__(self, n_heads: int, n_kv_heads: int, most: int, span: int, sms: int = 0):
+        group = n_heads // n_kv_heads
+        self.size = 32 if most <= 32 else 64 if most <= 64 else 128
+        self.heads, self.sms = n_heads, sms or sm_count()
+        self.row_blocks = n_kv_heads * -(-group // min(4, 1 << (group - 1).bit_length()))
+        self.key_tiles = span // 64
+        self.scale = self.ONE_HEAD if group == 1 else 1.0
+        self.known: dict = {}
+
+    def rows(self, rows: int) -> tuple:
+        """(cost, blocks over a row's keys, 1 for blocks of one warp or 0) of the row kernel."""
+        best = self.known.get(rows)
+        if best is None:
+            best = self.known[rows] = self._rows(rows)
+        return best
+
+    def _rows(self, rows: int) -> tuple:
+        best = (0.0, 1, 0)
+        for one in (0, 1) if rows > 0 else ():
+            warps, took, fit = (self.WARPS[self.size], 1)[one], self.ROUND[self.size][one], self.FIT[self.size][one]
+            for parts, filled in zip((1, 2, 4, 8), self.FILLED[self.size][one]):
+                if parts > 1 and parts // 2 * warps >= self.key_tiles:
+                    break
+                blocks, slots = rows * self.row_blocks * parts, max(1, self.sms * filled // 148) * fit
+                cost = self.LAUNCH + -(-blocks // slots) * -(-self.key_tiles // (parts * warps)) * took * self.scale
+                if best[0] == 0.0 or cost < best[0]:
+                    best = (cost, parts, one)
+        return best
+
+    def tiles(self, n_tiles: int) -> float:
+        return self.LAUNCH + -(-2 * n_tiles * self.heads // (self.sms * self.TILES_FIT[self.size])) * self.key_tiles * self.TILE[self.size]
 
 
-def f32_parts(rows: int, n_heads: int, n_kv_heads: int, sms: int = 0) -> int:
-    """Blocks over a row's keys: as many (a power of two up to a cluster's 8) as keep the grid within a block an SM (one fits)."""
-    blocks = max(1, rows) * n_kv_heads * -(-(n_heads // n_kv_heads) // 4)
-    parts = 8
-    while parts > 1 and blocks * parts > (sms or sm_count()):
-        parts //= 2
-    return parts
+_f32_costs = functools.lru_cache(maxsize=256)(F32Cost)
+
+
+def f32_launches(ctx, n_heads: int, n_kv_heads: int, most: int, window: int = 0, keep_first: int = 0, chunk: int = 0) -> tuple:
+    """What a 32-bit layer launches for a step: (single tokens at its head, blocks over a row's keys, 1 for blocks of one warp),
+    and for the prompt portions behind them (query tiles, or 0 where their rows go one by one, then blocks and warps again).
+    Worked out once a step for layers of the same sizes and mask; it is all that their launches depend on."""
+    key = ("f32_launches", n_heads, n_kv_heads, most, window, keep_first, chunk)
+    got = ctx.extras.get(key)
+    if got is None:
+        reach = chunk or (window + keep_first if window > 0 else 0)        # the most keys that the mask leaves a row, 0: all
+
+        def cost(longest):
+            span = min(longest, reach) if reach > 0 else longest
+            return _f32_costs(n_heads, n_kv_heads, most, max(64, 1 << (span - 1).bit_length()))
+        planned = None if ctx.decode_only else query_tiles(ctx)
+        lead, portions = ctx.num_tokens, (0, 1, 0)
+        if planned is not None:
+            _, _, n_prompt, lead = planned
+            behind = cost(ctx.portions_kv_len)
+            by_rows = behind.rows(ctx.num_tokens - lead)
+            portions = (n_prompt, 1, 0) if behind.tiles(n_prompt) <= by_rows[0] else (0,) + by_rows[1:]
+        got = ctx.extras[key] = (lead,) + cost(ctx.max_kv_len).rows(lead)[1:] + portions
+    return got
 
 
 def attention_f32(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: torch.Tensor, v_row: int, cache, ctx,
                   out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, vdim: int, scale: float, window: int = 0,
                   keep_first: int = 0, sink: bool = False, rate=None, step=None, chunk: int = 0) -> bool:
-    """The 32-bit kernels on a step, False where they do not take it: single tokens (and any step of few rows) row by row,
-    prompt portions in query tiles."""
+    """The 32-bit kernels on a step, False where they do not take it: single tokens row by row, prompt portions in query tiles
+    or, where those would leave most of the GPU idle, row by row too."""
     rows = q.shape[0]
     if not ops.attention_f32_takes(q, k_cache, k_row, v_cache, v_row, head_dim, vdim):
         return False
-    single, n_tiles, tiles = rows, 0, None
-    if rows > F32_ROWS and not ctx.decode_only:
-        if query_tiles(ctx) is None:
-            return False
-        tiles, _, n_tiles, single = query_tiles(ctx)
+    lead, parts, one, n_tiles, behind_parts, behind_one = f32_launches(ctx, n_heads, n_kv_heads, max(head_dim, vdim), window,
+                                                                       keep_first, chunk)
+    if max(lead, rows - lead if n_tiles == 0 else 0) > 65535:
+        return False
     args = (n_heads, n_kv_heads, head_dim, vdim, cache.page_size, scale, window, keep_first, sink, rate, step, chunk)
-    if single > 0:
-        ops.attention_f32_rows(q, k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions, ctx.row_slot, single,
-                               f32_parts(single, n_heads, n_kv_heads), out, *args)
+    if lead > 0:
+        ops.attention_f32_rows(q, k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions, ctx.row_slot, lead,
+                               parts, out, *args, warps=one)
     if n_tiles > 0:
-        ops.attention_f32_tiles(q, k_cache, k_row, v_cache, v_row, cache.block_table, tiles, n_tiles, out, *args)
+        ops.attention_f32_tiles(q, k_cache, k_row, v_cache, v_row, cache.block_table, query_tiles(ctx)[0], n_tiles, out, *args)
+    elif rows > lead:
+        ops.attention_f32_rows(q[lead:], k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions[lead:], ctx.row_slot[lead:],
+                               rows - lead, behind_parts, out[lead:], *args, warps=behind_one)
     return True
 
 

@@ -146,7 +146,7 @@ _SIGNATURES = {
         "dl_gemm_stream": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _P, _P]},
     "attention_f32": {
         "dl_attention_f32_tiles": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _P],
-        "dl_attention_f32_rows": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
+        "dl_attention_f32_rows": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
                                   _I, _P]},
     "gemm_simt": {"dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P]},
     "sampling": {
@@ -1995,14 +1995,14 @@ def attention_f32_rows(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cac
                        block_table: torch.Tensor, positions: torch.Tensor, row_request: torch.Tensor, rows: int, parts: int,
                        out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, vdim: int, page_size: int, scale: float,
                        window: int = 0, keep_first: int = 0, sink: bool = False, rate: Optional[torch.Tensor] = None,
-                       step: Optional[torch.Tensor] = None, chunk: int = 0) -> None:
-    """The same for the first `rows` rows of the step one by one, each row's keys over `parts` (1, 2, 4 or 8) blocks; the
-    result's bits do not depend on `parts`."""
+                       step: Optional[torch.Tensor] = None, chunk: int = 0, warps: int = 0) -> None:
+    """The same for the first `rows` rows of the step one by one, each row's keys over `parts` (1, 2, 4 or 8) blocks of one warp
+    (warps 1) or of as many as the kernel has (0); the result's bits depend on neither."""
     _attention_f32_args(q, k_cache, v_cache, block_table, out, n_heads, n_kv_heads, rate, step)
     _cuda(positions, row_request)
     _check(_fn("attention_f32", "dl_attention_f32_rows")(
         _p(q), q.stride(0), _p(k_cache), k_row, _p(v_cache), v_row, _p(block_table), block_table.stride(0), _p(positions),
-        _p(row_request), rows, parts, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, vdim, page_size, scale, window,
+        _p(row_request), rows, parts, warps, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, vdim, page_size, scale, window,
         int(keep_first), 1 if sink else 0, _p(rate), _p(step), int(chunk), _stream()), "attention_f32_rows")
 
 

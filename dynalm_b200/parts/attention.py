@@ -139,6 +139,9 @@ class PagedAttention:
 
     def graph_key(self, ctx) -> tuple:
         from ..kernels import attention as fast
+        s = self.spec
+        if self.rt.dtype == torch.float32:
+            return (("f32_attention",) + fast.f32_launches(ctx, s.num_heads, s.num_kv_heads, s.head_dim, int(s.get("window", 0))),)
         if fast.DECODE_PLANNED and fast.decode_uses_tensor_cores(self.spec):
             planned = ctx.extras.get(fast.decode_units_plan(self.spec).name)
             if planned is not None and planned[1][0] > 0:
@@ -318,9 +321,14 @@ class GatedNormedAttention(PagedAttention):
         return [fast.QUERY_TILES]                  # the masked flash kernel walks the step's query tiles
 
     def graph_key(self, ctx) -> tuple:
+        s = self.spec
+        if self.rt.dtype == torch.float32:
+            from ..kernels import attention as fast
+            return (("f32_attention",) + fast.f32_launches(ctx, s.num_heads, s.num_kv_heads, max(s.head_dim, s.value_dim), self.window,
+                                                           self.keep_first, self.chunk),)
         if self.same and self.plain_mask:
-            return super().graph_key(ctx) if self.rt.dtype == torch.bfloat16 else ()
-        return (("masked_flash_parts", self._decode_parts(ctx, ctx.num_tokens)),) if self.rt.dtype == torch.bfloat16 else ()
+            return super().graph_key(ctx)
+        return (("masked_flash_parts", self._decode_parts(ctx, ctx.num_tokens)),)
 
     def _decode_parts(self, ctx, rows: int) -> int:
         """Into how many parts the keys of `rows` single tokens are dealt (part of the launch shape, so of the graph key)."""

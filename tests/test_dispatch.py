@@ -281,3 +281,33 @@ def test_latents_with_a_scale_that_is_not_positive_go_over_the_records():
     for scale, expanded in ((0.07, True), (0.0, False), (-0.07, False)):
         spec = SimpleNamespace(head_dim=128, rot_dim=64, value_dim=128, kv_rank=48, scale=scale, get=lambda name, default=0: default)
         assert (latent.expand_plan(spec, 4, 512) is not None) == expanded
+
+
+def test_32_bit_attention_goes_where_it_costs_least(monkeypatch):
+    """By rows or by query tiles, and the row kernel's blocks: one warp a block and several blocks to an SM for many rows, all of a
+    row's keys in one round for few; what a mask leaves of the keys counts, and the launch follows the span in powers of two."""
+    from dynalm_b200.engine.step import StepShape
+    from types import SimpleNamespace
+    cost = lambda *a: attention.F32Cost(*a, sms=148)
+    assert cost(32, 8, 64, 64).rows(1)[1:] == (1, 0)              # one tile of keys: one block
+    assert cost(32, 8, 64, 1024).rows(1)[1:] == (4, 0)            # sixteen: four blocks of four warps
+    assert cost(24, 8, 128, 4096).rows(64)[1:] == (4, 1)          # many rows: blocks of one warp
+    assert cost(6, 6, 96, 64).rows(256)[1:] == (1, 1)
+    few, prompt = cost(4, 2, 16, 1024), cost(32, 8, 64, 512)
+    assert few.rows(70)[0] < few.tiles(1)                         # 70 rows behind 900 keys of a small model: 16 us, in tiles 81
+    assert prompt.tiles(3) < prompt.rows(300)[0]                  # a prompt of 300: in tiles 64, by rows 165
+    def launches(q_len, pos_start, *mask):
+        host = np.zeros(attention.QUERY_TILES.ints(4096, 32), dtype=np.int32)
+        first = np.cumsum([0] + q_len).tolist()
+        answer = attention.QUERY_TILES.fill(host, StepShape(q_len, first[:-1], pos_start, list(range(len(q_len))), first[-1]))
+        ctx = SimpleNamespace(num_tokens=first[-1], decode_only=max(q_len) == 1, extras={attention.QUERY_TILES.name: (None, answer)},
+                              max_kv_len=max(p + n for p, n in zip(pos_start, q_len)),
+                              portions_kv_len=max([p + n for p, n in zip(pos_start, q_len) if n > 1], default=0))
+        return attention.f32_launches(ctx, 32, 8, 64, *mask)
+    monkeypatch.setattr(attention, "sm_count", lambda: 148)
+    attention._f32_costs.cache_clear()
+    assert launches([1] * 3, [10, 2999, 5]) == (3, 4, 0, 0, 1, 0)
+    assert launches([1] * 3, [10, 2999, 5], 100, 20) == (3, 1, 0, 0, 1, 0) == launches([1] * 3, [10, 2999, 5], 0, 0, 50)
+    assert launches([1, 1, 300], [10, 2999, 0]) == (2, 4, 0, 3, 1, 0)            # the portion's own keys count, not the others'
+    assert launches([70], [3000])[3] == 1 and launches([5], [3000])[:4] == (0, 1, 0, 0)
+    attention._f32_costs.cache_clear()

@@ -323,6 +323,40 @@ def test_attention_f32(ops, heads, kvh, d, e, window, keep, sink, bias, chunk):
     assert torch.equal(out[5:], alone[0][5:]) and (out[:5] == 7.0).all()
 
 
+@pytest.mark.parametrize("heads,kvh,d,e,window,keep,chunk", [(4, 2, 16, 16, 0, 0, 0), (3, 3, 32, 20, 0, 0, 50), (7, 1, 64, 36, 90, 5, 0),
+                                                             (6, 6, 96, 96, 0, 0, 0), (4, 2, 128, 100, 33, 0, 0), (6, 2, 40, 128, 64, 70, 0)])
+def test_attention_f32_rows_with_any_blocks(ops, heads, kvh, d, e, window, keep, chunk):
+    """One, two and more heads of a group a block, blocks of one warp and of several, one or more of them a row: the same bits,
+    at every length from one key on, where tiles of 64 begin and end; unwritten slots hold no numbers. Bound as above."""
+    g = torch.Generator(device="cpu").manual_seed(71)
+    page, length = 16, 700
+    row = kvh * (d + e)
+    kc = torch.full((length // page + 4, page, row), float("nan"))
+    kc.view(-1, row)[:length] = torch.randn(length, row, generator=g)
+    table = torch.arange(kc.shape[0], dtype=torch.int32).view(1, -1).to(DEV)
+    kc = kc.to(DEV)
+    vc = kc.view(-1)[kvh * d:]
+    at = [0, 1, 7, 8, 31, 32, 33, 62, 63, 64, 65, 95, 96, 127, 128, 129, 191, 255, 256, 300, 511, 512, 575, 640, 699]
+    pos = torch.tensor(at, dtype=torch.int32, device=DEV)
+    req = torch.zeros(len(at), dtype=torch.int32, device=DEV)
+    q = torch.randn(len(at), heads * d, generator=g).to(DEV)
+    args = (heads, kvh, d, e, page, d ** -0.5, window, keep, False, None, None, chunk)
+    ref = torch.empty(len(at), heads * e, device=DEV)
+    ops.paged_attention_generic_kv(q, kc, row, vc, row, table, pos, req, ref, *args)
+    first = None
+    for parts in (1, 2, 4, 8):
+        for warps in (0, 1):
+            out = torch.full((len(at), heads * e), 7.0, device=DEV)
+            ops.attention_f32_rows(q, kc, row, vc, row, table, pos, req, len(at), parts, out, *args, warps=warps)
+            first = out if first is None else first
+            assert torch.equal(out, first), (parts, warps)
+    assert (first - ref).abs().max() <= 4e-5
+    tiles = torch.tensor([(0, i, 1, p) for i, p in enumerate(at)], dtype=torch.int32, device=DEV)
+    out = torch.empty(len(at), heads * e, device=DEV)
+    ops.attention_f32_tiles(q, kc, row, vc, row, table, tiles.view(-1), len(at), out, *args)
+    assert torch.equal(out, first)
+
+
 @pytest.mark.parametrize("window", [0, 5])
 def test_attention_f32_lets_no_key_without_a_number_pass(ops, window):
     """Keys that are no numbers, all that a row sees of a tile of 64: rows that see one give no numbers in every kernel and

@@ -193,3 +193,33 @@ def test_shapes_in_turn_beyond_the_places_are_not_captured_over_and_over(monkeyp
             assert len(kept["portions"]) == 32 and 1 <= len(kept["decode"]) <= 2
             assert eng.step_fn.graph_captures == 32 + len(kept["decode"])
     assert all(torch.equal(a, b) for a, b in zip(got[True], got[False]))
+
+
+@pytest.mark.parametrize("name", ["a", "e"])
+def test_32_bit_portions_replay_the_same_bits_at_every_span(name, monkeypatch):
+    """float32: portions of one size at spans of 64 to 1,024 keys, where rows and query tiles of the attention take turns."""
+    from dynalm_b200 import Engine, StepEntry
+    from dynalm_b200.engine.step import StepFunction
+    from dynalm_b200.kernels import ops
+    monkeypatch.setattr(StepFunction, "GRAPH_AFTER", 2)
+    cfg, seed = dict(TINY[name][0], max_position_embeddings=2048), TINY[name][1]
+    ids = torch.randint(0, 256, (1200,), generator=torch.Generator().manual_seed(5)).tolist()
+    got, seen = {}, set()
+    for graphs in (True, False):
+        with monkeypatch.context() as m:
+            if not graphs:
+                for kernel in ("attention_f32_rows", "attention_f32_tiles"):
+                    real = getattr(ops, kernel)
+                    m.setattr(ops, kernel, lambda *a, real=real, kernel=kernel, **k: (seen.add(kernel), real(*a, **k))[1])
+            eng = Engine(config=cfg, random_seed=seed, dtype="float32", ctx=4096, batch=256, max_running=2)
+            eng.step_fn.use_graphs = graphs
+            out = got[graphs] = []
+            eng.step([StepEntry("live", ids[:9])])
+            for again in range(3):
+                for at in range(again, 1100, 100):
+                    new = StepEntry("new", ids[at:at + 100], [99])
+                    out.append(eng.step([StepEntry("live", [ids[at]], [0]), new]).clone())
+                eng.end("new")
+        assert eng.step_fn.graph_captures >= 4 if graphs else eng.step_fn.graph_captures == 0
+    assert all(torch.equal(a, b) for a, b in zip(got[True], got[False]))
+    assert seen == {"attention_f32_rows", "attention_f32_tiles"}
