@@ -257,7 +257,7 @@ template <int D, int G, int W> struct FRows {
 // first to the last that the row sees are fetched and walked.
 template <int D, int FG, int FW>
 __global__ void __launch_bounds__(FW * 32)
-f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* __restrict__ row_request) {
+f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* __restrict__ row_request, int old_keys) {
   constexpr int DL = D / 32;             // values a lane
   using F = FRows<D, FG, FW>;
   constexpr int KS = D + 4, REC = D + 2;
@@ -314,8 +314,15 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
   };
 
   int base = kept > 0 ? 0 : lo / FT * FT;
+  // Where the row is the only one its request brings, the keys in front of it were left by earlier steps, and a tile of them is
+  // asked for before the wait on the kernel that writes this step's keys and queries (4 rows of 500 keys, 32:8 heads of 64, in a
+  // decode step: 13.7 -> 12 us).
+  const bool ahead = old_keys && tile_of(base) + FT <= pos;
+  if (!ahead) pdl_wait();
   fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, tile_of(base));
   fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, tile_of(base));
+  if (ahead) pdl_wait();
+  pdl_trigger();
   for (int e = tid; e < FG * D; e += FW * 32) {
     const int g = e / D, d = e % D;
     sq[e] = g < heads && d < at.head_dim ? at.q[static_cast<size_t>(row) * at.q_stride + static_cast<size_t>(head0 + g) * at.head_dim + d] : 0.0f;
@@ -483,7 +490,7 @@ int launch_f32_tiles(const F32Attention& at, const int4* tiles, int n_tiles, cud
 }
 
 template <int D, int FG, int FW>
-int launch_f32_rows_of(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts,
+int launch_f32_rows_of(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts, int old_keys,
                        cudaStream_t stream) {
   const int group = at.n_heads / at.n_kv_heads;
   const cudaError_t e = cudaFuncSetAttribute(f32_rows_kernel<D, FG, FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, FRows<D, FG, FW>::SMEM);
@@ -493,24 +500,33 @@ int launch_f32_rows_of(const F32Attention& at, const int* positions, const int* 
   cfg.blockDim = FW * 32;
   cfg.dynamicSmemBytes = FRows<D, FG, FW>::SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = parts;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (parts > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = parts;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl_mode() >= 1) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = parts > 1 ? 1 : 0;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, f32_rows_kernel<D, FG, FW>, at, positions, row_request));
+  cfg.numAttrs = n;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, f32_rows_kernel<D, FG, FW>, at, positions, row_request, old_keys));
 }
 
 template <int D>
-int launch_f32_rows(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts, int warps,
+int launch_f32_rows(const F32Attention& at, const int* positions, const int* row_request, int rows, int parts, int warps, int old_keys,
                     cudaStream_t stream) {
   constexpr int MOST_WARPS = D <= 64 ? 4 : 2;
   const int group = at.n_heads / at.n_kv_heads;
 #define DL_ROWS(G)                                                                                          \
-  return warps == 1 ? launch_f32_rows_of<D, G, 1>(at, positions, row_request, rows, parts, stream)          \
-                    : launch_f32_rows_of<D, G, MOST_WARPS>(at, positions, row_request, rows, parts, stream)
+  return warps == 1 ? launch_f32_rows_of<D, G, 1>(at, positions, row_request, rows, parts, old_keys, stream) \
+                    : launch_f32_rows_of<D, G, MOST_WARPS>(at, positions, row_request, rows, parts, old_keys, stream)
   if (group == 1) DL_ROWS(1);
   if (group == 2) DL_ROWS(2);
   DL_ROWS(4);
@@ -547,12 +563,13 @@ DL_EXPORT int dl_attention_f32_tiles(const void* q, int q_stride, const void* k_
 }
 
 // Rows 0 .. rows - 1, each the newest token of its request; `parts` (1, 2, 4 or 8): blocks over a row's keys; warps of a block: 1,
-// or 0 for as many as have room for a tile each (4, with more than 64 numbers 2).
+// or 0 for as many as have room for a tile each (4, with more than 64 numbers 2). old_keys: every row is the only one its request
+// brings, so that the keys in front of it lie there before this step.
 DL_EXPORT int dl_attention_f32_rows(const void* q, int q_stride, const void* k_cache, long long k_row, const void* v_cache,
                                     long long v_row, const int* block_table, int max_blocks, const int* positions,
                                     const int* row_request, int rows, int parts, int warps, void* out, int out_stride, int n_heads,
                                     int n_kv_heads, int head_dim, int vdim, int page_size, float scale, int window,
-                                    int keep_first, int sink, const float* rate, const float* dstep, int chunk,
+                                    int keep_first, int sink, const float* rate, const float* dstep, int chunk, int old_keys,
                                     cudaStream_t stream) {
   if (rows <= 0) return 0;
   const dl::F32Attention at = {static_cast<const float*>(q), static_cast<const float*>(k_cache), static_cast<const float*>(v_cache),
@@ -561,7 +578,7 @@ DL_EXPORT int dl_attention_f32_rows(const void* q, int q_stride, const void* k_c
   if (!dl::f32_sizes(at) || rows > 65535 || (parts != 1 && parts != 2 && parts != 4 && parts != 8) || warps < 0 || warps > 1)
     return DL_ERR_UNSUPPORTED;
   const int most = head_dim > vdim ? head_dim : vdim;
-  if (most <= 32) return dl::launch_f32_rows<32>(at, positions, row_request, rows, parts, warps, stream);
-  if (most <= 64) return dl::launch_f32_rows<64>(at, positions, row_request, rows, parts, warps, stream);
-  return dl::launch_f32_rows<128>(at, positions, row_request, rows, parts, warps, stream);
+  if (most <= 32) return dl::launch_f32_rows<32>(at, positions, row_request, rows, parts, warps, old_keys, stream);
+  if (most <= 64) return dl::launch_f32_rows<64>(at, positions, row_request, rows, parts, warps, old_keys, stream);
+  return dl::launch_f32_rows<128>(at, positions, row_request, rows, parts, warps, old_keys, stream);
 }

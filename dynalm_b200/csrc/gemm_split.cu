@@ -1,0 +1,954 @@
+// y = x W^T (+ bias) for float32 operands on the tensor cores, with the precision of 32-bit multiply-adds.
+//
+// A float32 is the sum of three bf16 (8 + 8 + 8 bits of mantissa, each part rounded to nearest, the split exact), so a
+// product of two is the sum of nine products of bf16 that the tensor core forms exactly. The six that matter are kept (of
+// the three that are left out the largest is 2^-26 of the product on average), smallest first:
+//   lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi          (a part of W times a part of x).
+// The tensor core cuts off what its 32-bit accumulator does not hold, so an accumulator is only used for 64 of k (24
+// steps of 16); the sums of the slices of 64 are added on the multiply-add lanes, rounded to nearest.
+//
+// The order of a sum is fixed by K alone, so a row's result does not depend on the other rows of the call, their number or
+// the tile it falls into: the slices of 64 of a sixteenth of k (rounded up to whole slices) in turn, then the sixteenths in turn.
+// Both kernels below follow it: mma.sync and tcgen05.mma round a step of 16 k alike (compared bit by bit in
+// tests/test_gemm_split_gpu.py), and either may deal the sixteenths to different warps or blocks.
+//
+// Numbers that are not finite (or round to no finite bf16) take no part in the instructions; rows and features that hold any
+// get those terms added in float32 at the end, so that infinities and NaN come out as from multiply-adds.
+#include "qkv_rope.cuh"
+#include "tcgen05.cuh"
+
+namespace dl {
+
+constexpr int GS_SLICE = 64;                                // k of a slice
+constexpr int GS_PARTS = 16;
+
+__host__ __device__ inline int gs_slices(int K) { return (K + GS_SLICE - 1) / GS_SLICE; }
+__host__ __device__ inline int gs_part(int K) { return (gs_slices(K) + GS_PARTS - 1) / GS_PARTS; }      // slices of a sixteenth
+
+// ---- the split --------------------------------------------------------------------------------------------------
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<const unsigned long long*>(&a)),
+      "l"(*reinterpret_cast<const unsigned long long*>(&b)));
+  return *reinterpret_cast<float2*>(&r);
+}
+// a - (the first, the second of the packed pair), both differences exact where it is a rounded to bf16
+__device__ __forceinline__ float2 left_over(float2 a, uint32_t pair) {
+  float2 r;
+  asm("{\n\t.reg .b16 x, y, m;\n\tmov.b32 {x, y}, %2;\n\tmov.b16 m, 0xbf80;\n\t"      // -1
+      "fma.rn.f32.bf16 %0, x, m, %3;\n\tfma.rn.f32.bf16 %1, y, m, %4;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "r"(pair), "f"(a.x), "f"(a.y));
+  return r;
+}
+// The upper halves of two words, packed.
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
+// Two numbers split into parts, as packed pairs: the first rounded, the second cut off the rest. `odd` (two bf16) becomes NaN
+// where one of the numbers has no finite parts.
+__device__ __forceinline__ void split2(float2 a, uint32_t& hi, uint32_t& mid, uint32_t& lo, uint32_t& odd) {
+  hi = pack2_bf16(a.x, a.y);
+  a = left_over(a, hi);
+  mid = upper_halves(a.x, a.y);
+  a.x -= __uint_as_float(__float_as_uint(a.x) & 0xffff0000u);
+  a.y -= __uint_as_float(__float_as_uint(a.y) & 0xffff0000u);
+  lo = upper_halves(a.x, a.y);
+  asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(odd) : "r"(lo), "r"(0u));
+}
+// Whether a number's parts are finite.
+__device__ __forceinline__ bool has_parts(float v) { return fabsf(__bfloat162float(__float2bfloat16_rn(v))) < INFINITY; }
+// Splits 16 numbers.
+__device__ __forceinline__ void split16(const float4 (&v)[4], uint32_t (&hi)[8], uint32_t (&mid)[8], uint32_t (&lo)[8], uint32_t& odd) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    split2(make_float2(v[i].x, v[i].y), hi[2 * i], mid[2 * i], lo[2 * i], odd);
+    split2(make_float2(v[i].z, v[i].w), hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1], odd);
+  }
+}
+// Whether anything was odd (else both halves are zeros, of either sign).
+__device__ __forceinline__ bool is_odd(uint32_t odd) { return (odd & 0x7fff7fffu) != 0; }
+__device__ __forceinline__ float4 with_parts(float4 v) {
+  return make_float4(has_parts(v.x) ? v.x : 0.0f, has_parts(v.y) ? v.y : 0.0f, has_parts(v.z) ? v.z : 0.0f, has_parts(v.w) ? v.w : 0.0f);
+}
+// The terms of a row of x and a row of W in which a number has no finite parts, in float32.
+__device__ __forceinline__ float gs_odd_terms(const float* x, const float* w, int k, int k_end) {
+  float t = 0.0f;
+#pragma unroll 1
+  for (; k < k_end && t == t; ++k)
+    if (!has_parts(x[k]) || !has_parts(w[k])) t = fmaf(x[k], w[k], t);
+  return t;
+}
+
+// ---- few rows -----------------------------------------------------------------------------------------------------
+//
+// Bound by the bytes of W, then by the instructions that split them. A block owns 16 features and up to 8 NT rows, each of
+// its warps one sixteenth of k or two. A lane copies the pieces of W and x that its own instructions need (16 bytes: four of
+// k) into a ring of its own in shared memory, half a slice at a time, so nothing is shared before the end; the first halves
+// of W are asked for before the wait on the kernel in front. Within a step of 16 k the four of a lane stand for the k that the
+// instruction gives that lane, in W and x alike.
+
+constexpr int GR_STAGES = 3;
+constexpr int GR_FEATS = 16;
+template <int NT> __host__ __device__ constexpr int gr_stage_pieces() { return 4 + 2 * NT; }      // 16 bytes a lane
+template <int NT, int WARPS> __host__ __device__ constexpr int gr_smem() {
+  return WARPS * GR_STAGES * gr_stage_pieces<NT>() * 512 + GS_PARTS * 8 * NT * GR_FEATS * 4;
+}
+
+__device__ __forceinline__ void gs_copy16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gs_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// ROPE: the q | k | v projection with the rotary encoding and the cache write on its way out (qkv_rope.cuh): a block of a q or k
+// head holds eight rotary pairs, features f and f + head_dim / 2. y takes the queries.
+template <int NT, int WARPS, bool ROPE>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 && NT == 1 ? 2 : 1)
+gemm_split_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ bias,
+                       float* __restrict__ y, int ldy, int M, int N, int K, float out_scale, const QkvRopeOf<float> rope) {
+  constexpr int PIECES = gr_stage_pieces<NT>(), ROWS = 8 * NT, FEATS = GR_FEATS, OWN = GS_PARTS / WARPS;
+  extern __shared__ __align__(16) float4 gr_smem_raw[];
+  x += static_cast<size_t>(blockIdx.y) * ROWS * ldx;
+  y += static_cast<size_t>(blockIdx.y) * ROWS * ldy;
+  M -= blockIdx.y * ROWS;
+  __shared__ int w_odd[FEATS], x_odd[ROWS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  // the block's features: eight from n0 on, eight from n1 on
+  int n0 = blockIdx.x * FEATS, n1 = n0 + 8, head = 0;
+  bool turned = false;
+  if constexpr (ROPE) {
+    const int per_head = rope.head_dim / FEATS;
+    head = blockIdx.x / per_head;                    // q heads, then k heads, then v heads
+    turned = head < rope.n_heads + rope.n_kv_heads;
+    if (turned) {
+      n0 = head * rope.head_dim + blockIdx.x % per_head * 8;
+      n1 = n0 + rope.head_dim / 2;
+    }
+  }
+  const int part = gs_part(K);
+  const int begin = min(gs_slices(K), warp * OWN * part), end = min(gs_slices(K), begin + OWN * part);
+  const int halves = 2 * (end - begin);
+  float4* ring = gr_smem_raw + warp * GR_STAGES * PIECES * 32 + lane;
+  float* sums = reinterpret_cast<float*>(gr_smem_raw + WARPS * GR_STAGES * PIECES * 32);      // [GS_PARTS][ROWS][FEATS]
+  if (threadIdx.x < FEATS) w_odd[threadIdx.x] = 0;
+  if (threadIdx.x < ROWS) x_odd[threadIdx.x] = 0;
+  __syncthreads();
+
+  // a half slice: of two features and of NT rows, two steps of 16 k each
+  const int k0 = begin * GS_SLICE + 4 * t;
+  const float* w_row[2];
+  const float* x_row[NT];
+  int x_bytes[NT];                                   // rows past M: zeros
+#pragma unroll
+  for (int i = 0; i < 2; ++i) w_row[i] = w + static_cast<size_t>(min((i ? n1 : n0) + g, N - 1)) * K + k0;
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    x_bytes[i] = 8 * i + g < M ? 16 : 0;
+    x_row[i] = x + (8 * i + g < M ? static_cast<size_t>(8 * i + g) * ldx : 0) + k0;
+  }
+  const uint32_t ring_at = smem_u32(ring);
+  const int whole = (K - begin * GS_SLICE) / 32;     // half slices before the one that k's end cuts short
+  auto load_w = [&](int h) {
+    const uint32_t to = ring_at + (h % GR_STAGES) * (PIECES * 512);
+    if (h < whole) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) gs_copy16(to + i * 512, w_row[i & 1] + h * 32 + (i >> 1) * 16, 16);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = h * 32 + (i >> 1) * 16;
+        gs_copy16(to + i * 512, k0 + k < K ? w_row[i & 1] + k : w, k0 + k < K ? 16 : 0);
+      }
+    }
+  };
+  auto load_x = [&](int h) {
+    const uint32_t to = ring_at + (h % GR_STAGES) * (PIECES * 512) + 4 * 512;
+    if (h < whole) {
+#pragma unroll
+      for (int i = 0; i < 2 * NT; ++i) gs_copy16(to + i * 512, x_row[i >> 1] + h * 32 + (i & 1) * 16, x_bytes[i >> 1]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2 * NT; ++i) {
+        const int k = h * 32 + (i & 1) * 16;
+        gs_copy16(to + i * 512, k0 + k < K ? x_row[i >> 1] + k : x, k0 + k < K ? x_bytes[i >> 1] : 0);
+      }
+    }
+  };
+  for (int h = 0; h < min(halves, GR_STAGES - 1); ++h) load_w(h);
+  pdl_wait();
+  pdl_trigger();
+  for (int h = 0; h < GR_STAGES - 1; ++h) {          // (the first group holds all of W that was asked for ahead)
+    if (h < halves) load_x(h);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  float sum[NT][4];
+  auto zero_sums = [&]() {
+#pragma unroll
+    for (int n = 0; n < NT; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0.0f;
+  };
+  auto keep_sums = [&](int p) {
+    float* to = sums + p * ROWS * FEATS;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) to[(n * 8 + 2 * t + (j & 1)) * FEATS + g + 8 * (j >> 1)] = sum[n][j];
+    zero_sums();
+  };
+  zero_sums();
+  int p = warp * OWN, left = part;
+  uint32_t wp[3][4][4], xp[3][NT][4][2];         // [part][step]
+#pragma unroll 1
+  for (int h = 0; h < halves; h += 2) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (h + i + GR_STAGES - 1 < halves) {
+        load_w(h + i + GR_STAGES - 1);
+        load_x(h + i + GR_STAGES - 1);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group %0;" ::"n"(GR_STAGES - 1) : "memory");
+      const float4* from = ring + (h + i) % GR_STAGES * PIECES * 32;
+      auto split = [&](auto read) {
+        uint32_t w_bad = 0, x_bad = 0, hi[8], mid[8], lo[8];
+        // feature g, step 0; g + 8; the same at step 1
+        const float4 v[4] = {read(from[0]), read(from[32]), read(from[64]), read(from[96])};
+        split16(v, hi, mid, lo, w_bad);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int s = 2 * i + j / 4, r = (j >> 1 & 1) + 2 * (j & 1);
+          wp[0][s][r] = hi[j], wp[1][s][r] = mid[j], wp[2][s][r] = lo[j];
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {              // a step
+            const float4 u = read(from[(4 + 2 * n + k) * 32]);
+            split2(make_float2(u.x, u.y), xp[0][n][2 * i + k][0], xp[1][n][2 * i + k][0], xp[2][n][2 * i + k][0], x_bad);
+            split2(make_float2(u.z, u.w), xp[0][n][2 * i + k][1], xp[1][n][2 * i + k][1], xp[2][n][2 * i + k][1], x_bad);
+          }
+        return make_uint2(w_bad, x_bad);
+      };
+      const uint2 bad = split([](float4 v) { return v; });
+      if (is_odd(bad.x | bad.y)) {                   // again, with zeros in the place of the odd numbers
+        if (is_odd(bad.x)) w_odd[g] = w_odd[g + 8] = 1;
+        if (is_odd(bad.y)) {
+#pragma unroll
+          for (int n = 0; n < NT; ++n) x_odd[8 * n + g] = 1;
+        }
+        split([](float4 v) { return with_parts(v); });
+      }
+    }
+    float d[NT][4];
+    auto product = [&](int pw, int px, bool opens) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          if (opens && s == 0) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
+          gs_mma(d[n], wp[pw][s], xp[px][n][s][0], xp[px][n][s][1]);
+        }
+    };
+    product(2, 0, true);
+    product(0, 2, false);
+    product(1, 1, false);
+    product(1, 0, false);
+    product(0, 1, false);
+    product(0, 0, false);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[n][j] += d[n][j];
+    if (--left == 0) keep_sums(p++), left = part;
+  }
+  // the sixteenths that k's end cuts short or leaves empty
+  for (; p < (warp + 1) * OWN; ++p) keep_sums(p);
+  __syncthreads();
+  auto total = [&](int m, int f, int n) {
+    float v = sums[m * FEATS + f];
+#pragma unroll
+    for (int e = 1; e < GS_PARTS; ++e) v += sums[(e * ROWS + m) * FEATS + f];
+    if (w_odd[f] | x_odd[m]) v += gs_odd_terms(x + static_cast<size_t>(m) * ldx, w + static_cast<size_t>(n) * K, 0, K);
+    return v;
+  };
+  if constexpr (ROPE) {
+    for (int i = threadIdx.x; i < ROWS * 8; i += WARPS * 32) {
+      const int f = i & 7, m = i >> 3, hd = rope.head_dim;
+      if (m >= M) continue;
+      float a = total(m, f, n0 + f), b = total(m, f + 8, n1 + f);
+      const int pos = rope.positions[m], in_head = n0 + f - head * hd;
+      if (turned) {
+        const float theta = static_cast<float>(pos) * rope.pos_scale * rope.inv_freq[in_head];
+        float s, c;
+        sincosf(theta, &s, &c);
+        const float ra = a * c - b * s, rb = a * s + b * c;
+        a = ra, b = rb;
+      }
+      float* to;
+      if (head < rope.n_heads) {
+        to = y + static_cast<size_t>(m) * ldy + n0 + f;
+      } else {
+        const size_t slot = qkv_rope_slot(rope, m, pos);
+        if (slot == QKV_NO_SLOT) continue;
+        const int kvh = head - rope.n_heads - (turned ? 0 : rope.n_kv_heads);
+        to = (turned ? rope.k_cache : rope.v_cache) + (slot * rope.n_kv_heads + kvh) * hd + in_head;
+      }
+      to[0] = a;
+      to[n1 - n0] = b;
+    }
+  } else {
+    for (int i = threadIdx.x; i < ROWS * FEATS; i += WARPS * 32) {
+      const int f = i % FEATS, m = i / FEATS, n = n0 + f;
+      if (m >= M || n >= N) continue;
+      float v = total(m, f, n);
+      if (bias != nullptr) v += bias[n];
+      y[static_cast<size_t>(m) * ldy + n] = v * out_scale;
+    }
+  }
+}
+
+// ---- more rows --------------------------------------------------------------------------------------------------
+//
+// The product is computed transposed (y^T = W x^T): 128 features are the M side of an instruction and 16 to 128 rows its N
+// side. The parts of x are made by a kernel in front (gemm_split_parts_kernel: they are read by every block of features),
+// those of W here. Either a block walks all of k, or the eight blocks of a cluster take two sixteenths each and add up through
+// distributed shared memory. Roles of a block:
+//   warp 0          TMA: float32 slices of W (128 x 64); the first ones before the wait on the kernel in front
+//   warp 2          TMA: slices of the three parts of x (rows x 64)
+//   warp 1          issues the instructions and commits them, slice by slice (two accumulators)
+//   warps 4 .. 7    split W: a thread holds a feature's slice, and its three parts go to tensor memory, from where the
+//                   instructions read them
+//   warps 8 .. 15   add a slice's accumulator to the sums (a thread: a feature, half the rows) and store y
+// What bounds it: the instructions (six for one of a bf16 product, 4,096 multiply-adds a cycle and SM: 1,536 cycles a slice of 128
+// rows), and between them the chain from one slice's end over the next but one's split (about 1,400 cycles) to its start; a slice
+// takes 2,100. With the splitting and the adding up done by the same warps, one after the other, it took 2,600, with x split
+// here as well 3,200.
+
+constexpr int GS_BF = 128;                                  // features of a block
+constexpr int GS_ROWS = 128;                                // the most rows of a tile
+constexpr int GS_THREADS = 512;
+constexpr int GS_CLUSTER = 8;
+constexpr int GS_MAX_STAGES = 6;
+constexpr uint32_t GS_W_BYTES = GS_BF * GS_SLICE * 4;       // 32 KiB, two boxes of 32 k
+constexpr uint32_t GS_FEW_X_BYTES = 16 * GS_SLICE * 4;     // 4 KiB, as W
+constexpr uint32_t GS_A_COLS = 3 * GS_SLICE / 2;            // tensor-memory columns of a slice's three parts of W
+constexpr uint32_t GS_SMEM = 232448, GS_FIXED = 1024 /* alignment */ + 512 /* barriers, flags */;
+enum { GS_ERR_W_COPY = 61, GS_ERR_X_COPY = 62, GS_ERR_MMA = 63, GS_ERR_SUMS = 64, GS_ERR_SPLIT = 65 };
+__host__ __device__ constexpr uint32_t gs_part_bytes(int rows) { return rows * GS_SLICE * 2; }
+
+// Three parts of every row of x, [3][M][pitch] bf16 (zeros behind K), and whether the row holds a number without finite parts.
+__global__ void __launch_bounds__(256)
+gemm_split_parts_kernel(const float* __restrict__ x, int ldx, int K, bf16* __restrict__ parts, int pitch, int* __restrict__ odd_rows) {
+  const float* row = x + static_cast<size_t>(blockIdx.x) * ldx;
+  const size_t stride = static_cast<size_t>(gridDim.x) * pitch;
+  bf16* to = parts + static_cast<size_t>(blockIdx.x) * pitch;
+  pdl_wait();
+  pdl_trigger();
+  int odd = 0;
+  for (int k = threadIdx.x * 8; k < pitch; k += 256 * 8) {
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v[2] = {*reinterpret_cast<const float4*>(row + k), k + 4 < K ? *reinterpret_cast<const float4*>(row + k + 4) : zero};
+    uint32_t hi[4], mid[4], lo[4];
+    uint32_t bad = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      split2(make_float2(v[i].x, v[i].y), hi[2 * i], mid[2 * i], lo[2 * i], bad);
+      split2(make_float2(v[i].z, v[i].w), hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1], bad);
+    }
+    if (is_odd(bad)) {
+      odd = 1;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float4 kept = with_parts(v[i]);
+        split2(make_float2(kept.x, kept.y), hi[2 * i], mid[2 * i], lo[2 * i], bad);
+        split2(make_float2(kept.z, kept.w), hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1], bad);
+      }
+    }
+    *reinterpret_cast<uint4*>(to + k) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(to + stride + k) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    *reinterpret_cast<uint4*>(to + 2 * stride + k) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+  odd = __syncthreads_or(odd);
+  if (threadIdx.x == 0) odd_rows[blockIdx.x] = odd;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+               "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+               : "memory");
+}
+template <int REGS> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
+template <int REGS> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
+
+__device__ __forceinline__ float cluster_read(uint32_t addr, int rank) {
+  uint32_t at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
+struct GsArgs {
+  const float* x;
+  const float* w;
+  const float* bias;
+  float* y;
+  int* status;
+  int ldx, ldy, M, N, K;
+  const int* odd_rows;
+  int rows;            // rows of a tile (a multiple of 16)
+  int row_tiles, tiles, stages;
+  int cluster;         // blocks that share a tile's k: 1 or 8
+  int gated;           // FEW: 0, or the number F of gate rows of W = [gate; up]; y = silu(x Wg^T) (x Wu^T)
+  float out_scale;
+};
+
+// FEW: up to 16 rows (a.rows is 16), whose parts the block makes itself: warps 4 .. 7 and 12 .. 15 split half a slice of W each,
+// warps 8 .. 11 split x and add up. Bound by W's bytes: 134 MB (16 x 16384 x 2048) take 27.5 us, 21 of them the stream at 6.2 TB/s
+// and the rest the block's start. (x came by plain loads at first: 35 us, since a trip to L2 takes long beside that stream; four
+// slices at once instead of two, or 147 tiles of 112 features instead of 128: nothing.)
+template <bool FEW>
+__global__ void __launch_bounds__(GS_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const GsArgs a) {
+  constexpr int TMEM_COLS = 512;
+  constexpr int DEPTH = 2, ACC_COLS = FEW ? 16 : GS_ROWS;      // slices on their way at once, columns of an accumulator
+  constexpr uint32_t A_COL = DEPTH * ACC_COLS;
+  extern __shared__ unsigned char gs_raw[];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gs_raw) + 1023) & ~uintptr_t(1023));
+  const int rows = a.rows, stages = a.stages;
+  const uint32_t part_bytes = gs_part_bytes(rows);
+  unsigned char* x_ring = ring + stages * GS_W_BYTES;                             // FEW: [stages] of GS_FEW_X_BYTES
+  unsigned char* parts = x_ring + (FEW ? stages * GS_FEW_X_BYTES : 0);            // [DEPTH][3] of part_bytes
+  uint64_t* bars = reinterpret_cast<uint64_t*>(parts + 3 * DEPTH * part_bytes);
+  uint64_t* w_full = bars;                           // [stages] a slice of W has come
+  uint64_t* w_empty = bars + GS_MAX_STAGES;          // [stages] it is split
+  uint64_t* x_full = bars + 2 * GS_MAX_STAGES;       // [DEPTH] a slice of x's parts has come; FEW: [stages] a slice of x
+  uint64_t* ready = x_full + GS_MAX_STAGES;                  // [DEPTH] a slice's parts of W (FEW: and x) lie where the instructions read them
+  uint64_t* done = ready + DEPTH;                    // [DEPTH] its instructions have completed
+  uint64_t* drained = ready + 2 * DEPTH;             // [DEPTH] its accumulator has been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ready + 3 * DEPTH);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile unsigned char* w_odd = reinterpret_cast<volatile unsigned char*>(tmem_slot + 2);      // [GS_BF]
+  volatile unsigned char* x_odd = w_odd + GS_BF;                                                 // [16], FEW
+  float* exchange = reinterpret_cast<float*>(parts + 3 * DEPTH * part_bytes + 512);  // [16][GS_BF], FEW and gated
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = a.cluster > 1 ? static_cast<int>(cluster_rank()) : 0;
+  const int first_tile = static_cast<int>(blockIdx.x) / a.cluster, tile_step = static_cast<int>(gridDim.x) / a.cluster;
+  const int slices = gs_slices(a.K), part = gs_part(a.K);
+  const int begin = min(slices, rank * 2 * part), end = a.cluster > 1 ? min(slices, begin + 2 * part) : slices;
+  const int per_tile = end - begin;
+  const int my_tiles = first_tile < a.tiles ? (a.tiles - first_tile + tile_step - 1) / tile_step : 0;
+  const int total = my_tiles * per_tile;             // slices this block works through
+
+  if (threadIdx.x == 0) {
+    prefetch_tensor_map(&map_w);
+    prefetch_tensor_map(&map_x);
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&w_full[s], 1);
+      mbar_init(&w_empty[s], FEW ? 12 : 4);
+      if (FEW) mbar_init(&x_full[s], 1);
+    }
+    for (int b = 0; b < DEPTH; ++b) {
+      if (!FEW) mbar_init(&x_full[b], 1);
+      mbar_init(&ready[b], FEW ? 12 : 4);
+      mbar_init(&done[b], 1);
+      mbar_init(&drained[b], FEW ? 4 : 8);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // a slice of W: its tile, its number in the tile, its place in the ring
+  struct At {
+    int tile, c, s;
+  };
+  auto next = [&](At& at) {
+    if (++at.c == per_tile) at.c = 0, at.tile += tile_step;
+    if (++at.s == stages) at.s = 0;
+  };
+  auto load_w = [&](const At& at) {
+    const int k = (begin + at.c) * GS_SLICE, n0 = FEW && a.gated ? at.tile * (GS_BF / 2) : at.tile / a.row_tiles * GS_BF;
+    const int n1 = FEW && a.gated ? a.gated + n0 : n0 + GS_BF / 2;      // of the tile's second 64 features
+    unsigned char* to = ring + at.s * GS_W_BYTES;
+    mbar_expect_tx(&w_full[at.s], GS_W_BYTES);
+    tma_load_2d(to, &map_w, k, n0, &w_full[at.s]);
+    tma_load_2d(to + GS_W_BYTES / 4, &map_w, k, n1, &w_full[at.s]);
+    tma_load_2d(to + GS_W_BYTES / 2, &map_w, k + 32, n0, &w_full[at.s]);
+    tma_load_2d(to + GS_W_BYTES * 3 / 4, &map_w, k + 32, n1, &w_full[at.s]);
+  };
+  const int ahead = min(total, stages);
+  if (warp == 0) {                                   // (the thread that made the barriers asks for the first slices at once)
+    At at = {first_tile, 0, 0};
+    __syncwarp();
+    if (lane == 0)
+      for (int g = 0; g < ahead; ++g, next(at)) load_w(at);
+    __syncwarp();
+  }
+  if (threadIdx.x < GS_BF + 16) w_odd[threadIdx.x] = 0;
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_before_sync();
+  __syncthreads();
+  tcgen05_after_sync();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp < 4) {
+    fewer_registers<40>();
+    if (warp == 0) {
+      auto load_x = [&](const At& at) {              // FEW
+        const int k = (begin + at.c) * GS_SLICE;
+        unsigned char* to = x_ring + at.s * GS_FEW_X_BYTES;
+        mbar_expect_tx(&x_full[at.s], GS_FEW_X_BYTES);
+        tma_load_2d(to, &map_x, k, 0, &x_full[at.s]);
+        tma_load_2d(to + GS_FEW_X_BYTES / 2, &map_x, k + 32, 0, &x_full[at.s]);
+      };
+      pdl_wait();
+      pdl_trigger();
+      At at = {first_tile, 0, 0};
+      for (int g = 0; g < ahead; ++g, next(at))
+        if (FEW && elect_one()) load_x(at);
+      __syncwarp();
+      uint32_t parity = 0;
+      for (int g = ahead; g < total; ++g) {
+        if (!warp_wait(&w_empty[at.s], parity, a.status, GS_ERR_W_COPY, abort_flag)) break;
+        if (elect_one()) {
+          load_w(at);
+          if (FEW) load_x(at);
+        }
+        __syncwarp();
+        next(at);
+        if (at.s == 0) parity ^= 1;
+      }
+    } else {
+      pdl_wait();
+      pdl_trigger();
+      if (warp == 2 && !FEW) {
+        int tile = first_tile, c = 0;
+        for (int g = 0; g < total; ++g) {
+          const int b = g % DEPTH;
+          if (g >= DEPTH && !warp_wait(&done[b], (g / DEPTH & 1) ^ 1, a.status, GS_ERR_X_COPY, abort_flag)) break;
+          if (elect_one()) {
+            mbar_expect_tx(&x_full[b], 3 * part_bytes);
+            for (int p = 0; p < 3; ++p)
+              tma_load_2d(parts + (3 * b + p) * part_bytes, &map_x, (begin + c) * GS_SLICE, p * a.M + tile % a.row_tiles * rows, &x_full[b]);
+          }
+          __syncwarp();
+          if (++c == per_tile) c = 0, tile += tile_step;
+        }
+      } else if (warp == 1) {
+        const uint32_t idesc = umma_idesc(GS_BF, rows);
+        const uint64_t desc0 = umma_desc_sw128(smem_u32(parts));
+        const uint32_t step = part_bytes >> 4;
+        for (int g = 0; g < total; ++g) {
+          const uint32_t b = g % DEPTH, par = g / DEPTH & 1;
+          if (g >= DEPTH && !warp_wait(&drained[b], par ^ 1, a.status, GS_ERR_MMA, abort_flag)) break;
+          if (!FEW && !warp_wait(&x_full[b], par, a.status, GS_ERR_MMA, abort_flag)) break;
+          if (!warp_wait(&ready[b], par, a.status, GS_ERR_MMA, abort_flag)) break;
+          tcgen05_after_sync();
+          if (elect_one()) {
+            const uint32_t acc = tmem + b * ACC_COLS, w0 = tmem + A_COL + b * GS_A_COLS;
+            const uint64_t x0 = desc0 + 3 * b * step;
+            auto product = [&](int wp, int xp, uint32_t adds) {
+#pragma unroll
+              for (int k = 0; k < GS_SLICE / 16; ++k)
+                umma_bf16_ts(acc, w0 + wp * (GS_SLICE / 2) + 8 * k, x0 + xp * step + 2 * k, idesc, k > 0 ? 1u : adds);
+            };
+            product(2, 0, 0u);
+            product(0, 2, 1u);
+            product(1, 1, 1u);
+            product(1, 0, 1u);
+            product(0, 1, 1u);
+            product(0, 0, 1u);
+            umma_commit(&done[b]);
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else if (warp < 8 || (FEW && warp >= 12)) {
+    if constexpr (!FEW) fewer_registers<112>();
+    constexpr int PIECES = FEW ? 2 : 4;              // 16 of k each
+    const int f = (warp & 3) * 32 + lane, first = FEW && warp >= 12 ? 2 : 0;
+    int s = 0;
+    uint32_t parity = 0;
+    for (int g = 0; g < total; ++g) {
+      const uint32_t b = g % DEPTH;
+      // the place in tensor memory was slice g - DEPTH's: its instructions must have completed
+      if (g >= DEPTH && !warp_wait(&done[b], (g / DEPTH & 1) ^ 1, a.status, GS_ERR_SPLIT, abort_flag)) break;
+      if (!warp_wait(&w_full[s], parity, a.status, GS_ERR_SPLIT, abort_flag)) break;
+      tcgen05_after_sync();
+      const uint32_t at = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + A_COL + b * GS_A_COLS + 8 * first;
+      auto split = [&](auto read) {
+        uint32_t odd = 0;
+#pragma unroll
+        for (int c = 0; c < PIECES; c += 2) {
+          const unsigned char* row = ring + s * GS_W_BYTES + ((first + c) >> 1) * (GS_W_BYTES / 2) + f * 128;
+          uint32_t hi[16], mid[16], lo[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 v = read(*reinterpret_cast<const float4*>(row + ((i ^ (f & 7)) << 4)));
+            split2(make_float2(v.x, v.y), hi[2 * i], mid[2 * i], lo[2 * i], odd);
+            split2(make_float2(v.z, v.w), hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1], odd);
+          }
+          tmem_st16(at + 8 * c, hi);
+          tmem_st16(at + GS_SLICE / 2 + 8 * c, mid);
+          tmem_st16(at + GS_SLICE + 8 * c, lo);
+        }
+        return is_odd(odd);
+      };
+      const bool odd = split([](float4 v) { return v; });
+      if (__any_sync(0xffffffffu, odd)) {            // again, with zeros in the place of the odd numbers
+        if (odd) w_odd[f] = 1;
+        split([](float4 v) { return with_parts(v); });
+      }
+      tmem_st_wait();
+      tcgen05_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&ready[b]);
+        mbar_arrive(&w_empty[s]);
+      }
+      if (++s == stages) s = 0, parity ^= 1;
+    }
+    pdl_wait();
+    pdl_trigger();
+  } else {
+    if constexpr (!FEW) more_registers<176>();
+    pdl_wait();
+    pdl_trigger();
+    constexpr int COLS = FEW ? 16 : GS_ROWS / 2;     // the most rows a thread adds up
+    const int half = FEW ? 0 : (warp - 8) >> 2, f = (warp & 3) * 32 + lane, cols = FEW ? 16 : rows / 2;
+    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    float2 sum[COLS / 2], all[COLS / 2];       // of the running sixteenth, and of those before it
+    int tile = first_tile, c = begin, left = part;
+#pragma unroll
+    for (int j = 0; j < COLS / 2; ++j) sum[j] = all[j] = make_float2(0.0f, 0.0f);
+    // FEW: a thread splits eight numbers of a row of x
+    int xs = 0;                                      // the next slice's place in the ring
+    uint32_t x_parity = 0;
+    auto split_x = [&](uint32_t b) -> bool {
+      if (!warp_wait(&x_full[xs], x_parity, a.status, GS_ERR_SUMS, abort_flag)) return false;
+      const int r = (threadIdx.x & 127) >> 3, c = threadIdx.x & 7;
+      const unsigned char* from = x_ring + xs * GS_FEW_X_BYTES + (c >> 2) * (GS_FEW_X_BYTES / 2) + r * 128;
+      float4 v[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) v[i] = *reinterpret_cast<const float4*>(from + (((2 * (c & 3) + i) ^ (r & 7)) << 4));
+      uint32_t hi[4], mid[4], lo[4], odd = 0;
+      auto split = [&]() {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          split2(make_float2(v[i].x, v[i].y), hi[2 * i], mid[2 * i], lo[2 * i], odd);
+          split2(make_float2(v[i].z, v[i].w), hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1], odd);
+        }
+      };
+      split();
+      if (is_odd(odd)) {
+        x_odd[r] = 1;
+        v[0] = with_parts(v[0]), v[1] = with_parts(v[1]);
+        split();
+      }
+      unsigned char* to = parts + 3 * b * part_bytes + r * 128 + ((c ^ (r & 7)) << 4);
+      *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(to + part_bytes) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+      *reinterpret_cast<uint4*>(to + 2 * part_bytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&ready[b]);
+        mbar_arrive(&w_empty[xs]);
+      }
+      if (++xs == stages) xs = 0, x_parity ^= 1;
+      return true;
+    };
+    bool ok = true;
+    if (FEW) {
+#pragma unroll 1
+      for (int g = 0; g < min(total, DEPTH) && ok; ++g) ok = split_x(g);      // (the first slices' places are free)
+    }
+#pragma unroll 1
+    for (int g = 0; g < total && ok; ++g) {
+      const uint32_t b = g % DEPTH;
+      if (!warp_wait(&done[b], g / DEPTH & 1, a.status, GS_ERR_SUMS, abort_flag)) break;
+      tcgen05_after_sync();
+      const uint32_t at = tmem + lanes + b * ACC_COLS + half * cols;
+#pragma unroll
+      for (int j = 0; j < COLS; j += 32) {
+        if (j >= cols) break;
+        uint32_t v[32];
+        tmem_ld32(at + j, v);                        // (columns past cols: any number, never used)
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16 && j / 2 + i < COLS / 2; ++i)
+          sum[j / 2 + i] = add2(sum[j / 2 + i], make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+      }
+      tcgen05_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&drained[b]);
+      if (FEW && g + DEPTH < total) ok = split_x(b);          // slice g's instructions have completed: its place is free
+      --left;
+      ++c;
+      if (left != 0 && c != end) continue;
+      // the end of a sixteenth (of a cluster's two the second stays in `sum`)
+      const bool second = a.cluster > 1 && c > begin + part;
+      if (!second) {
+#pragma unroll
+        for (int j = 0; j < COLS / 2; ++j) all[j] = add2(all[j], sum[j]), sum[j] = make_float2(0.0f, 0.0f);
+      }
+      left = part;
+      if (c != end) continue;
+      // the end of the tile: y, or for the cluster's sum [sixteenth][row][feature] in place of the rings
+      const bool gated = FEW && a.gated != 0;
+      const bool shared = a.cluster > 1 || gated;
+      const int n = gated ? (f < GS_BF / 2 ? tile * (GS_BF / 2) + f : a.gated + tile * (GS_BF / 2) + f - GS_BF / 2)
+                          : tile / a.row_tiles * GS_BF + f;
+      const int m0 = tile % a.row_tiles * rows + half * cols;
+      const int here = shared ? cols : n < a.N ? min(cols, a.M - m0) : 0;
+      float* to = gated ? exchange + f : shared ? reinterpret_cast<float*>(ring) + half * cols * GS_BF + f : a.y + static_cast<size_t>(m0) * a.ldy + n;
+      const int pitch = shared ? GS_BF : a.ldy;
+      const float bias = !shared && a.bias != nullptr && n < a.N ? a.bias[n] : 0.0f, scale = shared ? 1.0f : a.out_scale;
+#pragma unroll
+      for (int j = 0; j < COLS; ++j)
+        if (j < here) to[static_cast<size_t>(j) * pitch] = ((j & 1 ? all[j / 2].y : all[j / 2].x) + bias) * scale;
+      if (!FEW && shared) {
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+          if (j < here) to[static_cast<size_t>(rows + j) * pitch] = j & 1 ? sum[j / 2].y : sum[j / 2].x;
+      }
+      bool odd = w_odd[f] != 0;
+      for (int j = lane; j < cols; j += 32) odd |= FEW ? x_odd[j] != 0 : m0 + j < a.M && a.odd_rows[m0 + j] != 0;
+      if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll 1
+        for (int j = 0; j < here; ++j)
+          if (n < a.N && m0 + j < a.M && (w_odd[f] != 0 || (FEW ? x_odd[j] != 0 : a.odd_rows[m0 + j] != 0)))
+            to[static_cast<size_t>(j) * pitch] += scale * gs_odd_terms(a.x + static_cast<size_t>(m0 + j) * a.ldx, a.w + static_cast<size_t>(n) * a.K,
+                                                                       begin * GS_SLICE, min(a.K, end * GS_SLICE));
+      }
+      if (gated) {                                   // (one warpgroup adds up)
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int n0 = tile * (GS_BF / 2), fo = threadIdx.x & 63;
+        for (int j = (threadIdx.x & 127) >> 6; j < a.M; j += 2)
+          if (n0 + fo < a.gated) {
+            const float gate = exchange[j * GS_BF + fo];
+            a.y[static_cast<size_t>(j) * a.ldy + n0 + fo] = gate / (1.0f + expf(-gate)) * exchange[j * GS_BF + GS_BF / 2 + fo];
+          }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      }
+#pragma unroll
+      for (int j = 0; j < COLS / 2; ++j) all[j] = make_float2(0.0f, 0.0f);
+      tile += tile_step, c = begin;
+    }
+  }
+  // common exit: every role arrives here, with or without a timeout
+  drain_after_abort(abort_flag);
+  tcgen05_before_sync();
+  __syncthreads();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  if (a.cluster > 1) {
+    // every block of the cluster adds up the sixteenths of 16 features
+    pdl_wait();                                                // (a block without any k has not waited yet)
+    cluster_sync_all();
+    const int have = (slices + part - 1) / part;               // sixteenths that hold any k
+    const int n0 = first_tile / a.row_tiles * GS_BF, m0 = first_tile % a.row_tiles * rows;
+    for (int i = threadIdx.x; i < rows * 16; i += GS_THREADS) {
+      const int f = rank * 16 + (i & 15), r = i >> 4, n = n0 + f, m = m0 + r;
+      if (n >= a.N || m >= a.M) continue;
+      const uint32_t at = smem_u32(reinterpret_cast<float*>(ring) + r * GS_BF + f);
+      float got[GS_PARTS];
+#pragma unroll
+      for (int e = 0; e < GS_PARTS; ++e)
+        if (e < have) got[e] = cluster_read(at + (e & 1) * rows * GS_BF * 4, e >> 1);
+      float v = got[0];
+#pragma unroll
+      for (int e = 1; e < GS_PARTS; ++e)
+        if (e < have) v += got[e];
+      if (a.bias != nullptr) v += a.bias[n];
+      a.y[static_cast<size_t>(m) * a.ldy + n] = v * a.out_scale;
+    }
+    cluster_sync_all();                                        // nobody leaves while its sums are being read
+  }
+}
+
+// rows x cols of row pitch `ld`, in boxes of box_rows x 128 bytes, 128-byte swizzle, zeros outside
+static inline int gs_map(CUtensorMap* map, const void* base, bool f32, long long rows, int cols, int ld, int box_rows) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (fn == nullptr) return DL_ERR_UNSUPPORTED;
+  const int size = f32 ? 4 : 2;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * size};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / size), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t elem[2] = {1, 1};
+  const CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
+                        dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 700000 + static_cast<int>(r);
+}
+
+template <int NT, int WARPS, bool ROPE = false>
+int gr_launch(const float* x, int ldx, const float* w, const float* bias, float* y, int ldy, int M, int N, int K, float out_scale,
+              cudaStream_t stream, const QkvRopeOf<float>& rope = {}) {
+  auto kernel = gemm_split_rows_kernel<NT, WARPS, ROPE>;
+  constexpr int SMEM = gr_smem<NT, WARPS>();
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return launch_streaming(kernel, dim3((N + GR_FEATS - 1) / GR_FEATS, (M + 8 * NT - 1) / (8 * NT)), dim3(WARPS * 32), SMEM, stream, x, ldx, w,
+                          bias, y, ldy, M, N, K, out_scale, rope);
+}
+
+template <bool FEW>
+int gs_launch(const CUtensorMap& map_w, const CUtensorMap& map_x, GsArgs a, cudaStream_t stream) {
+  const uint32_t other = GS_FIXED + 6 * gs_part_bytes(a.rows) + (FEW ? 16 * GS_BF * 4 : 0);
+  const uint32_t stage = GS_W_BYTES + (FEW ? GS_FEW_X_BYTES : 0);
+  a.stages = static_cast<int>((GS_SMEM - other) / stage);
+  a.stages = a.stages < GS_MAX_STAGES ? a.stages : GS_MAX_STAGES;
+  auto kernel = gemm_split_kernel<FEW>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(GS_SMEM));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.cluster > 1 ? a.tiles * a.cluster : (a.tiles < sm_count() ? a.tiles : sm_count()));
+  cfg.blockDim = dim3(GS_THREADS);
+  cfg.dynamicSmemBytes = other + a.stages * static_cast<size_t>(stage);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (a.cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = a.cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl_mode() >= 1) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x, a));
+}
+
+// How a product is dealt: by the kernel for few rows (in groups of 8 or 16), by the one for many with up to 16 rows whose parts
+// it makes itself, or with parts in scratch, in tiles of `rows` rows, by single blocks or by clusters.
+enum { GS_AUTO = 0, GS_GROUPS = 1, GS_FEW = 2, GS_TILES = 3, GS_CLUSTERS = 4 };
+
+struct GsChoice {
+  int kind, rows;
+};
+
+// The one that costs least, in us. Measured on B200 (weights that lie in memory; before: gemm_simt.cu):
+//   rows x features x k    2048 x 2048    3072 x 2048    16384 x 2048    2048 x 8192    128256 x 2048
+//   1                      11 -> 12       12 -> 12       23 -> 28        15 -> 16       151 -> 166
+//   8                      11 -> 11       13 -> 13       33 -> 28        21 -> 18       234 -> 174
+//   16                     11 -> 11       18 -> 14       61 -> 28        31 -> 23       468 -> 182
+//   64                     36 -> 33       42 -> 36       116 -> 40       118 -> 51      749 -> 256
+//   700                    161 -> 43      251 -> 52      1,049 -> 256    575 -> 138
+//   2,048                  392 -> 92      537 -> 133     2,737 -> 628    1,449 -> 350
+// Few rows: a block of GS_FEW streams all of k for 128 features, so it needs about a block an SM (2048 features by 16 blocks:
+// 22 us against 11 in groups); from there on it is ahead of the groups, which are bound by splitting (16 x 16384 x 2048: 28
+// against 50). Groups of 16 share W in L2; past about 2.6 blocks an SM the tiles are ahead (32 x 2048 x 2048 18 against 35).
+// Tiles: a round of blocks takes `slice` us for every slice of k, by the rows of a tile; a cluster's rounds are an eighth as
+// long, but its blocks are placed late and add up through one another's memory.
+inline GsChoice gs_choose(int M, int N, int K, int sms) {
+  const int blocks = (N + GS_BF - 1) / GS_BF;
+  if (M <= 16 && 5 * blocks >= 4 * sms) return {GS_FEW, 16};
+  const long long groups = static_cast<long long>((N + GR_FEATS - 1) / GR_FEATS) * ((M + 15) / 16);
+  if (M <= 16 || (M <= 64 && 10 * groups <= 26 * sms)) return {GS_GROUPS, 0};
+  static const double slice[] = {0.80, 0.80, 0.82, 0.88, 1.15, 1.20, 1.27, 1.38};       // 16, 32, .. 128 rows
+  GsChoice best = {GS_TILES, 128};
+  double least = 1e300;
+  for (int rows = 16; rows <= GS_ROWS; rows += 16) {
+    if (rows < M && rows < 64) continue;
+    const long long tiles = static_cast<long long>(blocks) * ((M + rows - 1) / rows);
+    const double each = slice[rows / 16 - 1];
+    const double alone = 7.0 + static_cast<double>((tiles + sms - 1) / sms) * gs_slices(K) * each;
+    const double shared = 45.0 + static_cast<double>((tiles * GS_CLUSTER + 127) / 128) * 2 * gs_part(K) * each * 1.9;
+    if (alone < least) least = alone, best = {GS_TILES, rows};
+    if (shared < least) least = shared, best = {GS_CLUSTERS, rows};
+    if (rows >= M) break;
+  }
+  return best;
+}
+
+}  // namespace dl
+
+// x [M, K] (row pitch ldx), w [N, K], y [M, N] (row pitch ldy), bias [N] or null, all float32; x and w 16-byte aligned, K and
+// ldx multiples of 4. parts: scratch of 3 M ceil(K / 8) 8 bf16, 16-byte aligned, and odd_rows: scratch of M ints (both may be null
+// for up to 16 rows). kind: how the work is dealt (see above; 0: what costs least), rows: rows of a tile (a multiple of 16 up to
+// 128; 0: what costs least). status: one device int, set to a nonzero code if a wait inside the kernel timed out.
+DL_EXPORT int dl_gemm_split(const float* x, int ldx, const float* w, const float* bias, float* y, int ldy, int M, int N, int K,
+                            float out_scale, void* parts, int* odd_rows, int kind, int rows, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (K & 3) || (ldx & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || status == nullptr ||
+      kind < 0 || kind > dl::GS_CLUSTERS || rows < 0 || rows > dl::GS_ROWS || (rows & 15) || M > (1 << 28))
+    return DL_ERR_UNSUPPORTED;
+  const dl::GsChoice choice = dl::gs_choose(M, N, K, dl::sm_count());
+  if (kind == dl::GS_AUTO) kind = choice.kind;
+  if (kind == dl::GS_GROUPS) {
+    // sixteen warps where a block has an SM to itself anyway (8 x 2048 x 8192: 18 us, with eight 20)
+    if ((M + 7) / 8 > 65535) return DL_ERR_UNSUPPORTED;
+    if (M > 8) return dl::gr_launch<2, 8>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, stream);
+    if ((N + dl::GR_FEATS - 1) / dl::GR_FEATS <= dl::sm_count()) return dl::gr_launch<1, 16>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, stream);
+    return dl::gr_launch<1, 8>(x, ldx, w, bias, y, ldy, M, N, K, out_scale, stream);
+  }
+  const bool few = kind == dl::GS_FEW;
+  if (few ? M > 16 : parts == nullptr || (reinterpret_cast<uintptr_t>(parts) & 15) || odd_rows == nullptr) return DL_ERR_UNSUPPORTED;
+  if (few) rows = 16;
+  else if (rows == 0) rows = choice.rows >= 16 && (choice.kind == dl::GS_TILES || choice.kind == dl::GS_CLUSTERS) ? choice.rows : 64;
+  const int row_tiles = (M + rows - 1) / rows;
+  const long long tiles = static_cast<long long>((N + dl::GS_BF - 1) / dl::GS_BF) * row_tiles;
+  if (tiles > (1ll << 27)) return DL_ERR_UNSUPPORTED;
+  CUtensorMap map_w, map_x = {};
+  int rc = dl::gs_map(&map_w, w, true, N, K, K, dl::GS_BF / 2);
+  if (rc != 0) return rc;
+  dl::GsArgs a = {x, w, bias, y, status, ldx, ldy, M, N, K, odd_rows, rows, row_tiles, static_cast<int>(tiles), 0, 1, 0, out_scale};
+  if (few) {
+    rc = dl::gs_map(&map_x, x, true, M, K, ldx, 16);
+    return rc != 0 ? rc : dl::gs_launch<true>(map_w, map_x, a, stream);
+  }
+  const int pitch = (K + 7) / 8 * 8;
+  rc = dl::gs_map(&map_x, parts, false, 3ll * M, pitch, pitch, rows);
+  if (rc != 0) return rc;
+  rc = dl::launch_streaming(dl::gemm_split_parts_kernel, dim3(M), dim3(256), 0, stream, x, ldx, K, static_cast<dl::bf16*>(parts), pitch, odd_rows);
+  if (rc != 0) return rc;
+  if (kind == dl::GS_CLUSTERS) a.cluster = dl::GS_CLUSTER;
+  return dl::gs_launch<false>(map_w, map_x, a, stream);
+}
+
+// The gated feed-forward's first half for up to 16 rows: w = [Wg; Wu] with 2 F rows, y [M, F] = silu(x Wg^T) (x Wu^T), the products
+// as dl_gemm_split gives them. Refused where F is too narrow to fill the SMs with blocks of 64 features each.
+DL_EXPORT int dl_gemm_split_swiglu(const float* x, int ldx, const float* w, float* y, int ldy, int M, int F, int K, int* status,
+                                   cudaStream_t stream) {
+  if (M <= 0 || F <= 0) return 0;
+  if (K <= 0 || (K & 3) || (ldx & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || status == nullptr ||
+      M > 16 || F > (1 << 29))
+    return DL_ERR_UNSUPPORTED;
+  const int tiles = (F + dl::GS_BF / 2 - 1) / (dl::GS_BF / 2);
+  if (5ll * tiles < 4ll * dl::sm_count()) return DL_ERR_UNSUPPORTED;
+  CUtensorMap map_w, map_x;
+  int rc = dl::gs_map(&map_w, w, true, 2 * F, K, K, dl::GS_BF / 2);
+  if (rc == 0) rc = dl::gs_map(&map_x, x, true, M, K, ldx, 16);
+  if (rc != 0) return rc;
+  const dl::GsArgs a = {x, w, nullptr, y, status, ldx, ldy, M, 2 * F, K, nullptr, 16, 1, tiles, 0, 1, F, 1.0f};
+  return dl::gs_launch<true>(map_w, map_x, a, stream);
+}
+
+// The q | k | v projection of up to 16 rows with the rotary encoding and the cache write in its epilogue: w [(n_heads + 2 n_kv_heads)
+// head_dim, K]; rotated q goes to q_out [M, ldq], rotated k and plain v to the caches [pages, page_size, n_kv_heads, head_dim]. The
+// whole head is rotated (head_dim a multiple of 16). The same bits as dl_gemm_split followed by dl_rope_cache_write.
+DL_EXPORT int dl_gemm_split_qkv_rope(const float* x, int ldx, const float* w, float* q_out, int ldq, int M, int K, const int* positions,
+                                     const int* row_request, const int* block_table, int max_blocks, float* k_cache, float* v_cache,
+                                     const float* inv_freq, float pos_scale, int n_heads, int n_kv_heads, int head_dim, int page_size,
+                                     cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (K <= 0 || (K & 3) || (ldx & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || M > 16 ||
+      head_dim <= 0 || (head_dim & 15) || n_heads <= 0 || n_kv_heads <= 0 || page_size <= 0 || inv_freq == nullptr)
+    return DL_ERR_UNSUPPORTED;
+  const dl::QkvRopeOf<float> rope = {positions, row_request, block_table, max_blocks, k_cache, v_cache, inv_freq, nullptr, pos_scale,
+                                     n_heads, n_kv_heads, head_dim, page_size};
+  const int N = (n_heads + 2 * n_kv_heads) * head_dim;
+  if (M > 8) return dl::gr_launch<2, 8, true>(x, ldx, w, nullptr, q_out, ldq, M, N, K, 1.0f, stream, rope);
+  if (N / dl::GR_FEATS <= dl::sm_count()) return dl::gr_launch<1, 16, true>(x, ldx, w, nullptr, q_out, ldq, M, N, K, 1.0f, stream, rope);
+  return dl::gr_launch<1, 8, true>(x, ldx, w, nullptr, q_out, ldq, M, N, K, 1.0f, stream, rope);
+}

@@ -443,9 +443,10 @@ def attention_f32(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cache: t
     if max(lead, rows - lead if n_tiles == 0 else 0) > 65535:
         return False
     args = (n_heads, n_kv_heads, head_dim, vdim, cache.page_size, scale, window, keep_first, sink, rate, step, chunk)
+    single = ctx.decode_only or query_tiles(ctx) is not None      # the rows at the step's head are single tokens
     if lead > 0:
         ops.attention_f32_rows(q, k_cache, k_row, v_cache, v_row, cache.block_table, ctx.positions, ctx.row_slot, lead,
-                               parts, out, *args, warps=one)
+                               parts, out, *args, warps=one, old_keys=single)
     if n_tiles > 0:
         ops.attention_f32_tiles(q, k_cache, k_row, v_cache, v_row, cache.block_table, query_tiles(ctx)[0], n_tiles, out, *args)
     elif rows > lead:

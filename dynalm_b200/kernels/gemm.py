@@ -1,7 +1,9 @@
 """y = x W^T (+ bias): picks the matrix-product kernel for a dtype and shape.
 
-float32 always runs the plain fixed-order kernel (csrc/gemm_simt.cu): the true 32-bit path uses no
-tensor cores and no reduced-precision mode. bfloat16 with at most 16 rows (decode) runs a
+float32 runs on operands split into three bf16 parts (csrc/gemm_split.cu), which keeps the precision of 32-bit
+multiply-adds, for matrices of at least 512 x 512, and the plain fixed-order kernel (csrc/gemm_simt.cu) below;
+which one a product takes is decided by its matrix alone, and in both a row's result does not depend on the other
+rows. bfloat16 with at most 16 rows (decode) runs a
 weight-streaming kernel, which can also apply SwiGLU on the way out or leave split-K partial sums for
 the consumer to add: the mma.sync one (csrc/gemm_skinny.cu) up to 8 rows, the tcgen05 one
 (csrc/gemm_stream_tcgen05.cu), which computes the product transposed, from 9 to 16 rows. bfloat16 with
@@ -108,11 +110,47 @@ def rotating_epilogue_pays(rows: int, features: int, head_dim: int) -> bool:
     return tiles >= ops.QKV_ROPE_TCGEN05_MIN_ROUNDS[head_dim] * sm_count()
 
 
+# The smallest matrix (features and k) whose float32 product is the one of split numbers. Measured, plain / split, us: 512 x 512
+# with 1 to 64 rows 11 to 12 / 11 to 13, with 700 29 / 23; 1024 x 1024 11 to 12 / 11 to 13, 53 / 24; its error against 64 bits is
+# the smaller one from there on (random operands, k 512: 0.96e-7 against 1.17e-7; 2,048: 1.1e-7 against 2.1e-7; 8,192: 1.2e-7
+# against 4.1e-7).
+SPLIT_MIN = 512
+
+
+def split_applies(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a float32 product takes the kernels of split numbers: what speaks against it, but for operands that lie oddly, is
+    in w's sizes alone, so that a row meets the same arithmetic whatever step it comes in."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and w.shape[0] >= SPLIT_MIN and w.shape[1] >= SPLIT_MIN
+            and w.shape[1] % 4 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
+            and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0)
+
+
+def split_scratch(x: torch.Tensor, w: torch.Tensor, runtime) -> Optional[torch.Tensor]:
+    """Scratch for a product of split numbers of as many rows as the runtime may bring; None when it does not apply or the device
+    has no room for it (then no step of this runtime gets any, whatever its rows)."""
+    if runtime is None or not split_applies(x, w):
+        return None
+    per_row = ops.split_scratch_row(w.shape[1])
+    return runtime.spare(f"split_parts_{per_row}", runtime.max_tokens * per_row, torch.uint8)
+
+
+def _linear_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor], out_scale: float, runtime) -> bool:
+    """The product of split numbers; False when the plain kernel has to run it."""
+    scratch = split_scratch(x, w, runtime) if out.stride(1) == 1 else None
+    if scratch is None:
+        return False
+    ops.gemm_split(x, w, out, bias, out_scale, scratch)
+    return True
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
-           out_scale: float = 1.0) -> torch.Tensor:
+           out_scale: float = 1.0, runtime=None) -> torch.Tensor:
     """out[M, N] = (x[M, K] @ w[N, K].T + bias[N]) * out_scale. x and w share a dtype; out may be
-    float32 for bfloat16 operands (logits)."""
+    float32 for bfloat16 operands (logits). `runtime`: where float32 products keep their scratch; without it they run the plain
+    kernel."""
     global LIBRARY_CALLS
+    if x.dtype == torch.float32 and _linear_split(x, w, out, bias, out_scale, runtime):
+        return out
     if x.dtype == torch.float32 or bias is not None:
         ops.gemm_simt(x, w, out, bias, out_scale)
         return out
@@ -153,17 +191,17 @@ def linear_partial(x: torch.Tensor, w: torch.Tensor, runtime, name: str) -> torc
             (ops.gemm_stream if stream else ops.gemm_skinny)(x, w, out, "store", 1.0)
             return out
     out = runtime.buffer(name, (M, N))
-    return linear(x, w, out)
+    return linear(x, w, out, runtime=runtime)
 
 
-def linear_short(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def linear_short(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, runtime=None) -> torch.Tensor:
     """out = x W^T for a short K (an inner vector of a few dozen or hundred numbers, x often a slice of wider rows): there is
     no K to split, so this package's products take every row count and however few tiles, float32 results included."""
     ok = (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
           and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and w.is_contiguous() and w.shape[0] % 8 == 0
           and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0)
     if not ok:
-        return linear(x, w, out)
+        return linear(x, w, out, runtime=runtime)
     if x.shape[0] <= ops.SKINNY_MAX_ROWS:
         ops.gemm_skinny(x, w, out, "store", 1.0)
     else:
@@ -178,7 +216,7 @@ def linear_partial_biased(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch
         return linear_partial(x, w, runtime, name)
     M, N = x.shape[0], w.shape[0]
     if x.dtype == torch.float32:
-        return linear(x, w, runtime.buffer(name, (M, N)), bias)
+        return linear(x, w, runtime.buffer(name, (M, N)), bias, runtime=runtime)
     if use_stream(x, w) or skinny_ok(x, w):
         out = linear_partial(x, w, runtime, name)
         ops.add_bias(out[0] if out.dim() == 3 else out, bias)
@@ -211,8 +249,11 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, runtime, inner: int)
     act = runtime.buffer("ffn_act", (rows, inner))
     if _gated_epilogue(x, w_gate_up, act, inner):
         return act
+    if split_scratch(x, w_gate_up, runtime) is not None and w_gate_up.shape[0] == 2 * inner and ops.split_swiglu_applies(rows, inner):
+        ops.gemm_split_swiglu(x, w_gate_up, act)      # (the same bits as the two steps below)
+        return act
     gate_up = runtime.buffer("ffn_gate_up", (rows, 2 * inner))
-    linear(x, w_gate_up, gate_up)
+    linear(x, w_gate_up, gate_up, runtime=runtime)
     ops.silu_mul(gate_up, act)
     return act
 
@@ -225,7 +266,7 @@ def linear_clamped_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, coeffs: torc
     if _gated_epilogue(x, w_gate_up, act, inner, coeffs):
         return act
     gate_up = runtime.buffer("ffn_gate_up", (rows, 2 * inner))
-    linear(x, w_gate_up, gate_up)
+    linear(x, w_gate_up, gate_up, runtime=runtime)
     ops.clamped_swiglu(gate_up, coeffs, act)
     return act
 
@@ -235,7 +276,7 @@ def linear_geglu(x: torch.Tensor, w_gate_up: torch.Tensor, runtime, inner: int) 
     rows = x.shape[0]
     act = runtime.buffer("ffn_act", (rows, inner))
     gate_up = runtime.buffer("ffn_gate_up", (rows, 2 * inner))
-    linear(x, w_gate_up, gate_up)
+    linear(x, w_gate_up, gate_up, runtime=runtime)
     ops.gelu_mul(gate_up, act)
     return act
 
@@ -258,7 +299,7 @@ def linear_act(x: torch.Tensor, w_up: torch.Tensor, runtime, inner: int, activat
     if x.dtype == torch.bfloat16 and tcgen05_ok(x, w_up, act, inner):
         ops.gemm_tcgen05(x, w_up, act, activation, coeffs=coeffs)
         return act
-    linear(x, w_up, act)
+    linear(x, w_up, act, runtime=runtime)
     if activation == "xielu":
         ops.xielu(act, act, coeffs)
         return act

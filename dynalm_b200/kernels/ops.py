@@ -15,6 +15,7 @@ import torch
 
 from ..errors import EngineError, InvalidArgument, Unsupported
 from . import lib as _lib
+from .device import sm_count
 
 DL_ERR_UNSUPPORTED = 10001
 
@@ -136,6 +137,10 @@ _SIGNATURES = {
     "gemm_skinny": {
         "dl_gemm_skinny": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _L, _P, _L, _P, _P],
         "dl_gemm_skinny_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _F, _I, _I, _I, _I, _P]},
+    "gemm_split": {
+        "dl_gemm_split": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _I, _P, _P],
+        "dl_gemm_split_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _F, _I, _I, _I, _I, _P],
+        "dl_gemm_split_swiglu": [_P, _I, _P, _P, _I, _I, _I, _I, _P, _P]},
     "gemm_tcgen05": {
         "dl_gemm_tcgen05": [_P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _P, _I, _P],
         "dl_gemm_tcgen05_tile_coords": [_I, _I, _I, _I, _P, _P],
@@ -147,7 +152,7 @@ _SIGNATURES = {
     "attention_f32": {
         "dl_attention_f32_tiles": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _P],
         "dl_attention_f32_rows": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
-                                  _I, _P]},
+                                  _I, _I, _P]},
     "gemm_simt": {"dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P]},
     "sampling": {
         "dl_argmax": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
@@ -1264,17 +1269,22 @@ def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, pos
                   page_size: int, angles: Optional[torch.Tensor] = None) -> None:
     """The q | k | v projection with rotary encoding and cache write in its epilogue: rotated q into
     q_out [rows, >= n_heads * head_dim], rotated k and plain v into the paged cache. The whole head is rotated
-    (inv_freq has head_dim / 2 entries). bfloat16. Up to 16 rows: the weight-streaming kernel
+    (inv_freq has head_dim / 2 entries). bfloat16: up to 16 rows the weight-streaming kernel
     (csrc/gemm_skinny.cu, head_dim a multiple of 16); more rows: the tcgen05 kernel (csrc/gemm_tcgen05.cu,
-    head_dim 64 or 128), which reads the step's (cos, sin) pairs from `angles` (see rope_angles) when given."""
+    head_dim 64 or 128), which reads the step's (cos, sin) pairs from `angles` (see rope_angles) when given. float32: up to
+    16 rows, the product of split numbers (csrc/gemm_split.cu, head_dim a multiple of 16)."""
     _cuda(x, w_qkv, q_out, positions, row_request, block_table, k_cache, v_cache, inv_freq)
     _rows_contiguous(x, "x")
     _rows_contiguous(q_out, "q_out")
     M, K = x.shape
-    if any(t.dtype != torch.bfloat16 for t in (x, w_qkv, q_out, k_cache, v_cache)):
-        raise Unsupported("gemm_qkv_rope: bfloat16 only")
-    few = M <= SKINNY_FAST_ROWS
-    if K % 8 or x.stride(0) % 8 or (head_dim % 16 if few else head_dim not in QKV_ROPE_TCGEN05_HEAD_DIMS):
+    exact = x.dtype == torch.float32
+    if x.dtype not in (torch.bfloat16, torch.float32) or any(t.dtype != x.dtype for t in (w_qkv, q_out, k_cache, v_cache)):
+        raise Unsupported("gemm_qkv_rope: bfloat16 or float32, one of them throughout")
+    if exact and M > SPLIT_FEW_ROWS:
+        raise Unsupported(f"gemm_qkv_rope: float32 up to {SPLIT_FEW_ROWS} rows")
+    few = exact or M <= SKINNY_FAST_ROWS
+    unit = 4 if exact else 8
+    if K % unit or x.stride(0) % unit or (head_dim % 16 if few else head_dim not in QKV_ROPE_TCGEN05_HEAD_DIMS):
         raise Unsupported(f"gemm_qkv_rope: {M} rows, K {K} and head_dim {head_dim}")
     if angles is not None and (angles.dtype != torch.float32 or angles.numel() < M * head_dim or not angles.is_contiguous()):
         raise InvalidArgument("gemm_qkv_rope: angles must be contiguous float32 [rows, head_dim / 2, 2]")
@@ -1299,6 +1309,13 @@ def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, pos
             _p(block_table), block_table.stride(0), _p(k_cache), _p(v_cache), _p(inv_freq), _p(angles), pos_scale, n_heads,
             n_kv_heads, head_dim, page_size, _p(_status_word(x.device)), tcgen05_pairs(M, w_qkv.shape[0]), _stream()),
                "gemm_tcgen05_qkv_rope")
+        return
+    if exact:
+        check_limits("gemm_split", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
+        _check(_fn("gemm_split", "dl_gemm_split_qkv_rope")(
+            _p(x), x.stride(0), _p(w_qkv), _p(q_out), q_out.stride(0), M, K, _p(positions), _p(row_request), _p(block_table),
+            block_table.stride(0), _p(k_cache), _p(v_cache), _p(inv_freq), pos_scale, n_heads, n_kv_heads, head_dim, page_size,
+            _stream()), "gemm_split_qkv_rope")
         return
     check_limits("gemm_skinny", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
     _check(_fn("gemm_skinny", "dl_gemm_skinny_qkv_rope")(
@@ -1428,6 +1445,59 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optiona
         raise InvalidArgument("gemm: bias must be float32 [N]")
     _check(_fn("gemm_simt", "dl_gemm_simt")(dtype_code(x.dtype), dtype_code(out.dtype), _p(x), x.stride(0), _p(w),
                                              _p(bias), _p(out), out.stride(0), M, N, K, out_scale, _stream()), "gemm_simt")
+
+
+SPLIT_FEW_ROWS = 16       # up to here the product of split numbers needs no scratch
+SPLIT_KINDS = {"auto": 0, "groups": 1, "few": 2, "tiles": 3, "clusters": 4}
+
+
+def split_scratch_row(k: int) -> int:
+    """Bytes of scratch that gemm_split needs for a row."""
+    return 6 * (-(-k // 8) * 8) + 4
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, out_scale: float = 1.0,
+               scratch: Optional[torch.Tensor] = None, kind: str = "auto", tile_rows: int = 0) -> None:
+    """out = (x W^T + bias) * out_scale in float32, each operand as three bf16 parts on the tensor cores; see
+    csrc/gemm_split.cu. A row's bits depend on nothing but the row, w, bias and out_scale. `scratch`: uint8, contiguous, of
+    split_scratch_row(K) bytes for every row; none is needed up to SPLIT_FEW_ROWS rows. `kind` and tile_rows (a multiple of 16, at
+    most 128; 0: by cost): how the work is dealt."""
+    _cuda(x, w, out, bias, scratch)
+    M, K = x.shape
+    N = w.shape[0]
+    _rows_contiguous(x, "x")
+    _rows_contiguous(out, "out")
+    if (x.dtype, w.dtype, out.dtype) != (torch.float32,) * 3 or not w.is_contiguous() or w.shape[1] != K or out.shape != (M, N):
+        raise InvalidArgument("gemm_split: x [M, K], w [N, K] contiguous and out [M, N], all float32")
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
+        raise InvalidArgument("gemm_split: bias must be float32 [N]")
+    parts = odd = None
+    if scratch is not None:
+        if scratch.dtype != torch.uint8 or not scratch.is_contiguous() or scratch.numel() < M * split_scratch_row(K):
+            raise InvalidArgument("gemm_split: scratch too small")
+        parts = scratch.data_ptr()
+        odd = parts + M * (split_scratch_row(K) - 4)
+    _check(_fn("gemm_split", "dl_gemm_split")(
+        _p(x), x.stride(0), _p(w), _p(bias), _p(out), out.stride(0), M, N, K, out_scale, parts, odd, SPLIT_KINDS[kind], tile_rows,
+        _p(_status_word(x.device)), _stream()), "gemm_split")
+
+
+def split_swiglu_applies(rows: int, inner: int) -> bool:
+    """Whether gemm_split_swiglu takes a gated product of these sizes (csrc/gemm_split.cu, dl_gemm_split_swiglu)."""
+    return rows <= SPLIT_FEW_ROWS and 5 * -(-inner // 64) >= 4 * sm_count()
+
+
+def gemm_split_swiglu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """out = silu(x Wg^T) * (x Wu^T) with w = [Wg; Wu], for up to SPLIT_FEW_ROWS rows, the products as gemm_split gives them."""
+    _cuda(x, w, out)
+    M, K = x.shape
+    F = w.shape[0] // 2
+    _rows_contiguous(x, "x")
+    _rows_contiguous(out, "out")
+    if ((x.dtype, w.dtype, out.dtype) != (torch.float32,) * 3 or not w.is_contiguous() or w.shape != (2 * F, K) or out.shape != (M, F)):
+        raise InvalidArgument("gemm_split_swiglu: x [M, K], w [2 F, K] contiguous and out [M, F], all float32")
+    _check(_fn("gemm_split", "dl_gemm_split_swiglu")(_p(x), x.stride(0), _p(w), _p(out), out.stride(0), M, F, K,
+                                                     _p(_status_word(x.device)), _stream()), "gemm_split_swiglu")
 
 
 SKINNY_MAX_ROWS = 64      # what the kernel takes
@@ -1995,15 +2065,17 @@ def attention_f32_rows(q: torch.Tensor, k_cache: torch.Tensor, k_row: int, v_cac
                        block_table: torch.Tensor, positions: torch.Tensor, row_request: torch.Tensor, rows: int, parts: int,
                        out: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: int, vdim: int, page_size: int, scale: float,
                        window: int = 0, keep_first: int = 0, sink: bool = False, rate: Optional[torch.Tensor] = None,
-                       step: Optional[torch.Tensor] = None, chunk: int = 0, warps: int = 0) -> None:
+                       step: Optional[torch.Tensor] = None, chunk: int = 0, warps: int = 0, old_keys: bool = False) -> None:
     """The same for the first `rows` rows of the step one by one, each row's keys over `parts` (1, 2, 4 or 8) blocks of one warp
-    (warps 1) or of as many as the kernel has (0); the result's bits depend on neither."""
+    (warps 1) or of as many as the kernel has (0); the result's bits depend on neither. `old_keys`: every row is the only one its
+    request brings, and all that earlier kernels but the last wrote of the caches and of `positions`, `row_request` and
+    `block_table` stands: keys in front of a row are then asked for before the last of them has ended."""
     _attention_f32_args(q, k_cache, v_cache, block_table, out, n_heads, n_kv_heads, rate, step)
     _cuda(positions, row_request)
     _check(_fn("attention_f32", "dl_attention_f32_rows")(
         _p(q), q.stride(0), _p(k_cache), k_row, _p(v_cache), v_row, _p(block_table), block_table.stride(0), _p(positions),
         _p(row_request), rows, parts, warps, _p(out), out.stride(0), n_heads, n_kv_heads, head_dim, vdim, page_size, scale, window,
-        int(keep_first), 1 if sink else 0, _p(rate), _p(step), int(chunk), _stream()), "attention_f32_rows")
+        int(keep_first), 1 if sink else 0, _p(rate), _p(step), int(chunk), 1 if old_keys else 0, _stream()), "attention_f32_rows")
 
 
 def gelu_mul(gate_up: torch.Tensor, out: torch.Tensor) -> None:

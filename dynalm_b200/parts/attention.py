@@ -14,7 +14,7 @@ import torch
 
 from ..errors import Unsupported
 from ..kernels import linear, ops
-from ..kernels.gemm import linear_partial, linear_partial_biased
+from ..kernels.gemm import linear_partial, linear_partial_biased, split_scratch
 from .base import POSITIONS, CacheSpec, TensorDecl, register_mixer
 
 
@@ -95,11 +95,11 @@ class PagedAttention:
             return self._attend_and_project(qkv, cache, ctx, rows)
         if owns_cache:
             qkv = rt.buffer("attn_qkv", (rows, self.q_width + 2 * self.kv_width))
-            linear(x, self.w_qkv, qkv, self.b_qkv)
+            linear(x, self.w_qkv, qkv, self.b_qkv, runtime=rt)
         else:
             # a layer that reads another entry's cache makes queries only
             qkv = rt.buffer("attn_qkv", (rows, self.q_width + 2 * self.kv_width))[:, :self.q_width]
-            linear(x, self.w_qkv[:self.q_width], qkv, self.b_qkv[:self.q_width] if self.b_qkv is not None else None)
+            linear(x, self.w_qkv[:self.q_width], qkv, self.b_qkv[:self.q_width] if self.b_qkv is not None else None, runtime=rt)
         if self.position is not None and table is None:
             q = qkv[:, :self.q_width].unflatten(1, (s.num_heads, s.head_dim))
             k = qkv[:, self.q_width:self.q_width + self.kv_width].unflatten(1, (s.num_kv_heads, s.head_dim)) \
@@ -111,10 +111,15 @@ class PagedAttention:
         return self._attend_and_project(qkv, cache, ctx, rows)
 
     def _fused_projection_applies(self, x: torch.Tensor, table) -> bool:
-        """bfloat16, no bias, the rotation covers the whole head, and either few rows (the weight-streaming
-        kernel) or enough tiles for the tcgen05 kernel with a head size it takes (ops.QKV_ROPE_TCGEN05_MIN_ROUNDS)."""
-        if not (table is not None and table[0] is not None and table[1] == self.spec.head_dim and self.b_qkv is None
-                and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0):
+        """No bias, the rotation covers the whole head, and in bfloat16 either few rows (the weight-streaming
+        kernel) or enough tiles for the tcgen05 kernel with a head size it takes (ops.QKV_ROPE_TCGEN05_MIN_ROUNDS), in float32
+        few rows where the product of split numbers applies."""
+        if not (table is not None and table[0] is not None and table[1] == self.spec.head_dim and self.b_qkv is None):
+            return False
+        if x.dtype == torch.float32:
+            return (x.shape[0] <= ops.SPLIT_FEW_ROWS and self.spec.head_dim % 16 == 0
+                    and split_scratch(x, self.w_qkv, self.rt) is not None)
+        if not (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0):
             return False
         if x.shape[0] <= ops.SKINNY_FAST_ROWS:
             return True
@@ -134,7 +139,7 @@ class PagedAttention:
         if self.b_o is None:
             return linear_partial(attn, self.w_o, rt, "mixer_out")
         out = rt.buffer("mixer_out", (rows, s.width))
-        linear(attn, self.w_o, out, self.b_o)
+        linear(attn, self.w_o, out, self.b_o, runtime=rt)
         return out
 
     def graph_key(self, ctx) -> tuple:
@@ -379,7 +384,7 @@ class GatedNormedAttention(PagedAttention):
         proj = rt.buffer("gattn_proj", (rows, self.w_qkv.shape[0]))
         by_projection = self.normed or (not self.head_normed and not self.head_first and not self.interleaved)
         # a bias joins in the kernel that turns and norms, where that kernel takes one; else in the product (the plain one)
-        linear(x, self.w_qkv, proj, self.b_qkv if (by_projection or self.gated) else None)
+        linear(x, self.w_qkv, proj, self.b_qkv if (by_projection or self.gated) else None, runtime=rt)
         k_cache, k_row, v_cache, v_row = self._kv(cache)
         if self.head_first:
             pos = self.position
@@ -421,7 +426,7 @@ class GatedNormedAttention(PagedAttention):
         s, rt = self.spec, self.rt
         rows = x.shape[0]
         proj = rt.buffer("gattn_proj", (rows, self.w_qkv.shape[0]))
-        linear(x, self.w_qkv, proj)
+        linear(x, self.w_qkv, proj, runtime=rt)
         q = rt.buffer("gattn_q", (rows, self.q_width))
         kept = cache.state.arrays[0] if cache.state is not None else None
         k_cache = v_cache = None

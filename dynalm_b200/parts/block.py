@@ -286,7 +286,7 @@ class SigmoidGate:
         if self.weight is None:
             return part.joined(h.shape[0])
         g = self.rt.buffer("stream_gate", (h.shape[0], self.spec.width))
-        return linear(h, self.weight, g)
+        return linear(h, self.weight, g, runtime=self.rt)
 
 
 @register_block("gated_pre_norm")

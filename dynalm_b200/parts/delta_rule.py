@@ -127,10 +127,10 @@ class GatedDeltaMixer:
         rows = x.shape[0]
         H, G, d, e = s.num_heads, s.num_kv_heads, s.head_dim, s.value_dim
         proj = rt.buffer("delta_proj", (rows, self.w_in.shape[0]))
-        linear(x, self.w_in, proj)
+        linear(x, self.w_in, proj, runtime=rt)
         two = None
         if self.w_two is not None:
-            two = linear_short(proj[:, :self.inner_cols], self.w_two, rt.buffer("delta_two", (rows, self.w_two.shape[0]), torch.float32))
+            two = linear_short(proj[:, :self.inner_cols], self.w_two, rt.buffer("delta_two", (rows, self.w_two.shape[0]), torch.float32), rt)
         u = rt.buffer("delta_conv", (rows, self.channels))
         ops.short_conv(proj, self.inner_cols, self.channels, self.taps, None, state, self.keep_off, ctx.positions, ctx.row_request,
                        ctx.row_slot, ctx.pos_start, u, act="silu")

@@ -118,7 +118,7 @@ class DiffAttention:
         # a layer that reads another layer's records makes queries only
         qkv = rt.buffer("diff_qkv", (rows, self.q_width + self.k_width + self.v_width)) if owns_cache else \
             rt.buffer("diff_q", (rows, self.q_width))
-        linear(x, self.w_qkv, qkv)
+        linear(x, self.w_qkv, qkv, runtime=rt)
         ops.qk_norm_cache_write(qkv, ctx.positions, ctx.row_slot, cache.block_table, records, 0, self.k_width,
                                 self.q_norm, self.k_norm, self.eps, float(s.get("temp_coef", 0.0)),
                                 int(s.get("temp_every", 0)), 2 * s.num_heads, 2 * s.num_kv_heads, s.head_dim,

@@ -64,7 +64,7 @@ class LogitsHead:
         self.softcap = float(getattr(spec, "softcap", 0.0))
 
     def forward(self, normed_rows: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-        linear(normed_rows, self.weight, out, None, self.out_scale)
+        linear(normed_rows, self.weight, out, None, self.out_scale, runtime=self.rt)
         if self.softcap > 0.0:
             ops.softcap(out, self.softcap)         # c * tanh(logits / c), in place on the float32 logits
         return out

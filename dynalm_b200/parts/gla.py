@@ -81,7 +81,7 @@ class GatedLinearAttention:
         rows = x.shape[0]
         H, d, e = s.num_heads, s.head_dim, s.value_dim
         proj = rt.buffer("gla_proj", (rows, self.w_in.shape[0]))
-        linear(x, self.w_in, proj)
+        linear(x, self.w_in, proj, runtime=rt)
         gate_col = 2 * self.qk + self.inner
         z = rt.buffer("gla_decay", (rows, self.qk), torch.float32)
         inner_vec = proj[:, gate_col + self.inner:]
@@ -89,7 +89,7 @@ class GatedLinearAttention:
             ops.gemm_simt(inner_vec, self.w_decay, z, self.b_decay, 1.0)
             z_bias = None
         else:
-            linear(inner_vec, self.w_decay, z)         # float32 sums; the bias joins where the decays are formed
+            linear(inner_vec, self.w_decay, z, runtime=rt)         # float32 sums; the bias joins where the decays are formed
             z_bias = self.b_decay
         o = rt.buffer("gla_o", (rows, self.inner), torch.float32)
         ops.gla_scan(proj, 0, self.qk, 2 * self.qk, z, self.tau, self.q_scale, state, ctx.q_start, ctx.state_slots, o,

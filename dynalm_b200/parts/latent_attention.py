@@ -135,13 +135,13 @@ class LatentAttention:
         rows = x.shape[0]
         (records,) = cache.arrays
         down = rt.buffer("latent_down", (rows, self.w_down.shape[0]))
-        linear(x, self.w_down, down)
+        linear(x, self.w_down, down, runtime=rt)
         if s.q_rank:
             cq = rt.buffer("latent_cq", (rows, s.q_rank))
             ops.latent_prep(down, s.q_rank, R, r, self.rot, self.dq_norm, self.dkv_norm, self.eps, self.freq, ctx.positions,
                             ctx.row_slot, cache.block_table, records, cache.page_size, cq, self.mag)
             q = rt.buffer("latent_q", (rows, H * (d + r)))
-            linear(cq, self.w_uq, q)
+            linear(cq, self.w_uq, q, runtime=rt)
         else:
             q = down[:, :self.q_cols]
             ops.latent_prep(down[:, self.q_cols:], 0, R, r, self.rot, None, self.dkv_norm, self.eps, self.freq, ctx.positions,

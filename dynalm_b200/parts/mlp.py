@@ -158,6 +158,6 @@ class TokenSide:
     def forward(self, x: torch.Tensor, ctx) -> torch.Tensor:
         """x: the stream in the compute dtype."""
         z = self.rt.buffer("token_side", (x.shape[0], self.spec.inner))
-        linear(x, self.w_gate, z)
+        linear(x, self.w_gate, z, runtime=self.rt)
         ops.token_gate(z, self.table, ctx.token_ids, z)
         return linear_partial(z, self.w_proj, self.rt, "token_side_out")

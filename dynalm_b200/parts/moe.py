@@ -118,7 +118,7 @@ class RoutedMLP:
         E, top = self.E, self.top
         pairs = rows * top
         logits = self._logits(rows)
-        linear(x, self.w_router, logits)                                  # float32 accumulation and result
+        linear(x, self.w_router, logits, runtime=rt)                                  # float32 accumulation and result
         ids = rt.buffer("moe_ids", (rows, top), torch.int32)
         weights = rt.buffer("moe_weights", (rows, top), torch.float32)
         ops.moe_route(logits[:, :E], top, self.groups, self.keep, self.scale, ids, weights, self.correction, bias=self.router_bias, **self.route)

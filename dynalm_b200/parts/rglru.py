@@ -81,7 +81,7 @@ class GatedLinearRecurrence:
         (state,) = cache.arrays
         rows = x.shape[0]
         proj = rt.buffer("rglru_proj", (rows, 2 * R))
-        linear(x, self.w_in, proj)
+        linear(x, self.w_in, proj, runtime=rt)
         u = rt.buffer("rglru_conv", (rows, R))
         ops.short_conv(proj, R, R, self.taps, self.conv_bias, state, self.keep_off, ctx.positions, ctx.row_request,
                        ctx.row_slot, ctx.pos_start, u, act="none", in_bias=self.x_bias)

@@ -89,7 +89,7 @@ class StateSpaceMixer:
         rows = x.shape[0]
         H, P, N, G = s.num_heads, s.head_dim, s.state, s.groups
         proj = rt.buffer("ssd_proj", (rows, 2 * self.inner + 2 * G * N + H))
-        linear(x, self.w_in, proj)
+        linear(x, self.w_in, proj, runtime=rt)
         u = rt.buffer("ssd_conv", (rows, self.channels))
         ops.ssm_conv(proj, self.inner, self.channels, self.taps, self.conv_bias, state, self.keep_off, ctx.positions,
                      ctx.row_request, ctx.row_slot, ctx.pos_start, u)

@@ -1,0 +1,118 @@
+"""The float32 product of split numbers (csrc/gemm_split.cu): every way of dealing the work gives a row the same bits, within a
+bound of the 64-bit product, and numbers that have no finite parts come out as from plain multiply-adds."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from dynalm_b200.kernels import ops
+    return ops
+
+
+def _scratch(ops, rows, k):
+    return torch.empty(rows * ops.split_scratch_row(k), dtype=torch.uint8, device=DEV)
+
+
+def _ways(rows):
+    """(kind, rows of a tile) that take so many rows."""
+    ways = [("auto", 0), ("groups", 0), ("tiles", 16), ("tiles", 48), ("tiles", 128), ("clusters", 32), ("clusters", 128)]
+    return ways + ([("few", 0)] if rows <= 16 else [])
+
+
+# (remainders of features, rows and k; fewer slices of k than the sixteenths it is dealt in; several tiles to a block)
+@pytest.mark.parametrize("N,K", [(512, 512), (130, 4), (300, 516), (7, 2052), (640, 1100), (20000, 96), (2048, 8192)])
+def test_every_way_gives_the_same_bits(ops, N, K):
+    g = torch.Generator(device="cpu").manual_seed(N + K)
+    x = (torch.randn(300, K, generator=g) * torch.exp(2 * torch.randn(300, K, generator=g))).to(DEV)
+    w = torch.randn(N, K, generator=g).to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    ref = (x.double() @ w.double().T + bias.double()) * 0.5
+    # a slice: 24 steps, of each of which up to 2^-23 is cut off; then the slices of a sixteenth and the sixteenths are added, and
+    # the products left out are 2^-24 of a product
+    bound = 0.5 * 2.0 ** -23 * (24 + K / 1024 + 18) * (x.double().abs() @ w.double().abs().T + bias.double().abs())
+    want = None
+    for rows in (300, 1, 5, 8, 9, 16, 17, 64, 129):
+        for kind, tile in _ways(rows):
+            out = torch.full((rows, N), 7.0, device=DEV)
+            ops.gemm_split(x[:rows], w, out, bias, 0.5, _scratch(ops, rows, K), kind, tile)
+            if want is None:
+                want = out
+                assert ((out.double() - ref).abs() <= bound).all()
+            assert torch.equal(out, want[:rows]), (rows, kind, tile)
+    # rows that lie apart by more than a row, from the end of the block
+    wide = torch.zeros(20, K + 8, device=DEV)
+    wide[:, 4:K + 4] = x[280:]
+    out = torch.empty(20, N + 3, device=DEV)
+    ops.gemm_split(wide[:, 4:K + 4], w, out[:, :N], bias, 0.5, _scratch(ops, 20, K))
+    assert torch.equal(out[:, :N], want[280:])
+    assert ops.gemm_tcgen05_status(DEV) == 0
+
+
+@pytest.mark.parametrize("K", [512, 2048, 8192])
+def test_error_is_no_larger_than_of_multiply_adds(ops, K):
+    g = torch.Generator(device="cpu").manual_seed(K)
+    x, w = torch.randn(64, K, generator=g).to(DEV), torch.randn(512, K, generator=g).to(DEV)
+    ref = x.double() @ w.double().T
+    split, plain = torch.empty(64, 512, device=DEV), torch.empty(64, 512, device=DEV)
+    ops.gemm_split(x, w, split, scratch=_scratch(ops, 64, K))
+    ops.gemm_simt(x, w, plain)
+    assert (split.double() - ref).norm() <= (plain.double() - ref).norm()
+
+
+@pytest.mark.parametrize("rows", [3, 16, 40])
+def test_numbers_without_finite_parts(ops, rows):
+    """Infinities, NaN and numbers that bf16 rounds to infinity: what multiply-adds give. Also beside the smallest numbers."""
+    K, N = 700, 600
+    g = torch.Generator(device="cpu").manual_seed(rows)
+    x, w = torch.randn(rows, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    x[0, 3], x[1, K - 1], x[2, 65] = float("inf"), float("nan"), 3.4e38
+    w[5, 7], w[9, 3], w[N - 1, 699] = float("-inf"), 0.0, float("inf")
+    w[11] *= 1e-38
+    plain = torch.empty(rows, N, device=DEV)
+    ops.gemm_simt(x, w, plain)
+    finite = torch.isfinite(plain)
+    for kind, tile in _ways(rows):
+        out = torch.empty(rows, N, device=DEV)
+        ops.gemm_split(x, w, out, None, 1.0, _scratch(ops, rows, K), kind, tile)
+        assert torch.equal(out[~finite].nan_to_num(1.5), plain[~finite].nan_to_num(1.5)), (kind, tile)
+        size = plain[finite].abs().clamp_min(1.0)
+        assert ((out[finite] - plain[finite]).abs() <= 2e-5 * size).all(), (kind, tile)
+
+
+@pytest.mark.parametrize("rows,F,K", [(1, 8192, 512), (7, 8300, 516), (16, 20000, 64)])
+def test_gated_product_is_its_two_steps(ops, rows, F, K):
+    g = torch.Generator(device="cpu").manual_seed(F)
+    x, w = torch.randn(rows, K, generator=g).to(DEV), (torch.randn(2 * F, K, generator=g) * 0.1).to(DEV)
+    x[0, 0] = float("inf")
+    assert ops.split_swiglu_applies(rows, F)
+    both, want, out = torch.empty(rows, 2 * F, device=DEV), torch.empty(rows, F, device=DEV), torch.empty(rows, F, device=DEV)
+    ops.gemm_split(x, w, both)
+    ops.silu_mul(both, want)
+    ops.gemm_split_swiglu(x, w, out)
+    assert torch.equal(out.nan_to_num(1.5), want.nan_to_num(1.5))
+
+
+@pytest.mark.parametrize("rows,heads,groups,dim,K", [(1, 4, 2, 32, 512), (7, 32, 8, 64, 516), (8, 3, 1, 128, 96), (16, 80, 40, 16, 64)])
+def test_rotating_projection_is_its_two_steps(ops, rows, heads, groups, dim, K):
+    g = torch.Generator(device="cpu").manual_seed(rows)
+    N, page = (heads + 2 * groups) * dim, 16
+    x, w = torch.randn(rows, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    w[0, 0] = float("inf")
+    positions = torch.randint(0, 3000, (rows,), generator=g, dtype=torch.int32).to(DEV)
+    slot = torch.arange(rows, dtype=torch.int32, device=DEV)
+    table = torch.arange(rows, dtype=torch.int32, device=DEV)[:, None].repeat(1, 200).contiguous()
+    inv = (500000.0 ** (-torch.arange(dim // 2, dtype=torch.float32) * 2 / dim)).to(DEV)
+    caches = [[torch.zeros(rows, page, groups, dim, device=DEV) for _ in "kv"] for _ in "ab"]
+    qkv, fused = torch.empty(rows, N, device=DEV), torch.empty(rows, N, device=DEV)
+    ops.gemm_split(x, w, qkv)
+    ops.rope_cache_write(qkv, positions, slot, table, *caches[0], inv, dim, 0.5, heads, groups, dim, page)
+    ops.gemm_qkv_rope(x, w, fused, positions, slot, table, *caches[1], inv, 0.5, heads, groups, dim, page)
+    assert torch.equal(qkv[:, :heads * dim].nan_to_num(1.5), fused[:, :heads * dim].nan_to_num(1.5))
+    assert all(torch.equal(a, b) for a, b in zip(*caches))
+    assert caches[0][0].abs().sum() > 0 and caches[0][1].abs().sum() > 0
