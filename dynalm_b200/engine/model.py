@@ -36,6 +36,7 @@ class Decoder:
         self.width = plan.embedding.width
         # for launch_memo: blocks of equal class and spec share a number; the layouts of their tensors are filled on use
         seen: Dict[tuple, int] = {}
+        self._key_functions = None
         self._run_kinds = [seen.setdefault((type(self.blocks[run.layer]), self.blocks[run.layer].spec), len(seen))
                            for run in self.order]
         self._run_layouts: Dict[int, tuple] = {}
@@ -60,12 +61,24 @@ class Decoder:
 
     def graph_key(self, ctx) -> tuple:
         """What, beyond the numbers of rows, the parts' launch shapes depend on for this step."""
-        key = ()
-        for b in self.blocks:
-            f = getattr(b, "graph_key", None)
-            if f is not None:
-                key += tuple(f(ctx))
-        return tuple(sorted(set(key)))
+        key = set()
+        for f in self._graph_keys():
+            key.update(f(ctx))
+        return tuple(sorted(key))
+
+    def _graph_keys(self) -> list:
+        """The `graph_key` of every block that may answer differently: of blocks of one class and spec whose parts depend on
+        nothing but the step and their own tensors (`replay_safe`) the first one's."""
+        if self._key_functions is None:
+            seen, found = set(), []
+            for run, kind in zip(self.order, self._run_kinds):
+                block = self.blocks[run.layer]
+                mark = kind if getattr(block, "replay_safe", False) else (kind, run.layer)
+                if mark not in seen and hasattr(block, "graph_key"):
+                    found.append(block.graph_key)
+                seen.add(mark)
+            self._key_functions = found
+        return self._key_functions
 
     def step_plans(self) -> list:
         """The step plans the layers' parts ask for, each once (by name): what a part wants computed on the host once

@@ -92,7 +92,11 @@ class _StepBuffers:
         if on_gpu:
             self.host = [h.pin_memory() for h in self.host]
         self.host_np = [h.numpy() for h in self.host]
-        self.events = [None] * self.RING
+        self.sections = [{name: h[sl] for name, sl in self.off.items()} for h in self.host_np]
+        self.events = [None] * self.RING         # of a slot that has been sent: reached when it may be written again
+        self._spare_events = [torch.cuda.Event() if on_gpu else None for _ in range(self.RING)]
+        self._stream = (None, None)              # handle and object of the stream of the last upload
+        self.count = np.arange(max_requests + 1, dtype=np.int32)
         self.dev = torch.zeros(self.size, dtype=torch.int32, device=self.device)
         self.tables = tables if tables is not None else torch.full((max(1, n_groups), max_requests, max_blocks), -1,
                                                                   dtype=torch.int32, device=self.device)
@@ -114,9 +118,11 @@ class _StepBuffers:
             sec = self.off[section]
             self.dev[sec].copy_(self.host[i][sec], non_blocking=True)
         if self.device.type == "cuda":
-            ev = torch.cuda.Event()
-            ev.record()
-            self.events[i] = ev
+            handle = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+            if self._stream[0] != handle:
+                self._stream = (handle, torch.cuda.current_stream())
+            self.events[i] = self._spare_events[i]
+            self.events[i].record(self._stream[1])
 
     def dev_view(self, name: str) -> torch.Tensor:
         return self.dev[self.off[name]]
@@ -251,20 +257,34 @@ class BatchBuilder:
         i = b.next_host()
         h = b.host_np[i]
         off = b.off
-        tok = h[off["token_ids"]]
-        pos = h[off["positions"]]
-        rreq = h[off["row_request"]]
-        rslot = h[off["row_slot"]]
-        lrows = h[off["logit_rows"]]
-        q_start = h[off["q_start"]]
-        pos_start = h[off["pos_start"]]
-        kv_len = h[off["kv_len"]]
-        slots = h[off["state_slots"]]
+        sec = b.sections[i]
+        tok, pos, rreq, rslot, lrows = (sec[n] for n in ("token_ids", "positions", "row_request", "row_slot", "logit_rows"))
+        q_start, pos_start, kv_len, slots = (sec[n] for n in ("q_start", "pos_start", "kv_len", "state_slots"))
         r0 = 0
         n_logit = 0
         portions_kv_len = 0
         h_q_len, h_q_start, h_pos_start, h_slots = [], [], [], []
-        for r, e in enumerate(entries):
+        single = total == len(entries)
+        if single:
+            # one token each (every decode step): whole arrays at once
+            n = total
+            h_q_len, h_q_start = [1] * n, list(range(n))
+            h_pos_start = [self.computed[e.request] for e in entries]
+            h_slots = [self.cache.slot_of(e.request) for e in entries]
+            wanted = [r for r, e in enumerate(entries) for _ in e.want]
+            starts = np.array(h_pos_start, dtype=np.int32)
+            tok[:n] = [e.tokens[0] for e in entries]
+            pos[:n] = starts
+            pos_start[:n] = starts
+            kv_len[:n] = starts + 1
+            rslot[:n] = h_slots
+            slots[:n] = rslot[:n]
+            rreq[:n] = b.count[:n]
+            q_start[:n] = b.count[:n]
+            n_logit = len(wanted)
+            lrows[:n_logit] = wanted
+            r0 = n
+        for r, e in enumerate(() if single else entries):
             n = len(e.tokens)
             start = self.computed[e.request]
             slot = self.cache.slot_of(e.request)
@@ -290,7 +310,8 @@ class BatchBuilder:
         shape = StepShape(h_q_len, h_q_start, h_pos_start, h_slots, total)
         extras = {}
         for plan in b.plans:
-            extras[plan.name] = (b.views[f"plan:{plan.name}"], plan.fill(h[off[f"plan:{plan.name}"]], shape))
+            place = "plan:" + plan.name
+            extras[plan.name] = (b.views[place], plan.fill(sec[place], shape))
         if feedback_src is not None:
             if total != len(entries) or len(feedback_src) != len(entries):
                 raise InvalidArgument("token feedback needs one token per entry and one source per entry")
@@ -315,8 +336,8 @@ class BatchBuilder:
             row_request=d["row_request"], row_slot=d["row_slot"], q_start=d["q_start"], pos_start=d["pos_start"],
             kv_len=d["kv_len"], state_slots=d["state_slots"], logit_rows=d["logit_rows"], num_logit_rows=n_logit,
             h_q_len=h_q_len, h_pos_start=h_pos_start, h_state_slots=h_slots, block_tables=self.tables,
-            decode_only=all(n == 1 for n in h_q_len), max_q_len=max(h_q_len),
-            max_kv_len=max(s + n for s, n in zip(h_pos_start, h_q_len)), portions_kv_len=portions_kv_len, extras=extras)
+            decode_only=single, max_q_len=max(h_q_len),
+            max_kv_len=max(h_pos_start) + 1 if single else max(s + n for s, n in zip(h_pos_start, h_q_len)), portions_kv_len=portions_kv_len, extras=extras)
 
     def finish(self, entries: Sequence[StepEntry]) -> None:
         """The step has been issued: count its tokens and let windows give pages back."""

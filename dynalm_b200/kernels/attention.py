@@ -45,6 +45,12 @@ class QueryTilePlan:
         lead = 0
         while lead < len(shape.q_len) and shape.q_len[lead] == 1:
             lead += 1
+        if lead == len(shape.q_len):               # single tokens alone: a tile each, those with the most keys first
+            flat = []
+            for r in sorted(range(lead), key=shape.pos_start.__getitem__, reverse=True):
+                flat += (shape.slots[r], shape.q_start[r], 1, shape.pos_start[r])
+            host[:len(flat)] = flat
+            return lead, 0, lead
         tiles = []
         for r, (n, r0, start, slot) in enumerate(zip(shape.q_len, shape.q_start, shape.pos_start, shape.slots)):
             for t0 in range(0, n, Q_TILE):

@@ -405,8 +405,13 @@ class Recording:
 _pinned_stream: Optional[int] = None
 
 
+def current_stream_handle() -> int:
+    """The handle of the current device's current stream (0.1 us; torch.cuda.current_stream() takes 3)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _stream() -> int:
-    return _pinned_stream if _pinned_stream is not None else torch.cuda.current_stream().cuda_stream
+    return _pinned_stream if _pinned_stream is not None else current_stream_handle()
 
 
 @contextlib.contextmanager
@@ -415,7 +420,7 @@ def pinned_stream():
     pass instead of one per launch (the lookup costs more than the launch)."""
     global _pinned_stream
     previous = _pinned_stream
-    _pinned_stream = torch.cuda.current_stream().cuda_stream
+    _pinned_stream = current_stream_handle()
     try:
         yield
     finally:
