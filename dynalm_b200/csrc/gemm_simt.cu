@@ -29,7 +29,7 @@
 //   64                      337 -> 41      363 -> 121      1,356 -> 142
 //   700                     307 -> 162     1,788 -> 1,049  1,205 -> 577
 //   2,048                   675 -> 394      4,919 -> 2,736  2,686 -> 1,449
-#include "common.cuh"
+#include "qkv_rope.cuh"
 
 #include <cooperative_groups.h>
 
@@ -59,17 +59,36 @@ constexpr int RWARPS = SPANS / 2;         // two spans a warp
 template <int R>
 __host__ __device__ constexpr int rows_stage_floats() { return 2 * RF * RW + 2 * R * RK; }
 
-template <int R>
+// What becomes of the sums of up to 16 rows on their way out: the gated activation silu(gate) up of W = [gate; up] (a block holds eight
+// gate and the eight matching up features), or the rotary encoding and the cache write of the q | k | v projection (qkv_rope.cuh;
+// a block of a q or k head holds eight rotary pairs). Both as activation.cu and rope_cache.cu work them out, which were launches of
+// their own (a step of a tiny model, 5 rows and 3 layers: 32 launches, now 26).
+enum { ROWS_STORE = 0, ROWS_SWIGLU = 1, ROWS_ROPE = 2 };
+
+template <int R, int OUT>
 __global__ void __launch_bounds__(RWARPS * 32)
 gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ w, const float* __restrict__ bias,
-                 float* __restrict__ y, int ldy, int M, int N, int K, float out_scale) {
+                 float* __restrict__ y, int ldy, int M, int N, int K, float out_scale, const QkvRopeOf<float> rope) {
   extern __shared__ __align__(16) float rows_smem[];
   const int m_first = blockIdx.y * R;
   x += static_cast<size_t>(m_first) * ldx;
   y += static_cast<size_t>(m_first) * ldy;
   M -= m_first;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, f = lane & 15, half = lane >> 4;
-  const int n0 = blockIdx.x * RF, span = span_length(K);
+  const int span = span_length(K);
+  // the block's features: eight from n0 on, eight from n1 on
+  int n0 = blockIdx.x * RF, n1 = n0 + RF / 2, head = 0;
+  bool turned = false;
+  if constexpr (OUT == ROWS_SWIGLU) n0 = blockIdx.x * (RF / 2), n1 = N / 2 + n0;
+  if constexpr (OUT == ROWS_ROPE) {
+    const int per_head = rope.head_dim / RF;
+    head = blockIdx.x / per_head;                   // q heads, then k heads, then v heads
+    turned = head < rope.n_heads + rope.n_kv_heads;
+    if (turned) {
+      n0 = head * rope.head_dim + blockIdx.x % per_head * (RF / 2);
+      n1 = n0 + rope.head_dim / 2;
+    }
+  }
   float* ring = rows_smem + warp * 2 * rows_stage_floats<R>();
   const int steps = span / RK;
 
@@ -80,7 +99,7 @@ gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__
     for (int i = 0; i < 2 * RF * RK / 4 / 32; ++i) {
       const int e = i * 32 + lane, c = e & 7, row = e >> 3;         // row: half * 16 + feature
       const int k = (2 * warp + (row >> 4)) * span + s * RK + c * 4;
-      const int n = min(n0 + (row & 15), N - 1);
+      const int n = min((row & 8 ? n1 : n0) + (row & 7), N - 1);
       cp_async16_zfill(st + row * RW + c * 4, w + static_cast<size_t>(n) * K + (k < K ? k : 0), k < K ? 16 : 0);
     }
   };
@@ -132,9 +151,9 @@ gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__
 #pragma unroll
   for (int m = 0; m < R; ++m) rows_smem[((2 * warp + half) * R + m) * RF + f] = acc[m];
   __syncthreads();
-  const int t = threadIdx.x, m = t >> 4, n = n0 + f;
-  if (t < RF * R && m < M && n < N) {
-    const float* s = rows_smem + m * RF + f;
+  const int t = threadIdx.x;
+  auto sum_of = [&](int m, int i) {
+    const float* s = rows_smem + m * RF + i;
     float total = 0.0f;
 #pragma unroll
     for (int q = 0; q < QUARTERS; ++q) {
@@ -143,8 +162,41 @@ gemm_rows_kernel(const float* __restrict__ x, int ldx, const float* __restrict__
       for (int j = 1; j < SPANS / QUARTERS; ++j) part += s[(4 * q + j) * R * RF];
       total = q == 0 ? part : total + part;
     }
+    return total;
+  };
+  if constexpr (OUT == ROWS_STORE) {
+    const int m = t >> 4, n = n0 + f;
+    if (t >= RF * R || m >= M || n >= N) return;
+    float total = sum_of(m, f);
     if (bias) total += bias[n];
     y[static_cast<size_t>(m) * ldy + n] = total * out_scale;
+  } else {
+    const int m = t >> 3, i = t & 7;
+    if (t >= RF / 2 * R || m >= M) return;
+    float a = sum_of(m, i), b = sum_of(m, i + RF / 2);
+    if constexpr (OUT == ROWS_SWIGLU) {
+      if (n0 + i < N / 2) y[static_cast<size_t>(m) * ldy + n0 + i] = a / (1.0f + expf(-a)) * b;
+    } else {
+      const int pos = rope.positions[m], hd = rope.head_dim, in_head = n0 + i - head * hd;
+      if (turned) {
+        const float theta = static_cast<float>(pos) * rope.pos_scale * rope.inv_freq[in_head];
+        float s, c;
+        sincosf(theta, &s, &c);
+        const float ra = a * c - b * s, rb = a * s + b * c;
+        a = ra, b = rb;
+      }
+      float* to;
+      if (head < rope.n_heads) {
+        to = y + static_cast<size_t>(m) * ldy + n0 + i;
+      } else {
+        const size_t slot = qkv_rope_slot(rope, m, pos);
+        if (slot == QKV_NO_SLOT) return;
+        const int kvh = head - rope.n_heads - (turned ? 0 : rope.n_kv_heads);
+        to = (turned ? rope.k_cache : rope.v_cache) + (slot * rope.n_kv_heads + kvh) * hd + in_head;
+      }
+      to[0] = a;
+      to[n1 - n0] = b;
+    }
   }
 }
 
@@ -372,15 +424,16 @@ int launch_tiles(const void* x, int ldx, const void* w, const float* bias, void*
                                              static_cast<TO*>(y), ldy, M, N, K, out_scale, wide));
 }
 
-template <int R>
+template <int R, int OUT = ROWS_STORE>
 int launch_rows(const float* x, int ldx, const float* w, const float* bias, float* y, int ldy, int M, int N, int K,
-                float out_scale, cudaStream_t stream) {
+                float out_scale, cudaStream_t stream, const QkvRopeOf<float>& rope = {}) {
   constexpr int SMEM = RWARPS * 2 * rows_stage_floats<R>() * 4;
-  auto kernel = gemm_rows_kernel<R>;
+  auto kernel = gemm_rows_kernel<R, OUT>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
-  return launch_streaming(kernel, dim3((N + RF - 1) / RF, (M + R - 1) / R), dim3(RWARPS * 32), SMEM, stream, x, ldx, w, bias, y, ldy, M, N, K,
-                          out_scale);
+  const int blocks = OUT == ROWS_SWIGLU ? (N / 2 + RF / 2 - 1) / (RF / 2) : (N + RF - 1) / RF;
+  return launch_streaming(kernel, dim3(blocks, (M + R - 1) / R), dim3(RWARPS * 32), SMEM, stream, x, ldx, w, bias, y, ldy, M, N, K,
+                          out_scale, rope);
 }
 
 }  // namespace dl
@@ -432,4 +485,41 @@ DL_EXPORT int dl_gemm_simt(int in_dtype, int out_dtype, const void* x, int ldx, 
 #undef DL_LAUNCH
 #undef DL_TILES
   return DL_ERR_UNSUPPORTED;
+}
+
+// The gated feed-forward's first half for up to 16 rows, float32: w = [Wg; Wu] with 2 F rows, y [M, F] = silu(x Wg^T) (x Wu^T), the
+// same bits as the product followed by dl_silu_mul. x and w 16-byte aligned, K and ldx multiples of 4.
+DL_EXPORT int dl_gemm_simt_swiglu(const float* x, int ldx, const float* w, float* y, int ldy, int M, int F, int K, cudaStream_t stream) {
+  if (M <= 0 || F <= 0) return 0;
+  if (K <= 0 || (K & 3) || (ldx & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || M > 16 || F > (1 << 29))
+    return DL_ERR_UNSUPPORTED;
+#define DL_ROWS(R) return dl::launch_rows<R, dl::ROWS_SWIGLU>(x, ldx, w, nullptr, y, ldy, M, 2 * F, K, 1.0f, stream)
+  if (M == 1) DL_ROWS(1);
+  if (M == 2) DL_ROWS(2);
+  if (M <= 4) DL_ROWS(4);
+  if (M <= 8) DL_ROWS(8);
+  DL_ROWS(16);
+#undef DL_ROWS
+}
+
+// The q | k | v projection of up to 16 rows, float32, with the rotary encoding and the cache write: as dl_gemm_split_qkv_rope, the
+// same bits as dl_gemm_simt followed by dl_rope_cache_write.
+DL_EXPORT int dl_gemm_simt_qkv_rope(const float* x, int ldx, const float* w, float* q_out, int ldq, int M, int K, const int* positions,
+                                    const int* row_request, const int* block_table, int max_blocks, float* k_cache, float* v_cache,
+                                    const float* inv_freq, float pos_scale, int n_heads, int n_kv_heads, int head_dim, int page_size,
+                                    cudaStream_t stream) {
+  if (M <= 0) return 0;
+  if (K <= 0 || (K & 3) || (ldx & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) || M > 16 ||
+      head_dim <= 0 || head_dim % dl::RF || n_heads <= 0 || n_kv_heads <= 0 || page_size <= 0 || inv_freq == nullptr)
+    return DL_ERR_UNSUPPORTED;
+  const dl::QkvRopeOf<float> rope = {positions, row_request, block_table, max_blocks, k_cache, v_cache, inv_freq, nullptr, pos_scale,
+                                     n_heads, n_kv_heads, head_dim, page_size};
+  const int N = (n_heads + 2 * n_kv_heads) * head_dim;
+#define DL_ROWS(R) return dl::launch_rows<R, dl::ROWS_ROPE>(x, ldx, w, nullptr, q_out, ldq, M, N, K, 1.0f, stream, rope)
+  if (M == 1) DL_ROWS(1);
+  if (M == 2) DL_ROWS(2);
+  if (M <= 4) DL_ROWS(4);
+  if (M <= 8) DL_ROWS(8);
+  DL_ROWS(16);
+#undef DL_ROWS
 }

@@ -125,6 +125,14 @@ def split_applies(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0)
 
 
+def plain_few_applies(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a float32 product of few rows that does not take the kernels of split numbers may have an epilogue of its own
+    (csrc/gemm_simt.cu, gemm_rows_kernel): matrices too small for those, so the answer does not hang on scratch."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] <= ops.SPLIT_FEW_ROWS
+            and min(w.shape) < SPLIT_MIN and w.shape[1] % 4 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0
+            and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0)
+
+
 def split_scratch(x: torch.Tensor, w: torch.Tensor, runtime) -> Optional[torch.Tensor]:
     """Scratch for a product of split numbers of as many rows as the runtime may bring; None when it does not apply or the device
     has no room for it (then no step of this runtime gets any, whatever its rows)."""
@@ -251,6 +259,9 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, runtime, inner: int)
         return act
     if split_scratch(x, w_gate_up, runtime) is not None and w_gate_up.shape[0] == 2 * inner and ops.split_swiglu_applies(rows, inner):
         ops.gemm_split_swiglu(x, w_gate_up, act)      # (the same bits as the two steps below)
+        return act
+    if plain_few_applies(x, w_gate_up) and w_gate_up.shape[0] == 2 * inner:
+        ops.gemm_simt_swiglu(x, w_gate_up, act)       # (likewise)
         return act
     gate_up = runtime.buffer("ffn_gate_up", (rows, 2 * inner))
     linear(x, w_gate_up, gate_up, runtime=runtime)

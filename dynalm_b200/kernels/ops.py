@@ -153,7 +153,10 @@ _SIGNATURES = {
         "dl_attention_f32_tiles": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _I, _P],
         "dl_attention_f32_rows": [_P, _I, _P, _L, _P, _L, _P, _I, _P, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P,
                                   _I, _I, _P]},
-    "gemm_simt": {"dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P]},
+    "gemm_simt": {
+        "dl_gemm_simt": [_I, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _F, _P],
+        "dl_gemm_simt_swiglu": [_P, _I, _P, _P, _I, _I, _I, _I, _P],
+        "dl_gemm_simt_qkv_rope": [_P, _I, _P, _P, _I, _I, _I, _P, _P, _P, _I, _P, _P, _P, _F, _I, _I, _I, _I, _P]},
     "sampling": {
         "dl_argmax": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
         "dl_sample_temperature": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
@@ -1271,13 +1274,14 @@ def rope_angles(positions: torch.Tensor, inv_freq: torch.Tensor, pos_scale: floa
 def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, positions: torch.Tensor,
                   row_request: torch.Tensor, block_table: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                   inv_freq: torch.Tensor, pos_scale: float, n_heads: int, n_kv_heads: int, head_dim: int,
-                  page_size: int, angles: Optional[torch.Tensor] = None) -> None:
+                  page_size: int, angles: Optional[torch.Tensor] = None, plain: bool = False) -> None:
     """The q | k | v projection with rotary encoding and cache write in its epilogue: rotated q into
     q_out [rows, >= n_heads * head_dim], rotated k and plain v into the paged cache. The whole head is rotated
     (inv_freq has head_dim / 2 entries). bfloat16: up to 16 rows the weight-streaming kernel
     (csrc/gemm_skinny.cu, head_dim a multiple of 16); more rows: the tcgen05 kernel (csrc/gemm_tcgen05.cu,
     head_dim 64 or 128), which reads the step's (cos, sin) pairs from `angles` (see rope_angles) when given. float32: up to
-    16 rows, the product of split numbers (csrc/gemm_split.cu, head_dim a multiple of 16)."""
+    16 rows, head_dim a multiple of 16, the product of split numbers (csrc/gemm_split.cu) or with `plain` the one of
+    csrc/gemm_simt.cu."""
     _cuda(x, w_qkv, q_out, positions, row_request, block_table, k_cache, v_cache, inv_freq)
     _rows_contiguous(x, "x")
     _rows_contiguous(q_out, "q_out")
@@ -1316,11 +1320,12 @@ def gemm_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, pos
                "gemm_tcgen05_qkv_rope")
         return
     if exact:
-        check_limits("gemm_split", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
-        _check(_fn("gemm_split", "dl_gemm_split_qkv_rope")(
+        library = "gemm_simt" if plain else "gemm_split"
+        check_limits(library, pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
+        _check(_fn(library, f"dl_{library}_qkv_rope")(
             _p(x), x.stride(0), _p(w_qkv), _p(q_out), q_out.stride(0), M, K, _p(positions), _p(row_request), _p(block_table),
             block_table.stride(0), _p(k_cache), _p(v_cache), _p(inv_freq), pos_scale, n_heads, n_kv_heads, head_dim, page_size,
-            _stream()), "gemm_split_qkv_rope")
+            _stream()), f"{library}_qkv_rope")
         return
     check_limits("gemm_skinny", pages=k_cache.shape[0], requests=block_table.shape[0], rows=M)
     _check(_fn("gemm_skinny", "dl_gemm_skinny_qkv_rope")(
@@ -1492,17 +1497,27 @@ def split_swiglu_applies(rows: int, inner: int) -> bool:
     return rows <= SPLIT_FEW_ROWS and 5 * -(-inner // 64) >= 4 * sm_count()
 
 
+def gemm_simt_swiglu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """out = silu(x Wg^T) * (x Wu^T) with w = [Wg; Wu], float32, for up to SPLIT_FEW_ROWS rows, as gemm_simt and silu_mul give it."""
+    _swiglu_f32("gemm_simt", x, w, out)
+
+
 def gemm_split_swiglu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out = silu(x Wg^T) * (x Wu^T) with w = [Wg; Wu], for up to SPLIT_FEW_ROWS rows, the products as gemm_split gives them."""
+    """out = silu(x Wg^T) * (x Wu^T) with w = [Wg; Wu], for up to SPLIT_FEW_ROWS rows, as gemm_split and silu_mul give it."""
+    _swiglu_f32("gemm_split", x, w, out)
+
+
+def _swiglu_f32(library: str, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _cuda(x, w, out)
     M, K = x.shape
     F = w.shape[0] // 2
     _rows_contiguous(x, "x")
     _rows_contiguous(out, "out")
     if ((x.dtype, w.dtype, out.dtype) != (torch.float32,) * 3 or not w.is_contiguous() or w.shape != (2 * F, K) or out.shape != (M, F)):
-        raise InvalidArgument("gemm_split_swiglu: x [M, K], w [2 F, K] contiguous and out [M, F], all float32")
-    _check(_fn("gemm_split", "dl_gemm_split_swiglu")(_p(x), x.stride(0), _p(w), _p(out), out.stride(0), M, F, K,
-                                                     _p(_status_word(x.device)), _stream()), "gemm_split_swiglu")
+        raise InvalidArgument(f"{library}_swiglu: x [M, K], w [2 F, K] contiguous and out [M, F], all float32")
+    status = (_p(_status_word(x.device)),) if library == "gemm_split" else ()
+    _check(_fn(library, f"dl_{library}_swiglu")(_p(x), x.stride(0), _p(w), _p(out), out.stride(0), M, F, K, *status, _stream()),
+           f"{library}_swiglu")
 
 
 SKINNY_MAX_ROWS = 64      # what the kernel takes

@@ -14,7 +14,7 @@ import torch
 
 from ..errors import Unsupported
 from ..kernels import linear, ops
-from ..kernels.gemm import linear_partial, linear_partial_biased, split_scratch
+from ..kernels.gemm import linear_partial, linear_partial_biased, plain_few_applies, split_scratch
 from .base import POSITIONS, CacheSpec, TensorDecl, register_mixer
 
 
@@ -91,7 +91,8 @@ class PagedAttention:
             step_angles = getattr(self.position, "step_angles", None)
             angles = step_angles(ctx, rt) if rows > ops.SKINNY_FAST_ROWS and step_angles is not None else None
             ops.gemm_qkv_rope(x, self.w_qkv, qkv, ctx.positions, ctx.row_slot, cache.block_table, k_cache, v_cache,
-                              table[0], table[2], s.num_heads, s.num_kv_heads, s.head_dim, cache.page_size, angles)
+                              table[0], table[2], s.num_heads, s.num_kv_heads, s.head_dim, cache.page_size, angles,
+                              plain=plain_few_applies(x, self.w_qkv))
             return self._attend_and_project(qkv, cache, ctx, rows)
         if owns_cache:
             qkv = rt.buffer("attn_qkv", (rows, self.q_width + 2 * self.kv_width))
@@ -118,7 +119,7 @@ class PagedAttention:
             return False
         if x.dtype == torch.float32:
             return (x.shape[0] <= ops.SPLIT_FEW_ROWS and self.spec.head_dim % 16 == 0
-                    and split_scratch(x, self.w_qkv, self.rt) is not None)
+                    and (plain_few_applies(x, self.w_qkv) or split_scratch(x, self.w_qkv, self.rt) is not None))
         if not (x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0):
             return False
         if x.shape[0] <= ops.SKINNY_FAST_ROWS:

@@ -85,21 +85,25 @@ def test_numbers_without_finite_parts(ops, rows):
         assert ((out[finite] - plain[finite]).abs() <= 2e-5 * size).all(), (kind, tile)
 
 
+@pytest.mark.parametrize("plain", [False, True])
 @pytest.mark.parametrize("rows,F,K", [(1, 8192, 512), (7, 8300, 516), (16, 20000, 64)])
-def test_gated_product_is_its_two_steps(ops, rows, F, K):
+def test_gated_product_is_its_two_steps(ops, rows, F, K, plain):
     g = torch.Generator(device="cpu").manual_seed(F)
+    if plain:
+        F = F // 8 % 300 + 5
     x, w = torch.randn(rows, K, generator=g).to(DEV), (torch.randn(2 * F, K, generator=g) * 0.1).to(DEV)
     x[0, 0] = float("inf")
-    assert ops.split_swiglu_applies(rows, F)
+    assert plain or ops.split_swiglu_applies(rows, F)
     both, want, out = torch.empty(rows, 2 * F, device=DEV), torch.empty(rows, F, device=DEV), torch.empty(rows, F, device=DEV)
-    ops.gemm_split(x, w, both)
+    (ops.gemm_simt if plain else ops.gemm_split)(x, w, both)
     ops.silu_mul(both, want)
-    ops.gemm_split_swiglu(x, w, out)
+    (ops.gemm_simt_swiglu if plain else ops.gemm_split_swiglu)(x, w, out)
     assert torch.equal(out.nan_to_num(1.5), want.nan_to_num(1.5))
 
 
+@pytest.mark.parametrize("plain", [False, True])
 @pytest.mark.parametrize("rows,heads,groups,dim,K", [(1, 4, 2, 32, 512), (7, 32, 8, 64, 516), (8, 3, 1, 128, 96), (16, 80, 40, 16, 64)])
-def test_rotating_projection_is_its_two_steps(ops, rows, heads, groups, dim, K):
+def test_rotating_projection_is_its_two_steps(ops, rows, heads, groups, dim, K, plain):
     g = torch.Generator(device="cpu").manual_seed(rows)
     N, page = (heads + 2 * groups) * dim, 16
     x, w = torch.randn(rows, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
@@ -110,9 +114,9 @@ def test_rotating_projection_is_its_two_steps(ops, rows, heads, groups, dim, K):
     inv = (500000.0 ** (-torch.arange(dim // 2, dtype=torch.float32) * 2 / dim)).to(DEV)
     caches = [[torch.zeros(rows, page, groups, dim, device=DEV) for _ in "kv"] for _ in "ab"]
     qkv, fused = torch.empty(rows, N, device=DEV), torch.empty(rows, N, device=DEV)
-    ops.gemm_split(x, w, qkv)
+    (ops.gemm_simt if plain else ops.gemm_split)(x, w, qkv)
     ops.rope_cache_write(qkv, positions, slot, table, *caches[0], inv, dim, 0.5, heads, groups, dim, page)
-    ops.gemm_qkv_rope(x, w, fused, positions, slot, table, *caches[1], inv, 0.5, heads, groups, dim, page)
+    ops.gemm_qkv_rope(x, w, fused, positions, slot, table, *caches[1], inv, 0.5, heads, groups, dim, page, plain=plain)
     assert torch.equal(qkv[:, :heads * dim].nan_to_num(1.5), fused[:, :heads * dim].nan_to_num(1.5))
     assert all(torch.equal(a, b) for a, b in zip(*caches))
     assert caches[0][0].abs().sum() > 0 and caches[0][1].abs().sum() > 0
