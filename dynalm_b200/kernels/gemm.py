@@ -59,12 +59,33 @@ def skinny_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
 STREAM_ROWS = min(int(os.environ.get("DYNALM_STREAM_ROWS", "16")), ops.STREAM_MAX_ROWS)
 
 
-def use_stream(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return (x.dtype == torch.bfloat16 and 8 < x.shape[0] <= STREAM_ROWS and x.shape[1] % 8 == 0
+# The gated product, which has no K to split, goes on with it up to 31 rows (2 x 8192 x 2048: 14.3 us at 17 and 24 rows against 19.4 of the
+# tcgen05 product, 14.2 against 14.6 at 32, 16.1 against 14.4 at 48).
+GATED_ROWS = max(STREAM_ROWS, 31) if STREAM_ROWS else 0
+
+
+def use_stream(x: torch.Tensor, w: torch.Tensor, most: int = STREAM_ROWS) -> bool:
+    return (x.dtype == torch.bfloat16 and 8 < x.shape[0] <= most and x.shape[1] % 8 == 0
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.is_contiguous()
             and w.data_ptr() % 16 == 0)
 
 
+def stream_deep_splits(x: torch.Tensor, w: torch.Tensor) -> int:
+    """K splits with which the streaming product takes more rows than STREAM_ROWS for a consumer that adds partial sums; 0: it
+    does not."""
+    M, K = x.shape
+    if not (STREAM_ROWS < M <= DEEP_ROWS and K >= DEEP_K and x.dtype == torch.bfloat16 and K % 8 == 0 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0):
+        return 0
+    splits = min(8, sm_count() // max(1, -(-w.shape[0] // 128)), K // 256)
+    return splits if splits == 8 else 0
+
+
+# Products whose sums a norm adds: rows and k from which on the streaming product with eight K splits, 128 blocks or so, is ahead of
+# the library's split-K kernels (us, weights in memory, 2048 x 8192: 24 rows 8.6 against 13.1, 48 rows 10.1 against 13.1, of which
+# the norm takes back half a us; with the six splits that 3,072 features leave 24 rows 11.0 against 14.3 alone but no gain in a
+# whole step, and none for 64 rows). Whole decode steps of the 1B shape: 20 rows 1,180 -> 1,119 us, 30 rows 1,155 -> 1,112.
+DEEP_ROWS, DEEP_K = 48, 4096
 STREAM_MAX_SPLITS = 6      # more partial sums cost the norm that adds them more than they save (0.98 against 1.00 ms)
 
 
@@ -198,6 +219,12 @@ def linear_partial(x: torch.Tensor, w: torch.Tensor, runtime, name: str) -> torc
             out = flat[:parts * M * N].view(parts, M, N)
             (ops.gemm_stream if stream else ops.gemm_skinny)(x, w, out, "store", 1.0)
             return out
+    parts = stream_deep_splits(x, w)
+    if parts > 0:
+        flat = runtime.flat(f"{name}_parts_{N}", 16 * ops.SKINNY_MAX_ROWS * N, torch.float32)
+        out = flat[:parts * M * N].view(parts, M, N)
+        ops.gemm_stream(x, w, out, "store", 1.0)
+        return out
     out = runtime.buffer(name, (M, N))
     return linear(x, w, out, runtime=runtime)
 
@@ -239,7 +266,7 @@ def _gated_epilogue(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor,
     of them takes the product."""
     if x.dtype != torch.bfloat16:
         return False
-    if use_stream(x, w_gate_up):
+    if use_stream(x, w_gate_up, GATED_ROWS):
         ops.gemm_stream(x, w_gate_up, act, "swiglu", coeffs=coeffs)
     elif skinny_ok(x, w_gate_up):
         ops.gemm_skinny(x, w_gate_up, act, "swiglu", coeffs=coeffs)

@@ -311,3 +311,15 @@ def test_32_bit_attention_goes_where_it_costs_least(monkeypatch):
     assert launches([1, 1, 300], [10, 2999, 0]) == (2, 4, 0, 3, 1, 0)            # the portion's own keys count, not the others'
     assert launches([70], [3000])[3] == 1 and launches([5], [3000])[:4] == (0, 1, 0, 0)
     attention._f32_costs.cache_clear()
+
+
+def test_deep_narrow_products_of_some_rows_stream_with_eight_splits():
+    def splits(rows, n, k):
+        return gemm.stream_deep_splits(*_xw(rows, n, k))
+    assert splits(17, 2048, 8192) == 8 and splits(48, 2048, 12288) == 8 and splits(24, 2048, 4096) == 8
+    assert not splits(16, 2048, 8192) and not splits(49, 2048, 8192)         # few rows have their own kernels, more the library
+    assert not splits(24, 3072, 8192) and not splits(24, 2048, 2048)         # six splits, or too few slices of k
+    x, w = _xw(31, 16384, 2048)
+    assert gemm.use_stream(x, w, gemm.GATED_ROWS) and not gemm.use_stream(x, w)
+    x, w = _xw(32, 16384, 2048)
+    assert not gemm.use_stream(x, w, gemm.GATED_ROWS)
