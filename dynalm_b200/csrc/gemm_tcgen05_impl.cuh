@@ -432,10 +432,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
             const int col = n0 + c0 + j;
-            if (col < n_end)                       // a multiple of 4 in this mode
+            if (col < n_end) {                     // a multiple of 4 in this mode
+              const float4 add = coeffs != nullptr ? *reinterpret_cast<const float4*>(coeffs + col) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
               *reinterpret_cast<float4*>(out + col) =
-                  make_float4(__uint_as_float(v[j]) * out_scale, __uint_as_float(v[j + 1]) * out_scale,
-                              __uint_as_float(v[j + 2]) * out_scale, __uint_as_float(v[j + 3]) * out_scale);
+                  make_float4(fmaf(__uint_as_float(v[j]), out_scale, add.x), fmaf(__uint_as_float(v[j + 1]), out_scale, add.y),
+                              fmaf(__uint_as_float(v[j + 2]), out_scale, add.z), fmaf(__uint_as_float(v[j + 3]), out_scale, add.w));
+            }
           }
         }
       } else {
@@ -575,7 +577,7 @@ static int t5_run(cudaLaunchConfig_t cfg, const CUtensorMap& map_x, const CUtens
 // mode 0: y bf16 [M, N] (N % 8 == 0); mode 1: y fp32 [M, N] (N % 4 == 0); mode 2: w = [gate; up] with N = 2F rows,
 // y bf16 [M, F] = silu(x Wg^T) * (x Wu^T) (F % 8 == 0), or with coeffs (N + 4 float32, 16-byte aligned: common.cuh,
 // CLAMPED_HEADER) the gated activation with clamped halves and biases; mode 4: y bf16 [M, N] = max(x W^T, 0)^2; mode 5: = gelu_tanh(x W^T);
-// mode 7: = xIELU(x W^T) with coeffs = two float32 on the device. status: one device int, set to a nonzero code if a wait
+// mode 7: = xIELU(x W^T) with coeffs = two float32 on the device; mode 1 with coeffs: N float32 (16-byte aligned) that are added. status: one device int, set to a nonzero code if a wait
 // inside the kernel timed out (left untouched otherwise).
 static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, int mode, float out_scale,
                      int* status, const dl::QkvRope& rope, int pairs, cudaStream_t stream, const float* coeffs = nullptr) {
@@ -583,7 +585,7 @@ static int t5_launch(const void* x, int ldx, const void* w, void* y, int ldy, in
   if (K <= 0 || (K & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) ||
       status == nullptr || mode < 0 || (mode > 5 && mode != dl::T5_OUT_XIELU) || (mode == dl::T5_OUT_XIELU && coeffs == nullptr))
     return DL_ERR_UNSUPPORTED;
-  if (mode == dl::T5_OUT_SWIGLU && (reinterpret_cast<uintptr_t>(coeffs) & 15)) return DL_ERR_UNSUPPORTED;
+  if ((mode == dl::T5_OUT_SWIGLU || mode == dl::T5_OUT_F32) && (reinterpret_cast<uintptr_t>(coeffs) & 15)) return DL_ERR_UNSUPPORTED;
   const int feats = mode == dl::T5_OUT_SWIGLU ? N / 2 : N;
   if ((mode == dl::T5_OUT_SWIGLU && (N & 1)) || (mode == dl::T5_OUT_F32 ? (feats & 3) || (ldy & 3) : (feats & 7) || (ldy & 7)) ||
       (reinterpret_cast<uintptr_t>(y) & 15))

@@ -51,17 +51,13 @@ __global__ void ssm_conv_kernel(const T* __restrict__ proj, int proj_stride, int
 // The same with a thread on 8 (bfloat16) or 4 (float32) neighbouring channels of a row, 16 bytes a load: for channel
 // counts, first columns and row pitches that are multiples of that.
 template <typename T>
-__global__ void ssm_conv_vec_kernel(const T* __restrict__ proj, int proj_stride, int col0, int channels,
-                                    const float* __restrict__ taps, const float* __restrict__ bias, int K,
-                                    const float* __restrict__ state, size_t state_stride, size_t keep_off,
-                                    const int* __restrict__ positions, const int* __restrict__ row_request,
-                                    const int* __restrict__ row_slot, const int* __restrict__ pos_start,
-                                    T* __restrict__ out, int rows, int act, const float* __restrict__ in_bias) {
+__device__ __forceinline__ void conv_row_vec(const T* __restrict__ proj, int proj_stride, int col0, int channels,
+                                             const float* __restrict__ taps, const float* __restrict__ bias, int K,
+                                             const float* __restrict__ state, size_t state_stride, size_t keep_off,
+                                             const int* __restrict__ positions, const int* __restrict__ row_request,
+                                             const int* __restrict__ row_slot, const int* __restrict__ pos_start,
+                                             T* __restrict__ out, int act, const float* __restrict__ in_bias, int row, int ch) {
   constexpr int V = PerVec<T>::n;
-  const int per_row = channels / V;
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= static_cast<size_t>(rows) * per_row) return;
-  const int row = static_cast<int>(idx / per_row), ch = static_cast<int>(idx % per_row) * V;
   const int pos = positions[row];
   const int first = pos_start[ck_request(row_request[row])];
   const float* kept = state + static_cast<size_t>(ck_request(row_slot[row])) * state_stride + keep_off;
@@ -98,6 +94,86 @@ __global__ void ssm_conv_vec_kernel(const T* __restrict__ proj, int proj_stride,
     for (int j = 0; j < V; ++j) acc[j] = silu_f(acc[j]);
   }
   *reinterpret_cast<Vec16*>(out + static_cast<size_t>(row) * channels + ch) = pack<T>(acc);
+}
+
+template <typename T>
+__global__ void ssm_conv_vec_kernel(const T* __restrict__ proj, int proj_stride, int col0, int channels,
+                                    const float* __restrict__ taps, const float* __restrict__ bias, int K,
+                                    const float* __restrict__ state, size_t state_stride, size_t keep_off,
+                                    const int* __restrict__ positions, const int* __restrict__ row_request,
+                                    const int* __restrict__ row_slot, const int* __restrict__ pos_start,
+                                    T* __restrict__ out, int rows, int act, const float* __restrict__ in_bias) {
+  constexpr int V = PerVec<T>::n;
+  const int per_row = channels / V;
+  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (idx >= static_cast<size_t>(rows) * per_row) return;
+  conv_row_vec<T>(proj, proj_stride, col0, channels, taps, bias, K, state, state_stride, keep_off, positions, row_request, row_slot,
+                  pos_start, out, act, in_bias, static_cast<int>(idx / per_row), static_cast<int>(idx % per_row) * V);
+}
+
+// The same for portions of prompts, bfloat16 and four taps: a thread works out CONV_RUN rows in a row, so that the taps are read
+// once for all of them and an input for four, and asks for all of its inputs at once. Rows whose inputs do not all lie in the step
+// (a portion's first ones, single tokens) go one by one. The same bits. (A thread a row was bound by issue and by the taps' way
+// through L1: 1,777 rows of 4,352 channels 34 us, now 25.)
+constexpr int CONV_RUN = 4;
+__global__ void __launch_bounds__(256)
+ssm_conv_runs_kernel(const bf16* __restrict__ proj, int proj_stride, int col0, int channels, const float* __restrict__ taps,
+                     const float* __restrict__ bias, const float* __restrict__ state, size_t state_stride, size_t keep_off,
+                     const int* __restrict__ positions, const int* __restrict__ row_request, const int* __restrict__ row_slot,
+                     const int* __restrict__ pos_start, bf16* __restrict__ out, int rows, int act) {
+  constexpr int K = 4, V = 8;
+  const int per_row = channels / V;
+  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int row0 = static_cast<int>(idx / per_row) * CONV_RUN, ch = static_cast<int>(idx % per_row) * V;
+  if (row0 >= rows) return;
+  const int request = ck_request(row_request[row0]);
+  const bool whole = row0 + CONV_RUN <= rows && row_request[row0 + CONV_RUN - 1] == request && positions[row0] - pos_start[request] >= K - 1;
+  if (!whole) {
+#pragma unroll 1
+    for (int row = row0; row < min(rows, row0 + CONV_RUN); ++row)
+      conv_row_vec<bf16>(proj, proj_stride, col0, channels, taps, bias, K, state, state_stride, keep_off, positions, row_request, row_slot,
+                         pos_start, out, act, nullptr, row, ch);
+    return;
+  }
+  Vec16 in[CONV_RUN + K - 1];
+#pragma unroll
+  for (int i = 0; i < CONV_RUN + K - 1; ++i)
+    in[i] = *reinterpret_cast<const Vec16*>(proj + static_cast<size_t>(row0 - (K - 1) + i) * proj_stride + col0 + ch);
+  float t[K][V], b[V];
+#pragma unroll
+  for (int j = 0; j < V; j += 4) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float4 t4 = *reinterpret_cast<const float4*>(taps + static_cast<size_t>(k) * channels + ch + j);
+      t[k][j] = t4.x, t[k][j + 1] = t4.y, t[k][j + 2] = t4.z, t[k][j + 3] = t4.w;
+    }
+    const float4 b4 = bias ? *reinterpret_cast<const float4*>(bias + ch + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    b[j] = b4.x, b[j + 1] = b4.y, b[j + 2] = b4.z, b[j + 3] = b4.w;
+  }
+  float acc[CONV_RUN][V];
+#pragma unroll
+  for (int r = 0; r < CONV_RUN; ++r)
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[r][j] = b[j];
+#pragma unroll
+  for (int i = 0; i < CONV_RUN + K - 1; ++i) {         // (an input's rows in turn: each row's sum is oldest input first)
+    float v[V];
+    unpack<bf16>(in[i], v);
+#pragma unroll
+    for (int r = 0; r < CONV_RUN; ++r) {
+      if (i < r || i >= r + K) continue;
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[r][j] = fmaf(t[i - r][j], v[j], acc[r][j]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < CONV_RUN; ++r) {
+    if (act) {
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[r][j] = silu_f(acc[r][j]);
+    }
+    *reinterpret_cast<Vec16*>(out + static_cast<size_t>(row0 + r) * channels + ch) = pack<bf16>(acc[r]);
+  }
 }
 
 // After the convolution of a step: the last K - 1 inputs of every request, oldest first. One thread per (request,
@@ -302,33 +378,49 @@ namespace dl {
 // Between the two passes over the segments of long portions: per request of `long_requests` (first segment, segments,
 // slot, -) and element of the state, the state before every segment in place of what the segment added, and the
 // request's new state.
-__global__ void ssm_carry_kernel(float* __restrict__ state, size_t state_stride, float* __restrict__ scratch,
-                                 const float* __restrict__ seg_decay, const int* __restrict__ long_requests, int H,
-                                 int per_head) {
+// A thread takes one number or, where the sizes and addresses allow 16 bytes, four neighbouring ones.
+template <int V>
+__global__ void __launch_bounds__(256)
+ssm_carry_kernel(float* __restrict__ state, size_t state_stride, float* __restrict__ scratch, const float* __restrict__ seg_decay,
+                 const int* __restrict__ long_requests, int H, int per_head) {
   const int4 req = reinterpret_cast<const int4*>(long_requests)[blockIdx.y];
   const size_t per_seg = static_cast<size_t>(H) * per_head;
-  const size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const size_t e = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * V;
   if (e >= per_seg) return;
   const int h = static_cast<int>(e / per_head);
   float* slot = state + static_cast<size_t>(ck_request(req.z)) * state_stride;
-  float S = slot[e];
+  float S[V];
+  auto load = [](float (&to)[V], const float* from) {
+    if constexpr (V == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(from);
+      to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
+    } else {
+      to[0] = *from;
+    }
+  };
+  auto store = [](float* to, const float (&from)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4*>(to) = make_float4(from[0], from[1], from[2], from[3]);
+    else *to = from[0];
+  };
+  load(S, slot + e);
   constexpr int AHEAD = 8;                       // segments whose numbers are asked for at a time: none depends on S
   for (int c0 = 0; c0 < req.y; c0 += AHEAD) {
-    float added[AHEAD], decay[AHEAD];
+    float added[AHEAD][V], decay[AHEAD];
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const size_t seg = static_cast<size_t>(req.x + min(c0 + k, req.y - 1));
-      added[k] = scratch[seg * per_seg + e];
+      load(added[k], scratch + seg * per_seg + e);
       decay[k] = seg_decay[seg * H + h];
     }
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       if (c0 + k >= req.y) break;
-      scratch[static_cast<size_t>(req.x + c0 + k) * per_seg + e] = S;
-      S = fmaf(decay[k], S, added[k]);
+      store(scratch + static_cast<size_t>(req.x + c0 + k) * per_seg + e, S);
+#pragma unroll
+      for (int j = 0; j < V; ++j) S[j] = fmaf(decay[k], S[j], added[k][j]);
     }
   }
-  slot[e] = S;
+  store(slot + e, S);
 }
 
 // ---- gated norm -----------------------------------------------------------------------------------------------
@@ -430,6 +522,14 @@ DL_EXPORT int dl_short_conv(int dtype, const void* proj, int proj_stride, int co
                     (reinterpret_cast<uintptr_t>(taps) & 15) == 0 && (bias == nullptr || (reinterpret_cast<uintptr_t>(bias) & 15) == 0);
   const size_t items = static_cast<size_t>(rows) * (wide ? channels / vec : channels);
   const unsigned blocks = static_cast<unsigned>((items + threads - 1) / threads);
+  // runs of rows from 256 rows on: below, a thread a row fills the SMs better (200 rows of 4,352 channels: 7.5 us)
+  if (dtype == 1 && wide && K == 4 && rows >= 256 && in_bias == nullptr) {
+    const size_t runs = static_cast<size_t>((rows + dl::CONV_RUN - 1) / dl::CONV_RUN) * (channels / vec);
+    dl::ssm_conv_runs_kernel<<<static_cast<unsigned>((runs + threads - 1) / threads), threads, 0, stream>>>(
+        static_cast<const dl::bf16*>(proj), proj_stride, col0, channels, taps, bias, state, static_cast<size_t>(state_stride),
+        static_cast<size_t>(keep_off), positions, row_request, row_slot, pos_start, static_cast<dl::bf16*>(out), rows, act);
+    return dl::launch_status();
+  }
 #define DL_LAUNCH(KERNEL, T)                                                                                         \
   dl::KERNEL<T><<<blocks, threads, 0, stream>>>(static_cast<const T*>(proj), proj_stride, col0, channels, taps, bias, K, \
                                                 state, static_cast<size_t>(state_stride), static_cast<size_t>(keep_off), \
@@ -530,8 +630,8 @@ DL_EXPORT int dl_ssm_scan(int dtype, const void* u, int u_stride, const void* pr
   DL_MODE(dl::SCAN_WHOLE, requests);
   // The matrix form takes bfloat16 inputs with 64 or 128 rows of state and channels a head, in whole runs of 16 bytes; other
   // sizes, float32 inputs (whose terms would not be exact) and segments that may be longer than its fixed arrays are walked. Measured on B200 (64 heads of 64, 128 rows, 8 groups;
-  // prompts of 394 and 1,383 tokens; us a layer): first pass 41 against 167 walked, outputs 70 against 219; the carry between
-  // them, with the segments' numbers asked for eight at a time, 21 against 39.
+  // prompts of 394 and 1,383 tokens; us a layer): first pass 34 against 167 walked, outputs 63 against 219; the carry between
+  // them, with the segments' numbers asked for eight at a time 21 against 39, and four numbers a thread 10.
   const bool matrices = dtype == 1 && (N == 64 || N == 128) && (P == 64 || P == 128) && whole_up_to <= dl::SEG_T && u_stride % 8 == 0 &&
                         (reinterpret_cast<uintptr_t>(u) & 15) == 0 && (reinterpret_cast<uintptr_t>(scratch) & 15) == 0 &&
                         (reinterpret_cast<uintptr_t>(y) & 7) == 0;
@@ -552,8 +652,11 @@ DL_EXPORT int dl_ssm_scan(int dtype, const void* u, int u_stride, const void* pr
     }
     const int per_head = N * P;
     const size_t per_seg = static_cast<size_t>(H) * per_head;
-    dl::ssm_carry_kernel<<<dim3(static_cast<unsigned>((per_seg + 255) / 256), n_long), 256, 0, stream>>>(
-        state, static_cast<size_t>(state_stride), scratch, seg_decay, long_requests, H, per_head);
+    const bool four = per_head % 4 == 0 && state_stride % 4 == 0 &&
+                      ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
+    const dim3 grid(static_cast<unsigned>((per_seg / (four ? 4 : 1) + 255) / 256), n_long);
+    if (four) dl::ssm_carry_kernel<4><<<grid, 256, 0, stream>>>(state, static_cast<size_t>(state_stride), scratch, seg_decay, long_requests, H, per_head);
+    else dl::ssm_carry_kernel<1><<<grid, 256, 0, stream>>>(state, static_cast<size_t>(state_stride), scratch, seg_decay, long_requests, H, per_head);
     if (matrices) {
       const int code = DL_SIZES(DL_OUTPUTS);
       if (code != 0) return code;

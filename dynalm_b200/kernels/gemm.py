@@ -256,7 +256,11 @@ def linear_partial_biased(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch
         out = linear_partial(x, w, runtime, name)
         ops.add_bias(out[0] if out.dim() == 3 else out, bias)
         return out
-    out = linear(x, w, runtime.buffer(name + "_wide", (M, N), torch.float32))
+    out = runtime.buffer(name + "_wide", (M, N), torch.float32)
+    if tcgen05_ok(x, w, out, N) and bias.is_contiguous() and bias.data_ptr() % 16 == 0:
+        ops.gemm_tcgen05(x, w, out, "biased", coeffs=bias)
+        return out
+    linear(x, w, out, runtime=runtime)
     ops.add_bias(out, bias)
     return out
 

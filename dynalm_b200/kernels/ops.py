@@ -1535,7 +1535,13 @@ def clamped_coeffs(limit: float, gate_scale: float, bias: Optional[torch.Tensor]
 
 
 def _epilogue_coeffs(mode: str, coeffs: Optional[torch.Tensor], features: int) -> None:
-    """xielu takes its two coefficients, swiglu those of clamped halves (clamped_coeffs) or none."""
+    """xielu takes its two coefficients, swiglu those of clamped halves (clamped_coeffs) or none, a plain float32 result of the
+    tcgen05 product ("biased") a number to add to every feature."""
+    if mode == "biased":
+        if coeffs is None or coeffs.dtype != torch.float32 or coeffs.numel() != features or not coeffs.is_contiguous() or coeffs.data_ptr() % 16:
+            raise InvalidArgument("a biased product goes with a float32 number for every feature, 16-byte aligned")
+        _cuda(coeffs)
+        return
     if mode == "swiglu":
         if coeffs is not None and (coeffs.dtype != torch.float32 or coeffs.numel() != CLAMPED_HEADER + features or coeffs.data_ptr() % 16):
             raise InvalidArgument("swiglu with clamped halves goes with clamped_coeffs on the device")
@@ -1590,7 +1596,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str 
 
     x [M, K] and w [N, K] bfloat16; out [M, N] bfloat16 or float32, or with mode "swiglu"
     (w = [gate; up]) out [M, N/2] bfloat16, or with mode "relu2" out [M, N] bfloat16 = max(x W^T, 0)^2; "gelu_tanh" and
-    "xielu" (with `coeffs`, see ops.xielu) likewise."""
+    "xielu" (with `coeffs`, see ops.xielu) likewise; "biased": out float32 = x W^T + coeffs."""
     _epilogue_coeffs(mode, coeffs, w.shape[0])
     _cuda(x, w, out)
     _rows_contiguous(x, "x")
@@ -1605,6 +1611,8 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: str 
             raise Unsupported("gemm_tcgen05: swiglu needs out [M, N/2] bfloat16 with N/2 a multiple of 8")
         code = 2
     else:
+        if mode == "biased" and out.dtype != torch.float32:
+            raise InvalidArgument("gemm_tcgen05: a biased product leaves float32")
         if out.shape != (M, N):
             raise InvalidArgument("gemm_tcgen05: out [M, N]")
         if out.dtype == torch.bfloat16:

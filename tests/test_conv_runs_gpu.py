@@ -1,0 +1,66 @@
+"""Kernels that took in what had been a launch or a thread of its own give the same bits: the short convolution over runs of
+rows (runs that lie in one request, that cross from one to the next, that begin at a request's start, with kept inputs or nothing
+in front, and the remainder at the end of the step), and a product with its bias."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("lengths,starts", [([300], [0]), ([1, 1, 140, 159], [7, 0, 2, 0]), ([3, 250, 2, 6], [0, 5, 1, 0])])
+def test_runs_of_rows_are_its_rows(lengths, starts):
+    from dynalm_b200.kernels import ops
+    g = torch.Generator(device="cpu").manual_seed(sum(lengths))
+    rows, channels, col0, pitch, keep_off = sum(lengths), 136, 16, 168, 5
+    proj = torch.randn(rows, pitch, generator=g).to(DEV, torch.bfloat16)
+    taps, bias = torch.randn(4, channels, generator=g).to(DEV), torch.randn(channels, generator=g).to(DEV)
+    state = torch.randn(len(lengths), keep_off + 3 * channels, generator=g).to(DEV)
+
+    def run(first, pieces):
+        n = sum(lengths[r] for r in pieces)
+        i32 = dict(dtype=torch.int32, device=DEV)
+        positions = torch.tensor([starts[r] + t for r in pieces for t in range(lengths[r])], **i32)
+        request = torch.tensor([i for i, r in enumerate(pieces) for _ in range(lengths[r])], **i32)
+        slot = torch.tensor([r for r in pieces for _ in range(lengths[r])], **i32)
+        out = torch.empty(n, channels, dtype=torch.bfloat16, device=DEV)
+        ops.ssm_conv(proj[first:first + n], col0, channels, taps, bias, state, keep_off, positions, request, slot,
+                     torch.tensor([starts[r] for r in pieces], **i32), out)
+        return out
+
+    whole, first = run(0, list(range(len(lengths)))), 0
+    for r, n in enumerate(lengths):
+        step = 200                                             # (below 256 rows a thread takes a row)
+        for at in range(0, n, step):
+            if n <= step:
+                assert torch.equal(whole[first:first + n], run(first, [r]))
+                break
+            # a long portion in pieces: the rows in front of a piece stand in for what the request would have kept
+            sub = [starts[r] + at]
+            m = min(step, n - at)
+            i32 = dict(dtype=torch.int32, device=DEV)
+            kept = state[r:r + 1].clone()
+            for j in range(3):
+                p = at - 3 + j
+                if at > 0:
+                    kept[0, keep_off + j * channels:keep_off + (j + 1) * channels] = proj[first + p, col0:col0 + channels].float()
+            out = torch.empty(m, channels, dtype=torch.bfloat16, device=DEV)
+            ops.ssm_conv(proj[first + at:first + at + m], col0, channels, taps, bias, kept, keep_off,
+                         torch.arange(sub[0], sub[0] + m, **i32), torch.zeros(m, **i32), torch.zeros(m, **i32),
+                         torch.tensor(sub, **i32), out)
+            assert torch.equal(whole[first + at:first + at + m], out)
+        first += n
+
+
+def test_a_biased_product_is_its_two_steps():
+    from dynalm_b200.kernels import ops
+    g = torch.Generator(device="cpu").manual_seed(9)
+    x, w = torch.randn(300, 264, generator=g).to(DEV, torch.bfloat16), torch.randn(1100, 264, generator=g).to(DEV, torch.bfloat16)
+    bias = torch.randn(1100, generator=g).to(DEV)
+    two, one = torch.empty(300, 1100, device=DEV), torch.empty(300, 1100, device=DEV)
+    ops.gemm_tcgen05(x, w, two)
+    ops.add_bias(two, bias)
+    ops.gemm_tcgen05(x, w, one, "biased", coeffs=bias)
+    assert torch.equal(one, two)
