@@ -74,16 +74,39 @@ __device__ __forceinline__ void cp_async16_f32(void* dst, const void* src, int b
                : "memory");
 }
 
+// Two float32 numbers of neighbouring query rows, as the packed multiply-add takes them (each half an fma of its own).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma_pair(f32x2& acc, f32x2 a, f32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void halves_of(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// R query rows and 4 keys (D / 16 values) a thread: 16 / R warps of 2 R rows.
+template <int D> struct FTiles {
+  static constexpr int R = 4, THREADS = FT / R * 16;
+  static constexpr int KS = D + 4, QS = 2 * D + 4, PS = 2 * FT + 4;       // floats of a key, of a pair of queries, of a pair's weights
+  static constexpr int SMEM = (FT / 2 * QS + FT * KS + FT * D + FT / 2 * PS) * 4;
+};
+
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(FTiles<D>::THREADS)
 f32_tiles_kernel(F32Attention at, const int4* __restrict__ tiles) {
-  constexpr int KS = D + 4, PS = FT + 4, DV = D / 16;        // DV values of a row a thread: tx * 4 + 64 j, or tx * DV below 64
-  constexpr int RUN = DV < 4 ? DV : 4;
+  using F = FTiles<D>;
+  constexpr int R = F::R, P = R / 2, THREADS = F::THREADS, KS = F::KS, QS = F::QS, PS = F::PS;
+  constexpr int DV = D / 16, RUN = DV < 4 ? DV : 4;          // DV values of a row a thread: tx * 4 + 64 j, or tx * DV below 64
   extern __shared__ __align__(16) float f32_smem[];
-  float* sq = f32_smem;                  // [FT][KS]
-  float* sk = sq + FT * KS;              // [FT][KS]
+  float* sq = f32_smem;                  // [FT / 2][QS]: rows 2 i and 2 i + 1, number by number
+  float* sk = sq + FT / 2 * QS;          // [FT][KS]
   float* sv = sk + FT * KS;              // [FT][D]
-  float* sp = sv + FT * D;               // [FT][PS]
+  float* sp = sv + FT * D;               // [FT / 2][PS]: like the queries
+  __shared__ int s_slots[2 * FT];
   // the last tiles first: they walk the most keys, and the short ones fill what is left at the end (a prompt of 700 tokens, 32:8
   // heads of 64: 154 -> 138 us)
   const int unit = static_cast<int>((gridDim.x - 1 - blockIdx.x) / at.n_heads);
@@ -98,135 +121,218 @@ f32_tiles_kernel(F32Attention at, const int4* __restrict__ tiles) {
 
   const int last = pos0 + rows - 1, lo = first_key(at, pos0);
   const int kept = lo > 0 ? min(at.keep_first, lo) : 0;      // (keys that a later row's window has passed are kept ones too)
-  const int kept_last = first_key(at, last) > 0 ? min(at.keep_first, first_key(at, last)) : 0;
+  const int lo_last = first_key(at, last), kept_last = lo_last > 0 ? min(at.keep_first, lo_last) : 0;
   const int kept_most = max(kept, kept_last);
-  // one run of 16 bytes of key or value t; zeros for a key that no row of the block sees
-  auto fetch = [&](float* dst, int stride, const float* cache, long long row, int size, int per, int t0) {
-    for (int e = tid; e < FT * per; e += 256) {
-      const int r = e / per, c = (e - r * per) * 4, t = t0 + r;
-      const bool there = t <= last && (t >= lo || t < kept_most);
-      const float* src = cache;
-      if (there) {
-        const size_t slot = static_cast<size_t>(ck_page(table, t / at.page_size, at.max_blocks)) * at.page_size + t % at.page_size;
-        src = cache + slot * row + static_cast<size_t>(kvh) * size + c;
+  // where key t0 + tid lies, by the first threads, a tile ahead of its fetches: -1 for a key that no row of the block sees
+  auto look_up = [&](int* slots, int t0) {
+    if (tid < FT) {
+      const int t = t0 + tid;
+      slots[tid] = t <= last && (t >= lo || t < kept_most)
+                       ? ck_page(table, t / at.page_size, at.max_blocks) * at.page_size + t % at.page_size : -1;
+    }
+  };
+  // a tile's keys or values, 16 bytes a thread and trip (D / 4 threads a key, whatever its size); zeros for one that is not seen
+  auto fetch = [&](float* dst, int stride, const float* cache, long long row, int size, int per, const int* slots) {
+    constexpr int LANES = D / 4, KEYS = THREADS / LANES;
+    const int c = tid % LANES, r0 = tid / LANES;
+    const float* from = cache + static_cast<size_t>(kvh) * size + c * 4;
+    if (c < per) {
+#pragma unroll
+      for (int r = r0; r < FT; r += KEYS) {
+        const int slot = slots[r];
+        cp_async16_f32(dst + r * stride + c * 4, from + (slot < 0 ? 0 : slot * row), slot < 0 ? 0 : 16);
       }
-      cp_async16_f32(dst + r * stride + c, src, there ? 16 : 0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   auto seen_tile = [&](int t0) { return t0 + FT > lo || t0 < kept_most; };
 
-  for (int e = tid; e < FT * d4; e += 256) {
-    const int r = e / d4, c = (e - r * d4) * 4;
-    cp_async16_f32(sq + r * KS + c, at.q + static_cast<size_t>(row0 + min(r, rows - 1)) * at.q_stride + static_cast<size_t>(head) * at.head_dim + c, 16);
-  }
   int t0 = kept_most > 0 ? 0 : lo / FT * FT;
-  fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, t0);
+  int* slots = s_slots;                  // of this tile, and behind them of the next
+  look_up(slots, t0);
+  __syncthreads();
+  fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, slots);
+  for (int e = tid; e < FT / 2 * d4; e += THREADS) {
+    const int r = e / d4, c = (e - r * d4) * 4;
+    const float* q = at.q + static_cast<size_t>(head) * at.head_dim + c;
+    const float4 u = *reinterpret_cast<const float4*>(q + static_cast<size_t>(row0 + min(2 * r, rows - 1)) * at.q_stride);
+    const float4 w = *reinterpret_cast<const float4*>(q + static_cast<size_t>(row0 + min(2 * r + 1, rows - 1)) * at.q_stride);
+    float4* to = reinterpret_cast<float4*>(sq + r * QS + 2 * c);
+    to[0] = make_float4(u.x, w.x, u.y, w.y);
+    to[1] = make_float4(u.z, w.z, u.w, w.w);
+  }
 
-  float o[4][DV], m_run[4], l_run[4];
+  float o[R][DV], m_run[R], l_run[R];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < R; ++i) {
     m_run[i] = -INFINITY, l_run[i] = 0.0f;
 #pragma unroll
     for (int j = 0; j < DV; ++j) o[i][j] = 0.0f;
   }
+  const int warp_pos = pos0 + (tid >> 5) * 2 * R;            // the position of the warp's first row
   while (t0 <= last) {
     int next = t0 + FT;
     while (next <= last && !seen_tile(next)) next += FT;
-    fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, t0);
+    fetch(sv, D, at.v_cache, at.v_row, at.vdim, e4, slots);
+    slots = s_slots + (slots == s_slots ? FT : 0);
+    if (next <= last) look_up(slots, next);
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    // scores of rows ty * 4 .. + 3 and keys tx + 16 j
-    float s[4][4];
+    // scores of rows ty * R .. + R - 1 and keys tx + 16 j
+    f32x2 s2[P][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
-#pragma unroll 4
-    for (int c = 0; c < d4; ++c) {
-      float4 a[4], b[4];
+      for (int j = 0; j < 4; ++j) s2[i][j] = 0;
+    const int end = min(FT, warp_pos + 2 * R - t0);          // behind the last key that a row of the warp sees
+    if (end > 0) {
+#pragma unroll 2
+      for (int c = 0; c < d4; ++c) {
+        float4 b[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sq + (ty * 4 + i) * KS + c * 4);
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * KS + c * 4);
+        ulonglong2 a[P][2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * KS + c * 4);
+        for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+          for (int h = 0; h < 2; ++h) a[i][h] = *reinterpret_cast<const ulonglong2*>(sq + (ty * P + i) * QS + c * 8 + h * 4);
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float k = x == 0 ? b[j].x : x == 1 ? b[j].y : x == 2 ? b[j].z : b[j].w;
+            const f32x2 kk = pair_of(k, k);
+#pragma unroll
+            for (int i = 0; i < P; ++i) fma_pair(s2[i][j], (x & 1) ? a[i][x >> 1].y : a[i][x >> 1].x, kk);
+          }
+      }
+    }
+    float c_run[R], c_tile[R], l_tile[R];
+    // whether every row of the warp sees every key of the tile
+    const bool all = t0 + FT - 1 <= warp_pos && t0 >= lo_last;
+    // (every step for all rows at once and without a branch between them: row by row, with a branch at a key without weight, a
+    // tile's softmax took 4,000 to 5,000 cycles, as long as its products)
+    float s[R][4], m[R];
+#pragma unroll
+    for (int i = 0; i < P; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float s0, s1;
+        halves_of(s2[i][j], s0, s1);
+        s[2 * i][j] = __fmul_rn(s0, at.scale), s[2 * i + 1][j] = __fmul_rn(s1, at.scale);
+      }
+    if (at.rate != nullptr) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = biased(at, s[i][j], head, pos0 + ty * R + i - (t0 + tx + 16 * j));
+    }
+    if (!all) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const int pos = pos0 + ty * R + i, from = first_key(at, pos), keep = from > 0 ? min(at.keep_first, from) : 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
-          s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
-          s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
-          s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+          const int t = t0 + tx + 16 * j;
+          s[i][j] = t <= pos && (t >= from || t < keep) ? s[i][j] : -INFINITY;
         }
+      }
     }
-    float c_run[4], c_tile[4], l_tile[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int pos = pos0 + ty * 4 + i, from = first_key(at, pos), keep = from > 0 ? min(at.keep_first, from) : 0;
-      float m = -INFINITY;
+    for (int i = 0; i < R; ++i) m[i] = fmaxf(fmaxf(fmaxf(fmaxf(-INFINITY, s[i][0]), s[i][1]), s[i][2]), s[i][3]);
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], w));
+    bool zero = false;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int t = t0 + tx + 16 * j;
-        const bool seen = t <= pos && (t >= from || t < keep);
-        s[i][j] = seen ? biased(at, __fmul_rn(s[i][j], at.scale), head, pos - t) : -INFINITY;
-        m = fmaxf(m, s[i][j]);
+        const float e = expf(s[i][j] - m[i]);
+        s[i][j] = s[i][j] == -INFINITY ? 0.0f : e;
+        zero |= s[i][j] == 0.0f;
       }
 #pragma unroll
-      for (int w = 8; w > 0; w >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, w));
-      float l = 0.0f;
+    for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = s[i][j] == -INFINITY ? 0.0f : expf(s[i][j] - m);
-        sp[(ty * 4 + i) * PS + tx + 16 * j] = p;
-        l = j == 0 ? p : l + p;
-      }
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<float2*>(sp + (ty * P + i) * PS + 2 * (tx + 16 * j)) = make_float2(s[2 * i][j], s[2 * i + 1][j]);
 #pragma unroll
-      for (int w = 8; w > 0; w >>= 1) l += __shfl_xor_sync(0xffffffffu, l, w);
-      l_tile[i] = l;
-      merge_factors(m_run[i], m, c_run[i], c_tile[i]);
+    for (int i = 0; i < R; ++i) l_tile[i] = s[i][0] + s[i][1] + s[i][2] + s[i][3];
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1)
+#pragma unroll
+      for (int i = 0; i < R; ++i) l_tile[i] += __shfl_xor_sync(0xffffffffu, l_tile[i], w);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float top = fmaxf(m_run[i], m[i]), e_run = expf(m_run[i] - top), e_tile = expf(m[i] - top);
+      c_run[i] = m_run[i] == -INFINITY ? 0.0f : e_run;
+      c_tile[i] = m[i] == -INFINITY ? 0.0f : e_tile;
+      m_run[i] = top;
     }
+    const bool any_zero = __any_sync(0xffffffffu, zero);
     __syncthreads();                       // the keys have been read, the p's are there
-    if (next <= last) fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, next);
+    if (next <= last) fetch(sk, KS, at.k_cache, at.k_row, at.head_dim, d4, slots);
     else asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    float acc[4][DV];
+    f32x2 acc[P][DV];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < P; ++i)
 #pragma unroll
-      for (int j = 0; j < DV; ++j) acc[i][j] = 0.0f;
-#pragma unroll 4
-    for (int k = 0; k < FT; k += 4) {
-      float4 p[4];
+      for (int j = 0; j < DV; ++j) acc[i][j] = 0;
+    // a key with a weight of zero is not multiplied in; where the warp has none, nothing need be asked of its weights
+    auto weigh = [&](auto picked, int keys) {
+#pragma unroll 2
+      for (int k = 0; k < keys; k += 2) {
+        ulonglong2 w[P];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(sp + (ty * 4 + i) * PS + k);
+        for (int i = 0; i < P; ++i) w[i] = *reinterpret_cast<const ulonglong2*>(sp + (ty * P + i) * PS + 2 * k);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        float v[DV];
+        for (int kk = 0; kk < 2; ++kk) {
+          float v[DV];
 #pragma unroll
-        for (int j = 0; j < DV / RUN; ++j)
+          for (int j = 0; j < DV / RUN; ++j)
 #pragma unroll
-          for (int h = 0; h < RUN; ++h) v[j * RUN + h] = sv[(k + kk) * D + tx * RUN + 64 * j + h];
+            for (int h = 0; h < RUN; ++h) v[j * RUN + h] = sv[(k + kk) * D + tx * RUN + 64 * j + h];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+          for (int i = 0; i < P; ++i) {
+            const f32x2 wi = kk ? w[i].y : w[i].x;
+            float w0, w1;
+            halves_of(wi, w0, w1);
 #pragma unroll
-          for (int j = 0; j < DV; ++j) acc[i][j] = w != 0.0f ? fmaf(w, v[j], acc[i][j]) : acc[i][j];
+            for (int j = 0; j < DV; ++j) {
+              if constexpr (decltype(picked)::value) {
+                float a0, a1;
+                halves_of(acc[i][j], a0, a1);
+                acc[i][j] = pair_of(w0 != 0.0f ? fmaf(w0, v[j], a0) : a0, w1 != 0.0f ? fmaf(w1, v[j], a1) : a1);
+              } else {
+                fma_pair(acc[i][j], wi, pair_of(v[j], v[j]));
+              }
+            }
+          }
         }
       }
-    }
+    };
+    if (any_zero) weigh(std::true_type(), end);
+    else weigh(std::false_type(), FT);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < R; ++i) {
       l_run[i] = two_products(l_run[i], c_run[i], l_tile[i], c_tile[i]);
 #pragma unroll
-      for (int j = 0; j < DV; ++j) o[i][j] = two_products(o[i][j], c_run[i], acc[i][j], c_tile[i]);
+      for (int j = 0; j < DV; ++j) {
+        float a0, a1;
+        halves_of(acc[i / 2][j], a0, a1);
+        o[i][j] = two_products(o[i][j], c_run[i], (i & 1) ? a1 : a0, c_tile[i]);
+      }
     }
     t0 = next;
     __syncthreads();                       // the values and the p's have been read
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty * 4 + i;
+  for (int i = 0; i < R; ++i) {
+    const int r = ty * R + i;
     if (at.sink) {                         // one more score of 0 in the denominator; it carries no value
       float c_run, c_tile;
       merge_factors(m_run[i], 0.0f, c_run, c_tile);
@@ -485,11 +591,11 @@ f32_rows_kernel(F32Attention at, const int* __restrict__ positions, const int* _
 
 template <int D>
 int launch_f32_tiles(const F32Attention& at, const int4* tiles, int n_tiles, cudaStream_t stream) {
-  constexpr int SMEM = (2 * FT * (D + 4) + FT * D + FT * (FT + 4)) * 4;
+  constexpr int SMEM = FTiles<D>::SMEM;
   const cudaError_t e = cudaFuncSetAttribute(f32_tiles_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (2ll * n_tiles * at.n_heads > 0x7fffffffll) return DL_ERR_UNSUPPORTED;
-  f32_tiles_kernel<D><<<2 * n_tiles * at.n_heads, 256, SMEM, stream>>>(at, tiles);
+  f32_tiles_kernel<D><<<2 * n_tiles * at.n_heads, FTiles<D>::THREADS, SMEM, stream>>>(at, tiles);
   return launch_status();
 }
 
