@@ -374,7 +374,7 @@ class F32Cost:
     # SMs of 148 that clusters of 1, 2, 4 and 8 blocks fill round after round (with eight of 144 KB one of two stays empty)
     FILLED = {32: ((148, 148, 140, 112), (148, 148, 140, 128)), 64: ((148, 148, 128, 64), (148, 148, 140, 128)),
               128: ((148, 148, 128, 112), (148, 148, 140, 128))}
-    TILE, TILES_FIT = {32: 5.0, 64: 8.1, 128: 13.6}, {32: 2, 64: 2, 128: 1}      # a tile of keys of a block of 64 query rows
+    TILE, TILES_FIT = {32: 3.0, 64: 5.2, 128: 6.8}, {32: 2, 64: 2, 128: 1}      # a tile of keys of a block of 64 query rows
     LAUNCH = 5.0
 
     def __init__(self, n_heads: int, n_kv_heads: int, most: int, span: int, sms: int = 0):
