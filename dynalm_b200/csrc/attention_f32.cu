@@ -12,7 +12,8 @@
 // so that no infinity reaches a row that does not see it.
 //
 // * f32_tiles_kernel: 64 query rows of one request and one head a block, 256 threads, 4 x 4 scores and 4 rows x D / 16
-//   values a thread; keys and values by cp.async, the next tile's keys on their way while the values are multiplied.
+//   values a thread, as packed pairs of rows; keys and values by cp.async, the next tile's keys on their way while the values are
+//   multiplied, the pages of the tile after it looked up by then.
 // * f32_rows_kernel: a row's keys over the warps of up to eight blocks (a cluster along the keys), a tile of 64 a warp, for
 //   up to four query heads of one KV head at once, so that a key is read once for them. A warp asks for its whole tile of
 //   keys and values at once (cp.async), and for the next tile's as soon as a buffer has been read: with a few rows it is the
@@ -20,10 +21,15 @@
 //   several blocks, and are merged in the order of the keys. Which of its launches is taken, and where query tiles give
 //   way to rows: F32Cost in kernels/attention.py.
 //
-// Bound by the multiply-add lanes (tiles) and by trips to memory (rows). Measured on B200 against attention_generic.cu, us a
-// layer: 32:8 heads of 64, a prompt of 700 tokens 1,410 -> 146, single tokens: five of 450 keys 70 -> 12, 64 of 3,000 1,573 ->
+// Bound by the multiply-add lanes (tiles: of 13,200 cycles that a tile of 64 keys takes a block, two to an SM, 9,900 are products,
+// where the lanes need 8,200 for both blocks) and by trips to memory (rows). Measured on B200 against attention_generic.cu, us a
+// layer: 32:8 heads of 64, a prompt of 700 tokens 1,410 -> 87, single tokens: five of 450 keys 70 -> 12, 64 of 3,000 1,573 ->
 // 389; 24:8 heads of 128, 64 of 3,000 2,157 -> 754; six heads of 96, 256 of 700 546 -> 347; 4:2 heads of 16, 100 rows behind
-// 3,000 keys 102 -> 64. Behind the plain kernel with a handful of keys alone: 256 rows of 8 keys, 24:8 heads of 128, 56 -> 86.
+// 3,000 keys 102 -> 64.
+//
+// The tiles with a division and a walk to the block table for every 16 bytes, the softmax row by row with branches, and single
+// multiply-adds -> as they are, us: 32:8 heads of 64, prompts of 700 / 2,048 / four of 350 tokens 155 / 876 / 153 -> 87 / 520 / 101;
+// 24:8 heads of 128, 700 / 2,000 tokens 253 / 1,446 -> 107 / 782; 100 rows behind 3,000 keys, 4:2 heads of 16 244 -> 148.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -88,7 +94,9 @@ __device__ __forceinline__ void halves_of(f32x2 v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// R query rows and 4 keys (D / 16 values) a thread: 16 / R warps of 2 R rows.
+// R query rows and 4 keys (D / 16 values) a thread: a warp holds 2 R rows. Four rows, eight warps a block: with eight rows and four
+// warps a key is read half as often, but a tile's chain is longer (32:8 heads of 64, us: a prompt of 700 tokens 87 / 93, of 2,048
+// 520 / 471, 100 rows behind 300 keys 43 / 49). With single multiply-adds in the place of packed ones 93, 565 and 45.
 template <int D> struct FTiles {
   static constexpr int R = 4, THREADS = FT / R * 16;
   static constexpr int KS = D + 4, QS = 2 * D + 4, PS = 2 * FT + 4;       // floats of a key, of a pair of queries, of a pair's weights

@@ -364,8 +364,9 @@ class F32Cost:
     Measured on B200 over 1 to 256 rows of 8 to 3,000 keys, nine shapes of heads: the launch with the least cost is on average 3 %
     behind the fastest of all. Blocks of one warp, several to an SM, are the better ones for many rows (64 rows of 3,000 keys, 24:8
     heads of 128: 1,210 us with two warps a block, 754 in four blocks of one), blocks of several warps for few (one row of 3,000
-    keys: 79 and 43 us). Query tiles against rows, us: 70 rows behind 900 keys, 4:2 heads of 16 81 / 16, 32:8 heads of 64 132 /
-    135, 24:8 heads of 128 219 / 407; a prompt of 300 rows 28 / 17, 64 / 165, 72 / 381."""
+    keys: 79 and 43 us). Query tiles against rows, us: 70 rows behind 900 keys, 4:2 heads of 16 52 / 17, 32:8 heads of 64 91 /
+    135, 24:8 heads of 128 148 / 330; a prompt of 300 rows 20 / 23, 35 / 290, 52 / 298. TILE is what chose best between the two over 8
+    to 300 rows behind up to 2,500 keys of eight shapes (on average 1 to 2 % behind the faster one)."""
 
     WARPS = {32: 4, 64: 4, 128: 2}                      # of a block that is not one warp, a tile each
     ROUND = {32: (6.5, 6.5), 64: (8.4, 11.6), 128: (12.8, 14.0)}      # a tile for each warp of the block; for its only one
@@ -374,7 +375,7 @@ class F32Cost:
     # SMs of 148 that clusters of 1, 2, 4 and 8 blocks fill round after round (with eight of 144 KB one of two stays empty)
     FILLED = {32: ((148, 148, 140, 112), (148, 148, 140, 128)), 64: ((148, 148, 128, 64), (148, 148, 140, 128)),
               128: ((148, 148, 128, 112), (148, 148, 140, 128))}
-    TILE, TILES_FIT = {32: 3.0, 64: 5.2, 128: 6.8}, {32: 2, 64: 2, 128: 1}      # a tile of keys of a block of 64 query rows
+    TILE, TILES_FIT = {32: 2.3, 64: 5.1, 128: 9.0}, {32: 2, 64: 2, 128: 1}      # a tile of keys of a block of 64 query rows
     LAUNCH = 5.0
 
     def __init__(self, n_heads: int, n_kv_heads: int, most: int, span: int, sms: int = 0):
