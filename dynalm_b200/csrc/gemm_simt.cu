@@ -1,7 +1,7 @@
 // y = x W^T (+ bias): the plain matrix product, fp32 accumulation on the CUDA cores.
 //
-// This is the matrix product of the true 32-bit path (no tensor cores, no reduced-precision mode)
-// and the fallback for shapes the tensor-core kernels refuse. x: [M, K] (row stride ldx), W: [N, K] row-major,
+// The 32-bit path's product for matrices with fewer than 512 features or numbers of k (larger ones: gemm_split.cu) and
+// the fallback for shapes the tensor-core kernels refuse; no reduced-precision mode. x: [M, K] (row stride ldx), W: [N, K] row-major,
 // y: [M, N] (row stride ldy), bias: fp32 [N] or null.
 //
 // Every output element is a sum in an order that K alone fixes, so its value does not depend on the number of rows in the

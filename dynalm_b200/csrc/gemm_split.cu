@@ -1,6 +1,7 @@
 // y = x W^T (+ bias) for float32 operands on the tensor cores, with the precision of 32-bit multiply-adds.
 //
-// A float32 is the sum of three bf16 (8 + 8 + 8 bits of mantissa, each part rounded to nearest, the split exact), so a
+// A float32 is the sum of three bf16 (8 + 8 + 8 bits of mantissa, the first rounded to nearest, the others cut off the
+// rest, the split exact), so a
 // product of two is the sum of nine products of bf16 that the tensor core forms exactly. The six that matter are kept (of
 // the three that are left out the largest is 2^-26 of the product on average), smallest first:
 //   lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi          (a part of W times a part of x).
